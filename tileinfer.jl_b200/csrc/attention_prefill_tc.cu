@@ -21,6 +21,7 @@
 // scores, softmax statistics and sums in 32-bit, P rounded to the storage type for the second product.
 #include "tcgen05.cuh"
 #include "tensor_map.h"
+#include "packed_f32.cuh"
 
 namespace {
 
@@ -60,30 +61,6 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// Two 32-bit floats in one 64-bit register, for the packed FMA-pipe instructions of sm_100 (one issue
-// slot for two lanes of work).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
 // A row's scores r (unscaled) capped, in base-2 units: cap log2(e) tanh(x), x = scale r / cap. Where no row of the warp has |x| > 1/2 the
 // odd series of tanh to its seventh term (the rest is below 1e-7 of x there) does it on the FMA units, two lanes an instruction, which
 // leaves the exponential unit to the softmax; else the closed form.

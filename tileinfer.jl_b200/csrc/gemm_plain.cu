@@ -1,16 +1,26 @@
 // Plain matrix product y[n, out] = x[n, in] · W[out, in]ᵀ on the CUDA cores, for any sizes
 // and either element type. Inputs are widened to 32-bit, every product is a 32-bit fused
-// multiply-add (no tensor-core or reduced-precision mode), and each output element sums its
-// k terms in ascending order whatever n is: a row's result is bit-identical in a step of
+// multiply-add (no tensor-core or reduced-precision mode), and the order in which an output
+// element adds its k terms is fixed by `in` alone: a row's result is bit-identical in a step of
 // one token and in a step of thousands. It is the 32-bit path's product and the fallback of
 // the bfloat16 path for sizes the tensor-core kernel refuses.
+//
+// The order, common to the four kernels below: k is cut into segments of GP_SEGMENT terms. In a
+// segment the terms of even k and those of odd k are two chains of fused multiply-adds from zero
+// in ascending order (the two halves of a packed fma.rn.f32x2, which takes one issue slot where two
+// fused multiply-adds take two); a segment's sum is even + odd, and the segments' sums are added in
+// ascending order. Terms beyond `in` are zeros. Short chains are what lets several warps share one
+// output row's k (a single chain of 21,504 terms is 44 us of latency alone), and they lose less to
+// rounding than one long chain: against 64-bit sums a product of k = 4,096 is 2.9e-7 off.
 //
 // AntoineBut/TileInfer.jl: weights stay [out, in] row-major, y = Wᵀx with 32-bit
 // accumulation and one rounding (src/ops/reference.jl:23-26, src/ops/tile/linear.jl:12-13);
 // the logits leave in 32-bit after that rounding (src/ops/tile/linear.jl:26).
 #include "common.cuh"
 #include "mma_util.cuh"
+#include "packed_f32.cuh"
 
+#define GP_SEGMENT 512
 #define GP_BM 64      // tokens per tile
 #define GP_BN 64      // output features per tile
 #define GP_BK 16
@@ -19,6 +29,17 @@
 #define TI_EPI_XIELU 1
 #define TI_EPI_F32_OUT 2   // round to the storage type, store 32-bit (logits)
 
+// One output: rounded to the storage type, through the epilogue, stored.
+template <typename T>
+__device__ __forceinline__ void store_output(void* y, long long ldy, int r, int c, float sum, int epilogue, const XieluParams& act) {
+    float v = rnd<T>(sum);
+    if (epilogue == TI_EPI_XIELU) v = xielu_value<T>(v, act);
+    if (epilogue >= TI_EPI_GELU_ERF) v = gelu_epilogue(v, epilogue);
+    if (epilogue == TI_EPI_F32_OUT) ((float*)y)[(size_t)r * ldy + c] = v;
+    else ((T*)y)[(size_t)r * ldy + c] = from_f32<T>(v);
+}
+
+// ---- rows that cannot be read 16 bytes at a time: 64 x 64 tiles, element by element
 template <typename T>
 __global__ void __launch_bounds__(256) gemm_plain_kernel(void* __restrict__ y, long long ldy, const T* x,
                                                         long long ldx, const T* __restrict__ W, int n, int out,
@@ -28,11 +49,11 @@ __global__ void __launch_bounds__(256) gemm_plain_kernel(void* __restrict__ y, l
     const int tid = threadIdx.x;
     const int m0 = blockIdx.y * GP_BM, n0 = blockIdx.x * GP_BN;
     const int tr = tid / 16, tc = tid % 16;       // 16 x 16 threads, 4 x 4 outputs each
-    float acc[4][4];
+    float acc[2][4][4], total[4][4];              // even and odd chains of the segment; the segments before it
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) acc[0][i][j] = acc[1][i][j] = total[i][j] = 0.f;
 
     // Each thread stages 4 consecutive k of one row of each operand tile.
     const int lrow = tid / 4, lk = (tid % 4) * 4;
@@ -57,9 +78,20 @@ __global__ void __launch_bounds__(256) gemm_plain_kernel(void* __restrict__ y, l
 #pragma unroll
             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
         }
         __syncthreads();
+        if ((k0 + GP_BK) % GP_SEGMENT == 0 || k0 + GP_BK >= in) {
+            const bool first = k0 < GP_SEGMENT;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float s = acc[0][i][j] + acc[1][i][j];
+                    total[i][j] = first ? s : total[i][j] + s;
+                    acc[0][i][j] = acc[1][i][j] = 0.f;
+                }
+        }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -68,113 +100,13 @@ __global__ void __launch_bounds__(256) gemm_plain_kernel(void* __restrict__ y, l
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int c = n0 + tc * 4 + j;
-            if (c >= out) continue;
-            float v = rnd<T>(acc[i][j]);
-            if (epilogue == TI_EPI_XIELU) v = xielu_value<T>(v, act);
-            if (epilogue >= TI_EPI_GELU_ERF) v = gelu_epilogue(v, epilogue);
-            if (epilogue == TI_EPI_F32_OUT) ((float*)y)[(size_t)r * ldy + c] = v;
-            else ((T*)y)[(size_t)r * ldy + c] = from_f32<T>(v);
+            if (c < out) store_output<T>(y, ldy, r, c, total[i][j], epilogue, act);
         }
     }
 }
 
-// The same product in larger tiles for steps of many tokens whose rows can be read 16 bytes at a time:
-// 128 tokens x 128 features per block, 8 x 8 outputs per thread, the next k block's global loads in flight
-// while the current one is multiplied. Every output still sums its k terms in ascending order with single
-// fused multiply-adds from zero, so the bits are those of the kernels above and below.
-#define GB_T 128
-#define GB_BK 8
-
-template <typename T> __device__ __forceinline__ void load4(const T* p, float (&v)[4]);
-template <> __device__ __forceinline__ void load4<float>(const float* p, float (&v)[4]) {
-    const float4 t = __ldcg(reinterpret_cast<const float4*>(p));
-    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
-}
-template <> __device__ __forceinline__ void load4<bf16>(const bf16* p, float (&v)[4]) {
-    const uint2 t = __ldcg(reinterpret_cast<const uint2*>(p));
-    v[0] = __uint_as_float(t.x << 16); v[1] = __uint_as_float(t.x & 0xffff0000u);
-    v[2] = __uint_as_float(t.y << 16); v[3] = __uint_as_float(t.y & 0xffff0000u);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) gemm_plain_wide_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
-                                                             const T* __restrict__ W, int n, int out, int in, int epilogue,
-                                                             XieluParams act) {
-    __shared__ __align__(16) float As[2][GB_BK][GB_T + 4];
-    __shared__ __align__(16) float Bs[2][GB_BK][GB_T + 4];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * GB_T, n0 = blockIdx.x * GB_T;
-    const int ty = tid / 16, tx = tid % 16;            // 8 tokens x 8 features each
-    const int lrow = tid / 2, lk = (tid % 2) * 4;      // staging: 4 consecutive k of one row of each operand
-    const bool a_ok = m0 + lrow < n, b_ok = n0 + lrow < out;
-    const T* a_src = x + (size_t)(a_ok ? m0 + lrow : 0) * ldx + lk;
-    const T* b_src = W + (size_t)(b_ok ? n0 + lrow : 0) * in + lk;
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    float ra[4], rb[4];
-    auto fetch = [&](int k0) {                          // in % 4 == 0: a vector of 4 is inside the row or outside it
-        const bool k_ok = k0 + lk < in;
-        if (a_ok && k_ok) load4<T>(a_src + k0, ra); else { ra[0] = ra[1] = ra[2] = ra[3] = 0.f; }
-        if (b_ok && k_ok) load4<T>(b_src + k0, rb); else { rb[0] = rb[1] = rb[2] = rb[3] = 0.f; }
-    };
-    auto stage = [&](int buf) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            As[buf][lk + e][lrow] = ra[e];
-            Bs[buf][lk + e][lrow] = rb[e];
-        }
-    };
-    pdl_wait();
-    pdl_launch_dependents();
-    fetch(0);
-    stage(0);
-    __syncthreads();
-    int buf = 0;
-    for (int k0 = 0; k0 < in; k0 += GB_BK) {
-        const bool more = k0 + GB_BK < in;
-        if (more) fetch(k0 + GB_BK);
-#pragma unroll
-        for (int kk = 0; kk < GB_BK; ++kk) {
-            float a[8], b[8];
-            *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 8]);
-            *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(&As[buf][kk][ty * 8 + 4]);
-            *reinterpret_cast<float4*>(b) = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 8]);
-            *reinterpret_cast<float4*>(b + 4) = *reinterpret_cast<const float4*>(&Bs[buf][kk][tx * 8 + 4]);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        if (more) stage(buf ^ 1);
-        __syncthreads();
-        buf ^= 1;
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = m0 + ty * 8 + i;
-        if (r >= n) continue;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int c = n0 + tx * 8 + j;
-            if (c >= out) continue;
-            float v = rnd<T>(acc[i][j]);
-            if (epilogue == TI_EPI_XIELU) v = xielu_value<T>(v, act);
-            if (epilogue >= TI_EPI_GELU_ERF) v = gelu_epilogue(v, epilogue);
-            if (epilogue == TI_EPI_F32_OUT) ((float*)y)[(size_t)r * ldy + c] = v;
-            else ((T*)y)[(size_t)r * ldy + c] = from_f32<T>(v);
-        }
-    }
-}
-
-// The same product for steps of few tokens (decode): a block owns GV_ROWS output features and streams their
-// weight rows once, in k blocks that are staged in shared memory with 16-byte loads; a thread owns one
-// feature and every GV_SLOTS-th token and sums its k terms in ascending order with single fused
-// multiply-adds, starting from zero: the same chain as the tiled kernel above, so a row's result has the
-// same bits whichever of the two ran. With 8 tokens the tiled kernel would compute 64 token rows of which 56
-// are padding and run out/64 blocks; this one runs out/16 blocks that do nothing but stream.
+// The same for steps of few tokens: a block owns GV_ROWS output features and streams their weight rows once, in k blocks
+// staged in shared memory; a thread owns one feature and every GV_SLOTS-th token.
 #define GV_ROWS 16
 #define GV_SLOTS 8
 #define GV_BK 64
@@ -189,165 +121,384 @@ __global__ void __launch_bounds__(GV_ROWS * GV_SLOTS) gemv_plain_kernel(void* __
     const int tid = threadIdx.x;
     const int row = tid % GV_ROWS, slot = tid / GV_ROWS;
     const int m0 = blockIdx.x * GV_ROWS;
-    float acc[TPT];
+    float acc[2][TPT], total[TPT];
 #pragma unroll
-    for (int j = 0; j < TPT; ++j) acc[j] = 0.f;
-    constexpr int VEC = 16 / sizeof(T);                   // elements per 16-byte load
-    const bool wide = (in % VEC) == 0 && (((uintptr_t)W) & 15) == 0;
-    // Weights do not depend on the previous kernel: the first block of them is on its way before the wait.
-    auto load_w = [&](int k0) {
-        if (wide) {
-            for (int i = tid; i < GV_ROWS * (GV_BK / VEC); i += GV_ROWS * GV_SLOTS) {
-                const int r = i / (GV_BK / VEC), kv = (i % (GV_BK / VEC)) * VEC;
-                const int c = m0 + r, k = k0 + kv;
-                if (c < out && k < in) {                  // in % VEC == 0: a vector is inside the row or outside it
-                    Vec16<T> v;
-                    v.load(W + (size_t)c * in + k);
-#pragma unroll
-                    for (int e = 0; e < VEC; ++e) Ws[r][kv + e] = v.v[e];
-                } else {
-#pragma unroll
-                    for (int e = 0; e < VEC; ++e) Ws[r][kv + e] = 0.f;
-                }
-            }
-        } else {
-            for (int i = tid; i < GV_ROWS * GV_BK; i += GV_ROWS * GV_SLOTS) {
-                const int r = i / GV_BK, kk = i % GV_BK;
-                const int c = m0 + r, k = k0 + kk;
-                Ws[r][kk] = (c < out && k < in) ? to_f32(W[(size_t)c * in + k]) : 0.f;
-            }
-        }
-    };
-    load_w(0);
+    for (int j = 0; j < TPT; ++j) acc[0][j] = acc[1][j] = total[j] = 0.f;
     pdl_wait();
     pdl_launch_dependents();
     for (int k0 = 0; k0 < in; k0 += GV_BK) {
-        if (k0 > 0) load_w(k0);
+        for (int i = tid; i < GV_ROWS * GV_BK; i += GV_ROWS * GV_SLOTS) {
+            const int r = i / GV_BK, kk = i % GV_BK;
+            const int c = m0 + r, k = k0 + kk;
+            Ws[r][kk] = (c < out && k < in) ? to_f32(W[(size_t)c * in + k]) : 0.f;
+        }
         for (int i = tid; i < n * GV_BK; i += GV_ROWS * GV_SLOTS) {
             const int t = i / GV_BK, kk = i % GV_BK;
             Xs[t * (GV_BK + 1) + kk] = (k0 + kk < in) ? to_f32(__ldcg(x + (size_t)t * ldx + k0 + kk)) : 0.f;
         }
         __syncthreads();
-        const int kmax = min(GV_BK, in - k0);             // terms beyond `in` are not added (the tiled kernel adds +0 there: the same sum)
 #pragma unroll 4
-        for (int kk = 0; kk < kmax; ++kk) {
-            const float w = Ws[row][kk];
-#pragma unroll
-            for (int j = 0; j < TPT; ++j) {
-                const int t = slot + j * GV_SLOTS;
-                if (t < n) acc[j] = fmaf(Xs[t * (GV_BK + 1) + kk], w, acc[j]);
-            }
-        }
-        __syncthreads();
-    }
-    const int c = m0 + row;
-    if (c >= out) return;
-#pragma unroll
-    for (int j = 0; j < TPT; ++j) {
-        const int t = slot + j * GV_SLOTS;
-        if (t >= n) continue;
-        float v = rnd<T>(acc[j]);
-        if (epilogue == TI_EPI_XIELU) v = xielu_value<T>(v, act);
-            if (epilogue >= TI_EPI_GELU_ERF) v = gelu_epilogue(v, epilogue);
-        if (epilogue == TI_EPI_F32_OUT) ((float*)y)[(size_t)t * ldy + c] = v;
-        else ((T*)y)[(size_t)t * ldy + c] = from_f32<T>(v);
-    }
-}
-
-// The weight-streaming kernel with its k blocks in flight: the same block shape and the same sums, but the
-// weight rows' and the tokens' k blocks are copied to shared memory with 16-byte cp.async several stages ahead
-// (raw, widened when they are read), so that a block has tens of kilobytes in flight instead of one k block.
-// It needs rows that can be read 16 bytes at a time; the kernel above serves the rest.
-template <typename T, int TPT, int STAGES>
-__global__ void __launch_bounds__(GV_ROWS * GV_SLOTS) gemv_plain_pipe_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
-                                                                              const T* __restrict__ W, int n, int out, int in, int epilogue,
-                                                                              XieluParams act) {
-    extern __shared__ __align__(16) unsigned char pipe_smem[];
-    constexpr int VEC = 16 / sizeof(T);                    // elements per 16-byte chunk
-    constexpr int CHUNKS = GV_BK / VEC;                    // chunks per row of a k block
-    constexpr int ROW = GV_BK + VEC;                       // elements between rows in shared memory (16 bytes of padding)
-    const int stage_elems = (GV_ROWS + n) * ROW;
-    T* stages = reinterpret_cast<T*>(pipe_smem);
-    const int tid = threadIdx.x;
-    const int row = tid % GV_ROWS, slot = tid / GV_ROWS;
-    const int m0 = blockIdx.x * GV_ROWS;
-    float acc[TPT];
-#pragma unroll
-    for (int j = 0; j < TPT; ++j) acc[j] = 0.f;
-    const int tiles = (in + GV_BK - 1) / GV_BK;
-    auto issue = [&](int tile) {
-        if (tile < tiles) {
-            T* ws = stages + (size_t)(tile % STAGES) * stage_elems;
-            T* xs = ws + GV_ROWS * ROW;
-            const int k0 = tile * GV_BK;
-            for (int i = tid; i < (GV_ROWS + n) * CHUNKS; i += GV_ROWS * GV_SLOTS) {
-                const int r = i / CHUNKS, k = k0 + (i % CHUNKS) * VEC;
-                T* dst = (r < GV_ROWS ? ws + r * ROW : xs + (r - GV_ROWS) * ROW) + (i % CHUNKS) * VEC;
-                const bool inside = k < in && (r >= GV_ROWS || m0 + r < out);      // in % VEC == 0: a chunk is inside the row or outside it
-                if (inside) cp_async16(smem_u32(dst), r < GV_ROWS ? W + (size_t)(m0 + r) * in + k : x + (size_t)(r - GV_ROWS) * ldx + k);
-                else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
-            }
-        }
-        cp_async_commit();
-    };
-    pdl_wait();
-    pdl_launch_dependents();
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) issue(s);
-    for (int tile = 0; tile < tiles; ++tile) {
-        cp_async_wait<STAGES - 2>();
-        __syncthreads();                                   // this tile has landed, and the stage refilled below is no longer read
-        issue(tile + STAGES - 1);
-        const T* ws = stages + (size_t)(tile % STAGES) * stage_elems + row * ROW;
-        const T* xs = stages + (size_t)(tile % STAGES) * stage_elems + GV_ROWS * ROW;
-        const int chunks = min(GV_BK, in - tile * GV_BK) / VEC;      // in % VEC == 0
-        // 16 bytes of the row and of each token at a time (shared-memory reads, not arithmetic, bound this loop);
-        // the k terms are still added one by one in ascending order.
-#pragma unroll 2
-        for (int c = 0; c < chunks; ++c) {
-            Vec16<T> w;
-            w.load(ws + c * VEC);
+        for (int kk = 0; kk < GV_BK; kk += 2) {
+            const float w0 = Ws[row][kk], w1 = Ws[row][kk + 1];
 #pragma unroll
             for (int j = 0; j < TPT; ++j) {
                 const int t = slot + j * GV_SLOTS;
                 if (t < n) {
-                    Vec16<T> xv;
-                    xv.load(xs + t * ROW + c * VEC);
-#pragma unroll
-                    for (int e = 0; e < VEC; ++e) acc[j] = fmaf(xv.v[e], w.v[e], acc[j]);
+                    acc[0][j] = fmaf(Xs[t * (GV_BK + 1) + kk], w0, acc[0][j]);
+                    acc[1][j] = fmaf(Xs[t * (GV_BK + 1) + kk + 1], w1, acc[1][j]);
                 }
             }
         }
+        __syncthreads();
+        if ((k0 + GV_BK) % GP_SEGMENT == 0 || k0 + GV_BK >= in) {
+#pragma unroll
+            for (int j = 0; j < TPT; ++j) {
+                const float s = acc[0][j] + acc[1][j];
+                total[j] = k0 < GP_SEGMENT ? s : total[j] + s;
+                acc[0][j] = acc[1][j] = 0.f;
+            }
+        }
     }
-    cp_async_wait<0>();
     const int c = m0 + row;
     if (c >= out) return;
 #pragma unroll
     for (int j = 0; j < TPT; ++j) {
         const int t = slot + j * GV_SLOTS;
-        if (t >= n) continue;
-        float v = rnd<T>(acc[j]);
-        if (epilogue == TI_EPI_XIELU) v = xielu_value<T>(v, act);
-            if (epilogue >= TI_EPI_GELU_ERF) v = gelu_epilogue(v, epilogue);
-        if (epilogue == TI_EPI_F32_OUT) ((float*)y)[(size_t)t * ldy + c] = v;
-        else ((T*)y)[(size_t)t * ldy + c] = from_f32<T>(v);
+        if (t < n) store_output<T>(y, ldy, t, c, total[j], epilogue, act);
     }
 }
 
-template <typename T, int TPT, int STAGES>
-static int launch_gemv_pipe(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
-                            const XieluParams& act, cudaStream_t stream) {
-    constexpr int VEC = 16 / sizeof(T);
-    const size_t smem = (size_t)STAGES * (GV_ROWS + n) * (GV_BK + VEC) * sizeof(T);
-    static size_t configured = 0;
-    if (smem > configured) {
-        const cudaError_t e = cudaFuncSetAttribute(gemv_plain_pipe_kernel<T, TPT, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(STAGES * (GV_ROWS + TPT * GV_SLOTS) * (GV_BK + VEC) * sizeof(T)));
-        if (e != cudaSuccess) return ti_fail("gemv_plain: %s", cudaGetErrorString(e));
-        configured = STAGES * (GV_ROWS + TPT * GV_SLOTS) * (GV_BK + VEC) * sizeof(T);
+// ---- rows that can be read 16 bytes at a time
+//
+// Both kernels stage k blocks of 128 bytes a row (32 floats or 64 bfloat16 values) by 16-byte cp.async as they lie in memory; rows
+// are 144 bytes apart in shared memory, so eight consecutive rows' 16-byte pieces fall into different banks. Four consecutive
+// k of a row are one read: the packed multiply-add's operands are (k, k + 1) pairs of both sides, with no transposition and no
+// duplicated element.
+#define GT_ROW 144
+#define GT_BYTES 128
+
+template <typename T> struct Quad;                         // four consecutive k of a row as two packed pairs
+template <> struct Quad<float> {
+    f32x2 p[2];
+    static constexpr int BYTES = 16;
+    __device__ __forceinline__ void load(const unsigned char* s) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(s);
+        p[0] = t.x; p[1] = t.y;
     }
-    ti_launch(gemv_plain_pipe_kernel<T, TPT, STAGES>, dim3((out + GV_ROWS - 1) / GV_ROWS), dim3(GV_ROWS * GV_SLOTS), smem, stream, y, ldy, x, ldx, W, n,
-              out, in, epilogue, act);
+};
+template <> struct Quad<bf16> {
+    f32x2 p[2];
+    static constexpr int BYTES = 8;
+    __device__ __forceinline__ void load(const unsigned char* s) {
+        const uint2 t = *reinterpret_cast<const uint2*>(s);
+        p[0] = pack2(__uint_as_float(t.x << 16), __uint_as_float(t.x & 0xffff0000u));
+        p[1] = pack2(__uint_as_float(t.y << 16), __uint_as_float(t.y & 0xffff0000u));
+    }
+};
+
+// 16 bytes to shared memory, or 16 zero bytes (nothing is read from `src` then).
+__device__ __forceinline__ void stage16(unsigned dst, const void* src, bool inside) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(inside ? 16 : 0));
+}
+
+// Steps of up to 32 tokens: weights are streamed once. A block owns 16 * RPT output rows, its warps take the segments of k in
+// turn, each with a ring of STAGES k blocks of its own (no block barrier but one per round of segments, where the round's sums
+// are added up in ascending order). A lane owns RPT rows and half of the tokens (TPL each), so a row's quad is read once for
+// TPL tokens and a token's quad, the same for 16 lanes, is one broadcast.
+// What bounds it: weight bytes and, from 8 tokens on, shared-memory reads (a row's quad is read by one lane pair, a token's by 16
+// lanes; neighbouring lanes share both, which halves the reads' passes). Measured at 8 tokens: up projection (21,504 x 4,096, 352
+// MB) 77 us, 4.6 TB/s, where one chain per output and 16 bytes per token and thread took 220; down (4,096 x 21,504) 83 us (335).
+template <typename T, int TPL, int RPT, int STAGES>
+__global__ void __launch_bounds__(256) gemv_plain_stream_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
+                                                                const T* __restrict__ W, int n, int out, int in, int epilogue,
+                                                                XieluParams act) {
+    extern __shared__ __align__(16) unsigned char gv_smem[];
+    constexpr int ROWS = 16 * RPT, TOKENS = 2 * TPL;
+    constexpr int BK = GT_BYTES / (int)sizeof(T), PER_SEG = GP_SEGMENT / BK, VEC = 16 / (int)sizeof(T);
+    constexpr int STAGE = (ROWS + TOKENS) * GT_ROW;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    const int row = lane & 15, half = lane >> 4;
+    const int m0 = blockIdx.x * ROWS, t0 = blockIdx.y * TOKENS;
+    n = min(TOKENS, n - t0);
+    x += (size_t)t0 * ldx;
+    unsigned char* ring = gv_smem + (size_t)warp * (STAGES * STAGE);
+    float* sums = reinterpret_cast<float*>(gv_smem + (size_t)warps * (STAGES * STAGE));     // [2][warps][TOKENS][ROWS]
+    float* total = sums + 2 * warps * TOKENS * ROWS;                                         // [TOKENS][ROWS]
+    const int segments = (in + GP_SEGMENT - 1) / GP_SEGMENT, rounds = (segments + warps - 1) / warps;
+    // This warp's k blocks: segments warp, warp + warps, ..., each of PER_SEG blocks but perhaps the last one of all.
+    const int mine = warp < segments ? (segments - 1 - warp) / warps + 1 : 0;
+    const int last_blocks = (in - (segments - 1) * GP_SEGMENT + BK - 1) / BK;
+    const bool has_last = mine > 0 && (mine - 1) * warps + warp == segments - 1;
+    const int tiles = mine * PER_SEG - (has_last ? PER_SEG - last_blocks : 0);
+    auto k_of = [&](int tile) { return ((tile / PER_SEG) * warps + warp) * GP_SEGMENT + (tile % PER_SEG) * BK; };
+    auto issue_w = [&](int tile) {
+        if (tile < tiles) {
+            const int k0 = k_of(tile);
+            unsigned char* s = ring + (tile % STAGES) * STAGE;
+#pragma unroll
+            for (int i = 0; i < ROWS * 8 / 32; ++i) {
+                const int r = (i * 32 + lane) >> 3, c = lane & 7, k = k0 + c * VEC;
+                const bool inside = m0 + r < out && k < in;                 // in % VEC == 0: a vector is inside the row or outside it
+                stage16(smem_u32(s + r * GT_ROW + c * 16), inside ? W + (size_t)(m0 + r) * in + k : W, inside);
+            }
+        }
+    };
+    auto issue_x = [&](int tile) {
+        if (tile < tiles) {
+            const int k0 = k_of(tile);
+            unsigned char* s = ring + (tile % STAGES) * STAGE + ROWS * GT_ROW;
+#pragma unroll
+            for (int i = 0; i < (TOKENS * 8 + 31) / 32; ++i) {
+                const int r = (i * 32 + lane) >> 3, c = lane & 7, k = k0 + c * VEC;
+                if (TOKENS * 8 < 32 && r >= TOKENS) continue;
+                const bool inside = r < n && k < in;
+                stage16(smem_u32(s + r * GT_ROW + c * 16), inside ? x + (size_t)r * ldx + k : x, inside);
+            }
+        }
+    };
+    // Weights do not depend on the kernel before: the first k blocks are on their way before the wait.
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) issue_w(s);
+    pdl_wait();
+    pdl_launch_dependents();
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) { issue_x(s); cp_async_commit(); }
+    f32x2 acc[RPT][TPL];
+    int tile = 0;
+    for (int round = 0; round < rounds; ++round) {
+#pragma unroll
+        for (int q = 0; q < RPT; ++q)
+#pragma unroll
+            for (int j = 0; j < TPL; ++j) acc[q][j] = 0ull;
+        const int end = min(tiles, (round + 1) * PER_SEG);
+        for (; tile < end; ++tile) {
+            cp_async_wait<STAGES - 2>();
+            __syncwarp();                                   // every lane's copies of this k block have landed, and the stage refilled below is no longer read
+            issue_w(tile + STAGES - 1);
+            issue_x(tile + STAGES - 1);
+            cp_async_commit();
+            const unsigned char* s = ring + (tile % STAGES) * STAGE;
+            const unsigned char* ws = s + row * GT_ROW;
+            const unsigned char* xs = s + (ROWS + half) * GT_ROW;
+#pragma unroll
+            for (int c = 0; c < BK / 4; ++c) {
+                Quad<T> w[RPT];
+#pragma unroll
+                for (int q = 0; q < RPT; ++q) w[q].load(ws + q * 16 * GT_ROW + c * Quad<T>::BYTES);
+#pragma unroll
+                for (int j = 0; j < TPL; ++j) {
+                    Quad<T> v;
+                    v.load(xs + 2 * j * GT_ROW + c * Quad<T>::BYTES);
+#pragma unroll
+                    for (int q = 0; q < RPT; ++q) acc[q][j] = fma2(v.p[1], w[q].p[1], fma2(v.p[0], w[q].p[0], acc[q][j]));
+                }
+            }
+        }
+        if (round < mine) {
+            float* to = sums + ((round & 1) * warps + warp) * (TOKENS * ROWS);
+#pragma unroll
+            for (int q = 0; q < RPT; ++q)
+#pragma unroll
+                for (int j = 0; j < TPL; ++j) {
+                    float e, o;
+                    unpack2(acc[q][j], e, o);
+                    to[(2 * j + half) * ROWS + q * 16 + row] = e + o;
+                }
+        }
+        __syncthreads();                                    // the other buffer is written in the next round, after every thread has read it
+        const int here = min(warps, segments - round * warps);
+        for (int i = tid; i < n * ROWS; i += blockDim.x) {
+            const float* from = sums + (round & 1) * warps * (TOKENS * ROWS) + i;
+            float t = round == 0 ? from[0] : total[i] + from[0];
+            for (int w = 1; w < here; ++w) t += from[w * (TOKENS * ROWS)];
+            if (round + 1 < rounds) total[i] = t;
+            else if (m0 + i % ROWS < out) store_output<T>(y, ldy, t0 + i / ROWS, m0 + i % ROWS, t, epilogue, act);
+        }
+    }
+    cp_async_wait<0>();
+}
+
+// Steps of more tokens: tiles of 16 TI tokens x 16 TJ features, 256 threads with TI x TJ outputs each, k blocks in a ring of
+// shared-memory stages. A thread's tokens and features are 16 apart, so the lanes of a warp (8 features x 4 tokens) read
+// consecutive rows. The sums of the segments before the current one wait in shared memory.
+// What bounds it: the FMA units, at 0.7 of their rate at the clock that a long run of them settles at (ncu: 1.6 GHz; a
+// thread's fragments come in 16-byte reads of which every second or fourth lane's is its own). 512 tokens x 21,504 x 4,096: 2,230
+// us, 40 TFLOP/s; tiles staged with k outermost, 8 x 8 outputs a thread and single multiply-adds took 4,500.
+template <typename T, int TI, int TJ, int STAGES>
+__global__ void __launch_bounds__(256) gemm_plain_tile_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
+                                                             const T* __restrict__ W, int n, int out, int in, int epilogue,
+                                                             XieluParams act) {
+    extern __shared__ __align__(16) unsigned char gt_smem[];
+    constexpr int TM = 16 * TI, TN = 16 * TJ;
+    constexpr int BK = GT_BYTES / (int)sizeof(T), PER_SEG = GP_SEGMENT / BK, VEC = 16 / (int)sizeof(T);
+    constexpr int STAGE = (TM + TN) * GT_ROW;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    const int tx = (lane & 7) + 8 * (warp & 1), ty = (lane >> 3) + 4 * (warp >> 1);
+    float* total = reinterpret_cast<float*>(gt_smem + STAGES * STAGE);        // [TI * TJ][256]
+    const int blocks = (in + BK - 1) / BK;
+    const int lrow = tid >> 3, lc = tid & 7;                                 // staging: 32 rows of 8 pieces at a time
+    auto issue = [&](int b, bool weights, bool tokens) {
+        if (b < blocks) {
+            unsigned char* s = gt_smem + (b % STAGES) * STAGE + lrow * GT_ROW + lc * 16;
+            const int k = b * BK + lc * VEC;
+            const bool k_ok = k < in;
+            if (tokens) {
+#pragma unroll
+                for (int i = 0; i < TM / 32; ++i) {
+                    const int r = m0 + lrow + 32 * i;
+                    const bool inside = k_ok && r < n;
+                    stage16(smem_u32(s + 32 * i * GT_ROW), inside ? x + (size_t)r * ldx + k : x, inside);
+                }
+            }
+            if (weights) {
+#pragma unroll
+                for (int i = 0; i < TN / 32; ++i) {
+                    const int c = n0 + lrow + 32 * i;
+                    const bool inside = k_ok && c < out;
+                    stage16(smem_u32(s + (TM + 32 * i) * GT_ROW), inside ? W + (size_t)c * in + k : W, inside);
+                }
+            }
+        }
+    };
+#pragma unroll
+    for (int b = 0; b < STAGES - 1; ++b) issue(b, true, false);
+    pdl_wait();
+    pdl_launch_dependents();
+#pragma unroll
+    for (int b = 0; b < STAGES - 1; ++b) { issue(b, false, true); cp_async_commit(); }
+    f32x2 acc[TI][TJ];
+#pragma unroll
+    for (int i = 0; i < TI; ++i)
+#pragma unroll
+        for (int j = 0; j < TJ; ++j) acc[i][j] = 0ull;
+    for (int b = 0; b < blocks; ++b) {
+        cp_async_wait<STAGES - 2>();
+        __syncthreads();                                    // this k block has landed, and the stage refilled below is no longer read
+        issue(b + STAGES - 1, true, true);
+        cp_async_commit();
+        const unsigned char* as = gt_smem + (b % STAGES) * STAGE + ty * GT_ROW;
+        const unsigned char* bs = gt_smem + (b % STAGES) * STAGE + (TM + tx) * GT_ROW;
+#pragma unroll
+        for (int c = 0; c < BK / 4; ++c) {
+            Quad<T> w[TJ];
+#pragma unroll
+            for (int j = 0; j < TJ; ++j) w[j].load(bs + j * 16 * GT_ROW + c * Quad<T>::BYTES);
+#pragma unroll
+            for (int i = 0; i < TI; ++i) {
+                Quad<T> v;
+                v.load(as + i * 16 * GT_ROW + c * Quad<T>::BYTES);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int j = 0; j < TJ; ++j) acc[i][j] = fma2(v.p[h], w[j].p[h], acc[i][j]);
+            }
+        }
+        if ((b + 1) % PER_SEG == 0 && b + 1 < blocks) {     // a segment ends, and more follow
+#pragma unroll
+            for (int i = 0; i < TI; ++i)
+#pragma unroll
+                for (int j = 0; j < TJ; ++j) {
+                    float e, o;
+                    unpack2(acc[i][j], e, o);
+                    float* t = total + (i * TJ + j) * 256 + tid;
+                    *t = b < PER_SEG ? e + o : *t + (e + o);
+                    acc[i][j] = 0ull;
+                }
+        }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < TI; ++i) {
+        const int r = m0 + ty + 16 * i;
+#pragma unroll
+        for (int j = 0; j < TJ; ++j) {
+            const int c = n0 + tx + 16 * j;
+            float e, o;
+            unpack2(acc[i][j], e, o);
+            const float s = blocks > PER_SEG ? total[(i * TJ + j) * 256 + tid] + (e + o) : e + o;
+            if (r < n && c < out) store_output<T>(y, ldy, r, c, s, epilogue, act);
+        }
+    }
+}
+
+template <typename K> static cudaError_t allow_smem(K kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+template <typename T, int TPL, int RPT, int STAGES>
+static int launch_stream(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
+                         const XieluParams& act, cudaStream_t stream) {
+    constexpr int ROWS = 16 * RPT, MAX_WARPS = 8;
+    constexpr size_t PER_WARP = (size_t)STAGES * (ROWS + 2 * TPL) * GT_ROW + 2 * 2 * TPL * ROWS * sizeof(float);
+    constexpr size_t TOTAL = 2 * TPL * ROWS * sizeof(float);
+    static const cudaError_t allowed = allow_smem(gemv_plain_stream_kernel<T, TPL, RPT, STAGES>, MAX_WARPS * PER_WARP + TOTAL);
+    if (allowed != cudaSuccess) return ti_fail("gemv_plain: %s", cudaGetErrorString(allowed));
+    const int segments = (in + GP_SEGMENT - 1) / GP_SEGMENT, rounds = (segments + MAX_WARPS - 1) / MAX_WARPS;
+    const int warps = (segments + rounds - 1) / rounds;                        // as few as the rounds need: the last round is full
+    ti_launch(gemv_plain_stream_kernel<T, TPL, RPT, STAGES>, dim3((out + ROWS - 1) / ROWS, (n + 2 * TPL - 1) / (2 * TPL)), dim3(32 * warps), warps * PER_WARP + TOTAL, stream, y,
+              ldy, x, ldx, W, n, out, in, epilogue, act);
     return ti_check_launch("gemv_plain");
+}
+
+template <typename T, int TI, int TJ, int STAGES>
+static int launch_tile(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
+                       const XieluParams& act, cudaStream_t stream) {
+    constexpr size_t SMEM = (size_t)STAGES * 16 * (TI + TJ) * GT_ROW + (size_t)TI * TJ * 256 * sizeof(float);
+    static const cudaError_t allowed = allow_smem(gemm_plain_tile_kernel<T, TI, TJ, STAGES>, SMEM);
+    if (allowed != cudaSuccess) return ti_fail("gemm_plain: %s", cudaGetErrorString(allowed));
+    const dim3 grid((out + 16 * TJ - 1) / (16 * TJ), (n + 16 * TI - 1) / (16 * TI));
+    TI_REQUIRE(grid.y <= 65535, "gemm: too many rows (%d) for one launch", n);
+    ti_launch(gemm_plain_tile_kernel<T, TI, TJ, STAGES>, grid, dim3(256), SMEM, stream, y, ldy, x, ldx, W, n, out, in, epilogue, act);
+    return ti_check_launch("gemm_plain_tile");
+}
+
+// Tokens x features per thread of the tile kernel: the shape whose rounds of tiles over the SMs take the least time, by what a
+// round and a launch's first and last tile cost (in units of k, from sweeps of 64 to 2,048 tokens x 2,048 to 21,504 features at k =
+// 4,096: microseconds per round 447 / 235 / 132 / 92, and 0 / 15 / 23 / 22 once; 512 tokens x 4,096 features take 449 / 471 / 518 / 660
+// us, 128 x 4,096 take 448 / 255 / 155 / 260, 512 x 6,144 take 893 / 691 / 771 / 1,027). The sums do not depend on the shape.
+struct TileShape { int ti, tj; float round, once; };
+static const TileShape TILE_SHAPES[] = {{8, 8, 447.f, 0.f}, {8, 4, 235.f, 15.f}, {4, 4, 132.f, 23.f}, {2, 4, 92.f, 22.f}};
+
+extern "C" int ti_gemm_plain_shape(int n, int out, int sms) {
+    int best = 0;
+    float least = 0.f;
+    for (int s = 0; s < 4; ++s) {
+        const TileShape& t = TILE_SHAPES[s];
+        const long long tiles = (long long)((n + 16 * t.ti - 1) / (16 * t.ti)) * ((out + 16 * t.tj - 1) / (16 * t.tj));
+        const float time = (float)((tiles + sms - 1) / sms) * t.round + t.once;
+        if (s == 0 || time < least) { best = s; least = time; }
+    }
+    return best;
+}
+
+// Up to 64 tokens the weight-streaming kernel is the faster one (two token groups of 32 read the weights twice, the second time from
+// L2): 64 tokens x 4,096 / 21,504 features of k = 4,096 take 74 / 355 us against 115 / 402 in tiles; at 100 tokens the two are level.
+#define GT_STREAM_TOKENS 64
+
+template <typename T>
+static int launch_vectors(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
+                          const XieluParams& act, cudaStream_t stream) {
+#define GT_ARGS y, ldy, x, ldx, W, n, out, in, epilogue, act, stream
+    if (n <= GT_STREAM_TOKENS) {
+        // 32 rows a block halve what is read of the tokens, where that leaves blocks for six tenths of the SMs (8 tokens: 4,096
+        // rows 17.8 us against 24.5 with 16 rows a block, 2,048 rows of k = 2,048 13.8 against 10.7). More blocks than SMs take two
+        // stages, so that two blocks fit an SM (6,144 rows: 26.9 us against 33.0); fewer take a deeper ring (4,096 rows x 21,504: 83 us against 98).
+        const int sms = ti_sm_count(), groups = (n + 31) / 32, blocks = (out + 31) / 32 * groups;
+        const bool tall = 5 * blocks >= 3 * sms, many = blocks > sms;
+        if (n <= 2) return !tall ? launch_stream<T, 1, 1, 6>(GT_ARGS) : many ? launch_stream<T, 1, 2, 2>(GT_ARGS) : launch_stream<T, 1, 2, 5>(GT_ARGS);
+        if (n <= 4) return !tall ? launch_stream<T, 2, 1, 5>(GT_ARGS) : many ? launch_stream<T, 2, 2, 2>(GT_ARGS) : launch_stream<T, 2, 2, 4>(GT_ARGS);
+        if (n <= 8) return !tall ? launch_stream<T, 4, 1, 5>(GT_ARGS) : many ? launch_stream<T, 4, 2, 2>(GT_ARGS) : launch_stream<T, 4, 2, 4>(GT_ARGS);
+        if (n <= 16) return tall ? launch_stream<T, 8, 2, 3>(GT_ARGS) : launch_stream<T, 8, 1, 4>(GT_ARGS);
+        return tall ? launch_stream<T, 16, 2, 2>(GT_ARGS) : launch_stream<T, 16, 1, 3>(GT_ARGS);
+    }
+    switch (ti_gemm_plain_shape(n, out, ti_sm_count())) {
+        case 0: return launch_tile<T, 8, 8, 2>(GT_ARGS);
+        case 1: return launch_tile<T, 8, 4, 2>(GT_ARGS);
+        case 2: return launch_tile<T, 4, 4, 3>(GT_ARGS);
+        default: return launch_tile<T, 2, 4, 4>(GT_ARGS);
+    }
+#undef GT_ARGS
 }
 
 extern "C" int ti_gemm_plain(void* y, long long ldy, const void* x, long long ldx, const void* W, int n, int out, int in,
@@ -356,19 +507,12 @@ extern "C" int ti_gemm_plain(void* y, long long ldy, const void* x, long long ld
     if (n == 0) return 0;
     TI_REQUIRE(n > 0 && out > 0 && in > 0, "gemm: bad sizes n=%d out=%d in=%d", n, out, in);
     TI_REQUIRE((epilogue >= 0 && epilogue <= 2) || (epilogue >= TI_EPI_GELU_ERF && epilogue <= TI_EPI_LAST), "gemm: unknown epilogue %d", epilogue);
-    dim3 grid((out + GP_BN - 1) / GP_BN, (n + GP_BM - 1) / GP_BM);
-    TI_REQUIRE(grid.y <= 65535, "gemm: too many rows (%d) for one launch", n);
     XieluParams act{alpha_p, alpha_n, beta, eps};
+    const int vec = dtype == TI_F32 ? 4 : 8;               // elements of a 16-byte piece
+    if (in % vec == 0 && ldx % vec == 0 && aligned16(x) && aligned16(W)) {
+        TI_DISPATCH_DTYPE(dtype, return launch_vectors<T>(y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act, stream));
+    }
     if (n <= GV_MAX_TOKENS) {                              // few tokens: the weight-streaming form (same sums, bit for bit)
-        const int vec = dtype == TI_F32 ? 4 : 8;           // elements of a 16-byte chunk
-        if (in % vec == 0 && ldx % vec == 0 && aligned16(x) && aligned16(W)) {
-            TI_DISPATCH_DTYPE(dtype, {
-                if (n <= GV_SLOTS) return launch_gemv_pipe<T, 1, 8>(y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act, stream);
-                if (n <= 2 * GV_SLOTS) return launch_gemv_pipe<T, 2, 6>(y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act, stream);
-                if (n <= 4 * GV_SLOTS) return launch_gemv_pipe<T, 4, 4>(y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act, stream);
-                return launch_gemv_pipe<T, 8, 3>(y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act, stream);
-            });
-        }
         const size_t smem = (size_t)n * (GV_BK + 1) * sizeof(float);
         const dim3 blocks((out + GV_ROWS - 1) / GV_ROWS), threads(GV_ROWS * GV_SLOTS);
 #define GV_LAUNCH(TPT) ti_launch(gemv_plain_kernel<T, TPT>, blocks, threads, smem, stream, y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act)
@@ -381,15 +525,9 @@ extern "C" int ti_gemm_plain(void* y, long long ldy, const void* x, long long ld
 #undef GV_LAUNCH
         return ti_check_launch("gemv_plain");
     }
-    const int vec_bytes = dtype == TI_F32 ? 16 : 8;     // four elements
-    if (n > GB_T / 2 && in % 4 == 0 && ldx % 4 == 0 && ((uintptr_t)x % vec_bytes) == 0 && ((uintptr_t)W % vec_bytes) == 0) {
-        dim3 wide((out + GB_T - 1) / GB_T, (n + GB_T - 1) / GB_T);
-        TI_REQUIRE(wide.y <= 65535, "gemm: too many rows (%d) for one launch", n);
-        TI_DISPATCH_DTYPE(dtype, (ti_launch(gemm_plain_wide_kernel<T>, dim3(wide), dim3(256), 0, stream, y, ldy, (const T*)x, ldx, (const T*)W, n,
-                                            out, in, epilogue, act)));
-        return ti_check_launch("gemm_plain_wide");
-    }
-    TI_DISPATCH_DTYPE(dtype, (ti_launch(gemm_plain_kernel<T>, dim3(grid), dim3(256), 0, stream, y, ldy, (const T*)x, ldx, (const T*)W, n, out, in,
+    const dim3 grid((out + GP_BN - 1) / GP_BN, (n + GP_BM - 1) / GP_BM);
+    TI_REQUIRE(grid.y <= 65535, "gemm: too many rows (%d) for one launch", n);
+    TI_DISPATCH_DTYPE(dtype, (ti_launch(gemm_plain_kernel<T>, grid, dim3(256), 0, stream, y, ldy, (const T*)x, ldx, (const T*)W, n, out, in,
                                                                           epilogue, act)));
     return ti_check_launch("gemm_plain");
 }
