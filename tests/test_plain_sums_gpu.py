@@ -1,0 +1,78 @@
+"""The 32-bit path's product and attention at the sizes where their kernels change over: edges of tiles, of k segments and of key
+chunks, and that the bits depend on none of it."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from tileinfer_b200.kernels import ops
+    return ops
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("out,k", [(15, 8), (33, 504), (100, 512), (2000, 520), (5000, 1032), (4100, 2056), (260, 8 * 1037)])
+def test_product_bits_do_not_depend_on_the_kernel(ops, dtype, out, k):
+    """Weight streaming by 1 to 64 tokens (16 or 32 rows a block, shallow or deep rings), every tile shape, and the two kernels
+    for rows that cannot be read 16 bytes at a time: one order of additions, so one set of bits."""
+    g = torch.Generator().manual_seed(out + k)
+    x = torch.randn(700, k, generator=g).to(dtype).cuda()
+    w = (torch.randn(out, k, generator=g) * k ** -0.5).to(dtype).cuda()
+    odd = torch.zeros(700, k + 1, dtype=dtype, device="cuda")
+    odd[:, :k] = x
+    want = x.double() @ w.double().t()
+    # Two chains of 256 terms, their sum, and the segments' sums one after the other: so many roundings of partial sums.
+    bound = (min(k, 512) / 2 + 1 + k / 512) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    first = None
+    for n in (700, 300, 129, 128, 65, 64, 33, 32, 17, 16, 9, 8, 5, 4, 3, 2, 1):
+        for rows in (x[:n], odd[:n, :k]):
+            y = torch.full((n, out), float("nan"), dtype=torch.float32, device="cuda")
+            ops.gemm_plain(y, rows, w, ops.EPI_F32_OUT)
+            if first is None:
+                first = y
+                if dtype == torch.float32:
+                    assert bool(((y.double() - want).abs() <= bound).all())
+                else:                                    # one rounding to bfloat16 on top
+                    assert bool(((y.double() - want).abs() <= bound + want.abs() * 2.0 ** -8).all())
+            assert torch.equal(y, first[:n]), (n, rows.stride(0))
+
+
+@pytest.mark.parametrize("D,nq,nkv", [(4, 3, 3), (20, 5, 1), (33, 4, 2), (64, 8, 1), (96, 4, 4), (128, 12, 2), (132, 2, 1), (256, 4, 2), (512, 2, 2)])
+def test_attention_over_chunk_edges(ops, D, nq, nkv):
+    """Positions on both sides of the 256-key chunks, alone and in one launch (the same bits), against 64-bit arithmetic; without a
+    window, with one, with kept first positions, and in chunks of visibility."""
+    page, last = 16, 800
+    g = torch.Generator().manual_seed(D)
+    pages = -(-last // page)
+    k, v = (torch.randn(pages + 3, nkv, page, D, generator=g).cuda() for _ in range(2))
+    order = torch.randperm(pages + 3, generator=g)[:pages]
+    table = torch.zeros(2, pages, dtype=torch.int32)
+    table[1] = order.int()
+    table = table.cuda()
+    positions = [0, 1, 30, 31, 32, 255, 256, 257, 511, 512, 600, 799]
+    q = torch.randn(len(positions), nq, D, generator=g).cuda()
+    keys, values = (c[order.cuda()].permute(0, 2, 1, 3).reshape(-1, nkv, D).double() for c in (k, v))
+    scale = D ** -0.5
+    for window, keep, chunk in ((0, 0, 0), (70, 0, 0), (300, 40, 0), (0, 0, 100)):
+        def run(rows):
+            pos = torch.tensor([positions[r] for r in rows], dtype=torch.int32, device="cuda")
+            out = torch.empty(len(rows), nq * D, device="cuda")
+            ops.attention_plain(out, q[rows].contiguous(), k, v, table, torch.ones_like(pos), pos, scale, nq, nkv, D, page, window, chunk=chunk, keep=keep)
+            return out.view(len(rows), nq, D)
+        together = run(list(range(len(positions))))
+        for r, p in enumerate(positions):
+            seen = torch.arange(p + 1, device="cuda")
+            low = max(p + 1 - window if window else 0, p // chunk * chunk if chunk else 0)
+            seen = seen[(seen >= low) | (seen < keep)] if window else seen[seen >= low]
+            for h in range(nq):
+                s = (keys[seen, h // (nq // nkv)] @ q[r, h].double()) * scale
+                want = torch.softmax(s, 0) @ values[seen, h // (nq // nkv)]
+                # Roundings: the score's D products scaled (its error enters as a factor), an exponential and a sum over the keys.
+                size = float((q[r, h].abs().double() @ keys[seen, h // (nq // nkv)].abs().t()).max()) * scale
+                bound = 2.0 ** -24 * (2 * D * size + 4 * math.sqrt(len(seen)) + 16) * float(values.abs().max())
+                assert float((together[r, h].double() - want).abs().max()) <= bound, (p, h, window)
+            assert torch.equal(run([r])[0], together[r])
