@@ -123,7 +123,6 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
     const int tokens_per_block = 2 * tokens_per_tile;
 
     pdl_wait();
-    pdl_launch_dependents();
 
     // Which sequence and which block of its new tokens; later blocks (longer prefixes) run first.
     int b = 0, blk = (int)(gridDim.x / p.kv_heads) - 1 - (int)(blockIdx.x / p.kv_heads);
@@ -176,6 +175,9 @@ __global__ void __launch_bounds__(THREADS, 1) attention_prefill_tc_kernel(const 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    // Only a block that holds its tensor memory lets the successor start: a product's block takes its own before it waits, and beside
+    // one that had not, the two would wait for each other.
+    pdl_launch_dependents();
     const unsigned tmem_base = *tmem_slot;
 
     if (warp == 8) {

@@ -34,6 +34,13 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // kernel launched as a programmatic dependent starts before its predecessor has finished writing.
 extern int ti_pdl_enabled;
 
+// Loads through L2 (`__ldcg`) of one bfloat16 value are an asm statement without `volatile` in cuda_bf16.hpp: the compiler may move it,
+// ahead of the wait for the predecessor or out of the condition that keeps its address inside a buffer (a row's neighbour beyond the
+// last token). The other types' are volatile. Kernels therefore load through these.
+template <typename T> __device__ __forceinline__ T l2_load(const T* p) { return __ldcg(p); }
+__device__ __forceinline__ bf16 l2_load(const bf16* p) { return __ushort_as_bfloat16(__ldcg(reinterpret_cast<const unsigned short*>(p))); }
+#define __ldcg(...) l2_load(__VA_ARGS__)
+
 // Wait for the predecessor, then let the successor start: at most two kernels overlap. (Releasing the
 // successor before waiting, so that more kernels are resident at once, was measured on the decode
 // step and was slower: blocks that sit waiting take residency away from the kernel that is running.)
