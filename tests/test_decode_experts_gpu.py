@@ -1,0 +1,58 @@
+"""The routed units of a step of few tokens streamed by pair (csrc/expert_stream.cu), at the sizes where they can go wrong, against 64-bit
+arithmetic on the same numbers."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+
+
+@pytest.mark.parametrize("units,out,k,tokens,per_token", [(3, 8, 8, 1, 2), (5, 24, 40, 3, 2), (34, 40, 264, 8, 5), (4, 56, 520, 16, 3), (64, 16, 1032, 2, 7),
+                                                          (9, 136, 2048, 12, 4)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_units_streamed_by_pair(units, out, k, tokens, per_token, gated):
+    """Choices without a unit, units that more than 8 pairs share (the matrix goes over them again), fewer pairs than units and more,
+    rows beyond the last tile; the score on the input or not; the squared rectifier; a second product with a row per pair."""
+    from tileinfer_b200.kernels import fast
+    g = torch.Generator().manual_seed(units * 1000 + k)
+    x = torch.randn(tokens, k, generator=g).bfloat16()
+    w = (torch.randn(units, (2 if gated else 1) * out, k, generator=g) * k ** -0.5).bfloat16()
+    ids = torch.stack([torch.randperm(units, generator=g)[:per_token] if units >= per_token else torch.arange(per_token) % units for _ in range(tokens)]).int()
+    ids[:, 0] = units - 1                                # one unit that every token takes
+    if per_token > 2:
+        ids[tokens // 2, 1] = -1
+    scores = torch.rand(tokens, per_token, generator=g)
+    limits = torch.full((units,), 1.5)
+    pairs = tokens * per_token
+    for scaled in (False, True):
+        y = torch.full((pairs, out), 7.0, dtype=torch.bfloat16, device="cuda")
+        rows = torch.full((tokens, per_token), 99, dtype=torch.int32, device="cuda")
+        fast.grouped_stream(y, x.cuda(), w.cuda(), ids.cuda(), scores.cuda() if scaled else None, rows, per_token, gated=gated, relu2=not gated,
+                            limits=limits.cuda(), slope=1.7, shift=1.0)
+        assert torch.equal(rows.cpu().flatten(), torch.where(ids.flatten() >= 0, torch.arange(pairs), torch.tensor(-1)).int())
+        for p in range(pairs):
+            e, t = int(ids.flatten()[p]), p // per_token
+            if e < 0:
+                assert bool((y[p] == 7.0).all())
+                continue
+            row = (scores.flatten()[p] * x[t].float()).bfloat16() if scaled else x[t]
+            z = w[e].to(F64) @ row.to(F64)
+            # A 32-bit sum of k products off by k / 2 roundings of its terms at most, then one rounding to bfloat16.
+            off = k / 2 * 2.0 ** -24 * (w[e].to(F64).abs() @ row.to(F64).abs()) + z.abs() * 2.0 ** -8
+            if gated:
+                a, b = z[:out].clamp(max=1.5), z[out:].clamp(-1.5, 1.5)
+                want = a * torch.sigmoid(1.7 * a) * (b + 1.0)
+                bound = off[:out] * 1.2 * (b + 1.0).abs() + off[out:] * a.abs()             # slopes: |d/da| <= 1.2 |b + 1|, |d/db| <= |a|
+            else:
+                want = torch.relu(z) ** 2
+                bound = off * (2 * z.abs() + off)
+            assert bool(((y[p].cpu().to(F64) - want).abs() <= bound + want.abs() * 2.0 ** -7 + 1e-6).all()), p
+    down = (torch.randn(units, 24, out, generator=g) * out ** -0.5).bfloat16()
+    y2 = torch.zeros((pairs, 24), dtype=torch.bfloat16, device="cuda")
+    fast.grouped_stream(y2, y, down.cuda(), ids.cuda())
+    for p in range(pairs):
+        e = int(ids.flatten()[p])
+        if e >= 0:
+            want = down[e].to(F64) @ y[p].cpu().to(F64)
+            bound = out / 2 * 2.0 ** -24 * (down[e].to(F64).abs() @ y[p].cpu().to(F64).abs()) + want.abs() * 2.0 ** -8
+            assert bool(((y2[p].cpu().to(F64) - want).abs() <= bound + 1e-7).all())

@@ -26,6 +26,7 @@
 // accumulation, one rounding to the storage type, grouped tile order for L2 reuse.
 #include "tcgen05.cuh"
 #include "tensor_map.h"
+#include "expert_stream.h"
 
 
 namespace {
@@ -682,7 +683,8 @@ int many_dispatch(void* y, long long ldy, const void* x, long long ldx, const vo
 // [matrices, out, in]. `groups` (device): [0] = tiles in use, [1 + t] = the matrix of tile t; `rows` = the rows that x and
 // y hold (a multiple of `tile`, the capacity: tiles beyond groups[0] are not touched). Returns 2 for sizes it refuses.
 extern "C" int ti_gemm_tcgen05_grouped(void* y, const void* x, const void* W, const int* groups, int rows, int tile, int matrices,
-                                       int out, int in, int* status, cudaStream_t stream) {
+                                       int out, int in, int* status, const ExpertStream* pairs, cudaStream_t stream) {
+    if (pairs != nullptr) return expert_stream(y, x, W, *pairs, matrices, out, in, stream);     // few tokens: no tiles, no plan
     if (rows == 0) return 0;
     if (in % 8 != 0 || out % 8 != 0 || in < 8 || ((uintptr_t)W & 15) || ((uintptr_t)x & 15) || ((uintptr_t)y & 15) || rows % tile != 0 ||
         (tile != 32 && tile != 64 && tile != 128 && tile != 256) || (long long)matrices * out > 0x7fffffffLL) {
@@ -695,6 +697,8 @@ extern "C" int ti_gemm_tcgen05_grouped(void* y, const void* x, const void* W, co
     return many_dispatch(y, out, x, in, W, (long long)matrices * out, rows, out, in, tile, p, status, stream);
 }
 
+#define HEADS_STREAM_TOKENS 16
+
 // One matrix per head over all tokens: y[t, h, :] = W[h] x[t, h, :], W [heads, out_h, in_h], x [n, heads * in_h],
 // y [n, heads * out_h]. Returns 2 for sizes it refuses.
 extern "C" int ti_gemm_tcgen05_heads(void* y, const void* x, const void* W, int n, int heads, int out_h, int in_h, int* status,
@@ -705,6 +709,14 @@ extern "C" int ti_gemm_tcgen05_heads(void* y, const void* x, const void* W, int 
         return 2;
     }
     TI_REQUIRE(status != nullptr, "gemm_tcgen05_heads: status word missing");
+    // A step of few tokens: a small product per head, where tiles, barriers and tensor memory cost more than
+    // the product (8 tokens x 16 heads of 128 x 64 inside a step: about 8 us in tiles, 4.6 streamed).
+    if (n <= HEADS_STREAM_TOKENS) {
+        ExpertStream e = {};
+        e.pairs = n * heads;
+        e.per_row = 1;
+        return expert_stream(y, x, W, e, heads, out_h, in_h, stream);
+    }
     Params p;
     p.groups = nullptr; p.w_group_rows = 0; p.batch = heads; p.w_batch_rows = out_h; p.x_batch_k = in_h; p.y_batch_cols = out_h;
     const int bn = n > 128 ? 256 : n > 64 ? 128 : n > 32 ? 64 : 32;

@@ -3,6 +3,8 @@ outside what the fast kernels take, in which case the caller runs the plain CUDA
 kernel instead (same result up to rounding); it never returns a wrong result."""
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import library as _library
@@ -211,11 +213,49 @@ def grouped_linear(y, x, w, plan, tile) -> bool:
         return False
     experts, out, k = w.shape
     rc = lib().ti_gemm_tcgen05_grouped(y.data_ptr(), x.data_ptr(), w.data_ptr(), plan.data_ptr(), x.shape[0], tile, experts, out, k,
-                                       status_word().data_ptr(), _stream())
+                                       status_word().data_ptr(), None, _stream())
     if rc == 2:
         return False
     check(rc, "gemm_tcgen05_grouped")
     return True
+
+
+# A step of so few tokens streams the matrices of the units in use (csrc/expert_stream.cu); with more, a unit's pairs no longer fit one
+# operand of 8 and its matrices are gone over again. Both products, streamed against planned and grouped: 32 gated units of 1,024 x 2,048
+# with two shared, 8 tokens 62 against 85 us, 16 tokens 89 against 91, 24 tokens 111 against 97; plain units, 16 tokens 50 against 62;
+# 64 units of 1,408 x 4,096, 4 tokens 141 against 157, 16 tokens 357 against 363, 24 tokens 421 against 397.
+EXPERT_STREAM_TOKENS = 16
+
+
+def streams_experts(h, gate_up, down) -> bool:
+    """Whether a step with the inputs ``h`` [n, width] takes ``grouped_stream`` for its units (gate_up [units, rows, width], down
+    [units, width, inner]): 16-byte vectors along both products' k."""
+    return (h.dtype == torch.bfloat16 and 0 < h.shape[0] <= EXPERT_STREAM_TOKENS and h.is_contiguous() and gate_up.shape[2] % 8 == 0 and
+            down.shape[2] % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (h, gate_up, down)) and gate_up.shape[0] <= 65535)
+
+
+class _ExpertStream(ctypes.Structure):
+    """csrc/expert_stream.h's ExpertStream."""
+    _fields_ = [(n, ctypes.c_void_p) for n in ("ids", "scores", "pair_row", "limits")] + \
+               [(n, ctypes.c_int) for n in ("pairs", "per_row", "gated", "act")] + [("slope", ctypes.c_float), ("shift", ctypes.c_float)]
+
+
+def grouped_stream(y, x, w, ids, scores=None, pair_row=None, per_row=1, gated=False, relu2=False, limits=None, slope=0.0, shift=0.0):
+    """y [pairs, out] = act(w[ids[p]] x[p // per_row]) for every (token, choice) pair p with ids[p] >= 0, the matrices in use streamed
+    once (csrc/expert_stream.cu): ``gated``: w [units, 2 * out, in] holds gate rows then up rows and act is the clamped gated unit with
+    ``limits[unit]``; else w [units, out, in] and act is max(z, 0)^2 with ``relu2``, or nothing. ``scores``: a pair's row is times its score,
+    rounded. ``pair_row`` receives every pair's row of y (the pair itself, -1 for a choice without a unit)."""
+    pairs, (units, rows_w, k) = ids.numel(), w.shape
+    out = rows_w // 2 if gated else rows_w
+    ok = all(t is None or (t.is_cuda and t.is_contiguous() and t.dtype == d) for t, d in
+             ((y, torch.bfloat16), (x, torch.bfloat16), (w, torch.bfloat16), (ids, torch.int32), (scores, torch.float32), (pair_row, torch.int32),
+              (limits, torch.float32)))
+    if not ok or tuple(y.shape) != (pairs, out) or x.shape[1] != k or x.shape[0] * per_row != pairs:
+        raise KernelError(f"expert_stream: x {tuple(x.shape)}, w {tuple(w.shape)}, y {tuple(y.shape)} for {pairs} pairs")
+    ptr = lambda t: None if t is None else t.data_ptr()
+    args = _ExpertStream(ids.data_ptr(), ptr(scores), ptr(pair_row), ptr(limits), pairs, per_row, int(bool(gated)), int(bool(relu2)), slope, shift)
+    check(lib().ti_gemm_tcgen05_grouped(y.data_ptr(), x.data_ptr(), w.data_ptr(), None, pairs, 0, units, out, k, None, ctypes.byref(args), _stream()),
+          "expert_stream")
 
 
 def head_linear(y, x, w) -> bool:

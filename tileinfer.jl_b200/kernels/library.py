@@ -193,7 +193,7 @@ _SIGNATURES.update({
     "ti_expert_plan": [_P, _I, _I, _I, _I, _P, _P, _P, _P],
     "ti_expert_gather": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
     "ti_grouped_gemm": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _F, _F, _I, _P],
-    "ti_gemm_tcgen05_grouped": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P],
+    "ti_gemm_tcgen05_grouped": [_P, _P, _P, _P, _I, _I, _I, _I, _I, _P, _P, _P],
     "ti_gemm_tcgen05_heads": [_P, _P, _P, _I, _I, _I, _I, _P, _P],
     "ti_expert_combine": [_P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _P],
 })

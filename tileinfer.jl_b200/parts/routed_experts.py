@@ -149,12 +149,7 @@ class RoutedExperts(FeedForward):
             from ..kernels import fast
         ids = rt.buffer("experts.ids", (n, per_token), torch.int32)
         scores = rt.buffer("experts.scores", (n, per_token), torch.float32)
-        tile = fast.grouped_tile(pairs, self.units) if fast is not None else ops.EXPERT_TILE_ROWS
-        max_tiles, rows = ops.expert_plan_sizes(pairs, self.units, tile)
         pair_row = rt.buffer("experts.pair_row", (n, per_token), torch.int32)
-        row_pair = rt.buffer("experts.row_pair", (rows,), torch.int32)
-        plan = rt.buffer("experts.plan", (1 + max_tiles,), torch.int32)
-        xs = rt.buffer("experts.rows", (rows, W))
         logits = None
         if fast is not None:                     # the router's 32-bit sums from a product kernel, where one takes the sizes
             logits = fast.linear_f32(self.router_linear, h, rt.buffer("experts.logits", (n, self.router.shape[0]), torch.float32))
@@ -166,6 +161,33 @@ class RoutedExperts(FeedForward):
                               always=self.always, gate=self.gate_on, logit_bias=self.logit_bias, on_logits=self.on_logits)
         else:
             ops.router_topk(h, self.router, top, ids, scores, logits, always=self.always)
+        if fast is not None and fast.streams_experts(h, self.gate_up, self.down):
+            act, ys = rt.buffer("experts.act", (pairs, F)), rt.buffer("experts.out_rows", (pairs, W))
+            fast.grouped_stream(act, h, self.gate_up, ids, scores if self.scale_input else None, pair_row, per_token, gated=self.gated,
+                                relu2=not self.gated, limits=self.limits, slope=self.slope, shift=self.shift)
+            fast.grouped_stream(ys, act, self.down, ids)
+        else:
+            ys = self._grouped(h, ids, scores, pair_row, fast)
+        if self.scale_input:
+            return GatheredRows(ys, pair_row)    # the norm that reads the output adds a token's rows up itself
+        if self.rows_apart and pass_weight is None:
+            return GatheredRows(ys, pair_row, scores)
+        out = rt.buffer("feed_forward.delta", (n, W))
+        ops.expert_combine(out, ys, pair_row, scores, None, per_token, scale_output=True, h=h if pass_weight is not None else None,
+                           pass_weight=pass_weight)
+        return out
+
+    def _grouped(self, h, ids, scores, pair_row, fast):
+        """The units over rows grouped by unit and padded to tiles; ``pair_row`` receives the pairs' rows of the result."""
+        rt = self.rt
+        n, W = h.shape
+        F, per_token = self.spec.intermediate_size, self.top + self.always
+        pairs = n * per_token
+        tile = fast.grouped_tile(pairs, self.units) if fast is not None else ops.EXPERT_TILE_ROWS
+        max_tiles, rows = ops.expert_plan_sizes(pairs, self.units, tile)
+        row_pair = rt.buffer("experts.row_pair", (rows,), torch.int32)
+        plan = rt.buffer("experts.plan", (1 + max_tiles,), torch.int32)
+        xs = rt.buffer("experts.rows", (rows, W))
         ops.expert_plan(ids, self.units, tile, pair_row, row_pair, plan)
         ops.expert_gather(xs, h, pair_row, scores, per_token, self.scale_input)
         act = rt.buffer("experts.act", (rows, F))
@@ -181,11 +203,4 @@ class RoutedExperts(FeedForward):
         ys = rt.buffer("experts.out_rows", (rows, W))
         if not (fast is not None and fast.grouped_linear(ys, act, self.down, plan, tile)):
             ops.grouped_gemm(ys, act, self.down, plan, tile)
-        if self.scale_input:
-            return GatheredRows(ys, pair_row)    # the norm that reads the output adds a token's rows up itself
-        if self.rows_apart and pass_weight is None:
-            return GatheredRows(ys, pair_row, scores)
-        out = rt.buffer("feed_forward.delta", (n, W))
-        ops.expert_combine(out, ys, pair_row, scores, None, per_token, scale_output=True, h=h if pass_weight is not None else None,
-                           pass_weight=pass_weight)
-        return out
+        return ys
