@@ -48,7 +48,10 @@ struct ChunkArgs {
     float* ws;                   // [chunks, H, pitch]: S [D, V], then n [D]
     long long ws_pitch;
     float* total;                // [chunks, H]: e^(L_64)
+    int act = 0;                 // 1: q, k and v are SiLU of the rows, rounded to T
 };
+
+template <typename T> __device__ __forceinline__ float chunk_act(float v, int act) { return act ? rnd<T>(v / (1.0f + expf(-v))) : v; }
 
 // L and b of the chunk's tokens (beyond `count`: L stays, b is zero). 64 threads; the caller synchronises.
 __device__ __forceinline__ void chunk_decays(const ChunkArgs& a, int h, int t0, int count, double* L, float* add) {
@@ -112,7 +115,7 @@ __device__ __forceinline__ void stage_qk(const ChunkArgs& a, float* dst, int off
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < VEC; ++i) out[i] = v.v[i] * scale;
+                for (int i = 0; i < VEC; ++i) out[i] = chunk_act<T>(v.v[i], a.act) * scale;
             } else {
 #pragma unroll
                 for (int i = 0; i < VEC; ++i) out[i] = 0.f;
@@ -131,7 +134,7 @@ __device__ __forceinline__ void stage_qk(const ChunkArgs& a, float* dst, int off
                     const float w = to_f32(__ldcg(row + (low ? d + half : d - half)));
                     v = v * c.x + (low ? -1.f : 1.f) * (w * c.y);
                 }
-                v *= scale;
+                v = chunk_act<T>(v, a.act) * scale;
             }
             dst[s * MC_PITCH + d - d0] = v;
         }
@@ -154,9 +157,9 @@ __device__ __forceinline__ void stage_v(const ChunkArgs& a, float* dst, const fl
             Vec16<T> v;
             if (in) v.load_cg(src);
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) out[i] = in ? v.v[i] * w : 0.f;
+            for (int i = 0; i < VEC; ++i) out[i] = in ? chunk_act<T>(v.v[i], a.act) * w : 0.f;
         } else {
-            out[0] = in ? to_f32(__ldcg(src)) * w : 0.f;
+            out[0] = in ? chunk_act<T>(to_f32(__ldcg(src)), a.act) * w : 0.f;
         }
     }
 }
@@ -527,6 +530,15 @@ extern "C" int ti_memory_chunks(void* y, float* o, float* nq, const float* em, c
                          cos_sin != nullptr ? rotary : 0, q_scale, k_scale, ws, ti_memory_chunk_pitch(D, V), total};
     const ChunkOut out = {y, o, nq, em, w, gate_sigmoid, eps};
     return launch_chunks(a, out, state, state_stride, chunks, seq_slots, dtype, stream);
+}
+
+// Linear attention with a decay per head over prompts (csrc/lightning.cu): o [n, H * V] float, q, k and v through SiLU where `act`.
+int lightning_chunks(float* o, const void* rows, long long ld, int q_off, int k_off, int v_off, float* state, const float* decay, const int* cu_seqlens,
+                     const int* seq_slots, int B, int H, int D, int V, int act, float* ws, float* total, int chunks, int dtype, cudaStream_t stream) {
+    ChunkArgs a = {rows, ld, q_off, k_off, v_off, 0, cu_seqlens, nullptr, B, H, D, V, decay, nullptr, 0, 0, 1, nullptr, nullptr, 0, 1.f, 1.f, ws,
+                   ti_memory_chunk_pitch(D, V), total, act};
+    const ChunkOut out = {nullptr, o, nullptr, nullptr, nullptr, 0, 0.f};
+    return launch_chunks(a, out, state, (long long)H * D * V, chunks, seq_slots, dtype, stream);
 }
 
 // The state-space cell: rows [n, ld] of T with x (H * V columns) at x_off, B and C (groups * N each) at b_off and c_off; coef [n, H, 2] = (l, dt);

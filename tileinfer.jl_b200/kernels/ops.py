@@ -508,17 +508,30 @@ def sum_add_norm32(x, d1, d2, h, w_out, eps_out, offset_out=False):
                                   int(bool(offset_out)), eps_out, n, size, dtype_code(dtype), _stream()), "sum_add_norm32")
 
 
-def lightning_scan(o, rows, q_off, k_off, v_off, state, decay, cu_seqlens, seq_slots, batch, heads, dim, vdim, act=True):
+def _chunk_args(chunked, heads, dim, vdim):
+    if chunked is None:
+        return (None, None, 0)
+    chunks, ws, total = chunked
+    _need(ws, "ws", torch.float32); _need(total, "total", torch.float32)
+    if ws.numel() < chunks * heads * int(lib().ti_memory_chunk_pitch(dim, vdim)) or total.numel() < chunks * heads:
+        raise KernelError(f"lightning_scan: work space of {ws.numel()} floats for {chunks} chunks")
+    return (ws.data_ptr(), total.data_ptr(), chunks)
+
+
+def lightning_scan(o, rows, q_off, k_off, v_off, state, decay, cu_seqlens, seq_slots, batch, heads, dim, vdim, act=True, chunked=None):
     """The recurrence S = a_h S + k v^T, o = S^T q over the step's tokens of every sequence, from and to ``state``
     [slots, heads, dim, vdim] float32. ``rows`` [n, ld]: the projections' output with queries, keys and values from the given
-    columns on; ``act``: SiLU on them. o [n, heads * vdim] float32."""
+    columns on; ``act``: SiLU on them. o [n, heads * vdim] float32. ``chunked`` (chunks, work space, totals) as ``memory_chunk_sizes`` says:
+    the tokens are worked on in chunks side by side; the decays are then above zero."""
     _need(o, "o", torch.float32); _need(rows, "rows", contiguous=False); _need(state, "state", torch.float32); _need(decay, "decay", torch.float32)
     _need(cu_seqlens, "cu_seqlens", torch.int32); _need(seq_slots, "seq_slots", torch.int32)
     if rows.stride(1) != 1 or tuple(state.shape[1:]) != (heads, dim, vdim) or decay.numel() != heads:
         raise KernelError(f"lightning_scan: rows {tuple(rows.shape)}, state {tuple(state.shape)} for {heads} heads of {dim} x {vdim}")
     check(lib().ti_lightning_scan(o.data_ptr(), rows.data_ptr(), rows.stride(0), q_off, k_off, v_off, state.data_ptr(), decay.data_ptr(),
-                                  cu_seqlens.data_ptr(), seq_slots.data_ptr(), rows.shape[0], batch, heads, dim, vdim, int(bool(act)), dtype_code(rows.dtype),
-                                  _stream()), "lightning_scan")
+                                  cu_seqlens.data_ptr(), seq_slots.data_ptr(), rows.shape[0], batch, heads, dim, vdim, int(bool(act)), *_chunk_args(chunked, heads,
+                                  dim, vdim), dtype_code(rows.dtype), _stream()), "lightning_scan")
+    if chunked is not None:
+        _library.add_launches(2)                 # three kernels in place of one
 
 
 def lightning_out(y, o, gate, w, eps):

@@ -22,6 +22,7 @@ from ..config.spec import MixerSpec, TensorDecl
 from ..kernels import ops
 from .base import CacheRequest, Mixer, register_mixer
 from .linear import Linear
+from .matrix_memory import CHUNKED_FROM
 
 
 @register_mixer("lightning")
@@ -34,6 +35,8 @@ class LightningAttention(Mixer):
         if len(decay) != self.heads:
             raise ValueError(f"lightning: {len(decay)} decays for {self.heads} heads")
         self.decay = torch.tensor(decay, dtype=torch.float64).to(torch.float32).to(rt.device)
+        # Chunks work with the logarithms of the decays: a decay that has none (zero or below) keeps to the token-by-token scan.
+        self.chunks = bool((self.decay > 0).all())
         self.eps = float(o.get("norm_eps", 1e-6))
         self.gated = bool(o.get("gate", True))
         act = o.get("activation", "silu")
@@ -70,8 +73,12 @@ class LightningAttention(Mixer):
         rows = rt.buffer("lightning.rows", (n, self.proj.out_features))
         self.proj.forward(h, rows)
         o = rt.buffer("lightning.o", (n, H * V), torch.float32)
+        chunked = None
+        if self.chunks and step.max_q_len >= CHUNKED_FROM:
+            chunks, floats = ops.memory_chunk_sizes(step.host_q_lens, H, D, V)
+            chunked = (chunks, rt.buffer("memory.chunks", (floats,), torch.float32), rt.buffer("memory.totals", (chunks, H), torch.float32))
         ops.lightning_scan(o, rows, 0, H * D, 2 * H * D, cache.state, self.decay, step.cu_seqlens, step.seq_slots, step.n_seqs, H, D, V,
-                           act=self.act)
+                           act=self.act, chunked=chunked)
         y = rt.buffer("lightning.normed", (n, H * V))
         ops.lightning_out(y, o, rows[:, 2 * H * D + H * V:] if self.gated else None, self.norm_w, self.eps)
         out = rt.buffer("mixer.delta", (n, self.spec.hidden_size))
