@@ -13,7 +13,7 @@
 // between the loads and the one rounding on store is 32-bit. d is a sublayer's output: [n, size] in T, or the
 // 32-bit partial sums [s, n, size] of a product that was cut over k (added in split order, not rounded).
 // One block per row; the order of a row's sums depends on the row's size alone.
-#include "common.cuh"
+#include "row_quads.cuh"
 
 template <typename T>
 __global__ void embed_positions32_kernel(float* __restrict__ x, const T* __restrict__ table, const T* __restrict__ pos_table,
@@ -378,6 +378,111 @@ __global__ void branch_norm_add32_vec_kernel(float* x, const bf16* delta, const 
     }
 }
 
+// The same with a row in registers: a thread owns NQ quads, and everything it needs (branch, stream, and ahead of the wait for the kernel
+// before the weights and the bias) is asked for before the first sum. A decode step of 8 rows of 2,048: 4.5 -> 3.1 us.
+template <int NQ>
+__global__ void __launch_bounds__(512, NQ == 1 ? 2 : 1) branch_norm_add32_quads_kernel(float* x, const bf16* delta, const float* partials, int n_partials,
+                                                                                       size_t partial_stride, const int* gather, int per_row,
+                                                                                       const bf16* __restrict__ dbias, const bf16* __restrict__ w, int offset,
+                                                                                       float eps, float mult, bf16* __restrict__ h,
+                                                                                       const bf16* __restrict__ w_out, int offset_out, float eps_out, int size) {
+    __shared__ float scratch[33];
+    const int tid = threadIdx.x, threads = blockDim.x;
+    const size_t t = blockIdx.x;
+    float* row = x + t * size;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 g[NQ], go[NQ], db[NQ];
+    int at[NQ];
+    bool in[NQ];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+        at[k] = (tid + k * threads) * 4;
+        in[k] = at[k] < size;
+        g[k] = in[k] ? load_weight4(w + at[k]) : zero;
+        go[k] = in[k] && w_out != nullptr ? load_weight4(w_out + at[k]) : zero;
+        db[k] = in[k] && dbias != nullptr ? load_weight4(dbias + at[k]) : zero;
+    }
+    pdl_enter();
+    float4 xv[NQ];
+    float d[NQ][4], ss = 0.f, sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+        xv[k] = in[k] ? load_row4(row + at[k]) : zero;
+        float4 v = zero;
+        if (in[k]) {
+            if (partials != nullptr) {
+                const float* p = partials + t * size + at[k];
+                v = load_row4(p);
+                for (int s = 1; s < n_partials; ++s) {
+                    const float4 q = load_row4(p + (size_t)s * partial_stride);
+                    v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+                }
+            } else if (gather != nullptr) {
+                for (int j = 0; j < per_row; ++j) {
+                    const float4 q = load_row4(delta + (size_t)__ldcg(gather + t * per_row + j) * size + at[k]);
+                    v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+                }
+            } else {
+                v = load_row4(delta + t * size + at[k]);
+            }
+            if (dbias != nullptr) { v.x += db[k].x; v.y += db[k].y; v.z += db[k].z; v.w += db[k].w; }
+        }
+        d[k][0] = v.x; d[k][1] = v.y; d[k][2] = v.z; d[k][3] = v.w;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            ss = fmaf(d[k][e], d[k][e], ss);
+            sum += d[k][e];
+        }
+    }
+    float mean = 0.f;
+    if (offset & 2) {
+        mean = block_sum(sum, scratch) / (float)size;
+        ss = 0.f;
+#pragma unroll
+        for (int k = 0; k < NQ; ++k)
+            if (in[k])
+#pragma unroll
+                for (int e = 0; e < 4; ++e) ss = fmaf(d[k][e] - mean, d[k][e] - mean, ss);
+    }
+    const float inv = 1.0f / sqrtf(block_sum(ss, scratch) / (float)size + eps);
+    float ss2 = 0.f, sum2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+        if (!in[k]) continue;
+        const float xs[4] = {xv[k].x, xv[k].y, xv[k].z, xv[k].w}, gs[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            d[k][e] = xs[e] + mult * ((d[k][e] - mean) * inv * ((offset & 1) ? 1.0f + gs[e] : gs[e]));
+            ss2 = fmaf(d[k][e], d[k][e], ss2);
+            sum2 += d[k][e];
+        }
+        store_row4(row + at[k], d[k]);
+    }
+    if (h == nullptr) return;
+    float inv2 = 1.0f, mean2 = 0.f;
+    if (w_out != nullptr) {
+        if (offset_out & 2) {
+            mean2 = block_sum(sum2, scratch) / (float)size;
+            ss2 = 0.f;
+#pragma unroll
+            for (int k = 0; k < NQ; ++k)
+                if (in[k])
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) ss2 = fmaf(d[k][e] - mean2, d[k][e] - mean2, ss2);
+        }
+        inv2 = 1.0f / sqrtf(block_sum(ss2, scratch) / (float)size + eps_out);
+    }
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+        if (!in[k]) continue;
+        const float gs[4] = {go[k].x, go[k].y, go[k].z, go[k].w};
+        if (w_out != nullptr)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) d[k][e] = (d[k][e] - mean2) * inv2 * ((offset_out & 1) ? 1.0f + gs[e] : gs[e]);
+        store_row4(h + t * size + at[k], d[k]);
+    }
+}
+
 extern "C" int ti_branch_norm_add32(float* x, const void* delta, const float* partials, int n_partials, long long partial_stride,
                                     const int* gather, int per_row, const void* dbias, const void* w, int offset, float eps, float mult, void* h,
                                     const void* w_out, int offset_out, float eps_out, int n_rows, int size, int dtype, cudaStream_t stream) {
@@ -398,7 +503,12 @@ extern "C" int ti_branch_norm_add32(float* x, const void* delta, const float* pa
         }
         const bool vec = sizeof(T) == 2 && size % 4 == 0 && smem <= 48 * 1024 && aligned16(x) && (partials == nullptr || (aligned16(partials) && partial_stride % 4 == 0)) &&
                          (((uintptr_t)delta | (uintptr_t)dbias | (uintptr_t)w | (uintptr_t)h | (uintptr_t)w_out) & 7) == 0;
-        if (vec) {
+        if (vec && size <= 4096) {
+            const int quads = size / 4, per = quads > 512 ? 2 : 1, qt = ((quads + per - 1) / per + 31) / 32 * 32;
+            ti_launch(per == 1 ? branch_norm_add32_quads_kernel<1> : branch_norm_add32_quads_kernel<2>, dim3(n_rows), dim3(qt), 0, stream, x,
+                      (const bf16*)delta, partials, n_partials, (size_t)partial_stride, gather, per_row, (const bf16*)dbias, (const bf16*)w, offset, eps,
+                      mult, (bf16*)h, (const bf16*)w_out, offset_out, eps_out, size);
+        } else if (vec) {
             const int vt = size >= 2048 ? 256 : 128;
             ti_launch(branch_norm_add32_vec_kernel, dim3(n_rows), dim3(vt), smem, stream, x, (const bf16*)delta, partials, n_partials,
                       (size_t)partial_stride, gather, per_row, (const bf16*)dbias, (const bf16*)w, offset, eps, mult, (bf16*)h, (const bf16*)w_out,
