@@ -60,6 +60,7 @@ struct Params {
     int w_group_rows, m_fastest;
     int batch, w_batch_rows, x_batch_k;
     long long y_batch_cols;
+    int tile_n;                  // pair kernel: tokens per tile, a multiple of 32 up to 256
 };
 
 // MT: 128-row weight sub-tiles per block. With MT = 2 a block owns 256 weight rows: the token
@@ -409,6 +410,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                          const __grid_constant__ CUtensorMap map_y, void* __restrict__ y, Params p) {
     typedef PairCfg C;
     constexpr int BN = C::BN;
+    const int tile_n = p.tile_n;                           // tokens of a tile: half of them staged by each block
     extern __shared__ unsigned char smem_dyn[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
     unsigned char* tiles = smem;
@@ -446,14 +448,14 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             for (int kb = it.kb_lo; kb < it.kb_hi; ++kb) {
                 ok = mbar_wait(empty0 + 8 * stage, phase ^ 1, p.status, 1);
                 if (!ok) break;
-                if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * C::STAGE_BYTES);
+                if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * (C::A_BYTES + C::KB * (tile_n / 2) * BK * 2));
                 const unsigned bar = map_to_block(full0 + 8 * stage, 0);
                 const unsigned a_dst = smem_addr(tiles + (size_t)stage * C::STAGE_BYTES);
 #pragma unroll
                 for (int a = 0; a < C::KB; ++a) {
                     tma_load_2d_pair(a_dst + a * C::ATOM_BYTES, &map_w, (kb * C::KB + a) * BK, (it.m * 2 + (int)rank) * BM, bar);
                     tma_load_2d_pair(a_dst + C::A_BYTES + a * C::ATOM_BYTES, &map_x, (kb * C::KB + a) * BK,
-                                     it.n * BN + (int)rank * (BN / 2), bar);
+                                     it.n * tile_n + (int)rank * (tile_n / 2), bar);
                 }
                 if (++stage == C::STAGES) { stage = 0; phase ^= 1; }
             }
@@ -464,7 +466,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         unsigned phase = 0;
         int local = 0;
         bool ok = true;
-        constexpr unsigned IDESC = instr_desc_bf16(2 * BM, BN, false);
+        const unsigned idesc = instr_desc_bf16(2 * BM, tile_n, false);
         while (rank == 0 && lane == 0 && ok && it.next(p)) {
             const int acc = local & 1;
             const unsigned acc_phase = (local >> 1) & 1;
@@ -480,7 +482,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
 #pragma unroll
                 for (int k = 0; k < C::KB * BK / 16; ++k) {            // 16 k = 32 bytes along the swizzled row; 64 k = the next block of rows
                     const unsigned off = (k / 4) * C::ATOM_BYTES + (k % 4) * 32;
-                    umma_bf16_pair(d_tmem, smem_desc_sw128(a_addr + off), smem_desc_sw128(a_addr + C::A_BYTES + off), IDESC,
+                    umma_bf16_pair(d_tmem, smem_desc_sw128(a_addr + off), smem_desc_sw128(a_addr + C::A_BYTES + off), idesc,
                                    (kb > it.kb_lo || k > 0) ? 1u : 0u);
                 }
                 umma_commit_pair(empty0 + 8 * stage);      // the stage is free in both blocks once these MMAs have read it
@@ -503,8 +505,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * acc, acc_phase, p.status, 4));
             if (!ok) break;
             tc_fence_after();
-            const int n0 = it.n * BN;
-            const int n_valid = min(BN, p.N - n0);
+            const int n0 = it.n * tile_n;
+            const int n_valid = min(tile_n, p.N - n0);
             const int m_first = (it.m * 2 + (int)rank) * BM + quarter * 32;
             const unsigned t_row = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(acc * BN);
             epilogue_rows<BN, C::EPI_WARPS, C::OUT_BYTES>(t_row, m_first, lane, n0, n_valid, col_group, warp - 2, it.split, out_buf, out_tiles,
@@ -576,6 +578,23 @@ int launch_pair(void* y, const CUtensorMap& mw, const CUtensorMap& mx, const CUt
     return ti_check_launch("gemm_tcgen05 (pairs)");
 }
 
+// Tokens per tile of the pair kernel: the multiple of 32 from 128 to 256 that takes the least time by rounds of the pairs, each as
+// long as the tile's MMAs plus what does not shrink with the tile (in tokens: fitted to a sweep of 272 to 8,192 tokens x 3,072 to
+// 21,504 features, whose best width it misses by 0.3 % on average, 6 % at worst; widths of 256 throughout are 11 % longer). With 256
+// alone 1,283 tokens are padded to 1,536 and 96 tiles take two rounds of 74 pairs: the down projection (4,096 x 21,504) 230 us, in
+// tiles of 160 tokens 189; up (21,504 x 4,096) 187 -> 182 in tiles of 224; 512 tokens of q|k|v (6,144 x 4,096) 34 -> 30 in tiles of 192.
+#define PAIR_TILE_FIXED 112
+int pair_tile_tokens(int n, int m_tiles, int splits, int pairs) {
+    int best = 256;
+    long long least = -1;
+    for (int t = 256; t >= 128; t -= 32) {
+        const long long tiles = (long long)m_tiles * ((n + t - 1) / t) * splits;
+        const long long time = (tiles + pairs - 1) / pairs * (t + PAIR_TILE_FIXED);
+        if (least < 0 || time < least) { best = t; least = time; }
+    }
+    return best;
+}
+
 // Chooses the tile shape and kernel for one product. (Giving the rows of a ragged last wave to a second
 // launch with smaller tiles was measured and is slower: the few tiles of a last wave run faster than
 // those of a full one, with the memory system and the power budget to themselves.)
@@ -590,29 +609,31 @@ int gemm_dispatch(void* y, long long ldy, const void* x, long long ldx, const vo
     // stay, so the epilogue (xIELU included) overlaps the next tile, and a stage of 128 of k means one barrier
     // round trip per 1,024 tensor-core cycles. Measured on 2048 tokens: up projection with xIELU 257 us
     // (296 us with 128-row blocks of one SM), q|k|v 72 us (82 us), o 49 us (55 us).
-    // With a long k (the down projection) one block per SM with 256 weight rows, whose epilogue is not
-    // overlapped but rare, is a little faster still (233 us against 239 us), where it needs fewer waves.
-    int mt = 1;
     const long long n_t = (n + bn - 1) / bn;
-    if (bn == 256 && splits <= 1 && in >= 8192) {
-        const long long waves1 = (((out + BM - 1) / BM) * n_t + sm_count - 1) / sm_count;
-        const long long waves2 = (((out + 2 * BM - 1) / (2 * BM)) * n_t + sm_count - 1) / sm_count;
-        if (3 * waves2 < 2 * waves1) mt = 2;
-    }
     // (A product of a few hundred tokens with few output rows has fewer tiles than there are SM pairs: it may come cut
     // over k, each slice a tile of its own, leaving 32-bit partial sums.)
-    const bool pair = mt == 1 && bn == 256 && (splits <= 1 || (epilogue == EPI_PARTIAL && n > 256)) && out >= 2 * BM && pair_clusters(sm_count) > 0;
-    if (pair) mt = 2;
+    bool pair = bn == 256 && (splits <= 1 || (epilogue == EPI_PARTIAL && n > 256)) && out >= 2 * BM && pair_clusters(sm_count) > 0;
+    const int pair_n = pair ? pair_tile_tokens(n, (out + 2 * BM - 1) / (2 * BM), splits < 1 ? 1 : splits, pair_clusters(sm_count)) : bn;
+    // With a long k (the down projection) one block per SM with 256 weight rows, whose epilogue is not
+    // overlapped but rare, is a little faster still where pairs would take full tiles and it needs fewer waves
+    // (2,048 tokens 244 us against 250, 3,000 tokens 373 against 394; 1,283 tokens 239 against 189 in the pairs' smaller tiles).
+    int mt = pair ? 2 : 1;
+    if (bn == 256 && splits <= 1 && in >= 8192 && pair_n == bn) {
+        const long long waves1 = (((out + BM - 1) / BM) * n_t + sm_count - 1) / sm_count;
+        const long long waves2 = (((out + 2 * BM - 1) / (2 * BM)) * n_t + sm_count - 1) / sm_count;
+        if (3 * waves2 < 2 * waves1) { mt = 2; pair = false; }
+    }
     p.M = out;
     p.m_tiles = (out + mt * BM - 1) / (mt * BM);
-    p.n_tiles = (int)n_t;
+    p.tile_n = pair ? pair_n : bn;
+    p.n_tiles = pair ? (n + p.tile_n - 1) / p.tile_n : (int)n_t;
     p.k_blocks = pair ? (in + PairCfg::KB * BK - 1) / (PairCfg::KB * BK) : (in + BK - 1) / BK;     // the pair kernel's stages hold 128 of k
     p.splits = splits < 1 ? 1 : (splits > p.k_blocks ? p.k_blocks : splits);
     TI_REQUIRE(p.splits == 1 || epilogue == EPI_PARTIAL, "gemm_tcgen05: a split product leaves partial sums");
     p.ldy = ldy; p.epilogue = epilogue; p.act = act; p.status = status;
     CUtensorMap mw, mx, my;
     if (int rc = tensor_map(&mw, W, out, in, in, BM)) return rc;
-    if (int rc = tensor_map(&mx, x, n, in, ldx, pair ? bn / 2 : bn)) return rc;   // a pair's blocks load half a token tile each
+    if (int rc = tensor_map(&mx, x, n, in, ldx, pair ? p.tile_n / 2 : bn)) return rc;   // a pair's blocks load half a token tile each
     // A step of a few tokens: all blocks would ask L2 for the same token lines at the same time, so each weight
     // tile walks its k range from a start of its own (a function of the tile alone: a token's result does not
     // depend on the step it is in). With many tokens the tiles of a row of blocks share lines on purpose.
@@ -646,7 +667,7 @@ int sm_count_cached() {
 // Many matrices in one launch of the one-block-per-tile kernel, bfloat16 out. `bn`: tokens per tile.
 int many_dispatch(void* y, long long ldy, const void* x, long long ldx, const void* W, long long w_rows, int n, int out, int in, int bn,
                   Params p, int* status, cudaStream_t stream) {
-    p.N = n; p.K = in; p.M = out;
+    p.N = n; p.K = in; p.M = out; p.tile_n = bn;
     p.m_fastest = p.groups != nullptr && bn >= 128;
     // Token tiles of 128 with 256 weight rows per block: the token operand staged for a k block feeds two MMAs (tiles of
     // 128 x 128 are bound by the fill of shared memory).

@@ -87,6 +87,8 @@ def tc_splits(out_features: int, in_features: int, n: int) -> int:
     add partial sums: as many as fill the device's block slots (two per SM for token tiles of up to 64), at
     most 8, each at least 512 of k. Measured at 64 tokens: down projection 46 us in 3 slices, 35 us in 8;
     o 17 us in 2, 11 us in 8."""
+    if n > 768:
+        return 1        # tiles of fewer tokens fill the pairs as well and leave no partial sums (1,283 tokens: 189 us, in whole tiles 230)
     if n > 256:
         # A prompt of a few hundred tokens: tiles of 256 weight rows x 256 tokens on SM pairs. A product with few output
         # rows has fewer of them than there are pairs (the down projection of 512 tokens: 32 tiles for 74 pairs) and is
