@@ -48,8 +48,10 @@ def test_units_streamed_by_pair(units, out, k, tokens, per_token, gated):
                 bound = off * (2 * z.abs() + off)
             assert bool(((y[p].cpu().to(F64) - want).abs() <= bound + want.abs() * 2.0 ** -7 + 1e-6).all()), p
     down = (torch.randn(units, 24, out, generator=g) * out ** -0.5).bfloat16()
-    y2 = torch.zeros((pairs, 24), dtype=torch.bfloat16, device="cuda")
+    y2, y3 = torch.zeros((pairs, 24), dtype=torch.bfloat16, device="cuda"), torch.zeros((pairs, 24), dtype=torch.bfloat16, device="cuda")
     fast.grouped_stream(y2, y, down.cuda(), ids.cuda())
+    fast.grouped_stream(y3, y, down.cuda(), ids.cuda(), ahead=True)
+    assert torch.equal(y2, y3)
     for p in range(pairs):
         e = int(ids.flatten()[p])
         if e >= 0:

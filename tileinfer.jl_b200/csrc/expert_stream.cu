@@ -41,19 +41,22 @@ template <bool GATED, bool SCALE>
 __global__ void __launch_bounds__(ES_WARPS * 32, 2) expert_stream_kernel(bf16* __restrict__ y, const bf16* x, const bf16* __restrict__ W,
                                                                       const int* ids, const float* scores, int* __restrict__ pair_row, int pairs,
                                                                       int per_row, int by_pair, int out, int K, int act, const float* __restrict__ limits,
-                                                                      float slope, float shift) {
+                                                                      float slope, float shift, int ahead) {
     __shared__ float red[ES_WARPS][2][32][4];
     __shared__ int chosen[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int row0 = blockIdx.x * (GATED ? 16 : 32);
-    pdl_wait();
-    pdl_launch_dependents();
+    bool waited = !ahead;
+    if (waited) pdl_enter();
     const bool heads = ids == nullptr;                     // a matrix per head: pair p is token p / units, head p % units
     if (pair_row != nullptr && blockIdx.x == 0 && blockIdx.y == 0)     // a pair's result is its own row; a choice without a unit has none
         for (int p = threadIdx.x; p < pairs; p += ES_WARPS * 32) pair_row[p] = __ldcg(ids + p) >= 0 ? p : -1;
     // With `by_pair` a block's unit is that of pair blockIdx.y, if no pair before it chose the same one.
     const int unit = by_pair ? __ldcg(ids + blockIdx.y) : (int)blockIdx.y;
-    if (unit < 0) return;
+    if (unit < 0) {
+        if (!waited) pdl_wait();                           // no block ends before the kernel ahead: the next one counts on that
+        return;
+    }
     const bf16* w = W + (size_t)unit * (GATED ? 2 : 1) * out * K;
     const int next = GATED ? out : 16;                     // rows between the two tiles
     const uint4* wr[2][2];
@@ -83,7 +86,10 @@ __global__ void __launch_bounds__(ES_WARPS * 32, 2) expert_stream_kernel(bf16* _
             }
             seen += here;
         }
-        if (first >= seen || (by_pair && leader != (int)blockIdx.y)) return;      // the same for every thread of the block
+        if (first >= seen || (by_pair && leader != (int)blockIdx.y)) {           // the same for every thread of the block
+            if (!waited) pdl_wait();
+            return;
+        }
         if (warp == 0 && t == 0) chosen[g] = mine;
         const bf16* xrow = x + (size_t)(mine < 0 ? 0 : mine / per_row) * K;
         const float score = SCALE && mine >= 0 ? __ldcg(scores + mine) : 1.f;
@@ -102,7 +108,12 @@ __global__ void __launch_bounds__(ES_WARPS * 32, 2) expert_stream_kernel(bf16* _
                 for (int j = 0; j < 2; ++j)
 #pragma unroll
                     for (int i = 0; i < 2; ++i) a[j][i][u] = ok ? es_load_weights(wr[j][i] + idx) : zero;
-                v[u] = ok && mine >= 0 ? es_load_rows(reinterpret_cast<const uint4*>(xrow) + idx) : zero;
+            }
+            if (!waited) { pdl_enter(); waited = true; }   // the first weights are on their way
+#pragma unroll
+            for (int u = 0; u < ES_U; ++u) {
+                const int bb = b + u * ES_WARPS, idx = bb * 4 + t;
+                v[u] = bb < blocks && bb * 32 + 8 * t < K && mine >= 0 ? es_load_rows(reinterpret_cast<const uint4*>(xrow) + idx) : zero;
             }
 #pragma unroll
             for (int u = 0; u < ES_U; ++u) {
@@ -124,6 +135,7 @@ __global__ void __launch_bounds__(ES_WARPS * 32, 2) expert_stream_kernel(bf16* _
                 }
             }
         }
+        if (!waited) { pdl_enter(); waited = true; }       // a warp without work orders its writes after the kernel ahead too
 #pragma unroll
         for (int j = 0; j < 2; ++j) *reinterpret_cast<float4*>(red[warp][j][lane]) = make_float4(c[j][0], c[j][1], c[j][2], c[j][3]);
         __syncthreads();
@@ -159,6 +171,7 @@ int expert_stream(void* y, const void* x, const void* W, const ExpertStream& e, 
                units, out, in);
     TI_REQUIRE(in % 8 == 0 && aligned16(x) && aligned16(W), "expert_stream: rows of %d must be 16-byte vectors", in);
     TI_REQUIRE(!e.gated || e.limits != nullptr, "expert_stream: a gated unit needs its limits");
+    TI_REQUIRE(!e.ahead || (e.scores == nullptr && e.pair_row == nullptr), "expert_stream: scores and rows are the kernel before's");
     TI_REQUIRE(e.ids != nullptr || (e.pairs % units == 0 && e.pair_row == nullptr), "expert_stream: %d rows of %d heads", e.pairs, units);
     TI_REQUIRE(e.act == ES_ACT_NONE || e.act == ES_ACT_RELU2, "expert_stream: unknown activation %d", e.act);
     const int rows = e.gated ? 16 : 32;
@@ -167,7 +180,7 @@ int expert_stream(void* y, const void* x, const void* W, const ExpertStream& e, 
     const int by_pair = e.ids != nullptr && e.pairs < units;
     const dim3 grid((out + rows - 1) / rows, by_pair ? e.pairs : units), block(ES_WARPS * 32);
 #define ES_LAUNCH(G, S) ti_launch(expert_stream_kernel<G, S>, grid, block, 0, stream, (bf16*)y, (const bf16*)x, (const bf16*)W, e.ids, e.scores, e.pair_row, \
-                                  e.pairs, e.per_row, by_pair, out, in, e.act, e.limits, e.slope, e.shift)
+                                  e.pairs, e.per_row, by_pair, out, in, e.act, e.limits, e.slope, e.shift, e.ahead)
     if (e.gated) { if (e.scores != nullptr) ES_LAUNCH(true, true); else ES_LAUNCH(true, false); }
     else { if (e.scores != nullptr) ES_LAUNCH(false, true); else ES_LAUNCH(false, false); }
 #undef ES_LAUNCH

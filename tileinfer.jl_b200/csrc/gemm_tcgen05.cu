@@ -736,6 +736,7 @@ extern "C" int ti_gemm_tcgen05_heads(void* y, const void* x, const void* W, int 
         ExpertStream e = {};
         e.pairs = n * heads;
         e.per_row = 1;
+        e.ahead = 1;
         return expert_stream(y, x, W, e, heads, out_h, in_h, stream);
     }
     Params p;

@@ -239,14 +239,15 @@ def streams_experts(h, gate_up, down) -> bool:
 class _ExpertStream(ctypes.Structure):
     """csrc/expert_stream.h's ExpertStream."""
     _fields_ = [(n, ctypes.c_void_p) for n in ("ids", "scores", "pair_row", "limits")] + \
-               [(n, ctypes.c_int) for n in ("pairs", "per_row", "gated", "act")] + [("slope", ctypes.c_float), ("shift", ctypes.c_float)]
+               [(n, ctypes.c_int) for n in ("pairs", "per_row", "gated", "act", "ahead")] + [("slope", ctypes.c_float), ("shift", ctypes.c_float)]
 
 
-def grouped_stream(y, x, w, ids, scores=None, pair_row=None, per_row=1, gated=False, relu2=False, limits=None, slope=0.0, shift=0.0):
+def grouped_stream(y, x, w, ids, scores=None, pair_row=None, per_row=1, gated=False, relu2=False, limits=None, slope=0.0, shift=0.0, ahead=False):
     """y [pairs, out] = act(w[ids[p]] x[p // per_row]) for every (token, choice) pair p with ids[p] >= 0, the matrices in use streamed
     once (csrc/expert_stream.cu): ``gated``: w [units, 2 * out, in] holds gate rows then up rows and act is the clamped gated unit with
     ``limits[unit]``; else w [units, out, in] and act is max(z, 0)^2 with ``relu2``, or nothing. ``scores``: a pair's row is times its score,
-    rounded. ``pair_row`` receives every pair's row of y (the pair itself, -1 for a choice without a unit)."""
+    rounded. ``pair_row`` receives every pair's row of y (the pair itself, -1 for a choice without a unit). ``ahead``: the kernel right
+    before this one has not written ``ids`` (an earlier one has): they and the first weights are read while it still runs."""
     pairs, (units, rows_w, k) = ids.numel(), w.shape
     out = rows_w // 2 if gated else rows_w
     ok = all(t is None or (t.is_cuda and t.is_contiguous() and t.dtype == d) for t, d in
@@ -255,7 +256,7 @@ def grouped_stream(y, x, w, ids, scores=None, pair_row=None, per_row=1, gated=Fa
     if not ok or tuple(y.shape) != (pairs, out) or x.shape[1] != k or x.shape[0] * per_row != pairs:
         raise KernelError(f"expert_stream: x {tuple(x.shape)}, w {tuple(w.shape)}, y {tuple(y.shape)} for {pairs} pairs")
     ptr = lambda t: None if t is None else t.data_ptr()
-    args = _ExpertStream(ids.data_ptr(), ptr(scores), ptr(pair_row), ptr(limits), pairs, per_row, int(bool(gated)), int(bool(relu2)), slope, shift)
+    args = _ExpertStream(ids.data_ptr(), ptr(scores), ptr(pair_row), ptr(limits), pairs, per_row, int(bool(gated)), int(bool(relu2)), int(bool(ahead)), slope, shift)
     check(lib().ti_gemm_tcgen05_grouped(y.data_ptr(), x.data_ptr(), w.data_ptr(), None, pairs, 0, units, out, k, None, ctypes.byref(args), _stream()),
           "expert_stream")
 

@@ -165,7 +165,7 @@ class RoutedExperts(FeedForward):
             act, ys = rt.buffer("experts.act", (pairs, F)), rt.buffer("experts.out_rows", (pairs, W))
             fast.grouped_stream(act, h, self.gate_up, ids, scores if self.scale_input else None, pair_row, per_token, gated=self.gated,
                                 relu2=not self.gated, limits=self.limits, slope=self.slope, shift=self.shift)
-            fast.grouped_stream(ys, act, self.down, ids)
+            fast.grouped_stream(ys, act, self.down, ids, ahead=True)         # the first product lies between the router and this one
         else:
             ys = self._grouped(h, ids, scores, pair_row, fast)
         if self.scale_input:
