@@ -76,3 +76,26 @@ def test_attention_over_chunk_edges(ops, D, nq, nkv):
                 bound = 2.0 ** -24 * (2 * D * size + 4 * math.sqrt(len(seen)) + 16) * float(values.abs().max())
                 assert float((together[r, h].double() - want).abs().max()) <= bound, (p, h, window)
             assert torch.equal(run([r])[0], together[r])
+
+
+def test_attention_beyond_two_to_the_31_rows(ops):
+    """A pool of one-element heads with more rows than a 32-bit integer counts: a sequence whose pages lie at its end gets what the same
+    keys and values give in a pool of their own."""
+    page, nkv, nq, keys = 16, 2, 4, 300
+    g = torch.Generator().manual_seed(31)
+    used = -(-keys // page)
+    k, v = (torch.randn(used, nkv, page, 1, generator=g).bfloat16().cuda() for _ in range(2))
+    q = torch.randn(3, nq, 1, generator=g).bfloat16().cuda()
+    positions = torch.tensor([0, 255, keys - 1], dtype=torch.int32, device="cuda")
+
+    def run(k_pool, v_pool, first):
+        table = torch.arange(first, first + used, dtype=torch.int32, device="cuda")[None]
+        out = torch.empty(3, nq, dtype=torch.bfloat16, device="cuda")
+        ops.attention_plain(out, q, k_pool, v_pool, table, torch.zeros_like(positions), positions, 1.0, nq, nkv, 1, page)
+        return out
+
+    want = run(k, v, 0)
+    pages = 2 ** 31 // (nkv * page) + used                # 4.3 GB each; only the last pages are written and read
+    k_pool, v_pool = (torch.empty(pages, nkv, page, 1, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    k_pool[-used:], v_pool[-used:] = k, v
+    assert torch.equal(run(k_pool, v_pool, pages - used), want)

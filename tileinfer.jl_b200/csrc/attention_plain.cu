@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
     float* qs = smem;                                 // [AP_HEADS][Dq], zeros beyond D
     float* ps = smem + AP_HEADS * Dq;                 // [AP_CHUNK][AP_HEADS]
     float* part_sums = ps + AP_CHUNK * AP_HEADS;      // [AP_WARPS][Dq]
-    __shared__ int rows[AP_CHUNK];                    // a key's row in the cache, in rows of D elements
+    __shared__ long long rows[AP_CHUNK];              // a key's row in the cache, in rows of D elements (pools of small heads hold more than 2^31)
     __shared__ float maxima[AP_WARPS][AP_HEADS], sums[AP_WARPS][AP_HEADS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = nq / nkv;
@@ -102,14 +102,14 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
         const int hi = (c0 + AP_CHUNK - 1 < end) ? c0 + AP_CHUNK - 1 : end;       // inclusive
         const int j = c0 + tid;
         const bool mine = j >= lo && j <= hi;
-        const int row = mine ? (__ldcg(table + j / page_size) * nkv + kvh) * page_size + j % page_size : 0;
+        const long long row = mine ? ((long long)__ldcg(table + j / page_size) * nkv + kvh) * page_size + j % page_size : 0;
         __syncthreads();                              // the chunk before is done with rows and ps; q is there
         rows[tid] = row;
         float s[AP_HEADS];
 #pragma unroll
         for (int h = 0; h < AP_HEADS; ++h) s[h] = 0.f;
         if (mine) {
-            const T* krow = k_cache + (size_t)row * D;
+            const T* krow = k_cache + row * D;
 #pragma unroll 8
             for (int d0 = 0; d0 < Dq; d0 += 4) {
                 float kv[4];
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
         for (int g = a > 0 ? a / takes * takes : 0; g <= b; g += takes) {
             const int k = g + sub, i0 = 32 * warp + k;
             if (k < a || k > b) continue;
-            const T* vrow = v_cache + (size_t)rows[i0] * D;
+            const T* vrow = v_cache + rows[i0] * D;
             const float4 pv = *reinterpret_cast<const float4*>(ps + i0 * AP_HEADS);
             const float w[AP_HEADS] = {pv.x, pv.y, pv.z, pv.w};
 #pragma unroll
