@@ -87,12 +87,14 @@ def tc_splits(out_features: int, in_features: int, n: int) -> int:
     add partial sums: as many as fill the device's block slots (two per SM for token tiles of up to 64), at
     most 8, each at least 512 of k. Measured at 64 tokens: down projection 46 us in 3 slices, 35 us in 8;
     o 17 us in 2, 11 us in 8."""
-    if n > 768:
-        return 1        # tiles of fewer tokens fill the pairs as well and leave no partial sums (1,283 tokens: 189 us, in whole tiles 230)
     if n > 256:
         # A prompt of a few hundred tokens: tiles of 256 weight rows x 256 tokens on SM pairs. A product with few output
         # rows has fewer of them than there are pairs (the down projection of 512 tokens: 32 tiles for 74 pairs) and is
         # cut over k into the number of slices (up to 4, each at least 1,024 of k) that takes the fewest rounds of the pairs.
+        # The sums of a cut product reach a 32-bit stream without being rounded first.
+        # (The kernel then chooses tiles of 128 to 256 tokens by itself. With the consumer's reads counted, this choice takes 1 % longer on
+        # average than the best number of slices, 11 % at worst (512 tokens x 2,048 x 4,096), over 300 to 2,048 tokens of nine products on
+        # warm SMs; without cuts above 768 tokens 982 tokens x 2,048 x 8,192 take 50 us instead of 42, 1,283 x 4,096 x 21,504 224 instead of 201.)
         tiles = -(-out_features // 256) * -(-n // 256)
         pairs = max(1, sm_count() // 2)
         tile_us = in_features * 0.00585                  # 256 x 256 x k on two SMs at 11.2 TFLOP/s each
