@@ -45,3 +45,33 @@ def test_lightning_in_chunks(dtype, H, D, V, act):
     tol = 1e-4 if dtype == torch.float32 else 4e-3
     assert float((o.to(F64).view(n, H, V) - want).abs().max()) <= tol * max(1.0, float(want.abs().max()))
     assert torch.equal(state[4].cpu(), state0[4])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D,V", [(12, 20), (128, 128)])
+def test_an_infinity_does_not_reach_the_tokens_ahead_of_it(dtype, D, V):
+    """A query, key or value that is infinite or NaN, at every place of a group of four tokens: the outputs of earlier tokens of the sequence
+    and of the other sequences are the bits that they are without it; its own and later ones are not finite."""
+    from tileinfer_b200.kernels import ops
+    H, lengths = 2, [70, 130, 66]
+    g = torch.Generator().manual_seed(D)
+    n = sum(lengths)
+    clean = torch.randn(n, 2 * H * D + H * V, generator=g).to(dtype)
+    decay = torch.tensor([0.9, 0.998], device="cuda")
+    sp = _step(lengths, [0, 1, 2])
+    chunks, floats = ops.memory_chunk_sizes(lengths, H, D, V)
+
+    def run(rows):
+        state, o = torch.zeros(3, H, D, V, device="cuda"), torch.empty(n, H * V, device="cuda")
+        space = (chunks, torch.empty(floats, device="cuda"), torch.empty(chunks, H, device="cuda"))
+        ops.lightning_scan(o, rows.cuda(), 0, H * D, 2 * H * D, state, decay, sp.cu_seqlens, sp.seq_slots, 3, H, D, V, act=False, chunked=space)
+        return o
+    want = run(clean)
+    for t in (1, 2, 3, 4, 63, 65, 66, 67):                # places in the second sequence: first chunk, its last token, second chunk
+        for column, bad in ((2 * H * D + 1, float("inf")), (2 * H * D + 1, float("nan")), (H * D + 1, float("inf")), (1, float("nan"))):
+            rows = clean.clone()
+            rows[lengths[0] + t, column] = bad
+            got, at = run(rows), lengths[0] + t
+            assert torch.equal(got[:at], want[:at]), (t, column, bad)
+            assert torch.equal(got[lengths[0] + lengths[1]:], want[lengths[0] + lengths[1]:])
+            assert not bool(torch.isfinite(got[at, :V]).all())

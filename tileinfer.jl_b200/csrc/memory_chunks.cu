@@ -445,8 +445,9 @@ __global__ void __launch_bounds__(MC_THREADS, 2) memory_chunk_outputs_kernel(Chu
 #pragma unroll
         for (int j = 0; j < 8; ++j) acc[i][j] *= w;
     }
-    // The chunk's own share: P v. (P was written before the barriers above; a head of no rows does not exist.)
-    const int last = min(MC_TOKENS, ry * 4 + 4);         // later tokens' weights are zero
+    // The chunk's own share: P v. (P was written before the barriers above; a head of no rows does not exist.) Later tokens are left out
+    // by the choice of terms, not by a weight of zero: zero times an infinity or a NaN would reach the tokens ahead of it.
+    const int last = min(MC_TOKENS, ry * 4 + 4);
     for (int s16 = 0; s16 < last; s16 += 16) {
     float part[4][8];
 #pragma unroll
@@ -457,6 +458,7 @@ __global__ void __launch_bounds__(MC_THREADS, 2) memory_chunk_outputs_kernel(Chu
         float4 p4[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) p4[i] = *reinterpret_cast<const float4*>(P + (ry * 4 + i) * (MC_TOKENS + 4) + s);
+        const bool past_all = s < ry * 4;                // all four tokens are past for all four rows; else they are the rows' own
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const float4 s0 = *reinterpret_cast<const float4*>(vs + (s + k) * MC_SLAB + cx * 4), s1 = *reinterpret_cast<const float4*>(vs + (s + k) * MC_SLAB + 64 + cx * 4);
@@ -464,8 +466,9 @@ __global__ void __launch_bounds__(MC_THREADS, 2) memory_chunk_outputs_kernel(Chu
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float w = k == 0 ? p4[i].x : k == 1 ? p4[i].y : k == 2 ? p4[i].z : p4[i].w;
+                if (k <= i || past_all)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) part[i][j] = fmaf(w, sv[j], part[i][j]);
+                    for (int j = 0; j < 8; ++j) part[i][j] = fmaf(w, sv[j], part[i][j]);
             }
         }
     }
