@@ -99,3 +99,36 @@ def test_attention_beyond_two_to_the_31_rows(ops):
     k_pool, v_pool = (torch.empty(pages, nkv, page, 1, dtype=torch.bfloat16, device="cuda") for _ in range(2))
     k_pool[-used:], v_pool[-used:] = k, v
     assert torch.equal(run(k_pool, v_pool, pages - used), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("k", [40, 1031, 1042, 1544])      # one segment; an odd k; 2 modulo 8; several segments and a part of one, in 16-byte rows
+def test_every_tile_shape_and_width_of_copy(ops, dtype, k):
+    """Tiles of every shape with ragged edges, and steps of few tokens, with the operands' rows on 16 bytes, on 4, and on single elements:
+    one order of additions, so the bits of a token alone in rows of 16 bytes, and its distance to 64-bit sums."""
+    from tileinfer_b200.kernels import fast, lib
+    choose = lib().handle.ti_gemm_plain_shape
+    sizes = [(500, 4090), (390, 1999), (250, 2001), (100, 333), (1, 50), (7, 333), (13, 2001), (61, 100)]
+    assert {choose(n, out, fast.sm_count()) for n, out in sizes[:4]} == {0, 1, 2, 3}
+    g = torch.Generator(device="cuda").manual_seed(k)
+    wide = -(-k // 8) * 8                                  # the same k terms and zeros, in rows of 16 bytes
+    for n, out in sizes:
+        x = torch.zeros(n, wide, device="cuda", dtype=dtype)
+        w = torch.zeros(out, wide, device="cuda", dtype=dtype)
+        x[:, :k] = torch.randn(n, k, generator=g, device="cuda")
+        w[:, :k] = torch.randn(out, k, generator=g, device="cuda") * k ** -0.5
+        want = torch.empty(n, out, device="cuda")
+        for t in range(n):
+            ops.gemm_plain(want[t:t + 1], x[t:t + 1], w, ops.EPI_F32_OUT)
+        exact, mass = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+        bound = (min(k, 512) / 2 + 1 + k / 512) * 2.0 ** -24 * mass + (exact.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0.0)
+        assert bool(((want.double() - exact).abs() <= bound).all())
+        narrow = w[:, :k].contiguous()
+        for pad, base in ((0, 0), (1, 0), (2, 0), (8, 0), (8, 1), (8, 2)):      # the tokens' row pitch beyond k, and the first row's place
+            store = torch.full((base + n * (k + pad),), float("nan"), dtype=dtype, device="cuda")
+            rows = store[base:].view(n, k + pad)[:, :k]
+            rows.copy_(x[:, :k])
+            y = torch.full((n + 1, out), 7.0, device="cuda")
+            ops.gemm_plain(y[:n], rows, narrow, ops.EPI_F32_OUT)
+            assert torch.equal(y[:n], want), (n, out, pad, base)
+            assert bool((y[n] == 7.0).all())

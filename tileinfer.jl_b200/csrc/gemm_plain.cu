@@ -5,7 +5,7 @@
 // one token and in a step of thousands. It is the 32-bit path's product and the fallback of
 // the bfloat16 path for sizes the tensor-core kernel refuses.
 //
-// The order, common to the four kernels below: k is cut into segments of GP_SEGMENT terms. In a
+// The order, common to both kernels below: k is cut into segments of GP_SEGMENT terms. In a
 // segment the terms of even k and those of odd k are two chains of fused multiply-adds from zero
 // in ascending order (the two halves of a packed fma.rn.f32x2, which takes one issue slot where two
 // fused multiply-adds take two); a segment's sum is even + odd, and the segments' sums are added in
@@ -21,9 +21,6 @@
 #include "packed_f32.cuh"
 
 #define GP_SEGMENT 512
-#define GP_BM 64      // tokens per tile
-#define GP_BN 64      // output features per tile
-#define GP_BK 16
 
 #define TI_EPI_NONE 0
 #define TI_EPI_XIELU 1
@@ -39,141 +36,11 @@ __device__ __forceinline__ void store_output(void* y, long long ldy, int r, int 
     else ((T*)y)[(size_t)r * ldy + c] = from_f32<T>(v);
 }
 
-// ---- rows that cannot be read 16 bytes at a time: 64 x 64 tiles, element by element
-template <typename T>
-__global__ void __launch_bounds__(256) gemm_plain_kernel(void* __restrict__ y, long long ldy, const T* x,
-                                                        long long ldx, const T* __restrict__ W, int n, int out,
-                                                        int in, int epilogue, XieluParams act) {
-    __shared__ float As[GP_BK][GP_BM + 4];
-    __shared__ float Bs[GP_BK][GP_BN + 4];
-    const int tid = threadIdx.x;
-    const int m0 = blockIdx.y * GP_BM, n0 = blockIdx.x * GP_BN;
-    const int tr = tid / 16, tc = tid % 16;       // 16 x 16 threads, 4 x 4 outputs each
-    float acc[2][4][4], total[4][4];              // even and odd chains of the segment; the segments before it
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[0][i][j] = acc[1][i][j] = total[i][j] = 0.f;
-
-    // Each thread stages 4 consecutive k of one row of each operand tile.
-    const int lrow = tid / 4, lk = (tid % 4) * 4;
-    pdl_wait();
-    pdl_launch_dependents();
-    for (int k0 = 0; k0 < in; k0 += GP_BK) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int k = k0 + lk + i;
-            const int r = m0 + lrow, c = n0 + lrow;
-            As[lk + i][lrow] = (r < n && k < in) ? to_f32(__ldcg(x + (size_t)r * ldx + k)) : 0.f;
-            Bs[lk + i][lrow] = (c < out && k < in) ? to_f32(W[(size_t)c * in + k]) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GP_BK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][tr * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tc * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
-        }
-        __syncthreads();
-        if ((k0 + GP_BK) % GP_SEGMENT == 0 || k0 + GP_BK >= in) {
-            const bool first = k0 < GP_SEGMENT;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float s = acc[0][i][j] + acc[1][i][j];
-                    total[i][j] = first ? s : total[i][j] + s;
-                    acc[0][i][j] = acc[1][i][j] = 0.f;
-                }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = m0 + tr * 4 + i;
-        if (r >= n) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = n0 + tc * 4 + j;
-            if (c < out) store_output<T>(y, ldy, r, c, total[i][j], epilogue, act);
-        }
-    }
-}
-
-// The same for steps of few tokens: a block owns GV_ROWS output features and streams their weight rows once, in k blocks
-// staged in shared memory; a thread owns one feature and every GV_SLOTS-th token.
-#define GV_ROWS 16
-#define GV_SLOTS 8
-#define GV_BK 64
-#define GV_MAX_TOKENS 64
-
-template <typename T, int TPT>                           // TPT: tokens per thread (the step has at most TPT * GV_SLOTS tokens)
-__global__ void __launch_bounds__(GV_ROWS * GV_SLOTS) gemv_plain_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
-                                                                         const T* __restrict__ W, int n, int out, int in, int epilogue,
-                                                                         XieluParams act) {
-    __shared__ float Ws[GV_ROWS][GV_BK + 1];
-    extern __shared__ float Xs[];                         // [n][GV_BK + 1]
-    const int tid = threadIdx.x;
-    const int row = tid % GV_ROWS, slot = tid / GV_ROWS;
-    const int m0 = blockIdx.x * GV_ROWS;
-    float acc[2][TPT], total[TPT];
-#pragma unroll
-    for (int j = 0; j < TPT; ++j) acc[0][j] = acc[1][j] = total[j] = 0.f;
-    pdl_wait();
-    pdl_launch_dependents();
-    for (int k0 = 0; k0 < in; k0 += GV_BK) {
-        for (int i = tid; i < GV_ROWS * GV_BK; i += GV_ROWS * GV_SLOTS) {
-            const int r = i / GV_BK, kk = i % GV_BK;
-            const int c = m0 + r, k = k0 + kk;
-            Ws[r][kk] = (c < out && k < in) ? to_f32(W[(size_t)c * in + k]) : 0.f;
-        }
-        for (int i = tid; i < n * GV_BK; i += GV_ROWS * GV_SLOTS) {
-            const int t = i / GV_BK, kk = i % GV_BK;
-            Xs[t * (GV_BK + 1) + kk] = (k0 + kk < in) ? to_f32(__ldcg(x + (size_t)t * ldx + k0 + kk)) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll 4
-        for (int kk = 0; kk < GV_BK; kk += 2) {
-            const float w0 = Ws[row][kk], w1 = Ws[row][kk + 1];
-#pragma unroll
-            for (int j = 0; j < TPT; ++j) {
-                const int t = slot + j * GV_SLOTS;
-                if (t < n) {
-                    acc[0][j] = fmaf(Xs[t * (GV_BK + 1) + kk], w0, acc[0][j]);
-                    acc[1][j] = fmaf(Xs[t * (GV_BK + 1) + kk + 1], w1, acc[1][j]);
-                }
-            }
-        }
-        __syncthreads();
-        if ((k0 + GV_BK) % GP_SEGMENT == 0 || k0 + GV_BK >= in) {
-#pragma unroll
-            for (int j = 0; j < TPT; ++j) {
-                const float s = acc[0][j] + acc[1][j];
-                total[j] = k0 < GP_SEGMENT ? s : total[j] + s;
-                acc[0][j] = acc[1][j] = 0.f;
-            }
-        }
-    }
-    const int c = m0 + row;
-    if (c >= out) return;
-#pragma unroll
-    for (int j = 0; j < TPT; ++j) {
-        const int t = slot + j * GV_SLOTS;
-        if (t < n) store_output<T>(y, ldy, t, c, total[j], epilogue, act);
-    }
-}
-
-// ---- rows that can be read 16 bytes at a time
-//
-// Both kernels stage k blocks of 128 bytes a row (32 floats or 64 bfloat16 values) by 16-byte cp.async as they lie in memory; rows
-// are 144 bytes apart in shared memory, so eight consecutive rows' 16-byte pieces fall into different banks. Four consecutive
-// k of a row are one read: the packed multiply-add's operands are (k, k + 1) pairs of both sides, with no transposition and no
-// duplicated element.
+// Both kernels stage k blocks of 128 bytes a row (32 floats or 64 bfloat16 values) as they lie in memory, in pieces of PIECE bytes by
+// cp.async: 16 where every row of both operands starts on such a boundary, else 4, and single bfloat16 values, which no asynchronous
+// copy takes, through registers (as floats: the conversions are then one per element and not one per use). Rows are 144 bytes apart in
+// shared memory, so eight consecutive rows' 16-byte pieces fall into different banks. Four consecutive k of a row are one read: the
+// packed multiply-add's operands are (k, k + 1) pairs of both sides, with no transposition and no duplicated element.
 #define GT_ROW 144
 #define GT_BYTES 128
 
@@ -196,9 +63,48 @@ template <> struct Quad<bf16> {
     }
 };
 
-// 16 bytes to shared memory, or 16 zero bytes (nothing is read from `src` then).
+// 16 or 4 bytes to shared memory, or as many zero bytes (nothing is read from `src` then).
 __device__ __forceinline__ void stage16(unsigned dst, const void* src, bool inside) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(inside ? 16 : 0));
+}
+__device__ __forceinline__ void stage4(unsigned dst, const void* src, bool inside) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(inside ? 4 : 0));
+}
+// What lies in shared memory: the elements themselves, but single bfloat16 values, which pass through registers anyway, as floats.
+template <typename T, int PIECE> struct Staged {
+    typedef T type;
+    static constexpr int BYTES = PIECE;                    // of a piece there
+};
+template <> struct Staged<bf16, 2> {
+    typedef float type;
+    static constexpr int BYTES = 4;
+};
+// COUNT pieces of fewer than 16 bytes: `at(i, dst, src)` says where piece i goes and comes from and whether it lies inside the matrix. Of
+// single elements up to MOST loads leave together. (16-byte pieces, whose loops stand in the kernels, need no such care.)
+template <typename T, int PIECE, int COUNT, int MOST, typename F> __device__ __forceinline__ void stage_pieces(F at) {
+    if constexpr (PIECE == 4) {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) {
+            unsigned char* dst; const T* src;
+            const bool inside = at(i, dst, src);
+            stage4(smem_u32(dst), src, inside);
+        }
+    } else {
+        constexpr int AT_ONCE = COUNT <= MOST ? COUNT : 8;
+        static_assert(COUNT % AT_ONCE == 0 && sizeof(T) == PIECE, "whole rounds of single elements");
+#pragma unroll 1
+        for (int i0 = 0; i0 < COUNT; i0 += AT_ONCE) {
+            unsigned char* dst[AT_ONCE];
+            T v[AT_ONCE];
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) {
+                const T* src;
+                v[u] = at(i0 + u, dst[u], src) ? __ldcg(src) : from_f32<T>(0.f);
+            }
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) *reinterpret_cast<float*>(dst[u]) = to_f32(v[u]);
+        }
+    }
 }
 
 // Steps of up to 32 tokens: weights are streamed once. A block owns 16 * RPT output rows, its warps take the segments of k in
@@ -208,13 +114,15 @@ __device__ __forceinline__ void stage16(unsigned dst, const void* src, bool insi
 // What bounds it: weight bytes and, from 8 tokens on, shared-memory reads (a row's quad is read by one lane pair, a token's by 16
 // lanes; neighbouring lanes share both, which halves the reads' passes). Measured at 8 tokens: up projection (21,504 x 4,096, 352
 // MB) 77 us, 4.6 TB/s, where one chain per output and 16 bytes per token and thread took 220; down (4,096 x 21,504) 83 us (335).
-template <typename T, int TPL, int RPT, int STAGES>
+template <typename T, int TPL, int RPT, int STAGES, int PIECE>
 __global__ void __launch_bounds__(256) gemv_plain_stream_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
                                                                 const T* __restrict__ W, int n, int out, int in, int epilogue,
                                                                 XieluParams act) {
     extern __shared__ __align__(16) unsigned char gv_smem[];
     constexpr int ROWS = 16 * RPT, TOKENS = 2 * TPL;
-    constexpr int BK = GT_BYTES / (int)sizeof(T), PER_SEG = GP_SEGMENT / BK, VEC = 16 / (int)sizeof(T);
+    typedef typename Staged<T, PIECE>::type E;
+    constexpr int IN_ROW = Staged<T, PIECE>::BYTES, PER_ROW = GT_BYTES / IN_ROW, VEC = PIECE / (int)sizeof(T);
+    constexpr int BK = GT_BYTES / (int)sizeof(E), PER_SEG = GP_SEGMENT / BK;
     constexpr int STAGE = (ROWS + TOKENS) * GT_ROW;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
     const int row = lane & 15, half = lane >> 4;
@@ -231,15 +139,26 @@ __global__ void __launch_bounds__(256) gemv_plain_stream_kernel(void* __restrict
     const bool has_last = mine > 0 && (mine - 1) * warps + warp == segments - 1;
     const int tiles = mine * PER_SEG - (has_last ? PER_SEG - last_blocks : 0);
     auto k_of = [&](int tile) { return ((tile / PER_SEG) * warps + warp) * GP_SEGMENT + (tile % PER_SEG) * BK; };
+    // A warp's pieces of a k block: piece i * 32 + lane, PER_ROW of them a row; a piece is inside its row or outside it (in % VEC == 0).
     auto issue_w = [&](int tile) {
         if (tile < tiles) {
             const int k0 = k_of(tile);
             unsigned char* s = ring + (tile % STAGES) * STAGE;
+            if constexpr (PIECE == 16) {
 #pragma unroll
-            for (int i = 0; i < ROWS * 8 / 32; ++i) {
-                const int r = (i * 32 + lane) >> 3, c = lane & 7, k = k0 + c * VEC;
-                const bool inside = m0 + r < out && k < in;                 // in % VEC == 0: a vector is inside the row or outside it
-                stage16(smem_u32(s + r * GT_ROW + c * 16), inside ? W + (size_t)(m0 + r) * in + k : W, inside);
+                for (int i = 0; i < ROWS * 8 / 32; ++i) {
+                    const int r = (i * 32 + lane) >> 3, c = lane & 7, k = k0 + c * VEC;
+                    const bool inside = m0 + r < out && k < in;
+                    stage16(smem_u32(s + r * GT_ROW + c * 16), inside ? W + (size_t)(m0 + r) * in + k : W, inside);
+                }
+            } else {
+                stage_pieces<T, PIECE, ROWS * PER_ROW / 32, 16>([&](int i, unsigned char*& dst, const T*& src) {
+                    const int r = (i * 32 + lane) / PER_ROW, c = (i * 32 + lane) % PER_ROW, k = k0 + c * VEC;
+                    const bool inside = m0 + r < out && k < in;
+                    dst = s + r * GT_ROW + c * IN_ROW;
+                    src = inside ? W + (size_t)(m0 + r) * in + k : W;
+                    return inside;
+                });
             }
         }
     };
@@ -247,12 +166,22 @@ __global__ void __launch_bounds__(256) gemv_plain_stream_kernel(void* __restrict
         if (tile < tiles) {
             const int k0 = k_of(tile);
             unsigned char* s = ring + (tile % STAGES) * STAGE + ROWS * GT_ROW;
+            if constexpr (PIECE == 16) {
 #pragma unroll
-            for (int i = 0; i < (TOKENS * 8 + 31) / 32; ++i) {
-                const int r = (i * 32 + lane) >> 3, c = lane & 7, k = k0 + c * VEC;
-                if (TOKENS * 8 < 32 && r >= TOKENS) continue;
-                const bool inside = r < n && k < in;
-                stage16(smem_u32(s + r * GT_ROW + c * 16), inside ? x + (size_t)r * ldx + k : x, inside);
+                for (int i = 0; i < (TOKENS * 8 + 31) / 32; ++i) {
+                    const int r = (i * 32 + lane) >> 3, c = lane & 7, k = k0 + c * VEC;
+                    if (TOKENS * 8 < 32 && r >= TOKENS) continue;
+                    const bool inside = r < n && k < in;
+                    stage16(smem_u32(s + r * GT_ROW + c * 16), inside ? x + (size_t)r * ldx + k : x, inside);
+                }
+            } else {
+                stage_pieces<T, PIECE, TOKENS * PER_ROW / 32, 16>([&](int i, unsigned char*& dst, const T*& src) {
+                    const int r = (i * 32 + lane) / PER_ROW, c = (i * 32 + lane) % PER_ROW, k = k0 + c * VEC;
+                    const bool inside = r < n && k < in;
+                    dst = s + r * GT_ROW + c * IN_ROW;
+                    src = inside ? x + (size_t)r * ldx + k : x;
+                    return inside;
+                });
             }
         }
     };
@@ -282,13 +211,13 @@ __global__ void __launch_bounds__(256) gemv_plain_stream_kernel(void* __restrict
             const unsigned char* xs = s + (ROWS + half) * GT_ROW;
 #pragma unroll
             for (int c = 0; c < BK / 4; ++c) {
-                Quad<T> w[RPT];
+                Quad<E> w[RPT];
 #pragma unroll
-                for (int q = 0; q < RPT; ++q) w[q].load(ws + q * 16 * GT_ROW + c * Quad<T>::BYTES);
+                for (int q = 0; q < RPT; ++q) w[q].load(ws + q * 16 * GT_ROW + c * Quad<E>::BYTES);
 #pragma unroll
                 for (int j = 0; j < TPL; ++j) {
-                    Quad<T> v;
-                    v.load(xs + 2 * j * GT_ROW + c * Quad<T>::BYTES);
+                    Quad<E> v;
+                    v.load(xs + 2 * j * GT_ROW + c * Quad<E>::BYTES);
 #pragma unroll
                     for (int q = 0; q < RPT; ++q) acc[q][j] = fma2(v.p[1], w[q].p[1], fma2(v.p[0], w[q].p[0], acc[q][j]));
                 }
@@ -324,40 +253,63 @@ __global__ void __launch_bounds__(256) gemv_plain_stream_kernel(void* __restrict
 // What bounds it: the FMA units, at 0.7 of their rate at the clock that a long run of them settles at (ncu: 1.6 GHz; a
 // thread's fragments come in 16-byte reads of which every second or fourth lane's is its own). 512 tokens x 21,504 x 4,096: 2,230
 // us, 40 TFLOP/s; tiles staged with k outermost, 8 x 8 outputs a thread and single multiply-adds took 4,500.
-template <typename T, int TI, int TJ, int STAGES>
-__global__ void __launch_bounds__(256) gemm_plain_tile_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
+// (Single elements are not on their way while a k block is worked on, so two or three blocks share an SM; a lower bound of one block for
+// the others makes the compiler spend more registers: 512 tokens of the 32-bit model at 8B sizes 0.4 % longer.)
+template <typename T, int TI, int TJ, int STAGES, int PIECE>
+__global__ void __launch_bounds__(256, PIECE == 2 ? (TI * TJ <= 16 ? 3 : 2) : 0) gemm_plain_tile_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
                                                              const T* __restrict__ W, int n, int out, int in, int epilogue,
                                                              XieluParams act) {
     extern __shared__ __align__(16) unsigned char gt_smem[];
     constexpr int TM = 16 * TI, TN = 16 * TJ;
-    constexpr int BK = GT_BYTES / (int)sizeof(T), PER_SEG = GP_SEGMENT / BK, VEC = 16 / (int)sizeof(T);
-    constexpr int STAGE = (TM + TN) * GT_ROW;
+    typedef typename Staged<T, PIECE>::type E;
+    constexpr int IN_ROW = Staged<T, PIECE>::BYTES, PER_ROW = GT_BYTES / IN_ROW, VEC = PIECE / (int)sizeof(T);
+    constexpr int BK = GT_BYTES / (int)sizeof(E), PER_SEG = GP_SEGMENT / BK;
+    constexpr int STAGE = (TM + TN) * GT_ROW, STEP = 256 / PER_ROW;            // staging: STEP rows at a time
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     const int tx = (lane & 7) + 8 * (warp & 1), ty = (lane >> 3) + 4 * (warp >> 1);
     float* total = reinterpret_cast<float*>(gt_smem + STAGES * STAGE);        // [TI * TJ][256]
     const int blocks = (in + BK - 1) / BK;
-    const int lrow = tid >> 3, lc = tid & 7;                                 // staging: 32 rows of 8 pieces at a time
+    const int lrow = tid / PER_ROW, lc = tid % PER_ROW;
     auto issue = [&](int b, bool weights, bool tokens) {
         if (b < blocks) {
-            unsigned char* s = gt_smem + (b % STAGES) * STAGE + lrow * GT_ROW + lc * 16;
+            unsigned char* s = gt_smem + (b % STAGES) * STAGE + lrow * GT_ROW + lc * IN_ROW;
             const int k = b * BK + lc * VEC;
             const bool k_ok = k < in;
-            if (tokens) {
+            if constexpr (PIECE == 16) {
+                if (tokens) {
 #pragma unroll
-                for (int i = 0; i < TM / 32; ++i) {
-                    const int r = m0 + lrow + 32 * i;
-                    const bool inside = k_ok && r < n;
-                    stage16(smem_u32(s + 32 * i * GT_ROW), inside ? x + (size_t)r * ldx + k : x, inside);
+                    for (int i = 0; i < TM / 32; ++i) {
+                        const int r = m0 + lrow + 32 * i;
+                        const bool inside = k_ok && r < n;
+                        stage16(smem_u32(s + 32 * i * GT_ROW), inside ? x + (size_t)r * ldx + k : x, inside);
+                    }
                 }
-            }
-            if (weights) {
+                if (weights) {
 #pragma unroll
-                for (int i = 0; i < TN / 32; ++i) {
-                    const int c = n0 + lrow + 32 * i;
-                    const bool inside = k_ok && c < out;
-                    stage16(smem_u32(s + (TM + 32 * i) * GT_ROW), inside ? W + (size_t)c * in + k : W, inside);
+                    for (int i = 0; i < TN / 32; ++i) {
+                        const int c = n0 + lrow + 32 * i;
+                        const bool inside = k_ok && c < out;
+                        stage16(smem_u32(s + (TM + 32 * i) * GT_ROW), inside ? W + (size_t)c * in + k : W, inside);
+                    }
                 }
+            } else {
+                if (tokens)
+                    stage_pieces<T, PIECE, TM / STEP, 8>([&](int i, unsigned char*& dst, const T*& src) {
+                        const int r = m0 + lrow + STEP * i;
+                        const bool inside = k_ok && r < n;
+                        dst = s + STEP * i * GT_ROW;
+                        src = inside ? x + (size_t)r * ldx + k : x;
+                        return inside;
+                    });
+                if (weights)
+                    stage_pieces<T, PIECE, TN / STEP, 8>([&](int i, unsigned char*& dst, const T*& src) {
+                        const int c = n0 + lrow + STEP * i;
+                        const bool inside = k_ok && c < out;
+                        dst = s + (TM + STEP * i) * GT_ROW;
+                        src = inside ? W + (size_t)c * in + k : W;
+                        return inside;
+                    });
             }
         }
     };
@@ -381,13 +333,13 @@ __global__ void __launch_bounds__(256) gemm_plain_tile_kernel(void* __restrict__
         const unsigned char* bs = gt_smem + (b % STAGES) * STAGE + (TM + tx) * GT_ROW;
 #pragma unroll
         for (int c = 0; c < BK / 4; ++c) {
-            Quad<T> w[TJ];
+            Quad<E> w[TJ];
 #pragma unroll
-            for (int j = 0; j < TJ; ++j) w[j].load(bs + j * 16 * GT_ROW + c * Quad<T>::BYTES);
+            for (int j = 0; j < TJ; ++j) w[j].load(bs + j * 16 * GT_ROW + c * Quad<E>::BYTES);
 #pragma unroll
             for (int i = 0; i < TI; ++i) {
-                Quad<T> v;
-                v.load(as + i * 16 * GT_ROW + c * Quad<T>::BYTES);
+                Quad<E> v;
+                v.load(as + i * 16 * GT_ROW + c * Quad<E>::BYTES);
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -426,37 +378,39 @@ template <typename K> static cudaError_t allow_smem(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-template <typename T, int TPL, int RPT, int STAGES>
+template <typename T, int TPL, int RPT, int STAGES, int PIECE>
 static int launch_stream(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
                          const XieluParams& act, cudaStream_t stream) {
     constexpr int ROWS = 16 * RPT, MAX_WARPS = 8;
     constexpr size_t PER_WARP = (size_t)STAGES * (ROWS + 2 * TPL) * GT_ROW + 2 * 2 * TPL * ROWS * sizeof(float);
     constexpr size_t TOTAL = 2 * TPL * ROWS * sizeof(float);
-    static const cudaError_t allowed = allow_smem(gemv_plain_stream_kernel<T, TPL, RPT, STAGES>, MAX_WARPS * PER_WARP + TOTAL);
+    static const cudaError_t allowed = allow_smem(gemv_plain_stream_kernel<T, TPL, RPT, STAGES, PIECE>, MAX_WARPS * PER_WARP + TOTAL);
     if (allowed != cudaSuccess) return ti_fail("gemv_plain: %s", cudaGetErrorString(allowed));
     const int segments = (in + GP_SEGMENT - 1) / GP_SEGMENT, rounds = (segments + MAX_WARPS - 1) / MAX_WARPS;
     const int warps = (segments + rounds - 1) / rounds;                        // as few as the rounds need: the last round is full
-    ti_launch(gemv_plain_stream_kernel<T, TPL, RPT, STAGES>, dim3((out + ROWS - 1) / ROWS, (n + 2 * TPL - 1) / (2 * TPL)), dim3(32 * warps), warps * PER_WARP + TOTAL, stream, y,
+    ti_launch(gemv_plain_stream_kernel<T, TPL, RPT, STAGES, PIECE>, dim3((out + ROWS - 1) / ROWS, (n + 2 * TPL - 1) / (2 * TPL)), dim3(32 * warps), warps * PER_WARP + TOTAL, stream, y,
               ldy, x, ldx, W, n, out, in, epilogue, act);
     return ti_check_launch("gemv_plain");
 }
 
-template <typename T, int TI, int TJ, int STAGES>
+template <typename T, int TI, int TJ, int STAGES, int PIECE>
 static int launch_tile(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
                        const XieluParams& act, cudaStream_t stream) {
     constexpr size_t SMEM = (size_t)STAGES * 16 * (TI + TJ) * GT_ROW + (size_t)TI * TJ * 256 * sizeof(float);
-    static const cudaError_t allowed = allow_smem(gemm_plain_tile_kernel<T, TI, TJ, STAGES>, SMEM);
+    static const cudaError_t allowed = allow_smem(gemm_plain_tile_kernel<T, TI, TJ, STAGES, PIECE>, SMEM);
     if (allowed != cudaSuccess) return ti_fail("gemm_plain: %s", cudaGetErrorString(allowed));
     const dim3 grid((out + 16 * TJ - 1) / (16 * TJ), (n + 16 * TI - 1) / (16 * TI));
     TI_REQUIRE(grid.y <= 65535, "gemm: too many rows (%d) for one launch", n);
-    ti_launch(gemm_plain_tile_kernel<T, TI, TJ, STAGES>, grid, dim3(256), SMEM, stream, y, ldy, x, ldx, W, n, out, in, epilogue, act);
+    ti_launch(gemm_plain_tile_kernel<T, TI, TJ, STAGES, PIECE>, grid, dim3(256), SMEM, stream, y, ldy, x, ldx, W, n, out, in, epilogue, act);
     return ti_check_launch("gemm_plain_tile");
 }
 
 // Tokens x features per thread of the tile kernel: the shape whose rounds of tiles over the SMs take the least time, by what a
 // round and a launch's first and last tile cost (in units of k, from sweeps of 64 to 2,048 tokens x 2,048 to 21,504 features at k =
 // 4,096: microseconds per round 447 / 235 / 132 / 92, and 0 / 15 / 23 / 22 once; 512 tokens x 4,096 features take 449 / 471 / 518 / 660
-// us, 128 x 4,096 take 448 / 255 / 155 / 260, 512 x 6,144 take 893 / 691 / 771 / 1,027). The sums do not depend on the shape.
+// us, 128 x 4,096 take 448 / 255 / 155 / 260, 512 x 6,144 take 893 / 691 / 771 / 1,027). It does not ask for k: over k = 512 to 21,504,
+// 70 to 1,024 tokens and 1,024 to 21,504 features the choice takes 1.3 % longer than the best shape on average (3.2 % at k = 512, 0.0 at
+// 21,504; 20 % at worst, 1,024 tokens x 21,504 x 512), with the second cost weighed by k 1.9 %. The sums do not depend on the shape.
 struct TileShape { int ti, tj; float round, once; };
 static const TileShape TILE_SHAPES[] = {{8, 8, 447.f, 0.f}, {8, 4, 235.f, 15.f}, {4, 4, 132.f, 23.f}, {2, 4, 92.f, 22.f}};
 
@@ -476,27 +430,42 @@ extern "C" int ti_gemm_plain_shape(int n, int out, int sms) {
 // L2): 64 tokens x 4,096 / 21,504 features of k = 4,096 take 74 / 355 us against 115 / 402 in tiles; at 100 tokens the two are level.
 #define GT_STREAM_TOKENS 64
 
-template <typename T>
-static int launch_vectors(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
+template <typename T, int PIECE>
+static int launch_product(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
                           const XieluParams& act, cudaStream_t stream) {
 #define GT_ARGS y, ldy, x, ldx, W, n, out, in, epilogue, act, stream
     if (n <= GT_STREAM_TOKENS) {
-        // 32 rows a block halve what is read of the tokens, where that leaves blocks for six tenths of the SMs (8 tokens: 4,096
-        // rows 17.8 us against 24.5 with 16 rows a block, 2,048 rows of k = 2,048 13.8 against 10.7). More blocks than SMs take two
-        // stages, so that two blocks fit an SM (6,144 rows: 26.9 us against 33.0); fewer take a deeper ring (4,096 rows x 21,504: 83 us against 98).
-        const int sms = ti_sm_count(), groups = (n + 31) / 32, blocks = (out + 31) / 32 * groups;
-        const bool tall = 5 * blocks >= 3 * sms, many = blocks > sms;
-        if (n <= 2) return !tall ? launch_stream<T, 1, 1, 6>(GT_ARGS) : many ? launch_stream<T, 1, 2, 2>(GT_ARGS) : launch_stream<T, 1, 2, 5>(GT_ARGS);
-        if (n <= 4) return !tall ? launch_stream<T, 2, 1, 5>(GT_ARGS) : many ? launch_stream<T, 2, 2, 2>(GT_ARGS) : launch_stream<T, 2, 2, 4>(GT_ARGS);
-        if (n <= 8) return !tall ? launch_stream<T, 4, 1, 5>(GT_ARGS) : many ? launch_stream<T, 4, 2, 2>(GT_ARGS) : launch_stream<T, 4, 2, 4>(GT_ARGS);
-        if (n <= 16) return tall ? launch_stream<T, 8, 2, 3>(GT_ARGS) : launch_stream<T, 8, 1, 4>(GT_ARGS);
-        return tall ? launch_stream<T, 16, 2, 2>(GT_ARGS) : launch_stream<T, 16, 1, 3>(GT_ARGS);
+        if constexpr (PIECE == 16) {
+            // 32 rows a block halve what is read of the tokens, where that leaves blocks for six tenths of the SMs (8 tokens: 4,096
+            // rows 17.8 us against 24.5 with 16 rows a block, 2,048 rows of k = 2,048 13.8 against 10.7). More blocks than SMs take two
+            // stages, so that two blocks fit an SM (6,144 rows: 26.9 us against 33.0); fewer take a deeper ring (4,096 rows x 21,504: 83 us against 98).
+            const int sms = ti_sm_count(), groups = (n + 31) / 32, blocks = (out + 31) / 32 * groups;
+            const bool tall = 5 * blocks >= 3 * sms, many = blocks > sms;
+            if (n <= 2) return !tall ? launch_stream<T, 1, 1, 6, 16>(GT_ARGS) : many ? launch_stream<T, 1, 2, 2, 16>(GT_ARGS) : launch_stream<T, 1, 2, 5, 16>(GT_ARGS);
+            if (n <= 4) return !tall ? launch_stream<T, 2, 1, 5, 16>(GT_ARGS) : many ? launch_stream<T, 2, 2, 2, 16>(GT_ARGS) : launch_stream<T, 2, 2, 4, 16>(GT_ARGS);
+            if (n <= 8) return !tall ? launch_stream<T, 4, 1, 5, 16>(GT_ARGS) : many ? launch_stream<T, 4, 2, 2, 16>(GT_ARGS) : launch_stream<T, 4, 2, 4, 16>(GT_ARGS);
+            if (n <= 16) return tall ? launch_stream<T, 8, 2, 3, 16>(GT_ARGS) : launch_stream<T, 8, 1, 4, 16>(GT_ARGS);
+            return tall ? launch_stream<T, 16, 2, 2, 16>(GT_ARGS) : launch_stream<T, 16, 1, 3, 16>(GT_ARGS);
+        } else {
+            // Other rows, one set of blocks (microseconds; in brackets with blocks of 16 rows or tiles of 64 x 64 that staged element by element, 8-byte
+            // loads and tiles of 128 x 128 for bfloat16 rows of 4 modulo 8): bfloat16, 8 tokens x 4,096 x 4,100 35 (195), 512 tokens 536 (763);
+            // x 4,099 58 (199), 512 tokens 651 (865), 700 tokens 844 (879); 32-bit x 4,099, 8 tokens 48 (253), 512 tokens 510 (859).
+            if (n <= 2) return launch_stream<T, 1, 1, 4, PIECE>(GT_ARGS);
+            if (n <= 8) return launch_stream<T, 4, 1, 4, PIECE>(GT_ARGS);
+            if (n <= 16) return launch_stream<T, 8, 1, 4, PIECE>(GT_ARGS);
+            return launch_stream<T, 16, 2, 2, PIECE>(GT_ARGS);
+        }
     }
-    switch (ti_gemm_plain_shape(n, out, ti_sm_count())) {
-        case 0: return launch_tile<T, 8, 8, 2>(GT_ARGS);
-        case 1: return launch_tile<T, 8, 4, 2>(GT_ARGS);
-        case 2: return launch_tile<T, 4, 4, 3>(GT_ARGS);
-        default: return launch_tile<T, 2, 4, 4>(GT_ARGS);
+    const int shape = ti_gemm_plain_shape(n, out, ti_sm_count());
+    if constexpr (PIECE == 2) {                            // (8 x 8 outputs take longer at every size)
+        if (shape <= 1) return launch_tile<T, 8, 4, 2, 2>(GT_ARGS);
+        if (shape == 2) return launch_tile<T, 4, 4, 2, 2>(GT_ARGS);
+        return launch_tile<T, 2, 4, 2, 2>(GT_ARGS);
+    } else {
+        if (shape == 0) return launch_tile<T, 8, 8, 2, PIECE>(GT_ARGS);
+        if (shape == 1) return launch_tile<T, 8, 4, 2, PIECE>(GT_ARGS);
+        if (shape == 2) return launch_tile<T, 4, 4, 3, PIECE>(GT_ARGS);
+        return launch_tile<T, 2, 4, 4, PIECE>(GT_ARGS);
     }
 #undef GT_ARGS
 }
@@ -508,26 +477,12 @@ extern "C" int ti_gemm_plain(void* y, long long ldy, const void* x, long long ld
     TI_REQUIRE(n > 0 && out > 0 && in > 0, "gemm: bad sizes n=%d out=%d in=%d", n, out, in);
     TI_REQUIRE((epilogue >= 0 && epilogue <= 2) || (epilogue >= TI_EPI_GELU_ERF && epilogue <= TI_EPI_LAST), "gemm: unknown epilogue %d", epilogue);
     XieluParams act{alpha_p, alpha_n, beta, eps};
-    const int vec = dtype == TI_F32 ? 4 : 8;               // elements of a 16-byte piece
-    if (in % vec == 0 && ldx % vec == 0 && aligned16(x) && aligned16(W)) {
-        TI_DISPATCH_DTYPE(dtype, return launch_vectors<T>(y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act, stream));
-    }
-    if (n <= GV_MAX_TOKENS) {                              // few tokens: the weight-streaming form (same sums, bit for bit)
-        const size_t smem = (size_t)n * (GV_BK + 1) * sizeof(float);
-        const dim3 blocks((out + GV_ROWS - 1) / GV_ROWS), threads(GV_ROWS * GV_SLOTS);
-#define GV_LAUNCH(TPT) ti_launch(gemv_plain_kernel<T, TPT>, blocks, threads, smem, stream, y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act)
-        TI_DISPATCH_DTYPE(dtype, {
-            if (n <= GV_SLOTS) GV_LAUNCH(1);
-            else if (n <= 2 * GV_SLOTS) GV_LAUNCH(2);
-            else if (n <= 4 * GV_SLOTS) GV_LAUNCH(4);
-            else GV_LAUNCH(8);
-        });
-#undef GV_LAUNCH
-        return ti_check_launch("gemv_plain");
-    }
-    const dim3 grid((out + GP_BN - 1) / GP_BN, (n + GP_BM - 1) / GP_BM);
-    TI_REQUIRE(grid.y <= 65535, "gemm: too many rows (%d) for one launch", n);
-    TI_DISPATCH_DTYPE(dtype, (ti_launch(gemm_plain_kernel<T>, grid, dim3(256), 0, stream, y, ldy, (const T*)x, ldx, (const T*)W, n, out, in,
-                                                                          epilogue, act)));
-    return ti_check_launch("gemm_plain");
+    // The widest piece on whose boundaries all rows of both operands start.
+    const unsigned long long size = dtype == TI_F32 ? 4 : 2;
+    const unsigned long long off = (unsigned long long)in * size | (unsigned long long)ldx * size | (uintptr_t)x | (uintptr_t)W;
+#define GP_PRODUCT(T, PIECE) launch_product<T, PIECE>(y, ldy, (const T*)x, ldx, (const T*)W, n, out, in, epilogue, act, stream)
+    if (dtype == TI_F32) return off % 16 == 0 ? GP_PRODUCT(float, 16) : GP_PRODUCT(float, 4);
+    if (dtype == TI_BF16) return off % 16 == 0 ? GP_PRODUCT(bf16, 16) : off % 4 == 0 ? GP_PRODUCT(bf16, 4) : GP_PRODUCT(bf16, 2);
+#undef GP_PRODUCT
+    return ti_fail("unknown element type code %d", dtype);
 }
