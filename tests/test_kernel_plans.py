@@ -80,3 +80,16 @@ def test_the_attention_plan_in_the_step_planner_uses_the_same_split_policy():
         plan = fast.SplitKvPlan(kv_heads, page, pool)
         for batch in (1, 2, 3, 7, 8, 9, 18, 19, 37, 64, 100, 300):
             assert plan.splits(batch) == fast.decode_splits(batch, kv_heads, pool), (kv_heads, pool, batch)
+
+
+def test_linear_attention_in_chunks_only_where_they_pay():
+    """Sizes measured on both sides (148 SMs): long prompts go in chunks; short portions, many short prompts and a short prompt beside many
+    one-token sequences, where the chunks took up to ten times as long, walk token by token."""
+    from tileinfer_b200.kernels import ops
+    pay = lambda q_lens, H, D, V: ops.lightning_chunks_pay(q_lens, H, D, V, 148)
+    for H, D, V in ((16, 128, 128), (32, 128, 128), (8, 64, 64), (32, 64, 64), (4, 32, 32), (2, 256, 256), (16, 64, 128), (8, 128, 256)):
+        assert pay([2048], H, D, V) and pay([1000], H, D, V)
+        for q_lens in ([96], [192], [96] * 2, [96] * 8, [96] * 32, [100] + [1] * 7, [100] + [1] * 63, [100] + [1] * 199):
+            assert not pay(q_lens, H, D, V), (q_lens, H, D, V)
+    assert pay([500], 16, 128, 128) and pay([256] * 8, 16, 128, 128) and pay([500] * 2, 32, 128, 128)
+    assert not pay([100] * 64, 16, 128, 128) and not pay([300], 16, 128, 128) and not pay([500] * 2, 32, 64, 64)

@@ -862,6 +862,22 @@ def memory_chunk_sizes(q_lens, heads, dim, vdim):
     return chunks, chunks * heads * int(lib().ti_memory_chunk_pitch(dim, vdim))
 
 
+def lightning_chunks_pay(q_lens, heads, dim, vdim, sms) -> bool:
+    """Whether linear attention takes less time in chunks than token by token. The walk is bound by its longest sequence's chain, or by
+    (tokens x blocks of 32 value columns) once the SMs are full; the chunks by rounds of two blocks per SM, whatever part of
+    a chunk is there, by what does not fit L2 (work space and states), and by a little per sequence. Fitted to 1 to 200 sequences of 1 to 2,048
+    tokens at 2 to 32 heads of 32 x 32 to 256 x 256: 1 % longer than the better one on average, 27 % at worst (where the walk was kept: 32
+    sequences of 96 tokens at 256 x 256, 247 us against 194). 16 heads of 128 x 128, microseconds walked / in chunks: one sequence of 96
+    tokens 22 / 73, of 300 62 / 75, of 500 99 / 81, of 2,048 387 / 170; 64 sequences of 100 tokens 668 / 858; one of 100 beside 63 single
+    tokens 70 / 528."""
+    chunks = sum(-(-n // CHUNK_TOKENS) for n in q_lens)
+    slabs = -(-dim // 128)
+    walk = 3 + max((0.13 + 0.0007 * dim) * max(q_lens), 1.25e-5 * dim * sum(q_lens) * heads * -(-vdim // 32) * 148 / sms)
+    rounds = -(-chunks * heads * slabs * -(-vdim // 128) // (2 * sms))
+    megabytes = (chunks + len(q_lens)) * heads * dim * vdim * 4e-6
+    return rounds * (30 + 0.42 * min(dim, 128) + 40 * (slabs - 1)) + 2.5 * max(0.0, megabytes - 70) + 1.2 * len(q_lens) < walk
+
+
 def memory_chunks(rows, offs, state, step, heads, dim, vdim, ws, total, chunks, y=None, o=None, nq=None, em=None, decay=None, coef=None, rotation=None,
                   q_scale=1.0, k_scale=1.0, w=None, gate_sigmoid=False, eps=1e-6):
     """A step's tokens of retention (``decay``) or of the gated cell (``coef``, ``em`` of ``memory_gates``) in chunks: ``y`` the normed and

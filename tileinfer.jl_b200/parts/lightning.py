@@ -9,7 +9,7 @@ Per token, from the mixer's input h:
 
 The only thing a sequence keeps is S: a fixed-size state per layer (the cache's "state" kind), however long the sequence is.
 The four projections read the same input and run as one product; the recurrence (``csrc/lightning.cu``) reads its rows, applies
-the activation, and serves prompts and one-token steps alike. State, decay, o and the norm are 32-bit in every element type.
+the activation, and serves prompts and one-token steps alike, long prompts in chunks worked on side by side. State, decay, o and the norm are 32-bit in every element type.
 
 Record: ``num_heads``, ``head_dim`` (query/key size) and the options ``value_dim``, ``decay`` (one number per head), ``norm_eps``,
 ``gate`` (default True), ``activation`` ("silu" or "none").
@@ -19,10 +19,9 @@ from __future__ import annotations
 import torch
 
 from ..config.spec import MixerSpec, TensorDecl
-from ..kernels import ops
+from ..kernels import fast, ops
 from .base import CacheRequest, Mixer, register_mixer
 from .linear import Linear
-from .matrix_memory import CHUNKED_FROM
 
 
 @register_mixer("lightning")
@@ -74,7 +73,7 @@ class LightningAttention(Mixer):
         self.proj.forward(h, rows)
         o = rt.buffer("lightning.o", (n, H * V), torch.float32)
         chunked = None
-        if self.chunks and step.max_q_len >= CHUNKED_FROM:
+        if self.chunks and not step.is_decode and ops.lightning_chunks_pay(step.host_q_lens, H, D, V, fast.sm_count()):
             chunks, floats = ops.memory_chunk_sizes(step.host_q_lens, H, D, V)
             chunked = (chunks, rt.buffer("memory.chunks", (floats,), torch.float32), rt.buffer("memory.totals", (chunks, H), torch.float32))
         ops.lightning_scan(o, rows, 0, H * D, 2 * H * D, cache.state, self.decay, step.cu_seqlens, step.seq_slots, step.n_seqs, H, D, V,
