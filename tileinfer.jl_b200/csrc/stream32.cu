@@ -380,8 +380,11 @@ __global__ void branch_norm_add32_vec_kernel(float* x, const bf16* delta, const 
 
 // The same with a row in registers: a thread owns NQ quads, and everything it needs (branch, stream, and ahead of the wait for the kernel
 // before the weights and the bias) is asked for before the first sum. A decode step of 8 rows of 2,048: 4.5 -> 3.1 us.
-template <int NQ>
-__global__ void __launch_bounds__(512, NQ == 1 ? 2 : 1) branch_norm_add32_quads_kernel(float* x, const bf16* delta, const float* partials, int n_partials,
+// LATE: weights, bias and the stream are read where they are used, which leaves registers for more blocks per SM: steps of many rows are bound by memory
+// (2,048 rows of 2,048 / 2,880 / 4,096: 11.1 / 12.9 / 17.1 us, without it 15.3 / 32.3 / 34.4, rows staged in shared memory 11.9 / 14.9 /
+// 19.0). The same sums either way.
+template <int NQ, bool LATE>
+__global__ void __launch_bounds__(512, LATE ? 4 : NQ == 1 ? 2 : 1) branch_norm_add32_quads_kernel(float* x, const bf16* delta, const float* partials, int n_partials,
                                                                                        size_t partial_stride, const int* gather, int per_row,
                                                                                        const bf16* __restrict__ dbias, const bf16* __restrict__ w, int offset,
                                                                                        float eps, float mult, bf16* __restrict__ h,
@@ -398,6 +401,7 @@ __global__ void __launch_bounds__(512, NQ == 1 ? 2 : 1) branch_norm_add32_quads_
     for (int k = 0; k < NQ; ++k) {
         at[k] = (tid + k * threads) * 4;
         in[k] = at[k] < size;
+        if (LATE) continue;
         g[k] = in[k] ? load_weight4(w + at[k]) : zero;
         go[k] = in[k] && w_out != nullptr ? load_weight4(w_out + at[k]) : zero;
         db[k] = in[k] && dbias != nullptr ? load_weight4(dbias + at[k]) : zero;
@@ -407,7 +411,7 @@ __global__ void __launch_bounds__(512, NQ == 1 ? 2 : 1) branch_norm_add32_quads_
     float d[NQ][4], ss = 0.f, sum = 0.f;
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-        xv[k] = in[k] ? load_row4(row + at[k]) : zero;
+        if (!LATE) xv[k] = in[k] ? load_row4(row + at[k]) : zero;
         float4 v = zero;
         if (in[k]) {
             if (partials != nullptr) {
@@ -425,6 +429,7 @@ __global__ void __launch_bounds__(512, NQ == 1 ? 2 : 1) branch_norm_add32_quads_
             } else {
                 v = load_row4(delta + t * size + at[k]);
             }
+            if (LATE && dbias != nullptr) db[k] = load_weight4(dbias + at[k]);
             if (dbias != nullptr) { v.x += db[k].x; v.y += db[k].y; v.z += db[k].z; v.w += db[k].w; }
         }
         d[k][0] = v.x; d[k][1] = v.y; d[k][2] = v.z; d[k][3] = v.w;
@@ -449,6 +454,7 @@ __global__ void __launch_bounds__(512, NQ == 1 ? 2 : 1) branch_norm_add32_quads_
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
         if (!in[k]) continue;
+        if (LATE) { g[k] = load_weight4(w + at[k]); xv[k] = load_row4(row + at[k]); }
         const float xs[4] = {xv[k].x, xv[k].y, xv[k].z, xv[k].w}, gs[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -475,6 +481,7 @@ __global__ void __launch_bounds__(512, NQ == 1 ? 2 : 1) branch_norm_add32_quads_
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
         if (!in[k]) continue;
+        if (LATE && w_out != nullptr) go[k] = load_weight4(w_out + at[k]);
         const float gs[4] = {go[k].x, go[k].y, go[k].z, go[k].w};
         if (w_out != nullptr)
 #pragma unroll
@@ -505,7 +512,9 @@ extern "C" int ti_branch_norm_add32(float* x, const void* delta, const float* pa
                          (((uintptr_t)delta | (uintptr_t)dbias | (uintptr_t)w | (uintptr_t)h | (uintptr_t)w_out) & 7) == 0;
         if (vec && size <= 4096) {
             const int quads = size / 4, per = quads > 512 ? 2 : 1, qt = ((quads + per - 1) / per + 31) / 32 * 32;
-            ti_launch(per == 1 ? branch_norm_add32_quads_kernel<1> : branch_norm_add32_quads_kernel<2>, dim3(n_rows), dim3(qt), 0, stream, x,
+            const bool late = n_rows > 2 * ti_sm_count();
+            ti_launch(per == 1 ? (late ? branch_norm_add32_quads_kernel<1, true> : branch_norm_add32_quads_kernel<1, false>)
+                               : (late ? branch_norm_add32_quads_kernel<2, true> : branch_norm_add32_quads_kernel<2, false>), dim3(n_rows), dim3(qt), 0, stream, x,
                       (const bf16*)delta, partials, n_partials, (size_t)partial_stride, gather, per_row, (const bf16*)dbias, (const bf16*)w, offset, eps,
                       mult, (bf16*)h, (const bf16*)w_out, offset_out, eps_out, size);
         } else if (vec) {
