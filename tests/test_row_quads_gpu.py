@@ -44,3 +44,56 @@ def test_branch_norm(size, form, centred):
     assert bool(((h.to(F64) - want).abs() <= want.abs() * 2.0 ** -8 + (1e-5 if size > 4 else 1e-3)).all())
     few = run(5)
     assert torch.equal(few[0], x[:5]) and torch.equal(few[1], h[:5])
+
+
+# 24 + 40: one quad a thread; 336, 512 quads: two; 513, and ranks that are no whole quads: the general kernel.
+@pytest.mark.parametrize("q_rank,kv_rank,rot,spare", [(24, 40, 0, 0), (24, 40, 8, 4), (768, 512, 64, 0), (0, 512, 64, 8), (1536, 512, 0, 0), (1532, 448, 68, 0),
+                                                      (1536, 452, 64, 0), (1022, 130, 0, 0), (4, 4, 4, 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("form", ["rows", "partials"])
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_latent_inputs(q_rank, kv_rank, rot, spare, dtype, form, interleaved):
+    """A row's quads in registers and the general kernel (also the same numbers in rows off 4 elements), latents and the rotated key part."""
+    from tileinfer_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(q_rank + kv_rank + rot)
+    n, size, pool_row = 5, q_rank + kv_rank + rot, kv_rank + rot + spare
+    rows = torch.randn(n, size, generator=g, device="cuda").to(dtype) if form == "rows" else torch.randn(3, n, size, generator=g, device="cuda")
+    raw = rows.to(F64) if form == "rows" else rows.to(F64).sum(0)
+    mass = raw.abs() if form == "rows" else rows.to(F64).abs().sum(0)
+    wq, wkv = (torch.randn(r, generator=g, device="cuda").to(dtype) if r else None for r in (q_rank, kv_rank))
+    slots = torch.tensor([6, 0, 3, 8, 1], dtype=torch.int32, device="cuda")
+    positions = torch.tensor([2, 0, 7, 1, 5], dtype=torch.int32, device="cuda")
+    angles = torch.rand(8, max(rot // 2, 1), generator=g, device="cuda") * 6
+    table = torch.stack([angles.cos(), angles.sin()], -1).contiguous()
+    rotation = SimpleNamespace(rotary_dim=rot, cos_sin=table, interleaved=interleaved) if rot else None
+    off = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+
+    def check(given):
+        cq = torch.full((n, q_rank), 7.0, dtype=dtype, device="cuda") if q_rank else None
+        pool = torch.full((9, pool_row), 7.0, dtype=dtype, device="cuda")
+        ops.latent_inputs(given, cq, pool, wq, wkv, 1e-6, slots, q_rank, kv_rank, rotation=rotation, positions=positions if rot else None, pool_row=pool_row)
+        parts = [(pool[slots.long(), :kv_rank], slice(q_rank, q_rank + kv_rank), wkv)]
+        if q_rank:
+            parts.append((cq, slice(0, q_rank), wq))
+        for got, where, w in parts:
+            want = _rms(raw[:, where], w, 1e-6)
+            # An element's own sum of three terms off by two roundings of its terms; the root and the product by a few of the result.
+            bound = want.abs() * (off + 16 * 2.0 ** -24) + mass[:, where] / raw[:, where].pow(2).mean(-1, keepdim=True).sqrt() * w.to(F64).abs() * 2.0 ** -22
+            assert bool(((got.to(F64) - want).abs() <= bound).all())
+        if rot:
+            key, m, cs = raw[:, q_rank + kv_rank:], mass[:, q_rank + kv_rank:], table[positions.long()].to(F64)
+            first, second = (slice(0, rot, 2), slice(1, rot, 2)) if interleaved else (slice(0, rot // 2), slice(rot // 2, rot))
+            want, bound = torch.empty_like(key), torch.empty_like(key)
+            want[:, first] = key[:, first] * cs[..., 0] - key[:, second] * cs[..., 1]
+            want[:, second] = key[:, second] * cs[..., 0] + key[:, first] * cs[..., 1]
+            bound[:, first] = bound[:, second] = (m[:, first] + m[:, second]) * 2.0 ** -22
+            got = pool[slots.long(), kv_rank:kv_rank + rot].to(F64)
+            assert bool(((got - want).abs() <= bound + want.abs() * off).all())
+        assert bool((pool[slots.long(), kv_rank + rot:] == 0).all())
+        assert bool((pool[[2, 4, 5, 7]] == 7.0).all())
+
+    check(rows)
+    if form == "rows":                                   # rows a whole number of elements apart, but not of quads
+        wide = torch.zeros(n, size + 3, dtype=dtype, device="cuda")
+        wide[:, :size] = rows
+        check(wide[:, :size])

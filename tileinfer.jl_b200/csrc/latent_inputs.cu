@@ -64,7 +64,8 @@ __global__ void latent_inputs_kernel(const T* rows, size_t row_stride, const flo
 }
 
 // The same for ranks of whole quads: a thread owns up to LQ_PER quads of the row, kept in registers; the two sums meet in one reduction
-// and the weights are there before the kernel ahead has finished. A decode step of 8 rows of 768 + 128: 6.9 -> 2.3 us.
+// and the weights are there before the kernel ahead has finished. A decode step of 8 rows of 768 + 128: 6.9 -> 2.3 us. With two quads a thread the
+// block is as small as they allow: 8,192 rows of 768 + 256 + 32 take 19.8 us, in blocks of 256, where few threads have a second quad, 30.8.
 #define LQ_THREADS 256
 #define LQ_PER 2                                   // rows of up to 2,048 elements
 template <typename T>
@@ -177,7 +178,7 @@ extern "C" int ti_latent_inputs(const void* rows, long long row_stride, const fl
     const int quads = (q_rank + kv_rank + rot) / 4;
     if (q_rank % 4 == 0 && kv_rank % 4 == 0 && rot % 4 == 0 && pool_row % 4 == 0 && quads <= LQ_PER * LQ_THREADS && row_stride % 4 == 0 && in_row % 4 == 0 &&
         partial_stride % 4 == 0 && aligned16(rows) && aligned16(partials) && aligned16(cq) && aligned16(pool) && aligned16(wq) && aligned16(wkv)) {
-        const int threads = quads < LQ_THREADS ? (quads + 31) / 32 * 32 : LQ_THREADS;
+        const int per = quads > LQ_THREADS ? LQ_PER : 1, threads = ((quads + per - 1) / per + 31) / 32 * 32;
         TI_DISPATCH_DTYPE(dtype, (ti_launch(latent_inputs_quads_kernel<T>, dim3(n_tokens), dim3(threads), (size_t)rot * sizeof(float), stream, (const T*)rows,
                                             (size_t)row_stride, partials, n_partials, (size_t)partial_stride, (T*)cq, (T*)pool, (const T*)wq,
                                             (const T*)wkv, eps, slots, q_rank, kv_rank, rot, cos_sin, interleaved, positions, pool_row, (size_t)in_row)));
