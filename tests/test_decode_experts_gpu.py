@@ -58,3 +58,21 @@ def test_units_streamed_by_pair(units, out, k, tokens, per_token, gated):
             want = down[e].to(F64) @ y[p].cpu().to(F64)
             bound = out / 2 * 2.0 ** -24 * (down[e].to(F64).abs() @ y[p].cpu().to(F64).abs()) + want.abs() * 2.0 ** -8
             assert bool(((y2[p].cpu().to(F64) - want).abs() <= bound + 1e-7).all())
+
+
+@pytest.mark.parametrize("heads,out,k", [(3, 40, 8), (16, 128, 64), (5, 24, 264), (2, 136, 2056), (64, 520, 128), (130, 264, 128)])
+@pytest.mark.parametrize("n", [1, 8, 9, 16, 17])
+def test_product_with_a_matrix_per_head(heads, out, k, n):
+    """Streamed by head up to 16 tokens (a second pass over the matrices from 9 on), in tiles from 17 on and where the blocks would be too many;
+    outputs that are no whole tiles."""
+    from tileinfer_b200.kernels import fast
+    g = torch.Generator(device="cuda").manual_seed(heads * 100 + n)
+    x = torch.randn(n, heads, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(heads, out, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    y = torch.full((n + 1, heads, out), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert fast.head_linear(y[:n], x, w)
+    fast.check_status()
+    want, mass = (torch.einsum("hok,nhk->nho", a, b) for a, b in ((w.to(F64), x.to(F64)), (w.to(F64).abs(), x.to(F64).abs())))
+    # 32-bit sums of k products in any order, then one rounding to bfloat16.
+    assert bool(((y[:n].to(F64) - want).abs() <= k / 2 * 2.0 ** -24 * mass + want.abs() * 2.0 ** -8 + 1e-7).all())
+    assert bool((y[n] == 7.0).all())

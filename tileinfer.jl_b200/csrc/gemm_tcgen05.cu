@@ -731,8 +731,11 @@ extern "C" int ti_gemm_tcgen05_heads(void* y, const void* x, const void* W, int 
     }
     TI_REQUIRE(status != nullptr, "gemm_tcgen05_heads: status word missing");
     // A step of few tokens: a small product per head, where tiles, barriers and tensor memory cost more than
-    // the product (8 tokens x 16 heads of 128 x 64 inside a step: about 8 us in tiles, 4.6 streamed).
-    if (n <= HEADS_STREAM_TOKENS) {
+    // the product (8 tokens x 16 heads of 128 x 64 inside a step: about 8 us in tiles, 4.6 streamed). Streamed, a block is 32 rows of a
+    // head for up to 8 tokens, and 1,024 of them take what the tiles take (6.6 us; heads of 512 x 128: 64 heads, 8 tokens 6.6 against 6.6, 16 tokens
+    // 10.9 against 6.7; 128 heads, 8 tokens 12.1 against 8.8).
+    const long long passes = (long long)heads * ((out_h + 31) / 32) * ((n + 7) / 8);
+    if (n <= HEADS_STREAM_TOKENS && passes <= 7LL * sm_count_cached()) {
         ExpertStream e = {};
         e.pairs = n * heads;
         e.per_row = 1;
