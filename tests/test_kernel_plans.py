@@ -93,3 +93,18 @@ def test_linear_attention_in_chunks_only_where_they_pay():
             assert not pay(q_lens, H, D, V), (q_lens, H, D, V)
     assert pay([500], 16, 128, 128) and pay([256] * 8, 16, 128, 128) and pay([500] * 2, 32, 128, 128)
     assert not pay([100] * 64, 16, 128, 128) and not pay([300], 16, 128, 128) and not pay([500] * 2, 32, 64, 64)
+
+
+def test_many_units_in_use_are_not_streamed():
+    """Streamed up to 16 tokens, but not where more than 64 units are in use whose matrices are not small: the grouped products took less time."""
+    import torch
+    from tileinfer_b200.kernels import fast
+
+    def streams(tokens, units, per_token, width, inner):
+        meta = dict(dtype=torch.bfloat16, device="meta")
+        return fast.streams_experts(torch.empty(tokens, width, **meta), torch.empty(units, 2 * inner, width, **meta), torch.empty(units, width, inner, **meta),
+                                    per_token)
+    assert streams(8, 256, 8, 2048, 256) and not streams(10, 256, 8, 2048, 256) and not streams(16, 256, 8, 2048, 256)
+    assert streams(10, 128, 8, 2048, 768) and not streams(12, 128, 8, 2048, 768)
+    assert streams(16, 34, 6, 2048, 1024) and streams(16, 64, 6, 4096, 1408) and streams(16, 64, 8, 2048, 512) and not streams(17, 64, 6, 4096, 1408)
+    assert streams(16, 128, 8, 512, 128) and streams(16, 1, 1, 64, 64)

@@ -229,13 +229,22 @@ def grouped_linear(y, x, w, plan, tile) -> bool:
 # with two shared, 8 tokens 62 against 85 us, 16 tokens 89 against 91, 24 tokens 111 against 97; plain units, 16 tokens 50 against 62;
 # 64 units of 1,408 x 4,096, 4 tokens 141 against 157, 16 tokens 357 against 363, 24 tokens 421 against 397.
 EXPERT_STREAM_TOKENS = 16
+# More units in use than this (as many as pairs drawn at random reach) take longer streamed, unless their matrices are small: 256 units of 2,048
+# x 256, 8 a token, 8 / 10 / 16 tokens 64 / 82 / 129 us against 67 / 75 / 100; 128 units of 2,048 x 768 10 / 12 / 16 tokens 130 / 151 / 192
+# against 137 / 146 / 179; 64 units of 2,048 x 512 16 tokens 95 against 96; 128 plain units of 512 x 128 16 tokens 24 against 31.
+EXPERT_STREAM_UNITS = 64
+EXPERT_STREAM_BYTES = 64 << 20
 
 
-def streams_experts(h, gate_up, down) -> bool:
+def streams_experts(h, gate_up, down, per_token) -> bool:
     """Whether a step with the inputs ``h`` [n, width] takes ``grouped_stream`` for its units (gate_up [units, rows, width], down
-    [units, width, inner]): 16-byte vectors along both products' k."""
-    return (h.dtype == torch.bfloat16 and 0 < h.shape[0] <= EXPERT_STREAM_TOKENS and h.is_contiguous() and gate_up.shape[2] % 8 == 0 and
-            down.shape[2] % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (h, gate_up, down)) and gate_up.shape[0] <= 65535)
+    [units, width, inner], ``per_token`` of them a token): 16-byte vectors along both products' k."""
+    units, pairs = gate_up.shape[0], h.shape[0] * per_token
+    if not (h.dtype == torch.bfloat16 and 0 < h.shape[0] <= EXPERT_STREAM_TOKENS and h.is_contiguous() and gate_up.shape[2] % 8 == 0 and
+            down.shape[2] % 8 == 0 and all(t.data_ptr() % 16 == 0 for t in (h, gate_up, down)) and units <= 65535):
+        return False
+    used = units * (1.0 - (1.0 - 1.0 / units) ** pairs)
+    return used <= EXPERT_STREAM_UNITS or 2 * (gate_up.numel() + down.numel()) // units * min(pairs, units) <= EXPERT_STREAM_BYTES
 
 
 class _ExpertStream(ctypes.Structure):

@@ -161,7 +161,7 @@ class RoutedExperts(FeedForward):
                               always=self.always, gate=self.gate_on, logit_bias=self.logit_bias, on_logits=self.on_logits)
         else:
             ops.router_topk(h, self.router, top, ids, scores, logits, always=self.always)
-        if fast is not None and fast.streams_experts(h, self.gate_up, self.down):
+        if fast is not None and fast.streams_experts(h, self.gate_up, self.down, per_token):
             act, ys = rt.buffer("experts.act", (pairs, F)), rt.buffer("experts.out_rows", (pairs, W))
             fast.grouped_stream(act, h, self.gate_up, ids, scores if self.scale_input else None, pair_row, per_token, gated=self.gated,
                                 relu2=not self.gated, limits=self.limits, slope=self.slope, shift=self.shift)
