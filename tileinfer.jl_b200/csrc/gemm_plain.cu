@@ -16,6 +16,7 @@
 // AntoineBut/TileInfer.jl: weights stay [out, in] row-major, y = Wᵀx with 32-bit
 // accumulation and one rounding (src/ops/reference.jl:23-26, src/ops/tile/linear.jl:12-13);
 // the logits leave in 32-bit after that rounding (src/ops/tile/linear.jl:26).
+#include <type_traits>
 #include "common.cuh"
 #include "mma_util.cuh"
 #include "packed_f32.cuh"
@@ -255,6 +256,10 @@ __global__ void __launch_bounds__(256) gemv_plain_stream_kernel(void* __restrict
 // us, 40 TFLOP/s; tiles staged with k outermost, 8 x 8 outputs a thread and single multiply-adds took 4,500.
 // (Single elements are not on their way while a k block is worked on, so two or three blocks share an SM; a lower bound of one block for
 // the others makes the compiler spend more registers: 512 tokens of the 32-bit model at 8B sizes 0.4 % longer.)
+// bfloat16 in the largest tiles is widened once, into floats in shared memory, instead of by each of the 16 threads that read a row: 512 /
+// 1,000 tokens x 21,504 x 4,096 2,288 / 4,578 us (2,574 / 5,156 without). Smaller tiles would lose the blocks that share an SM to the floats' room.
+template <typename T, int TI, int TJ, int PIECE> struct Widens { static constexpr bool value = sizeof(typename Staged<T, PIECE>::type) == 2 && TI * TJ >= 64; };
+#define GT_WIDE_ROW (2 * GT_BYTES + 16)
 template <typename T, int TI, int TJ, int STAGES, int PIECE>
 __global__ void __launch_bounds__(256, PIECE == 2 ? (TI * TJ <= 16 ? 3 : 2) : 0) gemm_plain_tile_kernel(void* __restrict__ y, long long ldy, const T* x, long long ldx,
                                                              const T* __restrict__ W, int n, int out, int in, int epilogue,
@@ -262,6 +267,8 @@ __global__ void __launch_bounds__(256, PIECE == 2 ? (TI * TJ <= 16 ? 3 : 2) : 0)
     extern __shared__ __align__(16) unsigned char gt_smem[];
     constexpr int TM = 16 * TI, TN = 16 * TJ;
     typedef typename Staged<T, PIECE>::type E;
+    constexpr bool WIDE = Widens<T, TI, TJ, PIECE>::value;
+    typedef std::conditional_t<WIDE, float, E> F;           // what the products are taken of
     constexpr int IN_ROW = Staged<T, PIECE>::BYTES, PER_ROW = GT_BYTES / IN_ROW, VEC = PIECE / (int)sizeof(T);
     constexpr int BK = GT_BYTES / (int)sizeof(E), PER_SEG = GP_SEGMENT / BK;
     constexpr int STAGE = (TM + TN) * GT_ROW, STEP = 256 / PER_ROW;            // staging: STEP rows at a time
@@ -329,17 +336,30 @@ __global__ void __launch_bounds__(256, PIECE == 2 ? (TI * TJ <= 16 ? 3 : 2) : 0)
         __syncthreads();                                    // this k block has landed, and the stage refilled below is no longer read
         issue(b + STAGES - 1, true, true);
         cp_async_commit();
-        const unsigned char* as = gt_smem + (b % STAGES) * STAGE + ty * GT_ROW;
-        const unsigned char* bs = gt_smem + (b % STAGES) * STAGE + (TM + tx) * GT_ROW;
+        const unsigned char* from = gt_smem + (b % STAGES) * STAGE;
+        if constexpr (WIDE) {
+            unsigned char* wide = gt_smem + STAGES * STAGE + TI * TJ * 256 * sizeof(float);
+#pragma unroll
+            for (int i = 0; i < (TM + TN) / 16; ++i) {
+                const int r = (tid >> 4) + 16 * i, c = tid & 15;
+                const uint2 t = *reinterpret_cast<const uint2*>(from + r * GT_ROW + c * 8);
+                *reinterpret_cast<uint4*>(wide + r * GT_WIDE_ROW + c * 16) = make_uint4(t.x << 16, t.x & 0xffff0000u, t.y << 16, t.y & 0xffff0000u);
+            }
+            __syncthreads();
+            from = wide;
+        }
+        constexpr int ROW = WIDE ? GT_WIDE_ROW : GT_ROW;
+        const unsigned char* as = from + ty * ROW;
+        const unsigned char* bs = from + (TM + tx) * ROW;
 #pragma unroll
         for (int c = 0; c < BK / 4; ++c) {
-            Quad<E> w[TJ];
+            Quad<F> w[TJ];
 #pragma unroll
-            for (int j = 0; j < TJ; ++j) w[j].load(bs + j * 16 * GT_ROW + c * Quad<E>::BYTES);
+            for (int j = 0; j < TJ; ++j) w[j].load(bs + j * 16 * ROW + c * Quad<F>::BYTES);
 #pragma unroll
             for (int i = 0; i < TI; ++i) {
-                Quad<E> v;
-                v.load(as + i * 16 * GT_ROW + c * Quad<E>::BYTES);
+                Quad<F> v;
+                v.load(as + i * 16 * ROW + c * Quad<F>::BYTES);
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -396,7 +416,8 @@ static int launch_stream(void* y, long long ldy, const T* x, long long ldx, cons
 template <typename T, int TI, int TJ, int STAGES, int PIECE>
 static int launch_tile(void* y, long long ldy, const T* x, long long ldx, const T* W, int n, int out, int in, int epilogue,
                        const XieluParams& act, cudaStream_t stream) {
-    constexpr size_t SMEM = (size_t)STAGES * 16 * (TI + TJ) * GT_ROW + (size_t)TI * TJ * 256 * sizeof(float);
+    constexpr size_t SMEM = (size_t)STAGES * 16 * (TI + TJ) * GT_ROW + (size_t)TI * TJ * 256 * sizeof(float) +
+                            (Widens<T, TI, TJ, PIECE>::value ? (size_t)16 * (TI + TJ) * GT_WIDE_ROW : 0);
     static const cudaError_t allowed = allow_smem(gemm_plain_tile_kernel<T, TI, TJ, STAGES, PIECE>, SMEM);
     if (allowed != cudaSuccess) return ti_fail("gemm_plain: %s", cudaGetErrorString(allowed));
     const dim3 grid((out + 16 * TJ - 1) / (16 * TJ), (n + 16 * TI - 1) / (16 * TI));
