@@ -456,6 +456,11 @@ static int launch_product(void* y, long long ldy, const T* x, long long ldx, con
                           const XieluParams& act, cudaStream_t stream) {
 #define GT_ARGS y, ldy, x, ldx, W, n, out, in, epilogue, act, stream
     if (n <= GT_STREAM_TOKENS) {
+        // One segment of k is one warp a block, whose chain is the time: its tokens are shared out, four to a block, while the blocks take
+        // no more than about three rounds, of 1 KB rows (32-bit, 32 / 64 tokens: 512 x 512 22.5 / 22.5 -> 6.8 / 7.1 us, 300 x 64 6.8 / 6.9 -> 2.7 / 2.6,
+        // but 8,192 x 512 24.5 -> 25.2 with 32).
+        const long long row = in * (long long)sizeof(T) < 1024 ? 1024 : in * (long long)sizeof(T), fours = (long long)((out + 15) / 16) * ((n + 3) / 4);
+        if (in <= GP_SEGMENT && n > 4 && fours * row <= 42LL * 1024 * ti_sm_count()) return launch_stream<T, 2, 1, PIECE == 16 ? 5 : 4, PIECE>(GT_ARGS);
         if constexpr (PIECE == 16) {
             // 32 rows a block halve what is read of the tokens, where that leaves blocks for six tenths of the SMs (8 tokens: 4,096
             // rows 17.8 us against 24.5 with 16 rows a block, 2,048 rows of k = 2,048 13.8 against 10.7). More blocks than SMs take two
