@@ -17,8 +17,8 @@ def ops():
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("out,k", [(15, 8), (33, 504), (100, 512), (2000, 520), (5000, 1032), (4100, 2056), (260, 8 * 1037)])
 def test_product_bits_do_not_depend_on_the_kernel(ops, dtype, out, k):
-    """Weight streaming by 1 to 64 tokens (16 or 32 rows a block, shallow or deep rings), every tile shape, and the two kernels
-    for rows that cannot be read 16 bytes at a time: one order of additions, so one set of bits."""
+    """Weight streaming by 1 to 64 tokens (16 or 32 rows a block, shallow or deep rings), tiles, and rows that cannot be
+    read 16 bytes at a time (staged in smaller pieces): one order of additions, so one set of bits."""
     g = torch.Generator().manual_seed(out + k)
     x = torch.randn(700, k, generator=g).to(dtype).cuda()
     w = (torch.randn(out, k, generator=g) * k ** -0.5).to(dtype).cuda()
@@ -76,6 +76,34 @@ def test_attention_over_chunk_edges(ops, D, nq, nkv):
                 bound = 2.0 ** -24 * (2 * D * size + 4 * math.sqrt(len(seen)) + 16) * float(values.abs().max())
                 assert float((together[r, h].double() - want).abs().max()) <= bound, (p, h, window)
             assert torch.equal(run([r])[0], together[r])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D,nq,nkv", [(4, 3, 3), (33, 4, 2), (64, 10, 2), (100, 4, 2), (128, 4, 4), (128, 12, 2), (132, 3, 3), (192, 4, 2), (256, 6, 2), (260, 2, 2),
+                                      (512, 4, 2), (512, 5, 1)])
+def test_attention_of_many_tokens_has_the_bits_of_few(ops, dtype, D, nq, nkv):
+    """A launch of many blocks takes the kernels that put more of them on an SM, with fewer loads in flight each: the same bits as in launches
+    of few, for sets of one, two and up to four heads."""
+    from tileinfer_b200.kernels import fast
+    page, last = 16, 300
+    g = torch.Generator(device="cuda").manual_seed(D + nq)
+    pages = -(-last // page)
+    k, v = (torch.randn(pages, nkv, page, D, generator=g, device="cuda").to(dtype) for _ in range(2))
+    table = torch.randperm(pages, generator=g, device="cuda").int()[None]
+    n = 3 * fast.sm_count() + 1                          # a block per token, KV head and set
+    positions = torch.randint(0, last, (n,), generator=g, device="cuda").int()
+    q = torch.randn(n, nq, D, generator=g, device="cuda").to(dtype)
+
+    def run(lo, hi):
+        out = torch.empty(hi - lo, nq * D, dtype=dtype, device="cuda")
+        pos = positions[lo:hi].contiguous()
+        ops.attention_plain(out, q[lo:hi].contiguous(), k, v, table, torch.zeros_like(pos), pos, D ** -0.5, nq, nkv, D, page)
+        return out
+
+    together = run(0, n)
+    for lo in range(0, n, 37):
+        hi = min(n, lo + 37)
+        assert torch.equal(run(lo, hi), together[lo:hi]), lo
 
 
 def test_attention_beyond_two_to_the_31_rows(ops):

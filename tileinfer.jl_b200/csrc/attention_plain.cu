@@ -30,10 +30,44 @@ __device__ __forceinline__ void load_quad(const bf16* p, float (&v)[4]) {
     v[0] = __uint_as_float(t.x << 16); v[1] = __uint_as_float(t.x & 0xffff0000u);
     v[2] = __uint_as_float(t.y << 16); v[3] = __uint_as_float(t.y & 0xffff0000u);
 }
-template <typename T> __device__ __forceinline__ void load_quad_any(const T* row, int d, int D, bool quads, float (&v)[4]) {
-    if (quads) { load_quad(row + d, v); return; }
+// A quad of a row that cannot be read so, element by element, zeros beyond the row's end.
+template <typename T> __device__ __forceinline__ void load_elements(const T* row, int d, int D, float (&v)[4]) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) v[e] = d + e < D ? to_f32(__ldcg(row + d + e)) : 0.f;
+}
+// A set's HN probabilities of one key.
+template <int HN> __device__ __forceinline__ void load_set(const float* p, float (&v)[HN]) {
+    if constexpr (HN == 4) { const float4 t = *reinterpret_cast<const float4*>(p); v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w; }
+    else if constexpr (HN == 2) { const float2 t = *reinterpret_cast<const float2*>(p); v[0] = t.x; v[1] = t.y; }
+    else v[0] = *p;
+}
+// N quads of a key into the scores of a set's heads, terms in ascending dimension. `q`: the heads' queries, Dq apart, from the first quad on.
+template <int HN, int N> __device__ __forceinline__ void add_scores(const float (&k)[N][4], const float* q, int Dq, float (&s)[HN]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+#pragma unroll
+        for (int h = 0; h < HN; ++h) {
+            const float4 qv = *reinterpret_cast<const float4*>(q + h * Dq + 4 * i);
+            s[h] = fmaf(qv.w, k[i][3], fmaf(qv.z, k[i][2], fmaf(qv.y, k[i][1], fmaf(qv.x, k[i][0], s[h]))));
+        }
+}
+template <typename T, int HN, int N> __device__ __forceinline__ void score_quads(const T* k, const float* q, int Dq, float (&s)[HN]) {
+    float v[N][4];
+#pragma unroll
+    for (int i = 0; i < N; ++i) load_quad(k + 4 * i, v[i]);                        // all on their way before the first is used
+    add_scores<HN, N>(v, q, Dq, s);
+}
+
+// A key's quads of the value row, times its probabilities, into the sums of a set's heads.
+template <int NI, int HN> __device__ __forceinline__ void add_values(const float* p, const float (&v)[NI][4], float (&acc)[HN][NI][4]) {
+    float w[HN];
+    load_set<HN>(p, w);
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+        for (int h = 0; h < HN; ++h)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[h][i][e] = fmaf(w[h], v[i][e], acc[h][i][e]);
 }
 
 // One block per (token, KV head, set of up to AP_HEADS of its query heads): a key's and a value's row is read once for all the
@@ -46,8 +80,10 @@ template <typename T> __device__ __forceinline__ void load_quad_any(const T* row
 // numbers come from the block table once per chunk, and value rows are asked for eight at a time: 8 sequences of 12 to 255
 // positions, 32 / 8 heads of 128 take 35 us; with 128 threads, a table lookup ahead of every value row and one chain per
 // dimension over all keys they took 127 us.
-template <typename T, int NI>                     // NI: quads of a value row per lane (rows of up to 128 NI elements)
-__global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restrict__ out, const T* q, const T* k_cache,
+// NI: quads of a value row per lane (rows of up to 128 NI elements). HN: heads of a set, 1, 2 or 4 (the last set may have fewer).
+// AT_ONCE: quads that a thread has in flight. BLOCKS: what an SM is to hold.
+template <typename T, int NI, int HN, int AT_ONCE, int BLOCKS>
+__global__ void __launch_bounds__(AP_THREADS, BLOCKS) attention_plain_kernel(T* __restrict__ out, const T* q, const T* k_cache,
                                        const T* v_cache, const int* block_table,
                                        int table_stride, const int* tok_slot,
                                        const int* positions, float scale, int nq, int nkv, int D,
@@ -56,17 +92,17 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
                                        const float* __restrict__ slope, int keep) {
     extern __shared__ __align__(16) float smem[];
     const int Dq = (D + 3) & ~3;
-    float* qs = smem;                                 // [AP_HEADS][Dq], zeros beyond D
-    float* ps = smem + AP_HEADS * Dq;                 // [AP_CHUNK][AP_HEADS]
-    float* part_sums = ps + AP_CHUNK * AP_HEADS;      // [AP_WARPS][Dq]
+    float* qs = smem;                                 // [HN][Dq], zeros beyond D
+    float* ps = smem + HN * Dq;                 // [AP_CHUNK][HN]
+    float* part_sums = ps + AP_CHUNK * HN;            // [AP_WARPS][Dq]
     __shared__ long long rows[AP_CHUNK];              // a key's row in the cache, in rows of D elements (pools of small heads hold more than 2^31)
-    __shared__ float maxima[AP_WARPS][AP_HEADS], sums[AP_WARPS][AP_HEADS];
+    __shared__ float maxima[AP_WARPS][HN], sums[AP_WARPS][HN];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int group = nq / nkv;
-    const int sets = (group + AP_HEADS - 1) / AP_HEADS;
+    const int sets = (group + HN - 1) / HN;
     const int t = blockIdx.x, kvh = blockIdx.y / sets;
-    const int h0 = kvh * group + (blockIdx.y % sets) * AP_HEADS;           // first query head of the set
-    const int heads = min(AP_HEADS, kvh * group + group - h0);
+    const int h0 = kvh * group + (blockIdx.y % sets) * HN;           // first query head of the set
+    const int heads = min(HN, kvh * group + group - h0);
     // Lanes that share a value row, and how many rows a warp takes at a time.
     int lanes = 32;
     if (NI == 1) while (lanes > 1 && lanes * 2 >= Dq) lanes >>= 1;          // lanes * 4 >= Dq still holds
@@ -76,15 +112,15 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
     pdl_launch_dependents();
     const int p = __ldcg(positions + t);
     const int* table = block_table + (size_t)__ldcg(tok_slot + t) * table_stride;
-    for (int i = tid; i < AP_HEADS * Dq; i += AP_THREADS) {
+    for (int i = tid; i < HN * Dq; i += AP_THREADS) {
         const int h = i / Dq, d = i % Dq;
         qs[i] = h < heads && d < D ? to_f32(__ldcg(q + ((size_t)t * nq + h0 + h) * D + d)) : 0.f;
     }
 
-    float acc[AP_HEADS][NI][4];
-    float m[AP_HEADS], l[AP_HEADS];
+    float acc[HN][NI][4];
+    float m[HN], l[HN];
 #pragma unroll
-    for (int h = 0; h < AP_HEADS; ++h) {
+    for (int h = 0; h < HN; ++h) {
         m[h] = -INFINITY; l[h] = 0.f;
 #pragma unroll
         for (int i = 0; i < NI; ++i)
@@ -105,25 +141,28 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
         const long long row = mine ? ((long long)__ldcg(table + j / page_size) * nkv + kvh) * page_size + j % page_size : 0;
         __syncthreads();                              // the chunk before is done with rows and ps; q is there
         rows[tid] = row;
-        float s[AP_HEADS];
+        float s[HN];
 #pragma unroll
-        for (int h = 0; h < AP_HEADS; ++h) s[h] = 0.f;
+        for (int h = 0; h < HN; ++h) s[h] = 0.f;
         if (mine) {
             const T* krow = k_cache + row * D;
-#pragma unroll 8
-            for (int d0 = 0; d0 < Dq; d0 += 4) {
-                float kv[4];
-                load_quad_any(krow, d0, D, quads, kv);
-#pragma unroll
-                for (int h = 0; h < AP_HEADS; ++h) {
-                    if (h >= heads) continue;                                      // uniform across the block
-                    const float4 qv = *reinterpret_cast<const float4*>(qs + h * Dq + d0);
-                    s[h] = fmaf(qv.w, kv[3], fmaf(qv.z, kv[2], fmaf(qv.y, kv[1], fmaf(qv.x, kv[0], s[h]))));
+            int d = 0;
+            if (quads) {
+#pragma unroll 1
+                for (; d + 4 * AT_ONCE <= D; d += 4 * AT_ONCE) score_quads<T, HN, AT_ONCE>(krow + d, qs + d, Dq, s);
+#pragma unroll 1
+                for (; d < D; d += 4) score_quads<T, HN, 1>(krow + d, qs + d, Dq, s);
+            } else {
+#pragma unroll 1
+                for (; d < Dq; d += 4) {
+                    float kv[1][4];
+                    load_elements(krow, d, D, kv[0]);
+                    add_scores<HN, 1>(kv, qs + d, Dq, s);
                 }
             }
         }
 #pragma unroll
-        for (int h = 0; h < AP_HEADS; ++h) {
+        for (int h = 0; h < HN; ++h) {
             if (h >= heads) continue;
             if (mine) {
                 s[h] *= scale;
@@ -138,23 +177,23 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
             if (lane == 0) maxima[warp][h] = wm;
         }
         __syncthreads();
-        float factor[AP_HEADS];
+        float factor[HN];
 #pragma unroll
-        for (int h = 0; h < AP_HEADS; ++h) {
+        for (int h = 0; h < HN; ++h) {
             if (h >= heads) continue;
             float m_new = m[h];
 #pragma unroll
             for (int w = 0; w < AP_WARPS; ++w) m_new = fmaxf(m_new, maxima[w][h]);
             factor[h] = (m[h] == -INFINITY) ? 0.f : expf(m[h] - m_new);
             const float e = mine ? expf(s[h] - m_new) : 0.f;
-            ps[tid * AP_HEADS + h] = rnd<T>(e);
+            ps[tid * HN + h] = rnd<T>(e);
             const float ws = warp_sum(e);
             if (lane == 0) sums[warp][h] = ws;
             m[h] = m_new;
         }
         __syncthreads();
 #pragma unroll
-        for (int h = 0; h < AP_HEADS; ++h) {
+        for (int h = 0; h < HN; ++h) {
             if (h >= heads) continue;
             float total = 0.f;
 #pragma unroll
@@ -167,30 +206,39 @@ __global__ void __launch_bounds__(AP_THREADS) attention_plain_kernel(T* __restri
         }
         // This warp's keys of the chunk that are visible: from the first row group that holds one on.
         const int w0 = c0 + 32 * warp, a = max(lo, w0) - w0, b = min(hi, w0 + 31) - w0;
-#pragma unroll 8
-        for (int g = a > 0 ? a / takes * takes : 0; g <= b; g += takes) {
-            const int k = g + sub, i0 = 32 * warp + k;
-            if (k < a || k > b) continue;
-            const T* vrow = v_cache + rows[i0] * D;
-            const float4 pv = *reinterpret_cast<const float4*>(ps + i0 * AP_HEADS);
-            const float w[AP_HEADS] = {pv.x, pv.y, pv.z, pv.w};
+        const int g0 = a > 0 ? a / takes * takes : 0;
+        if (quads) {
+            // Rows in flight together: AT_ONCE quads a lane. In the place of a key that is not visible stands the cache's first row; nothing is added.
+            constexpr int ROWS = AT_ONCE / NI;
+#pragma unroll 1
+            for (int g = g0; g <= b; g += takes * ROWS) {
+                float v[ROWS][NI][4];
 #pragma unroll
-            for (int i = 0; i < NI; ++i) {
-                const int d = dl + 128 * i;
-                if (d >= D) continue;
-                float v[4];
-                load_quad_any(vrow, d, D, quads, v);
+                for (int r = 0; r < ROWS; ++r) {
+                    const T* vrow = v_cache + rows[32 * warp + min(g + r * takes + sub, 31)] * D;
 #pragma unroll
-                for (int h = 0; h < AP_HEADS; ++h) {
-                    if (h >= heads) continue;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[h][i][e] = fmaf(w[h], v[e], acc[h][i][e]);
+                    for (int i = 0; i < NI; ++i) load_quad(vrow + (dl + 128 * i < D ? dl + 128 * i : 0), v[r][i]);
                 }
+#pragma unroll
+                for (int r = 0; r < ROWS; ++r) {
+                    const int k = g + r * takes + sub;
+                    if (k >= a && k <= b) add_values<NI, HN>(ps + (32 * warp + k) * HN, v[r], acc);
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int g = g0; g <= b; g += takes) {
+                const int k = g + sub;
+                if (k < a || k > b) continue;
+                float v[NI][4];
+#pragma unroll
+                for (int i = 0; i < NI; ++i) load_elements(v_cache + rows[32 * warp + k] * D, dl + 128 * i, D, v[i]);
+                add_values<NI, HN>(ps + (32 * warp + k) * HN, v, acc);
             }
         }
     }
 #pragma unroll
-    for (int h = 0; h < AP_HEADS; ++h) {
+    for (int h = 0; h < HN; ++h) {
         if (h >= heads) continue;
         // A sink: one more term exp(sink_h) in the softmax's denominator, with no key and no value.
         if (sink != nullptr) l[h] += expf(sink[h0 + h] - m[h]);
@@ -230,16 +278,25 @@ extern "C" int ti_attention_plain_kept(void* out, const void* q, const void* k_c
     TI_REQUIRE(keep >= 0 && (keep == 0 || chunk == 0), "attention: kept positions beside a window, not beside chunks");
     TI_REQUIRE(D > 0 && D <= AP_MAX_D, "attention: head_dim %d exceeds %d", D, AP_MAX_D);
     TI_REQUIRE(nq > 0 && nkv > 0 && nq % nkv == 0, "attention: %d query heads do not divide into %d KV heads", nq, nkv);
-    const int sets = (nq / nkv + AP_HEADS - 1) / AP_HEADS;
+    const int group = nq / nkv, hn = group <= 2 ? group : AP_HEADS, sets = (group + hn - 1) / hn;
     TI_REQUIRE((long long)nkv * sets <= 65535, "attention: too many heads (%d)", nq);
     dim3 grid(n_tokens, nkv * sets);
     const int Dq = (D + 3) & ~3;
-    const size_t smem = (size_t)(AP_HEADS * Dq + AP_CHUNK * AP_HEADS + AP_WARPS * Dq) * sizeof(float);       // 28 KB at the largest head
-#define AP_LAUNCH(NI) ti_launch(attention_plain_kernel<T, NI>, dim3(grid), dim3(AP_THREADS), smem, stream, (T*)out, (const T*)q, (const T*)k_cache,  \
+    const size_t smem = (size_t)(hn * Dq + AP_CHUNK * hn + AP_WARPS * Dq) * sizeof(float);       // 28 KB at the largest head
+    // Many blocks hide one another's latency: more of them on an SM (8 prompts of 60 tokens, 32-bit, 8 / 16 heads of 64 / 128 on as many: 42 / 111 us, 129 / 439
+    // with two blocks an SM). Few have the longer run of loads each (one sequence of 20 / 2,000 positions, 32 / 4 heads of 64: 9 / 62 us).
+    const bool many = (long long)n_tokens * nkv * sets > 3LL * ti_sm_count();
+#define AP_ONE(NI, HN, AT_ONCE, BLOCKS) ti_launch(attention_plain_kernel<T, NI, HN, AT_ONCE, BLOCKS>, dim3(grid), dim3(AP_THREADS), smem, stream, (T*)out, (const T*)q, (const T*)k_cache,  \
                                 (const T*)v_cache, block_table, table_stride, tok_slot, positions, scale, nq, nkv, D, page_size, window, sink, chunk, \
                                 dist_bias, bias_len, cap, slope, window > 0 ? keep : 0)
-    TI_DISPATCH_DTYPE(dtype, { if (D <= 128) AP_LAUNCH(1); else if (D <= 256) AP_LAUNCH(2); else AP_LAUNCH(4); });
+#define AP_LAUNCH(NI, HN, LITTLE, BLOCKS) do { if (many) AP_ONE(NI, HN, LITTLE, BLOCKS); else AP_ONE(NI, HN, 8, 2); } while (0)
+    TI_DISPATCH_DTYPE(dtype, {
+        if (D <= 128) { if (hn == 1) AP_LAUNCH(1, 1, 4, 4); else if (hn == 2) AP_LAUNCH(1, 2, 4, 4); else AP_LAUNCH(1, 4, 4, 3); }
+        else if (D <= 256) { if (hn == 1) AP_LAUNCH(2, 1, 4, 4); else if (hn == 2) AP_LAUNCH(2, 2, 4, 3); else AP_LAUNCH(2, 4, 4, 2); }
+        else { if (hn == 1) AP_LAUNCH(4, 1, 4, 3); else if (hn == 2) AP_LAUNCH(4, 2, 4, 2); else AP_ONE(4, 4, 4, 2); }
+    });
 #undef AP_LAUNCH
+#undef AP_ONE
     return ti_check_launch("attention_plain");
 }
 
