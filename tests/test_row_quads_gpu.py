@@ -97,3 +97,43 @@ def test_latent_inputs(q_rank, kv_rank, rot, spare, dtype, form, interleaved):
         wide = torch.zeros(n, size + 3, dtype=dtype, device="cuda")
         wide[:, :size] = rows
         check(wide[:, :size])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nkv,D,taps,norm", [(16, 4, 128, 4, True), (32, 8, 64, 0, True), (6, 2, 36, 3, False), (5, 1, 256, 2, True)])
+def test_convolved_attention_inputs_shared_out(nq, nkv, D, taps, norm, dtype):
+    """A token's heads by one block, by a few in quads and by many channel by channel: the same bits, and those of 64-bit arithmetic within the
+    roundings."""
+    from tileinfer_b200.kernels import ops
+    g = torch.Generator(device="cuda").manual_seed(nq * D)
+    n, page, C = 260, 16, (nq + 2 * nkv) * D
+    rows = torch.randn(n, C, generator=g, device="cuda").to(dtype)
+    bias = torch.randn(C, generator=g, device="cuda").to(dtype)
+    conv = torch.randn(C, taps, generator=g, device="cuda").to(dtype) if taps else None
+    state = torch.randn(n, taps - 1, C, generator=g, device="cuda").to(dtype).float() if taps else None
+    wq, wk = ((torch.randn(D, generator=g, device="cuda") * 0.1 + 1).to(dtype) for _ in range(2)) if norm else (None, None)
+
+    def run(count):
+        q = torch.empty(count, nq, D, dtype=dtype, device="cuda")
+        k, v = (torch.empty(-(-count // page), nkv, page, D, dtype=dtype, device="cuda") for _ in range(2))
+        index = torch.arange(count + 1, device="cuda").int()
+        step = SimpleNamespace(positions=torch.full((count,), 9, dtype=torch.int32, device="cuda"), cu_seqlens=index, seq_slots=index[:count],
+                               kv_lens=torch.full((count,), 10, dtype=torch.int32, device="cuda"), n_seqs=count)
+        ops.conv_attention_inputs(rows[:count], bias, conv, taps, state, wq, wk, 1e-6, None, q, k, v, step, index[:count].contiguous(), nq, nkv, D, D, D, page,
+                                  head_norm=norm)
+        keys, values = (c.permute(0, 2, 1, 3).reshape(-1, nkv, D)[:count] for c in (k, v))
+        return torch.cat([q, keys, values], 1)
+
+    whole = run(n)
+    for count in (1, 8, 33, 70, 150):
+        assert torch.equal(run(count), whole[:count]), count
+    low = dtype == torch.bfloat16
+    own = (rows.to(F64) + bias.to(F64)).to(dtype).to(F64)
+    if taps:
+        own = ((state.to(F64) * conv.to(F64).T[:taps - 1]).sum(1) + own * conv.to(F64).T[taps - 1]).to(dtype).to(F64)
+    want = own.view(n, nq + 2 * nkv, D)
+    if norm:
+        want = torch.cat([_rms(want[:, :nq], wq, 1e-6), _rms(want[:, nq:nq + nkv], wk, 1e-6), want[:, nq + nkv:]], 1)
+    # bfloat16: a rounding before the last one may fall the other way, two units in the last place together; 32-bit: a few roundings of terms
+    # of up to 64.
+    assert bool(((whole.to(F64) - want).abs() <= (2.0 ** -6 if low else 2.0 ** -17) * want.abs().clamp(min=1.0)).all())

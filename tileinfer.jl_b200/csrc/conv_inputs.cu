@@ -250,16 +250,20 @@ extern "C" int ti_conv_attention_inputs(const void* proj, long long ld, const vo
     const int C = nq * D + (write_kv ? nkv * (shared_kv ? D : D + V) : 0);
     const size_t smem = (size_t)C * sizeof(float);
     TI_REQUIRE(smem <= 160 * 1024, "conv_attention_inputs: %d channels", C);
-    // Few tokens: their heads are shared out among several blocks each (a head's results do not depend on it).
+    // Few tokens: their heads are shared out among several blocks each (a head's results do not depend on it), as many as leave each SM a block or
+    // two, at least 256 channels a block: 64 tokens of 3,072 channels, 4 taps, in 64 / 128 / 192 / 256 / 576 blocks 7.4 / 5.5 / 5.4 / 8.5 / 12.7 us.
     int parts = 1;
     if (!shared_kv && (head_norm || (q_norm_w == nullptr && k_norm_w == nullptr))) {
-        parts = 4 * ti_sm_count() / n;
+        parts = 3 * ti_sm_count() / (2 * n);
         if (parts > C / CI_THREADS) parts = C / CI_THREADS;
         if (parts > nq) parts = nq;
         if (parts < 1) parts = 1;
     }
+    // Small shares of bfloat16 rows go channel by channel, where a thread's quad and its taps are one chain (one token, 12 blocks: 3.2 us
+    // against 3.5; 32-bit rows 3.3 against 3.1).
     const bool quads = taps <= 4 && D % 4 == 0 && V % 4 == 0 && Dp % 4 == 0 && ld % 4 == 0 && (cos_sin == nullptr || (rotary % 8 == 0 && !interleaved)) &&
-                       aligned16(proj) && aligned16(bias) && aligned16(conv) && aligned16(state) && aligned16(q_out) && aligned16(k_cache) && aligned16(v_cache);
+                       aligned16(proj) && aligned16(bias) && aligned16(conv) && aligned16(state) && aligned16(q_out) && aligned16(k_cache) && aligned16(v_cache) &&
+                       (parts == 1 || dtype == TI_F32 || C / parts >= 2 * CI_THREADS);
 #define CI_LAUNCH(TAPS)                                                                                                                       \
     do {                                                                                                                                      \
         if (quads) {                                                                                                                          \
