@@ -1,0 +1,116 @@
+"""Row kernels whose blocks depend on how many rows a step has: a row's bits do not depend on the step it is in. Their distance to
+64-bit arithmetic is measured where the kernels are tested alone (test_fasodra_gpu.py)."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from tileinfer_b200.kernels import ops
+    return ops
+
+
+def _step(lengths, slots=None):
+    cu = torch.tensor([0] + lengths).cumsum(0).int().cuda()
+    return SimpleNamespace(cu_seqlens=cu, seq_slots=torch.tensor(slots or list(range(len(lengths)))).int().cuda(), n_seqs=len(lengths))
+
+
+@pytest.mark.parametrize("size", [96, 1000, 1024, 2048, 4096, 5000])
+@pytest.mark.parametrize("streams", [1, 2, 3, 8])
+def test_stream_rows_in_small_and_large_steps(ops, size, streams):
+    g = torch.Generator(device="cuda").manual_seed(size + streams)
+    n = 400                                                # more rows than SMs
+    R = lambda *s, dtype=torch.float32: torch.randn(*s, generator=g, device="cuda").to(dtype)     # noqa: E731
+    x, delta, parts = R(n, streams * size), R(n, size, dtype=torch.bfloat16), R(3, n, size)
+    w, b = R(size, dtype=torch.bfloat16), R(size, dtype=torch.bfloat16)
+    mix, out, blend = ([0.3 + 0.1 * i for i in range(c)] for c in (streams * streams, streams, streams))
+    a = torch.tensor(blend, device="cuda")
+
+    def run(lo, hi):
+        got = []
+        for d in (delta[lo:hi].contiguous(), parts[:, lo:hi].contiguous()):
+            for centred in (True, False):
+                xs, h = x[lo:hi].clone(), torch.empty(hi - lo, size, dtype=torch.bfloat16, device="cuda")
+                ops.streams_update(xs, d, mix, out, blend, h, w, b, 1e-6, centred)
+                got += [xs, h]
+        h = torch.empty(hi - lo, size, dtype=torch.bfloat16, device="cuda")
+        ops.streams_read_norm(h, x[lo:hi].contiguous(), a, w, b, 1e-6)
+        pairs = torch.empty(hi - lo, size, device="cuda")
+        ops.pair_combine(pairs, delta[lo:hi].contiguous(), parts[:, lo:hi].contiguous(), w, b, 1e-6, 0.5, 2.0, torch.bfloat16)
+        return got + [h, pairs]
+
+    whole = run(0, n)
+    want = torch.einsum("st,nsc->ntc", torch.tensor(mix).view(streams, streams).double().cuda(), x.double().view(n, streams, size))
+    want = (want + torch.tensor(out).double().cuda()[:, None] * delta.double()[:, None, :]).reshape(n, -1)
+    assert float((whole[0].double() - want).abs().max()) <= 16 * 2.0 ** -24 * float(want.abs().max())
+    for lo, hi in ((0, 1), (3, 7), (100, 248)):
+        for one, all_ in zip(run(lo, hi), whole):
+            assert torch.equal(one, all_[lo:hi]), (lo, hi)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("W,K", [(40, 1), (257, 5), (2048, 5), (1024, 10)])
+def test_blends_in_runs_of_tokens(ops, dtype, W, K):
+    """Eight tokens a block and one: sequences that begin and end inside a run, rows before the step's first from the state."""
+    g = torch.Generator(device="cuda").manual_seed(W)
+    lengths = [1, 3, 900, 2, 7, 300, 1]
+    n, slots = sum(lengths), [4, 0, 6, 2, 1, 3, 5]
+    h = torch.randn(n, W, generator=g, device="cuda").to(dtype)
+    mu = torch.randn(K, W, generator=g, device="cuda").to(dtype)
+    prev = torch.randn(7, W, generator=g, device="cuda")
+
+    def run(cuts):
+        state, out = prev.clone(), torch.empty(K, n, W, dtype=dtype, device="cuda")
+        for first, last in zip(cuts, cuts[1:]):              # sequences first .. last - 1 in one step
+            lo, hi = sum(lengths[:first]), sum(lengths[:last])
+            piece = torch.empty(K, hi - lo, W, dtype=dtype, device="cuda")
+            ops.shift_blend(piece, h[lo:hi].contiguous(), mu, state, _step(lengths[first:last], slots[first:last]))
+            out[:, lo:hi] = piece
+        return out, state
+
+    whole, state = run([0, 7])
+    apart, state_apart = run([0, 2, 3, 5, 6, 7])
+    assert torch.equal(whole, apart) and torch.equal(state, state_apart)
+    at = 0
+    for length, slot in zip(lengths, slots):
+        rows = h[at:at + length].double()
+        before = torch.cat([prev[slot].double()[None], rows[:-1]])
+        want = rows[None] + (before - rows)[None] * mu.double()[:, None, :]
+        bound = (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22) * float(want.abs().max())
+        assert float((whole[:, at:at + length].double() - want).abs().max()) <= bound
+        assert torch.equal(state[slot], h[at + length - 1].float())
+        at += length
+
+
+@pytest.mark.parametrize("taps", [0, 1, 3, 4, 7])
+@pytest.mark.parametrize("G,D,HV", [(1, 24, 40), (3, 128, 384), (2, 300, 64), (4, 64, 1000)])
+def test_delta_inputs_in_runs_of_tokens(ops, taps, G, D, HV):
+    g = torch.Generator(device="cuda").manual_seed(D + taps)
+    C, lengths = 2 * G * D + HV, [2, 2000, 1, 5]
+    n, slots = sum(lengths), [2, 0, 3, 1]
+    proj = torch.randn(n, C, generator=g, device="cuda").bfloat16()
+    conv = torch.randn(C, max(1, taps), generator=g, device="cuda").bfloat16()
+    hist = torch.randn(4, max(1, taps - 1) * C, generator=g, device="cuda")
+    whole = torch.empty(n, C, device="cuda")
+    ops.delta_inputs(whole, proj, conv, taps, hist, _step(lengths, slots), G, D, HV, 1e-6)
+    at = 0
+    for length, slot in zip(lengths, slots):
+        rows = min(length, 40)                             # few tokens: one a block
+        part = torch.empty(rows, C, device="cuda")
+        ops.delta_inputs(part, proj[at:at + rows].contiguous(), conv, taps, hist, _step([rows], [slot]), G, D, HV, 1e-6)
+        assert torch.equal(part, whole[at:at + rows])
+        older = hist[slot, :max(0, taps - 1) * C].double().view(-1, C)
+        x = torch.cat([older, proj[at:at + length].double()])
+        y = x if taps == 0 else sum(conv[:, k].double() * x[k:k + length] for k in range(taps))
+        y = y * torch.sigmoid(y)
+        heads = y[:, :2 * G * D].view(length, 2 * G, D)
+        heads = heads / torch.sqrt((heads * heads).sum(-1, keepdim=True) + 1e-6)
+        heads[:, :G] *= D ** -0.5
+        want = torch.cat([heads.reshape(length, -1), y[:, 2 * G * D:]], 1)
+        # Sums of up to 7 products, an exponential, and sums over a head.
+        assert float((whole[at:at + length].double() - want).abs().max()) <= 2.0 ** -24 * 64 * max(1.0, float(y.abs().max()))
+        at += length

@@ -9,7 +9,16 @@
 
 #define HS_MAX_STREAMS 8
 
+// Sums over a row are added as by this many threads, element i by thread i modulo it, whatever a block's size is: a token's bits do not
+// depend on the step it is in.
 static int hs_threads(int size) { return size >= 4096 ? 512 : size >= 1024 ? 256 : 128; }
+// Threads of a row's block. With no more rows than SMs a row's time is the round trips of one thread's loads, one after the other: blocks as
+// large as the row, up to 1,024 threads (4 rows of 2,048, two copies: update 8.4 -> 5.3 us, read 6.1 -> 3.6).
+static int hs_block(int size, int n) {
+    if (n > ti_sm_count()) return hs_threads(size);
+    const int all = (size + 31) / 32 * 32;
+    return all > 1024 ? 1024 : all > hs_threads(size) ? all : hs_threads(size);
+}
 
 // x [n][S][size] <- x0 [n][size] in every copy.
 __global__ void streams_begin_kernel(float* __restrict__ x, const float* x0, int S, int size, size_t count) {
@@ -38,14 +47,23 @@ struct StreamTables {
     float in_next[HS_MAX_STREAMS];                 // a'[t]
 };
 
-// The layer norm of `row_u` [size] (shared memory; a thread reads back the elements it wrote) into dst.
-template <typename T>
+// The layer norm of `row_u` [size] (shared memory) into dst. Element i was written by thread i modulo the block's size, which added its own up
+// in `sum`; a block of more than `sum_threads` threads adds again in the order of so many, and so does one that did not (ADD).
+template <typename T, bool ADD>
 __device__ __forceinline__ void norm_row(T* __restrict__ dst, const float* row_u, float sum, const T* __restrict__ w, const T* __restrict__ b,
-                                         float eps, int centred, int size, float* scratch) {
+                                         float eps, int centred, int size, int sum_threads, float* scratch) {
+    const int first = threadIdx.x < sum_threads ? threadIdx.x : size;
+    if (ADD || blockDim.x != sum_threads) {
+        __syncthreads();
+        sum = 0.f;
+#pragma unroll 4
+        for (int i = centred ? first : size; i < size; i += sum_threads) sum += row_u[i];
+    }
     float mean = 0.f;
     if (centred) mean = block_sum(sum, scratch) / (float)size;
     float ss = 0.f;
-    for (int i = threadIdx.x; i < size; i += blockDim.x) {
+#pragma unroll 4
+    for (int i = first; i < size; i += sum_threads) {
         const float d = row_u[i] - mean;
         ss = fmaf(d, d, ss);
     }
@@ -57,14 +75,24 @@ __device__ __forceinline__ void norm_row(T* __restrict__ dst, const float* row_u
         dst[i] = from_f32<T>(v);
     }
 }
+// The norm's weights do not depend on the step's kernels: on their way to L2 before the wait, one request per 128 bytes. (Of many blocks the first
+// do it for all, and the others' requests for the same lines only queue.)
+#define HS_PREFETCH_ROWS 64
+template <typename T> __device__ __forceinline__ void prefetch_row(const T* p, int size) {
+    constexpr int PER = 128 / (int)sizeof(T);
+    if (p != nullptr && gridDim.x <= HS_PREFETCH_ROWS)
+        for (int i = threadIdx.x * PER; i < size; i += blockDim.x * PER) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+}
 
 // h = norm(sum_s a[s] x_s): the first reader's input (nothing to write back yet).
 template <typename T>
-__global__ void streams_read_norm_kernel(T* __restrict__ h, const float* x, const float* __restrict__ a, int S, const T* __restrict__ w,
-                                         const T* __restrict__ b, float eps, int centred, int size) {
+__global__ void __launch_bounds__(1024) streams_read_norm_kernel(T* __restrict__ h, const float* x, const float* __restrict__ a, int S, const T* __restrict__ w,
+                                         const T* __restrict__ b, float eps, int centred, int size, int sum_threads) {
     extern __shared__ float row_u[];
     __shared__ float scratch[33];
     const float* rows = x + (size_t)blockIdx.x * S * size;
+    prefetch_row(w, size);
+    prefetch_row(b, size);
     pdl_enter();
     float sum = 0.f;
     for (int i = threadIdx.x; i < size; i += blockDim.x) {
@@ -73,14 +101,15 @@ __global__ void streams_read_norm_kernel(T* __restrict__ h, const float* x, cons
         row_u[i] = u;
         sum += u;
     }
-    norm_row<T>(h + (size_t)blockIdx.x * size, row_u, sum, w, b, eps, centred, size, scratch);
+    norm_row<T, false>(h + (size_t)blockIdx.x * size, row_u, sum, w, b, eps, centred, size, sum_threads, scratch);
 }
 
 // Write a sublayer's output back and make the next reader's input. The output is `delta` [n][size] of T, or the sum of
 // `n_partials` 32-bit arrays [n][size] `partial_stride` apart (a product cut over k, or one unrounded 32-bit result).
 template <typename T>
 __global__ void streams_update_kernel(float* x, const T* delta, const float* partials, int n_partials, size_t partial_stride, StreamTables tab,
-                                      int S, T* __restrict__ h, const T* __restrict__ w, const T* __restrict__ b, float eps, int centred, int size) {
+                                      int S, T* __restrict__ h, const T* __restrict__ w, const T* __restrict__ b, float eps, int centred, int size,
+                                      int sum_threads) {
     extern __shared__ float row_u[];
     __shared__ float scratch[33];
     float* rows = x + (size_t)blockIdx.x * S * size;
@@ -114,7 +143,58 @@ __global__ void streams_update_kernel(float* x, const T* delta, const float* par
         sum += u;
     }
     if (h == nullptr) return;
-    norm_row<T>(h + (size_t)blockIdx.x * size, row_u, sum, w, b, eps, centred, size, scratch);
+    norm_row<T, false>(h + (size_t)blockIdx.x * size, row_u, sum, w, b, eps, centred, size, sum_threads, scratch);
+}
+
+// The same, at most MAXS copies; a thread asks for AT_ONCE elements of all of them before it works on the first (2,048 rows, two copies of 2,048: 32.0 ->
+// 23.4 us).
+template <typename T, int MAXS, int AT_ONCE, int MOST>
+__global__ void __launch_bounds__(MOST) streams_update_rows_kernel(float* x, const T* delta, const float* partials, int n_partials, size_t partial_stride, StreamTables tab,
+                                      int S, T* __restrict__ h, const T* __restrict__ w, const T* __restrict__ b, float eps, int centred, int size,
+                                      int sum_threads) {
+    extern __shared__ float row_u[];
+    __shared__ float scratch[33];
+    float* rows = x + (size_t)blockIdx.x * S * size;
+    if (h != nullptr) {
+        prefetch_row(w, size);
+        prefetch_row(b, size);
+    }
+    pdl_enter();
+    for (int i0 = threadIdx.x; i0 < size; i0 += blockDim.x * AT_ONCE) {
+        float y[AT_ONCE], old[AT_ONCE][MAXS];
+#pragma unroll
+        for (int k = 0; k < AT_ONCE; ++k) {
+            const int i = i0 + k * blockDim.x, in = i < size ? i : 0;
+            y[k] = partials != nullptr ? __ldcg(partials + (size_t)blockIdx.x * size + in) : to_f32(__ldcg(delta + (size_t)blockIdx.x * size + in));
+#pragma unroll
+            for (int s = 0; s < MAXS; ++s) old[k][s] = s < S ? __ldcg(rows + (size_t)s * size + in) : 0.f;
+        }
+        for (int s = 1; s < n_partials; ++s)
+#pragma unroll
+            for (int k = 0; k < AT_ONCE; ++k) {
+                const int i = i0 + k * blockDim.x;
+                y[k] += __ldcg(partials + (size_t)s * partial_stride + (size_t)blockIdx.x * size + (i < size ? i : 0));
+            }
+#pragma unroll
+        for (int k = 0; k < AT_ONCE; ++k) {
+            const int i = i0 + k * blockDim.x;
+            float u = 0.f;
+#pragma unroll
+            for (int t = 0; t < MAXS; ++t) {
+                if (t >= S) break;
+                float v = 0.f;
+#pragma unroll
+                for (int s = 0; s < MAXS; ++s)
+                    if (s < S) v = fmaf(tab.mix[s * HS_MAX_STREAMS + t], old[k][s], v);
+                v = fmaf(tab.out[t], y[k], v);
+                if (i < size) rows[(size_t)t * size + i] = v;
+                u = fmaf(tab.in_next[t], v, u);
+            }
+            if (i < size) row_u[i] = u;
+        }
+    }
+    if (h == nullptr) return;
+    norm_row<T, true>(h + (size_t)blockIdx.x * size, row_u, 0.f, w, b, eps, centred, size, sum_threads, scratch);
 }
 
 extern "C" int ti_streams_read_norm(void* h, const float* x, const float* a, int S, const void* w, const void* b, float eps, int centred, int n,
@@ -125,7 +205,8 @@ extern "C" int ti_streams_read_norm(void* h, const float* x, const float* a, int
     TI_REQUIRE(smem <= 160 * 1024, "streams_read_norm: rows of %d", size);
     TI_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(streams_read_norm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        ti_launch(streams_read_norm_kernel<T>, dim3(n), dim3(hs_threads(size)), smem, stream, (T*)h, x, a, S, (const T*)w, (const T*)b, eps, centred, size);
+        ti_launch(streams_read_norm_kernel<T>, dim3(n), dim3(hs_block(size, n)), smem, stream, (T*)h, x, a, S, (const T*)w, (const T*)b, eps, centred, size,
+                  hs_threads(size));
     });
     return ti_check_launch("streams_read_norm");
 }
@@ -145,10 +226,22 @@ extern "C" int ti_streams_update(float* x, const void* delta, const float* parti
     }
     const size_t smem = (size_t)size * sizeof(float);
     TI_REQUIRE(smem <= 160 * 1024, "streams_update: rows of %d", size);
+    const int threads = hs_block(size, n);
     TI_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(streams_update_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        ti_launch(streams_update_kernel<T>, dim3(n), dim3(hs_threads(size)), smem, stream, x, (const T*)delta, partials, n_partials,
-                  (size_t)partial_stride, tab, S, (T*)h, (const T*)w, (const T*)b, eps, centred, size);
+        auto launch = [&](auto kernel) {
+            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            ti_launch(kernel, dim3(n), dim3(threads), smem, stream, x, (const T*)delta, partials, n_partials, (size_t)partial_stride, tab, S, (T*)h,
+                      (const T*)w, (const T*)b, eps, centred, size, hs_threads(size));
+        };
+        // Many rows of 4,096 and more, or of many copies: their blocks' memory traffic is the bound, and a thread that asks for more at once only
+        // takes room from other blocks (2,048 rows of 4,096, two copies, four elements at once: 73 us
+        // against 65; four copies, two elements: 112 against 80).
+        if (n <= ti_sm_count()) {
+            if (S <= 2) launch(streams_update_rows_kernel<T, 2, 4, 1024>);
+            else if (S <= 4) launch(streams_update_rows_kernel<T, 4, 2, 1024>);
+            else launch(streams_update_rows_kernel<T, HS_MAX_STREAMS, 1, 1024>);
+        } else if (S <= 2 && size < 4096) launch(streams_update_rows_kernel<T, 2, 4, 256>);
+        else launch(streams_update_kernel<T>);
     });
     return ti_check_launch("streams_update");
 }

@@ -20,15 +20,28 @@
 __device__ __forceinline__ float rs_silu(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float rs_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
-// The sequence of the step that token t belongs to: the last b with cu[b] <= t.
-__device__ __forceinline__ int rs_sequence_of(const int* cu, int B, int t) {
-    int lo = 0, hi = B - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldcg(cu + mid) <= t) lo = mid; else hi = mid - 1;
+// Where the RUN tokens from `first` on lie: every token's sequence's first token of the step, that sequence's slot and the one after its last token.
+// Asked by a whole block ahead of the wait (the step's tables were uploaded before its first kernel). One warp looks, a lane per token:
+// thousands of warps that each go through the same few words queue for them at L2. With one token a sequence there is nothing to look for.
+template <int RUN> struct TokenRun {
+    int t0[RUN], t1[RUN], slot[RUN];
+    __device__ __forceinline__ void find(const int* cu, const int* slots, int B, int n, int first) {
+        if (threadIdx.x < RUN && first + (int)threadIdx.x < n) {
+            const int i = threadIdx.x, t = first + i;
+            int lo = 0, hi = B - 1;
+            if (n == B) lo = t;
+            else
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (__ldcg(cu + mid) <= t) lo = mid; else hi = mid - 1;
+                }
+            t0[i] = n == B ? t : __ldcg(cu + lo);
+            t1[i] = n == B ? t + 1 : __ldcg(cu + lo + 1);
+            slot[i] = __ldcg(slots + lo);
+        }
+        __syncthreads();
     }
-    return lo;
-}
+};
 
 // ------------------------------------------------------------------------------------------------ decay scan
 // rkv [n][ld] of T: r at r_off, k at k_off, v at v_off, heads of `D` side by side; dlog [n][H * D] float: the decay's logit
@@ -463,19 +476,38 @@ extern "C" int ti_delta_scan(float* o, const float* qkv, long long ld, const flo
 // out [K][n][W] of T (every blend a matrix of its own): out[k][t] = h_t + (h_(t-1) - h_t) * mu[k], h_(t-1) being the row before in the step, or for a sequence's
 // first token of the step the row `prev` [slots] (state rows `prev_stride` floats apart; zeros at a sequence's start). The
 // block of a sequence's first token then moves the state on to the sequence's last row of the step (it alone reads the state).
-template <typename T>
+// A thread has one channel of RUN tokens in a row: their rows and the blends' weights are read once, all loads in flight together
+// (five blends of 2,048 channels, against a block that goes through a token's channels: 4 tokens 8.0 -> 2.3 us, 2,048 tokens 30 -> 24).
+#define SB_BLENDS 8
+template <typename T, int RUN>
 __global__ void shift_blend_kernel(T* __restrict__ out, const T* h, const T* __restrict__ mu, int K, float* prev, long long prev_stride,
-                                   const int* cu_seqlens, const int* seq_slots, int B, int W) {
-    const int t = blockIdx.x;
+                                   const int* cu_seqlens, const int* seq_slots, int B, int n, int W) {
+    __shared__ TokenRun<RUN> run;
+    const int t = blockIdx.x * RUN, c = blockIdx.y * blockDim.x + threadIdx.x;
+    run.find(cu_seqlens, seq_slots, B, n, t);
+    const int count = min(RUN, n - t);
+    float weight[SB_BLENDS];
+#pragma unroll
+    for (int k = 0; k < SB_BLENDS; ++k) weight[k] = k < K && c < W ? to_f32(mu[(size_t)k * W + c]) : 0.f;
     pdl_enter();
-    const int b = rs_sequence_of(cu_seqlens, B, t);
-    const int t0 = __ldcg(cu_seqlens + b), last = __ldcg(cu_seqlens + b + 1) - 1;
-    float* st = prev + (size_t)__ldcg(seq_slots + b) * prev_stride;
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
-        const float cur = to_f32(__ldcg(h + (size_t)t * W + c));
-        const float before = t > t0 ? to_f32(__ldcg(h + (size_t)(t - 1) * W + c)) : __ldcg(st + c);
-        for (int k = 0; k < K; ++k) out[((size_t)k * gridDim.x + t) * W + c] = from_f32<T>(fmaf(before - cur, to_f32(mu[(size_t)k * W + c]), cur));
-        if (t == t0) st[c] = to_f32(__ldcg(h + (size_t)last * W + c));
+    if (c >= W) return;
+    float row[RUN + 1];
+#pragma unroll
+    for (int i = 0; i <= RUN; ++i) row[i] = t + i >= 1 && i <= count ? to_f32(__ldcg(h + (size_t)(t + i - 1) * W + c)) : 0.f;
+#pragma unroll
+    for (int i = 0; i < RUN; ++i) {
+        if (i >= count) break;
+        const float cur = row[i + 1];
+        float before = row[i];
+        if (t + i == run.t0[i]) {                            // the sequence's first token of the step
+            float* st = prev + (size_t)run.slot[i] * prev_stride + c;
+            before = __ldcg(st);
+            *st = to_f32(__ldcg(h + (size_t)(run.t1[i] - 1) * W + c));
+        }
+#pragma unroll
+        for (int k = 0; k < SB_BLENDS; ++k)
+            if (k < K) out[((size_t)k * n + t + i) * W + c] = from_f32<T>(fmaf(before - cur, weight[k], cur));
+        for (int k = SB_BLENDS; k < K; ++k) out[((size_t)k * n + t + i) * W + c] = from_f32<T>(fmaf(before - cur, to_f32(mu[(size_t)k * W + c]), cur));
     }
 }
 
@@ -483,8 +515,18 @@ extern "C" int ti_shift_blend(void* out, const void* h, const void* mu, int K, f
                               const int* seq_slots, int n, int B, int W, int dtype, cudaStream_t stream) {
     if (n == 0) return 0;
     TI_REQUIRE(K > 0 && W > 0 && B > 0, "shift_blend: %d blends of rows of %d", K, W);
-    TI_DISPATCH_DTYPE(dtype, (ti_launch(shift_blend_kernel<T>, dim3(n), dim3(W >= 1024 ? 256 : 128), 0, stream, (T*)out, (const T*)h, (const T*)mu, K,
-                                        prev, prev_stride, cu_seqlens, seq_slots, B, W)));
+    const int threads = W >= 1024 ? 256 : 128, parts = (W + threads - 1) / threads;
+    // Eight tokens in a row once single ones would be some 14 blocks an SM (2,048 channels, single / eight: 100 tokens 3.2 / 4.5 us, 300 6.7 / 5.8,
+    // 2,048 33 / 24; 384 channels, 600 tokens 4.1 / 4.7, 1,000 5.6 / 4.7), but not where every token begins its sequence (200 x 4,096: 9.2 / 11.8).
+    const bool runs = n > B && (long long)n * parts > 14LL * ti_sm_count();
+    TI_DISPATCH_DTYPE(dtype, {
+        if (runs)
+            ti_launch(shift_blend_kernel<T, 8>, dim3((n + 7) / 8, parts), dim3(threads), 0, stream, (T*)out, (const T*)h, (const T*)mu, K, prev, prev_stride,
+                      cu_seqlens, seq_slots, B, n, W);
+        else
+            ti_launch(shift_blend_kernel<T, 1>, dim3(n, parts), dim3(threads), 0, stream, (T*)out, (const T*)h, (const T*)mu, K, prev, prev_stride, cu_seqlens,
+                      seq_slots, B, n, W);
+    });
     return ti_check_launch("shift_blend");
 }
 
@@ -493,36 +535,64 @@ extern "C" int ti_shift_blend(void* out, const void* h, const void* mu, int K, f
 // convolution over time (conv [C][taps] of T, the last tap the current token's, zeros before the sequence's start; history from
 // the step's own rows or from `hist`: the sequence's last taps - 1 rows, state rows `hist_stride` floats apart) and SiLU; then
 // every q and k head becomes a unit vector x / sqrt(sum x^2 + unit_eps), q also times D^(-1/2). out [n][C] float.
+// A block has RUN tokens in a row and `per` channels, whole heads among the q and k channels. A thread reads a channel's rows and weights once
+// for all of them (TAPS weights, 0: so many that they are read again for every token), its loads in flight together
+// (4,096 channels, 4 taps, against a block that goes through a token's channels: 4 tokens 13.6 -> 2.3 us, 2,048 tokens 60 -> 54).
 #define DI_THREADS 256
-template <typename T>
+template <typename T, int RUN, int TAPS>
 __global__ void __launch_bounds__(DI_THREADS) delta_inputs_kernel(float* __restrict__ out, const T* proj, long long ld, const T* __restrict__ conv,
                                                                    int taps, const float* hist, long long hist_stride, const int* cu_seqlens,
-                                                                   const int* seq_slots, int B, int G, int D, int HV, float unit_eps) {
-    extern __shared__ float y[];
-    const int t = blockIdx.x, C = 2 * G * D + HV;
+                                                                   const int* seq_slots, int B, int n, int G, int D, int HV, float unit_eps, int per) {
+    extern __shared__ float y[];                             // [RUN][per]
+    __shared__ TokenRun<RUN> run;
+    const int t = blockIdx.x * RUN, C = 2 * G * D + HV, c0 = blockIdx.y * per, channels = min(per, C - c0), count = min(RUN, n - t);
+    run.find(cu_seqlens, seq_slots, B, n, t);
     pdl_enter();
-    const int b = rs_sequence_of(cu_seqlens, B, t);
-    const int t0 = __ldcg(cu_seqlens + b);
-    const float* st = hist + (size_t)__ldcg(seq_slots + b) * hist_stride;
-    for (int c = threadIdx.x; c < C; c += DI_THREADS) {
-        float acc;
-        if (taps <= 0) {
-            acc = to_f32(__ldcg(proj + (size_t)t * ld + c));
+    for (int i = threadIdx.x; i < channels; i += DI_THREADS) {
+        const int c = c0 + i;
+        // The row `back` before token t + j: of the step, or of the sequence's history, whose row taps - 1 - (t0 - token) counts back from the newest.
+        auto older = [&](int j, int back) {
+            return __ldcg(hist + (size_t)run.slot[j] * hist_stride + (size_t)(taps - 1 - (run.t0[j] - (t + j - back))) * C + c);
+        };
+        if (TAPS > 0) {
+            constexpr int KEEP = TAPS > 0 ? TAPS - 1 : 0;
+            float row[RUN + KEEP], weight[KEEP + 1];
+#pragma unroll
+            for (int k = 0; k < TAPS; ++k) weight[k] = to_f32(conv[(size_t)c * TAPS + k]);
+#pragma unroll
+            for (int j = 0; j < RUN + KEEP; ++j) {
+                const int tj = t + j - KEEP;
+                row[j] = tj >= run.t0[0] && tj < t + count ? to_f32(__ldcg(proj + (size_t)tj * ld + c)) : 0.f;
+            }
+#pragma unroll
+            for (int j = 0; j < RUN; ++j) {
+                if (j >= count) break;
+                float acc = 0.f;
+#pragma unroll
+                for (int k = 0; k < TAPS; ++k) {
+                    const int back = KEEP - k;
+                    acc = fmaf(weight[k], t + j - back >= run.t0[j] ? row[j + k] : older(j, back), acc);
+                }
+                y[j * per + i] = rs_silu(acc);
+            }
         } else {
-            acc = 0.f;
-            for (int j = 0; j < taps; ++j) {
-                const int back = taps - 1 - j, tj = t - back;
-                // Rows before the step's first of this sequence come from the state: its row taps - 1 - (t0 - tj) counts back from the newest.
-                const float x = tj >= t0 ? to_f32(__ldcg(proj + (size_t)tj * ld + c)) : __ldcg(st + (size_t)(taps - 1 - (t0 - tj)) * C + c);
-                acc = fmaf(to_f32(conv[(size_t)c * taps + j]), x, acc);
+            for (int j = 0; j < count; ++j) {
+                float acc = 0.f;
+                if (taps <= 0) acc = to_f32(__ldcg(proj + (size_t)(t + j) * ld + c));
+                for (int k = 0; k < taps; ++k) {
+                    const int back = taps - 1 - k;
+                    const float x = t + j - back >= run.t0[j] ? to_f32(__ldcg(proj + (size_t)(t + j - back) * ld + c)) : older(j, back);
+                    acc = fmaf(to_f32(conv[(size_t)c * taps + k]), x, acc);
+                }
+                y[j * per + i] = rs_silu(acc);
             }
         }
-        y[c] = rs_silu(acc);
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int hd = warp; hd < 2 * G; hd += DI_THREADS / 32) {              // a warp per q or k head
-        float* src = y + (size_t)hd * D;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head0 = c0 / D, heads = max(0, min(2 * G - head0, channels / D));
+    for (int e = warp; e < heads * count; e += DI_THREADS / 32) {              // a warp per q or k head of a token
+        const int hd = head0 + e % heads;
+        float* src = y + (e / heads) * per + (size_t)hd * D - c0;
         float ss = 0.f;
         for (int d = lane; d < D; d += 32) ss = fmaf(src[d], src[d], ss);
         float inv = 1.0f / sqrtf(warp_sum(ss) + unit_eps);
@@ -530,7 +600,8 @@ __global__ void __launch_bounds__(DI_THREADS) delta_inputs_kernel(float* __restr
         for (int d = lane; d < D; d += 32) src[d] *= inv;
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < C; c += DI_THREADS) out[(size_t)t * C + c] = y[c];
+    for (int j = 0; j < count; ++j)
+        for (int i = threadIdx.x; i < channels; i += DI_THREADS) out[(size_t)(t + j) * C + c0 + i] = y[j * per + i];
 }
 
 extern "C" int ti_delta_inputs(float* out, const void* proj, long long ld, const void* conv, int taps, const float* hist, long long hist_stride,
@@ -539,12 +610,20 @@ extern "C" int ti_delta_inputs(float* out, const void* proj, long long ld, const
     if (n == 0) return 0;
     const int C = 2 * G * D + HV;
     TI_REQUIRE(taps >= 0 && taps <= 64 && (taps <= 1 || hist != nullptr) && (taps == 0 || conv != nullptr), "delta_inputs: %d taps", taps);
-    const size_t smem = (size_t)C * sizeof(float);
-    TI_REQUIRE(smem <= 160 * 1024, "delta_inputs: %d channels", C);
+    TI_REQUIRE((size_t)C * sizeof(float) <= 160 * 1024, "delta_inputs: %d channels", C);
+    // Heads' worth of channels a block: about DI_THREADS of them; eight tokens in a row once single ones would be some 20 blocks an SM (4,096
+    // channels, single / eight: 100 tokens 5.7 / 6.8 us, 200 10.5 / 9.8, 2,048 89 / 54; 2,048 channels, 300 tokens 8.0 / 8.9, 600 14.7 / 11.9).
+    const int heads = D >= DI_THREADS ? 1 : DI_THREADS / D, per = heads * D < C ? heads * D : C, parts = (C + per - 1) / per;
+    const bool runs = (long long)n * parts > 20LL * ti_sm_count() && (size_t)8 * per * sizeof(float) <= 48 * 1024;
+    const size_t smem = (size_t)(runs ? 8 : 1) * per * sizeof(float);
     TI_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(delta_inputs_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        ti_launch(delta_inputs_kernel<T>, dim3(n), dim3(DI_THREADS), smem, stream, out, (const T*)proj, ld, (const T*)conv, taps, hist, hist_stride,
-                  cu_seqlens, seq_slots, B, G, D, HV, unit_eps);
+        auto launch = [&](auto kernel) {
+            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            ti_launch(kernel, dim3(runs ? (n + 7) / 8 : n, parts), dim3(DI_THREADS), smem, stream, out, (const T*)proj, ld, (const T*)conv, taps, hist, hist_stride,
+                      cu_seqlens, seq_slots, B, n, G, D, HV, unit_eps, per);
+        };
+        if (taps == 4) { if (runs) launch(delta_inputs_kernel<T, 8, 4>); else launch(delta_inputs_kernel<T, 1, 4>); }
+        else { if (runs) launch(delta_inputs_kernel<T, 8, 0>); else launch(delta_inputs_kernel<T, 1, 0>); }
     });
     return ti_check_launch("delta_inputs");
 }
@@ -644,10 +723,13 @@ __device__ __forceinline__ float pair_value(const T* d, const float* partials, i
     return to_f32(__ldcg(d + at));
 }
 
+// Squares are added as by `sum_threads` threads, element i by thread i modulo it, whatever a block's size is. With no more rows than SMs a block
+// has up to 1,024 threads, so that a row is a round trip or two
+// (4 rows of 2,048, two slices of sums each: 7.5 -> 4.1 us).
 template <typename T>
-__global__ void pair_combine_kernel(float* __restrict__ out, const T* a, const float* pa, int na, size_t sa_stride, const T* b, const float* pb,
+__global__ void __launch_bounds__(1024) pair_combine_kernel(float* __restrict__ out, const T* a, const float* pa, int na, size_t sa_stride, const T* b, const float* pb,
                                     int nb, size_t sb_stride, const T* __restrict__ wa, const T* __restrict__ wb, int normed, float eps,
-                                    float scale_a, float scale_b, int size) {
+                                    float scale_a, float scale_b, int size, int sum_threads) {
     extern __shared__ float rows[];                // [2][size]
     __shared__ float scratch[33];
     pdl_enter();
@@ -660,6 +742,15 @@ __global__ void pair_combine_kernel(float* __restrict__ out, const T* a, const f
     }
     float ia = 1.f, ib = 1.f;
     if (normed) {
+        if (blockDim.x != sum_threads) {
+            __syncthreads();
+            ssa = ssb = 0.f;
+#pragma unroll 4
+            for (int i = threadIdx.x < sum_threads ? threadIdx.x : size; i < size; i += sum_threads) {
+                ssa = fmaf(rows[i], rows[i], ssa);
+                ssb = fmaf(rows[size + i], rows[size + i], ssb);
+            }
+        }
         ia = 1.0f / sqrtf(block_sum(ssa, scratch) / (float)size + eps);
         ib = 1.0f / sqrtf(block_sum(ssb, scratch) / (float)size + eps);
     }
@@ -679,8 +770,10 @@ extern "C" int ti_pair_combine(float* out, const void* a, const float* pa, int n
     TI_REQUIRE(smem <= 160 * 1024, "pair_combine: rows of %d", size);
     TI_DISPATCH_DTYPE(dtype, {
         if (smem > 48 * 1024) cudaFuncSetAttribute(pair_combine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        ti_launch(pair_combine_kernel<T>, dim3(n), dim3(size >= 1024 ? 256 : 128), smem, stream, out, (const T*)a, pa, na, (size_t)sa_stride, (const T*)b,
-                  pb, nb, (size_t)sb_stride, (const T*)wa, (const T*)wb, normed, eps, scale_a, scale_b, size);
+        const int sum_threads = size >= 1024 ? 256 : 128, all = size > 1024 ? 1024 : (size + 31) / 32 * 32;
+        const int threads = n <= ti_sm_count() && all > sum_threads ? all : sum_threads;
+        ti_launch(pair_combine_kernel<T>, dim3(n), dim3(threads), smem, stream, out, (const T*)a, pa, na, (size_t)sa_stride, (const T*)b,
+                  pb, nb, (size_t)sb_stride, (const T*)wa, (const T*)wb, normed, eps, scale_a, scale_b, size, sum_threads);
     });
     return ti_check_launch("pair_combine");
 }
