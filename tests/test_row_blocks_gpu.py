@@ -1,5 +1,5 @@
-"""Row kernels whose blocks depend on how many rows a step has: a row's bits do not depend on the step it is in. Their distance to
-64-bit arithmetic is measured where the kernels are tested alone (test_fasodra_gpu.py)."""
+"""Row kernels whose blocks depend on how many rows a step has, and the recurrences' scans beside their one-token kernels: a row's bits do not
+depend on the step it is in. Their distance to 64-bit arithmetic is measured where the kernels are tested alone (test_fasodra_gpu.py)."""
 from types import SimpleNamespace
 
 import pytest
@@ -114,3 +114,42 @@ def test_delta_inputs_in_runs_of_tokens(ops, taps, G, D, HV):
         # Sums of up to 7 products, an exponential, and sums over a head.
         assert float((whole[at:at + length].double() - want).abs().max()) <= 2.0 ** -24 * 64 * max(1.0, float(y.abs().max()))
         at += length
+
+
+@pytest.mark.parametrize("H,D", [(3, 5), (2, 33), (32, 64), (1, 64), (5, 100), (2, 129), (1, 256)])
+def test_scans_have_the_bits_of_single_tokens(ops, H, D):
+    """Batches of tokens, a batch's remainder and tokens one by one: the same bits, for every number of row groups and blocks of all sizes."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    R = lambda *s: torch.randn(*s, generator=g, device="cuda")                                     # noqa: E731
+    lengths, G, V = [37, 16, 1, 30], H, D + 3
+    n = sum(lengths)
+    rkv, dlog, w0, u = R(n, 3 * H * D).bfloat16(), R(n, H * D), R(H * D) - 2, R(H * D)
+    C = 2 * G * D + H * V
+    wide = torch.zeros(n, (C + 3) // 4 * 4 + 4, device="cuda")
+    wide[:, :C] = R(n, C) * D ** -0.5
+    qkv = wide[:, :C].contiguous()
+    ba, a_log, dt = R(n, 2 * H), R(H) * 0.5, R(H) - 1
+
+    def run(portions):
+        s1, s2 = torch.zeros(4, H * D * D, device="cuda"), torch.zeros(4, H * D * V, device="cuda")
+        o1, o2 = torch.empty(n, H * D, device="cuda"), torch.empty(n, H * V, device="cuda")
+        fed = [0] * 4
+        starts = [sum(lengths[:b]) for b in range(4)]
+        for p in portions:
+            live = [b for b in range(4) if fed[b] < lengths[b]]
+            if not live:
+                break
+            take = [min(p, lengths[b] - fed[b]) for b in live]
+            rows = torch.cat([torch.arange(starts[b] + fed[b], starts[b] + fed[b] + m) for b, m in zip(live, take)]).cuda()
+            a, c = torch.empty(len(rows), H * D, device="cuda"), torch.empty(len(rows), H * V, device="cuda")
+            ops.decay_scan(a, rkv[rows].contiguous(), 0, H * D, 2 * H * D, dlog[rows].contiguous(), w0, u, s1, _step(take, live), H, D)
+            ops.delta_scan(c, qkv[rows].contiguous(), ba[rows].contiguous(), a_log, dt, s2, _step(take, live), H, G, D, V)
+            o1[rows], o2[rows] = a, c
+            for b, m in zip(live, take):
+                fed[b] += m
+        return o1, o2, s1, s2
+
+    whole = run([100])
+    for portions in ([17] * 4, [1] * 40):
+        for got, want in zip(run(portions), whole):
+            assert torch.equal(got, want)

@@ -65,6 +65,18 @@ inline cudaError_t ti_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Launch in plain stream order. For a kernel of few long blocks: those that come up beside the last blocks of the kernel before go where there is
+// room first, several to an SM that has just been left, and stay there.
+template <typename... KArgs, typename... Args>
+inline cudaError_t ti_launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 #define TI_REQUIRE(cond, ...)                \
     do {                                     \
         if (!(cond)) return ti_fail(__VA_ARGS__); \

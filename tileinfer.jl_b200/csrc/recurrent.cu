@@ -6,16 +6,18 @@
 //       S <- g_t S ;  e = beta_t (v_t - S^T k_t) ;  S <- S + k_t e^T ;  o_t = S^T q_t
 //       beta_t = sigmoid(b_t),  g_t = exp(-exp(A_log) * softplus(a_t + dt_bias))
 //
-// S is [dim][vdim] (key rows, value columns). A block owns 32 value columns of one (sequence, head): lane = column, warp w owns
-// the key rows 16 w .. 16 w + 15, sixteen state values per thread in registers. A step's tokens are walked in order from the
-// state that earlier steps left, in batches of RS_BATCH tokens staged in shared memory (activations, decays and gates are
-// computed while staging, in 32-bit); the partial sums of the warps are added in warp order, so a result depends on the
-// token's place in its sequence alone, not on the batch or on how the prompt was cut.
-#include "common.cuh"
+// S is [dim][vdim] (key rows, value columns). A warp owns CB value columns of one (sequence, head) with all their key rows: G = 32 / CB groups
+// of R rows a column, a lane has the rows of one group in registers (G is the least power of two that holds the key size). What a token
+// reads out of the state is added up over a column's groups by shuffles, so the warps of a block share nothing but the staged inputs.
+// A step's tokens are walked in order from the state that earlier steps left, in batches of RS_BATCH tokens staged in shared memory. The
+// sums over the groups have one order (partners G / 2, ..., 2, 1 apart), in the one-token kernels too, so a result depends on the token's
+// place in its sequence alone, not on the batch or on how the prompt was cut.
+#include "mma_util.cuh"
+#include "packed_f32.cuh"
 
-#define RS_ROWS 16
+#define RS_ROWS 16                 // key rows of a lane of the delta scan
 #define RS_BATCH 16
-#define RS_MAX_WARPS 16           // key sizes up to 256
+#define RS_MAX_KEY 256
 
 __device__ __forceinline__ float rs_silu(float z) { return z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float rs_softplus(float z) { return z > 20.f ? z : log1pf(expf(z)); }
@@ -43,141 +45,221 @@ template <int RUN> struct TokenRun {
     }
 };
 
+// ------------------------------------------------------------------------------------------------ what both scans share
+// The launch of a scan: G groups of R rows hold a key of D elements; a block has `warps` warps of 32 / G columns.
+struct ScanShape { int groups, warps; };
+// Blocks of `most` warps share the staged rows of a head; where so few leave most SMs idle, smaller ones (a token's time is its warp's own
+// chain, and staging takes a small part of it).
+static ScanShape scan_shape(int rows, int D, int cols, long long heads, int most, int least) {
+    ScanShape s = {1, most};
+    while (s.groups * rows < D) s.groups *= 2;
+    auto blocks = [&] { const int per = s.warps * (32 / s.groups); return (cols + per - 1) / per * heads; };
+    while (s.warps > least && 2 * blocks() < ti_sm_count()) s.warps /= 2;
+    return s;
+}
+template <int G> __device__ __forceinline__ float groups_sum(float v) {      // lanes of a column are 32 / G apart
+#pragma unroll
+    for (int m = 16; m >= 32 / G; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    return v;
+}
+// The same sum of G values that lie `stride` apart.
+template <int G> __device__ __forceinline__ float groups_sum(const float* from, int stride) {
+    float v[G];
+#pragma unroll
+    for (int i = 0; i < G; ++i) v[i] = from[i * stride];
+#pragma unroll
+    for (int m = G / 2; m >= 1; m >>= 1)
+#pragma unroll
+        for (int i = 0; i < m; ++i) v[i] += v[i + m];
+    return v[0];
+}
+// A staged row: a group's rows lie four floats further apart than they are many, so that a warp's 16-byte reads fall into different banks.
+template <int R> __device__ __forceinline__ int staged_at(int d) { return d + d / R * 4; }
+template <int R> __device__ __forceinline__ void read_rows(f32x2 (&to)[R / 2], const float* from) {
+#pragma unroll
+    for (int r = 0; r < R; r += 4) {
+        const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(from + r);
+        to[r / 2] = t.x; to[r / 2 + 1] = t.y;
+    }
+}
+template <int R> __device__ __forceinline__ void load_state(f32x2 (&s)[R / 2], const float* S, int row0, int col, int D, int V) {
+#pragma unroll
+    for (int r = 0; r < R; r += 2)
+        s[r / 2] = pack2(row0 + r < D && col < V ? __ldcg(S + (size_t)(row0 + r) * V + col) : 0.f,
+                         row0 + r + 1 < D && col < V ? __ldcg(S + (size_t)(row0 + r + 1) * V + col) : 0.f);
+}
+template <int R> __device__ __forceinline__ void store_state(float* S, const f32x2 (&s)[R / 2], int row0, int col, int D, int V) {
+#pragma unroll
+    for (int r = 0; r < R; r += 2) {
+        float lo, hi;
+        unpack2(s[r / 2], lo, hi);
+        if (row0 + r < D && col < V) S[(size_t)(row0 + r) * V + col] = lo;
+        if (row0 + r + 1 < D && col < V) S[(size_t)(row0 + r + 1) * V + col] = hi;
+    }
+}
+__device__ __forceinline__ float rows_sum(f32x2 a, f32x2 b) {
+    float p0, p1, p2, p3;
+    unpack2(a, p0, p1);
+    unpack2(b, p2, p3);
+    return (p0 + p1) + (p2 + p3);
+}
+// A load that stays where it is written (the compiler would move it down to its use, past the work that hides its latency).
+__device__ __forceinline__ float load_now(const float* p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ bf16 load_now(const bf16* p) {
+    unsigned short v;
+    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return __ushort_as_bfloat16(v);
+}
+__device__ __forceinline__ void copy4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src));
+}
+
 // ------------------------------------------------------------------------------------------------ decay scan
 // rkv [n][ld] of T: r at r_off, k at k_off, v at v_off, heads of `D` side by side; dlog [n][H * D] float: the decay's logit
 // before w0 [H * D] is added; u [H * D] float; state rows `state_stride` floats apart, a head's matrix at h * D * D.
-// R key rows per thread (8 up to key size 128, so that a token's chain of dependent operations is short; 16 beyond). The next
-// batch's rows are fetched into registers before this batch is worked on and laid into the other half of the staging buffers
-// after it, so their latency hides behind the recurrence; one barrier per batch.
-template <typename T, int R, int CB>
-__global__ void decay_scan_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
+// The next batch's rows are fetched into registers before this batch is worked on and laid into the other half of the staging buffers
+// after it, so their latency hides behind the recurrence; one barrier per batch. A thread stages one channel of tokens STEP apart.
+// What bounds it: instructions issued, a warp or two per scheduler, a third of them staging. The lanes' sums of a token meet in shared memory once
+// per batch. A prompt of 1,500 tokens (with 333, 64 and 7 beside it), 32 heads of 64, inside the step: 423 -> 309 us, against blocks of 32 columns
+// whose warps shared a column's rows; 2,048 tokens alone 405 -> 313, 8 heads 800 -> 392.
+template <typename T, int R, int G, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
                                   const float* __restrict__ w0, const float* __restrict__ u, float* state, long long state_stride,
                                   const int* cu_seqlens, const int* seq_slots, int H, int D) {
     extern __shared__ __align__(16) float sm[];
-    constexpr int SUBS = 32 / CB;                 // a warp's lanes: CB columns x SUBS groups of R rows
-    constexpr int PER = RS_BATCH * R * SUBS / 32; // staged elements of r, k, w per thread and batch: RS_BATCH * Dp / threads
-    constexpr int PV = (RS_BATCH * CB + 127) / 128;
-    const int warps = blockDim.x >> 5, Dp = warps * R * SUBS, threads = blockDim.x;
-    float* sr = sm;                               // [2][RS_BATCH][Dp]
-    float* sk = sr + 2 * RS_BATCH * Dp;
-    float* sw = sk + 2 * RS_BATCH * Dp;
-    float* sv = sw + 2 * RS_BATCH * Dp;           // [2][RS_BATCH][CB]
-    float* red = sv + 2 * RS_BATCH * CB;          // [2][RS_BATCH][warps][CB]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = lane % CB, sub = lane / CB;
-    const int col0 = blockIdx.x * CB, col = col0 + cl, h = blockIdx.y, b = blockIdx.z;
-    const int row0 = (warp * SUBS + sub) * R;
-    const bool early_v = threads >= 128;          // enough threads to fetch a batch's values ahead in PV registers each
-    pdl_enter();
+    constexpr int CB = 32 / G, Dp = R * G, ROW = G * (R + 4), THREADS = 32 * WARPS, COLS = WARPS * CB;
+    constexpr int CHANNELS = Dp < THREADS ? Dp : THREADS, STEP = THREADS / CHANNELS;       // threads of a row, rows at a time
+    constexpr int PER = RS_BATCH / STEP, PASSES = Dp / CHANNELS;                           // rows of a thread's channel, channels of a thread
+    constexpr int PV = (RS_BATCH * COLS + THREADS - 1) / THREADS;
+    float* sr = sm;                               // [2][RS_BATCH][ROW]
+    float* sk = sr + 2 * RS_BATCH * ROW;
+    float* sw = sk + 2 * RS_BATCH * ROW;
+    float* sv = sw + 2 * RS_BATCH * ROW;          // [2][RS_BATCH][COLS]
+    float* so = sv + 2 * RS_BATCH * COLS;         // [WARPS][RS_BATCH][32]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = warp * CB + lane % CB, sub = lane / CB;
+    const int col0 = blockIdx.x * COLS, col = col0 + cl, h = blockIdx.y, b = blockIdx.z, row0 = sub * R;
     const int t0 = __ldcg(cu_seqlens + b), t1 = __ldcg(cu_seqlens + b + 1);
     float* S = state + (size_t)__ldcg(seq_slots + b) * state_stride + (size_t)h * D * D;
-    float s[R], bonus[R];
+    const int ch = threadIdx.x % CHANNELS, i0 = threadIdx.x / CHANNELS;
+    float shift[PASSES];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const bool in = row0 + r < D && col < D;
-        s[r] = in ? __ldcg(S + (size_t)(row0 + r) * D + col) : 0.f;
-        bonus[r] = row0 + r < D ? u[h * D + row0 + r] : 0.f;
-    }
+    for (int q = 0; q < PASSES; ++q) shift[q] = ch + q * CHANNELS < D ? w0[h * D + ch + q * CHANNELS] : 0.f;
+    f32x2 bonus[R / 2];
+#pragma unroll
+    for (int r = 0; r < R; r += 2)
+        bonus[r / 2] = pack2(row0 + r < D ? u[h * D + row0 + r] : 0.f, row0 + r + 1 < D ? u[h * D + row0 + r + 1] : 0.f);
+    pdl_enter();
+    f32x2 s[R / 2];
+    load_state<R>(s, S, row0, col, D, D);
     // Fetched values stay as they were loaded (no conversion, no branch): a use right behind a load would make the warp wait for it,
     // one round trip to memory per load instead of one per batch. Rows outside the batch or the head read a valid address and
     // are zeroed when they are laid into shared memory.
     T fr[PER], fk[PER], fv[PV];
     float fd[PER];
-    auto fetch = [&](int base, int count) {
+    auto fetch = [&](int base, int count, int q) {
+        const int d = min(ch + q * CHANNELS, D - 1);
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            const int e = threadIdx.x + j * threads, i = e / Dp, d = e - i * Dp;
-            const bool in = i < count && d < D;
-            const size_t at = in ? (size_t)(base + i) * ld + h * D + d : 0;
-            fr[j] = __ldcg(rkv + at + r_off);
-            fk[j] = __ldcg(rkv + at + k_off);
-            fd[j] = __ldcg(dlog + (in ? (size_t)(base + i) * H * D + h * D + d : 0));
-        }
-        if (early_v) {
-#pragma unroll
-            for (int j = 0; j < PV; ++j) {
-                const int e = threadIdx.x + j * threads, i = e / CB, c = col0 + e % CB;
-                const bool in = e < RS_BATCH * CB && i < count && c < D;
-                fv[j] = __ldcg(rkv + (in ? (size_t)(base + i) * ld + v_off + h * D + c : 0));
-            }
+            const size_t t = base + min(i0 + j * STEP, count - 1);
+            fr[j] = load_now(rkv + t * ld + (r_off + h * D + d));
+            fk[j] = load_now(rkv + t * ld + (k_off + h * D + d));
+            fd[j] = load_now(dlog + t * (H * D) + (h * D + d));
         }
     };
-    auto stash = [&](int buf, int base, int count) {
+    auto stash = [&](int buf, int count, int q) {
+        const bool in_head = ch + q * CHANNELS < D;
+        const int to = buf * RS_BATCH * ROW + i0 * ROW + staged_at<R>(ch + q * CHANNELS);
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            const int e = threadIdx.x + j * threads, i = e / Dp, d = e - i * Dp;
-            const bool in = i < count && d < D;
-            sr[buf * RS_BATCH * Dp + e] = in ? to_f32(fr[j]) : 0.f;
-            sk[buf * RS_BATCH * Dp + e] = in ? to_f32(fk[j]) : 0.f;
-            sw[buf * RS_BATCH * Dp + e] = in ? expf(-expf(fd[j] + w0[h * D + d])) : 1.f;
+            const bool in = in_head && i0 + j * STEP < count;
+            sr[to + j * STEP * ROW] = in ? to_f32(fr[j]) : 0.f;
+            sk[to + j * STEP * ROW] = in ? to_f32(fk[j]) : 0.f;
+            sw[to + j * STEP * ROW] = in ? expf(-expf(fd[j] + shift[q])) : 1.f;
         }
-        if (early_v) {
+    };
+    auto fetch_values = [&](int base, int count) {
 #pragma unroll
-            for (int j = 0; j < PV; ++j) {
-                const int e = threadIdx.x + j * threads, i = e / CB, c = col0 + e % CB;
-                if (e < RS_BATCH * CB) sv[buf * RS_BATCH * CB + e] = (i < count && c < D) ? to_f32(fv[j]) : 0.f;
-            }
-        } else {                                  // a block of few threads (a small key size) reads its values late
-            for (int e = threadIdx.x; e < RS_BATCH * CB; e += threads) {
-                const int i = e / CB, c = col0 + e % CB;
-                sv[buf * RS_BATCH * CB + e] = (i < count && c < D) ? to_f32(__ldcg(rkv + (size_t)(base + i) * ld + v_off + h * D + c)) : 0.f;
-            }
+        for (int j = 0; j < PV; ++j) {
+            const int e = threadIdx.x + j * THREADS, i = e / COLS, c = col0 + e % COLS;
+            fv[j] = load_now(rkv + (size_t)(base + min(i, count - 1)) * ld + (v_off + h * D + min(c, D - 1)));
+        }
+    };
+    auto stash_values = [&](int buf, int count) {
+#pragma unroll
+        for (int j = 0; j < PV; ++j) {
+            const int e = threadIdx.x + j * THREADS, i = e / COLS, c = col0 + e % COLS;
+            if (e < RS_BATCH * COLS) sv[buf * RS_BATCH * COLS + e] = i < count && c < D ? to_f32(fv[j]) : 0.f;
+        }
+    };
+    auto rest = [&](int buf, int base, int count) {      // the channels that a thread has beyond its first
+#pragma unroll
+        for (int q = 1; q < PASSES; ++q) {
+            fetch(base, count, q);
+            stash(buf, count, q);
         }
     };
     if (t0 < t1) {
-        fetch(t0, min(RS_BATCH, t1 - t0));
-        stash(0, t0, min(RS_BATCH, t1 - t0));
+        const int count = min(RS_BATCH, t1 - t0);
+        fetch(t0, count, 0);
+        fetch_values(t0, count);
+        stash(0, count, 0);
+        stash_values(0, count);
+        rest(0, t0, count);
     }
     __syncthreads();
-    int it = 0;
-    for (int base = t0; base < t1; base += RS_BATCH, ++it) {
-        const int count = min(RS_BATCH, t1 - base), buf = it & 1;
-        const int next = base + RS_BATCH, next_count = min(RS_BATCH, t1 - next);
-        if (next < t1) fetch(next, next_count);
-        float* my_red = red + (size_t)buf * RS_BATCH * warps * CB;
-        for (int i = 0; i < count; ++i) {
-            const float v = sv[(buf * RS_BATCH + i) * CB + cl];
-            const float4* pr = reinterpret_cast<const float4*>(sr + (buf * RS_BATCH + i) * Dp + row0);
-            const float4* pk = reinterpret_cast<const float4*>(sk + (buf * RS_BATCH + i) * Dp + row0);
-            const float4* pw = reinterpret_cast<const float4*>(sw + (buf * RS_BATCH + i) * Dp + row0);
-            float part[4] = {0.f, 0.f, 0.f, 0.f};
+    int buf = 0;
+    float* mine = so + warp * RS_BATCH * 32;
+    for (int base = t0; base < t1; base += RS_BATCH, buf ^= 1) {
+        const int count = min(RS_BATCH, t1 - base), next = base + RS_BATCH, next_count = min(RS_BATCH, t1 - next);
+        if (next < t1) {
+            fetch(next, next_count, 0);
+            fetch_values(next, next_count);
+        }
+        // Whole batches (tokens beyond the last leave the state as it is: k = 0, v = 0, w = 1), several tokens' reads in flight: a token
+        // waits for the one before only in the state, one multiply-add an element.
+#pragma unroll 4
+        for (int i = 0; i < RS_BATCH; ++i) {
+            const int at = (buf * RS_BATCH + i) * ROW + sub * (R + 4);
+            const float v = sv[(buf * RS_BATCH + i) * COLS + cl];
+            f32x2 rr[R / 2], kk[R / 2], ww[R / 2], part[2] = {0ull, 0ull};
+            read_rows<R>(rr, sr + at);
+            read_rows<R>(kk, sk + at);
+            read_rows<R>(ww, sw + at);
+            const f32x2 v2 = pack2(v, v);
 #pragma unroll
-            for (int q = 0; q < R / 4; ++q) {
-                const float4 r4 = pr[q], k4 = pk[q], w4 = pw[q];
-                const float rr[4] = {r4.x, r4.y, r4.z, r4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w}, ww[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    const float kv = kk[c] * v;
-                    part[c] = fmaf(fmaf(bonus[4 * q + c], kv, s[4 * q + c]), rr[c], part[c]);
-                    s[4 * q + c] = fmaf(ww[c], s[4 * q + c], kv);
-                }
+            for (int r = 0; r < R / 2; ++r) {
+                const f32x2 kv = mul2(kk[r], v2);
+                part[r & 1] = fma2(fma2(bonus[r], kv, s[r]), rr[r], part[r & 1]);
+                s[r] = fma2(ww[r], s[r], kv);
             }
-            float total = (part[0] + part[1]) + (part[2] + part[3]);
-#pragma unroll
-            for (int m = CB; m < 32; m <<= 1) total += __shfl_xor_sync(0xffffffffu, total, m);      // the row groups of a column
-            if (sub == 0) my_red[(i * warps + warp) * CB + cl] = total;
+            mine[i * 32 + lane] = rows_sum(part[0], part[1]);
         }
-        if (next < t1) stash(buf ^ 1, next, next_count);
+        __syncwarp();
+        for (int e = lane; e < count * CB; e += 32) {         // a warp's own columns leave once per batch
+            const int i = e / CB, c = e % CB, to = col0 + warp * CB + c;
+            if (to < D) o[(size_t)(base + i) * H * D + h * D + to] = groups_sum<G>(mine + i * 32 + c, CB);
+        }
+        if (next < t1) {
+            stash(buf ^ 1, next_count, 0);
+            stash_values(buf ^ 1, next_count);
+            rest(buf ^ 1, next, next_count);
+        }
         __syncthreads();
-        for (int e = threadIdx.x; e < count * CB; e += threads) {
-            const int i = e / CB, c = col0 + e % CB;
-            float total = 0.f;
-            for (int w = 0; w < warps; ++w) total += my_red[(i * warps + w) * CB + e % CB];
-            if (c < D) o[(size_t)(base + i) * H * D + h * D + c] = total;
-        }
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-        if (row0 + r < D && col < D) S[(size_t)(row0 + r) * D + col] = s[r];
+    store_state<R>(S, s, row0, col, D, D);
 }
 
-// One token per sequence (a decode step): no staging; a thread reads its rows' r, k and decay logits itself (the lanes of a warp
-// read the same addresses), the warps' partial sums meet in a small array. The sums are added in the same order as in the scan.
-template <typename T, int R>
+// One token per sequence (a decode step): no staging; a warp has one group of rows of 32 columns, its lanes read the same r, k and decay
+// logits; the groups' sums meet in a small array and are added in the scan's order.
+template <typename T, int R, int G>
 __global__ void decay_token_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
                                    const float* __restrict__ w0, const float* __restrict__ u, float* state, long long state_stride,
                                    const int* seq_slots, int H, int D) {
-    __shared__ float red[RS_MAX_WARPS * 2 * 32];
-    const int warps = blockDim.x >> 5;
+    __shared__ float red[G * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int col = blockIdx.x * 32 + lane, h = blockIdx.y, t = blockIdx.z;
     const int row0 = warp * R;
@@ -210,196 +292,183 @@ __global__ void decay_token_kernel(float* __restrict__ o, const T* rkv, long lon
     for (int r = 0; r < R; ++r)
         if (row0 + r < D && col < D) S[(size_t)(row0 + r) * D + col] = s[r];
     __syncthreads();
-    if (warp == 0 && col < D) {
-        float total = 0.f;
-        for (int w = 0; w < warps; ++w) total += red[w * 32 + lane];
-        o[(size_t)t * H * D + h * D + col] = total;
-    }
+    if (warp == 0 && col < D) o[(size_t)t * H * D + h * D + col] = groups_sum<G>(red + lane, 32);
 }
 
-template <typename T, int R, int CB>
+template <typename T, int R, int G>
 static void launch_decay_scan(float* o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog, const float* w0, const float* u,
                               float* state, long long state_stride, const int* cu_seqlens, const int* seq_slots, int B, int H, int D, bool one_token,
-                              cudaStream_t stream) {
+                              int warps, cudaStream_t stream) {
     if (one_token) {
-        ti_launch(decay_token_kernel<T, R>, dim3((D + 31) / 32, H, B), dim3((D + R - 1) / R * 32), 0, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u, state,
+        ti_launch(decay_token_kernel<T, R, G>, dim3((D + 31) / 32, H, B), dim3(G * 32), 0, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u, state,
                   state_stride, seq_slots, H, D);
         return;
     }
-    constexpr int RW = R * (32 / CB);             // key rows of a warp
-    const int warps = (D + RW - 1) / RW;
-    const size_t smem = (size_t)(2 * 3 * RS_BATCH * warps * RW + 2 * RS_BATCH * CB + 2 * RS_BATCH * warps * CB) * sizeof(float);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(decay_scan_kernel<T, R, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ti_launch(decay_scan_kernel<T, R, CB>, dim3((D + CB - 1) / CB, H, B), dim3(warps * 32), smem, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u, state,
-              state_stride, cu_seqlens, seq_slots, H, D);
+    const int cols = warps * (32 / G);
+    const size_t smem = (size_t)(2 * 3 * RS_BATCH * G * (R + 4) + 2 * RS_BATCH * cols + RS_BATCH * warps * 32) * sizeof(float);
+    auto launch = [&](auto kernel) {
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        ti_launch_after(kernel, dim3((D + cols - 1) / cols, H, B), dim3(warps * 32), smem, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u, state, state_stride,
+                  cu_seqlens, seq_slots, H, D);
+    };
+    if (warps >= 4) launch(decay_scan_kernel<T, R, G, 4>);
+    else launch(decay_scan_kernel<T, R, G, 2>);
 }
 
 extern "C" int ti_decay_scan(float* o, const void* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog, const float* w0,
                              const float* u, float* state, long long state_stride, const int* cu_seqlens, const int* seq_slots, int n, int B,
                              int H, int D, int dtype, cudaStream_t stream) {
     if (n == 0 || B == 0) return 0;
-    TI_REQUIRE(D > 0 && D <= RS_MAX_WARPS * RS_ROWS && H > 0, "decay_scan: %d heads of %d (at most %d)", H, D, RS_MAX_WARPS * RS_ROWS);
-    // Very few (sequence, head) pairs: blocks of 16 or 8 columns, so that more SMs have one (the state's rows of a column are then
-    // shared out among the lanes of a warp as well as among the warps). Every block stages all key rows of its head, so narrower
-    // blocks multiply that work: with 64 blocks of 32 columns already (32 heads of 64, one prompt of 2,048 tokens) blocks of 16
-    // columns were slower (551 against 465 us), hence only below a quarter of the SMs.
-    const long long blocks32 = (long long)((D + 31) / 32) * H * B;
-    const int sms = ti_sm_count();
-#define RS_DECAY(R, CB) launch_decay_scan<T, R, CB>(o, (const T*)rkv, ld, r_off, k_off, v_off, dlog, w0, u, state, state_stride, cu_seqlens, seq_slots, B, H, D, n == B, stream)
+    TI_REQUIRE(D > 0 && D <= RS_MAX_KEY && H > 0, "decay_scan: %d heads of %d (at most %d)", H, D, RS_MAX_KEY);
+    // 8 rows a lane up to key size 128 (more warps for the same work), 16 beyond.
+    const ScanShape shape = scan_shape(D <= 128 ? 8 : 16, D, D, (long long)H * B, 4, 2);
+#define RS_DECAY(R, G) launch_decay_scan<T, R, G>(o, (const T*)rkv, ld, r_off, k_off, v_off, dlog, w0, u, state, state_stride, cu_seqlens, seq_slots, B, H, D, n == B, shape.warps, stream)
     TI_DISPATCH_DTYPE(dtype, {
-        if (D > 128) RS_DECAY(16, 32);
-        else if (n == B || blocks32 * 4 >= sms) RS_DECAY(8, 32);
-        else if (blocks32 * 8 >= sms) RS_DECAY(8, 16);
-        else RS_DECAY(8, 8);
+        if (D <= 128) {
+            if (shape.groups == 1) RS_DECAY(8, 1);
+            else if (shape.groups == 2) RS_DECAY(8, 2);
+            else if (shape.groups == 4) RS_DECAY(8, 4);
+            else if (shape.groups == 8) RS_DECAY(8, 8);
+            else RS_DECAY(8, 16);
+        } else RS_DECAY(16, 16);
     });
 #undef RS_DECAY
     return ti_check_launch("decay_scan");
 }
 
 // ------------------------------------------------------------------------------------------------ delta scan
-// qkv [n][ld] float: q heads (G of D) at 0, k heads (G of D) at G * D, v heads (H of V) at 2 G D, already activated and
-// normalised; ba [n][2 H] float: the logits of beta, then of the decay; head h reads q/k head h / (H / G). Sixteen key rows per
-// thread; what a token reads out of the state before it writes (S^T k) is summed over the warps through shared memory, one barrier
-// per token; the next batch's rows are fetched into registers while this batch is worked on.
-template <int CB>
-__global__ void delta_scan_kernel(float* __restrict__ o, const float* qkv, long long ld, const float* ba, const float* __restrict__ a_log,
+// qkv [n][ld] float: q heads (GQ of D) at 0, k heads (GQ of D) at GQ * D, v heads (H of V) at 2 GQ D, already activated and
+// normalised; ba [n][2 H] float: the logits of beta, then of the decay; head h reads q/k head h / (H / GQ). The next batch's rows are
+// on their way (cp.async, 16 bytes where `vec` says that all rows allow it) while this batch is worked on; one barrier per batch.
+// What bounds it: one token's chain, decay, products with k, their sum over the lanes of a column, the write. So the next token's k is read
+// ahead, the products with q are off the chain, and pairs of rows share an instruction. A prompt of 1,500 tokens
+// (with 333, 64 and 7 beside it), 16 heads of 128 x 128, inside the step: 965 -> 412 us, against blocks of 32 columns whose warps shared a column's rows
+// and met at a barrier per token; 2,048 tokens alone 972 -> 436, 4 heads 1,407 -> 451.
+template <int G>
+__global__ void __launch_bounds__(128) delta_scan_kernel(float* __restrict__ o, const float* qkv, long long ld, const float* ba, const float* __restrict__ a_log,
                                   const float* __restrict__ dt_bias, float* state, long long state_stride, const int* cu_seqlens,
-                                  const int* seq_slots, int H, int G, int D, int V) {
+                                  const int* seq_slots, int H, int GQ, int D, int V, int vec) {
     extern __shared__ __align__(16) float sm[];
-    constexpr int R = RS_ROWS, SUBS = 32 / CB;    // a warp's lanes: CB columns x SUBS groups of R rows
-    constexpr int PER = RS_BATCH * R * SUBS / 32, PV = RS_BATCH * CB / 32;
-    const int warps = blockDim.x >> 5, Dp = warps * R * SUBS, threads = blockDim.x;
-    float* sq = sm;                               // [2][RS_BATCH][Dp]
-    float* sk = sq + 2 * RS_BATCH * Dp;
-    float* sv = sk + 2 * RS_BATCH * Dp;           // [2][RS_BATCH][CB]
-    float* sg = sv + 2 * RS_BATCH * CB;           // [2][RS_BATCH][2]: decay, beta
-    float* red = sg + 2 * RS_BATCH * 2;           // [2][warps][CB]
-    float* red_o = red + 2 * warps * CB;          // [2][RS_BATCH][warps][CB]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = lane % CB, sub = lane / CB;
-    const int col0 = blockIdx.x * CB, col = col0 + cl, h = blockIdx.y, b = blockIdx.z;
-    const int g = h / (H / G), row0 = (warp * SUBS + sub) * R;
-    pdl_enter();
+    constexpr int R = RS_ROWS, CB = 32 / G, ROW = G * (R + 4);
+    const int threads = blockDim.x, cols = (threads >> 5) * CB;
+    float* sq = sm;                               // [2][RS_BATCH][ROW]
+    float* sk = sq + 2 * RS_BATCH * ROW;
+    float* sv = sk + 2 * RS_BATCH * ROW;          // [2][RS_BATCH][cols]
+    float* sg = sv + 2 * RS_BATCH * cols;         // [2][RS_BATCH][2]: decay, beta
+    float* so = sg + 2 * RS_BATCH * 2;            // [warps][RS_BATCH][32]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = warp * CB + lane % CB, sub = lane / CB;
+    const int col0 = blockIdx.x * cols, col = col0 + cl, h = blockIdx.y, b = blockIdx.z;
+    const int g = h / (H / GQ), row0 = sub * R;
     const int t0 = __ldcg(cu_seqlens + b), t1 = __ldcg(cu_seqlens + b + 1);
     float* S = state + (size_t)__ldcg(seq_slots + b) * state_stride + (size_t)h * D * V;
     const float rate = expf(a_log[h]), shift = dt_bias[h];
-    float s[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) s[r] = (row0 + r < D && col < V) ? __ldcg(S + (size_t)(row0 + r) * V + col) : 0.f;
-    float fq[PER], fk[PER], fv[PV], fg[2];
-    auto fetch = [&](int base, int count) {
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int e = threadIdx.x + j * threads, i = e / Dp, d = e - i * Dp;
-            fq[j] = 0.f; fk[j] = 0.f;
-            if (i < count && d < D) {
-                const float* row = qkv + (size_t)(base + i) * ld + g * D + d;
-                fq[j] = __ldcg(row);
-                fk[j] = __ldcg(row + G * D);
+    // 16-byte pieces: a thread has one column of rows `vec_rows` apart (threads beyond whole rows have none).
+    const int pieces = max(1, D >> 2), vec_rows = threads / pieces, vec_col = (int)threadIdx.x % pieces * 4;
+    const int vec_row = (int)threadIdx.x < vec_rows * pieces ? (int)threadIdx.x / pieces : RS_BATCH;
+    for (int e = threadIdx.x; e < 4 * RS_BATCH * ROW + 2 * RS_BATCH * cols; e += threads) sm[e] = 0.f;      // what lies beyond the last key or column stays zero
+    __syncthreads();
+    pdl_enter();
+    f32x2 s[R / 2];
+    load_state<R>(s, S, row0, col, D, V);
+    float fg[2] = {0.f, 0.f};
+    auto fetch = [&](int buf, int base, int count) {
+        const float* from = qkv + (size_t)base * ld + g * D;
+        if (vec) {
+            for (int i = vec_row; i < count; i += vec_rows) {
+                const int to = (buf * RS_BATCH + i) * ROW + staged_at<R>(vec_col);
+                cp_async16(smem_u32(sq + to), from + (size_t)i * ld + vec_col);
+                cp_async16(smem_u32(sk + to), from + (size_t)i * ld + GQ * D + vec_col);
+            }
+        } else {
+            for (int e = threadIdx.x; e < count * D; e += threads) {
+                const int i = e / D, d = e - i * D, to = (buf * RS_BATCH + i) * ROW + staged_at<R>(d);
+                copy4(sq + to, from + (size_t)i * ld + d);
+                copy4(sk + to, from + (size_t)i * ld + GQ * D + d);
             }
         }
-#pragma unroll
-        for (int j = 0; j < PV; ++j) {                // RS_BATCH * CB values over at least 32 threads
-            const int e = threadIdx.x + j * threads, i = e / CB, c = col0 + e % CB;
-            fv[j] = (e < RS_BATCH * CB && i < count && c < V) ? __ldcg(qkv + (size_t)(base + i) * ld + 2 * G * D + h * V + c) : 0.f;
+        for (int e = threadIdx.x; e < count * cols; e += threads) {
+            const int i = e / cols, c = col0 + e % cols;
+            if (c < V) copy4(sv + buf * RS_BATCH * cols + e, qkv + (size_t)(base + i) * ld + 2 * GQ * D + h * V + c);
         }
+        cp_async_commit();
         if (threadIdx.x < count) {
             const float* row = ba + (size_t)(base + threadIdx.x) * 2 * H;
-            fg[0] = __ldcg(row + H + h); fg[1] = __ldcg(row + h);
+            fg[0] = load_now(row + H + h); fg[1] = load_now(row + h);
         }
     };
-    auto stash = [&](int buf, int count) {
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            const int e = threadIdx.x + j * threads;
-            sq[buf * RS_BATCH * Dp + e] = fq[j];
-            sk[buf * RS_BATCH * Dp + e] = fk[j];
-        }
-#pragma unroll
-        for (int j = 0; j < PV; ++j) {
-            const int e = threadIdx.x + j * threads;
-            if (e < RS_BATCH * CB) sv[buf * RS_BATCH * CB + e] = fv[j];
-        }
+    auto land = [&](int buf, int count) {
         if (threadIdx.x < count) {
             sg[(buf * RS_BATCH + threadIdx.x) * 2] = expf(-rate * rs_softplus(fg[0] + shift));
             sg[(buf * RS_BATCH + threadIdx.x) * 2 + 1] = 1.0f / (1.0f + expf(-fg[1]));
         }
+        cp_async_wait<0>();
+        __syncthreads();
     };
     if (t0 < t1) {
-        fetch(t0, min(RS_BATCH, t1 - t0));
-        stash(0, min(RS_BATCH, t1 - t0));
+        fetch(0, t0, min(RS_BATCH, t1 - t0));
+        land(0, min(RS_BATCH, t1 - t0));
     }
-    __syncthreads();
-    int it = 0, flip = 0;
-    for (int base = t0; base < t1; base += RS_BATCH, ++it) {
-        const int count = min(RS_BATCH, t1 - base), buf = it & 1;
-        const int next = base + RS_BATCH, next_count = min(RS_BATCH, t1 - next);
-        if (next < t1) fetch(next, next_count);
-        float* my_red_o = red_o + (size_t)buf * RS_BATCH * warps * CB;
-        for (int i = 0; i < count; ++i, flip ^= 1) {
-            const float decay = sg[(buf * RS_BATCH + i) * 2], beta = sg[(buf * RS_BATCH + i) * 2 + 1];
-            const float4* pq = reinterpret_cast<const float4*>(sq + (buf * RS_BATCH + i) * Dp + row0);
-            const float4* pk = reinterpret_cast<const float4*>(sk + (buf * RS_BATCH + i) * Dp + row0);
-            float kk[R];
-            float part[4] = {0.f, 0.f, 0.f, 0.f};
+    int buf = 0;
+    float* mine = so + warp * RS_BATCH * 32;
+    for (int base = t0; base < t1; base += RS_BATCH, buf ^= 1) {
+        const int count = min(RS_BATCH, t1 - base), next = base + RS_BATCH, next_count = min(RS_BATCH, t1 - next);
+        if (next < t1) fetch(buf ^ 1, next, next_count);
+        const float* rows_q = sq + buf * RS_BATCH * ROW + sub * (R + 4);
+        const float* rows_k = sk + buf * RS_BATCH * ROW + sub * (R + 4);
+        const float* gates = sg + buf * RS_BATCH * 2;
+        // One token: `kk` and `decay` are its key rows and decay, `kn` and `decay_n` become the next one's.
+        auto token = [&](int i, const f32x2 (&kk)[R / 2], float decay, f32x2 (&kn)[R / 2], float& decay_n) {
+            const int after = min(i + 1, RS_BATCH - 1);
+            const float beta = gates[i * 2 + 1], v = sv[(buf * RS_BATCH + i) * cols + cl];
+            f32x2 qq[R / 2], part[2] = {0ull, 0ull}, out[2] = {0ull, 0ull};
+            const f32x2 decay2 = pack2(decay, decay);
 #pragma unroll
-            for (int q = 0; q < R / 4; ++q) {
-                const float4 k4 = pk[q];
-                kk[4 * q] = k4.x; kk[4 * q + 1] = k4.y; kk[4 * q + 2] = k4.z; kk[4 * q + 3] = k4.w;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    s[4 * q + c] *= decay;
-                    part[c] = fmaf(s[4 * q + c], kk[4 * q + c], part[c]);
-                }
+            for (int r = 0; r < R / 2; ++r) {
+                s[r] = mul2(s[r], decay2);
+                part[r & 1] = fma2(s[r], kk[r], part[r & 1]);
             }
-            float* buf_red = red + flip * warps * CB;
-            float mine = (part[0] + part[1]) + (part[2] + part[3]);
+            read_rows<R>(kn, rows_k + after * ROW);
+            read_rows<R>(qq, rows_q + i * ROW);
+            decay_n = gates[after * 2];
+            const float write = beta * (v - groups_sum<G>(rows_sum(part[0], part[1])));
+            const f32x2 write2 = pack2(write, write);
 #pragma unroll
-            for (int m = CB; m < 32; m <<= 1) mine += __shfl_xor_sync(0xffffffffu, mine, m);        // the row groups of a column
-            if (sub == 0) buf_red[warp * CB + cl] = mine;
-            __syncthreads();
-            float read = 0.f;
-            for (int w = 0; w < warps; ++w) read += buf_red[w * CB + cl];         // every warp adds in the same order
-            const float write = beta * (sv[(buf * RS_BATCH + i) * CB + cl] - read);
-            float out[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int q = 0; q < R / 4; ++q) {
-                const float4 q4 = pq[q];
-                const float qq[4] = {q4.x, q4.y, q4.z, q4.w};
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    s[4 * q + c] = fmaf(kk[4 * q + c], write, s[4 * q + c]);
-                    out[c] = fmaf(s[4 * q + c], qq[c], out[c]);
-                }
+            for (int r = 0; r < R / 2; ++r) {
+                s[r] = fma2(kk[r], write2, s[r]);
+                out[r & 1] = fma2(s[r], qq[r], out[r & 1]);
             }
-            float mine_o = (out[0] + out[1]) + (out[2] + out[3]);
-#pragma unroll
-            for (int m = CB; m < 32; m <<= 1) mine_o += __shfl_xor_sync(0xffffffffu, mine_o, m);
-            if (sub == 0) my_red_o[(i * warps + warp) * CB + cl] = mine_o;
+            mine[i * 32 + lane] = rows_sum(out[0], out[1]);
+        };
+        f32x2 ka[R / 2], kb[R / 2];
+        float decay_a = gates[0], decay_b;
+        read_rows<R>(ka, rows_k);
+        int i = 0;
+        for (; i + 1 < count; i += 2) {
+            token(i, ka, decay_a, kb, decay_b);
+            token(i + 1, kb, decay_b, ka, decay_a);
         }
-        if (next < t1) stash(buf ^ 1, next_count);
-        __syncthreads();
-        for (int e = threadIdx.x; e < count * CB; e += threads) {
-            const int i = e / CB, c = col0 + e % CB;
-            float total = 0.f;
-            for (int w = 0; w < warps; ++w) total += my_red_o[(i * warps + w) * CB + e % CB];
-            if (c < V) o[(size_t)(base + i) * H * V + h * V + c] = total;
+        if (i < count) token(i, ka, decay_a, kb, decay_b);
+        __syncwarp();
+        for (int e = lane; e < count * CB; e += 32) {         // a warp's own columns leave once per batch
+            const int i = e / CB, c = e % CB, to = col0 + warp * CB + c;
+            if (to < V) o[(size_t)(base + i) * H * V + h * V + to] = groups_sum<G>(mine + i * 32 + c, CB);
         }
+        __syncwarp();
+        if (next < t1) land(buf ^ 1, next_count);
     }
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-        if (row0 + r < D && col < V) S[(size_t)(row0 + r) * V + col] = s[r];
+    store_state<R>(S, s, row0, col, D, V);
 }
 
-// One token per sequence: as the scan's step for one token, without staging.
+// One token per sequence: as the scan's step for one token, without staging; a warp has one group of rows of 32 columns.
+template <int G>
 __global__ void delta_token_kernel(float* __restrict__ o, const float* qkv, long long ld, const float* ba, const float* __restrict__ a_log,
-                                   const float* __restrict__ dt_bias, float* state, long long state_stride, const int* seq_slots, int H, int G,
+                                   const float* __restrict__ dt_bias, float* state, long long state_stride, const int* seq_slots, int H, int GQ,
                                    int D, int V) {
     constexpr int R = RS_ROWS;
-    __shared__ float red[2 * RS_MAX_WARPS * 32];
-    const int warps = blockDim.x >> 5;
+    __shared__ float red[2 * G * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int col = blockIdx.x * 32 + lane, h = blockIdx.y, t = blockIdx.z;
-    const int g = h / (H / G), row0 = warp * R;
+    const int g = h / (H / GQ), row0 = warp * R;
     float* S = state + (size_t)__ldg(seq_slots + t) * state_stride + (size_t)h * D * V;
     float s[R];
 #pragma unroll
@@ -408,19 +477,17 @@ __global__ void delta_token_kernel(float* __restrict__ o, const float* qkv, long
     const float* row = qkv + (size_t)t * ld;
     const float decay = expf(-expf(a_log[h]) * rs_softplus(__ldcg(ba + (size_t)t * 2 * H + H + h) + dt_bias[h]));
     const float beta = 1.0f / (1.0f + expf(-__ldcg(ba + (size_t)t * 2 * H + h)));
-    const float v = col < V ? __ldcg(row + 2 * G * D + h * V + col) : 0.f;
+    const float v = col < V ? __ldcg(row + 2 * GQ * D + h * V + col) : 0.f;
     float kk[R], part[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        kk[r] = row0 + r < D ? __ldcg(row + G * D + g * D + row0 + r) : 0.f;
+        kk[r] = row0 + r < D ? __ldcg(row + GQ * D + g * D + row0 + r) : 0.f;
         s[r] *= decay;
         part[r & 3] = fmaf(s[r], kk[r], part[r & 3]);
     }
     red[warp * 32 + lane] = (part[0] + part[1]) + (part[2] + part[3]);
     __syncthreads();
-    float read = 0.f;
-    for (int w = 0; w < warps; ++w) read += red[w * 32 + lane];
-    const float write = beta * (v - read);
+    const float write = beta * (v - groups_sum<G>(red + lane, 32));
     float out[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -429,46 +496,43 @@ __global__ void delta_token_kernel(float* __restrict__ o, const float* qkv, long
         out[r & 3] = fmaf(s[r], qq, out[r & 3]);
         if (row0 + r < D && col < V) S[(size_t)(row0 + r) * V + col] = s[r];
     }
-    float* red_o = red + RS_MAX_WARPS * 32;
+    float* red_o = red + G * 32;
     red_o[warp * 32 + lane] = (out[0] + out[1]) + (out[2] + out[3]);
     __syncthreads();
-    if (warp == 0 && col < V) {
-        float total = 0.f;
-        for (int w = 0; w < warps; ++w) total += red_o[w * 32 + lane];
-        o[(size_t)t * H * V + h * V + col] = total;
-    }
+    if (warp == 0 && col < V) o[(size_t)t * H * V + h * V + col] = groups_sum<G>(red_o + lane, 32);
 }
 
-template <int CB>
+template <int G>
 static void launch_delta_scan(float* o, const float* qkv, long long ld, const float* ba, const float* a_log, const float* dt_bias, float* state,
-                              long long state_stride, const int* cu_seqlens, const int* seq_slots, int B, int H, int G, int D, int V, cudaStream_t stream) {
-    constexpr int RW = RS_ROWS * (32 / CB);       // key rows of a warp
-    const int warps = (D + RW - 1) / RW;
-    const size_t smem = (size_t)(2 * 2 * RS_BATCH * warps * RW + 2 * RS_BATCH * CB + 2 * RS_BATCH * 2 + 2 * warps * CB + 2 * RS_BATCH * warps * CB) * sizeof(float);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(delta_scan_kernel<CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ti_launch(delta_scan_kernel<CB>, dim3((V + CB - 1) / CB, H, B), dim3(warps * 32), smem, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride,
-              cu_seqlens, seq_slots, H, G, D, V);
+                              long long state_stride, const int* cu_seqlens, const int* seq_slots, int B, int H, int GQ, int D, int V, bool one_token,
+                              int warps, cudaStream_t stream) {
+    if (one_token) {
+        ti_launch(delta_token_kernel<G>, dim3((V + 31) / 32, H, B), dim3(G * 32), 0, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride, seq_slots,
+                  H, GQ, D, V);
+        return;
+    }
+    const int cols = warps * (32 / G);
+    const size_t smem = (size_t)(4 * RS_BATCH * G * (RS_ROWS + 4) + 2 * RS_BATCH * cols + 4 * RS_BATCH + RS_BATCH * warps * 32) * sizeof(float);
+    const int vec = D % 4 == 0 && ld % 4 == 0 && aligned16(qkv) && warps * 32 >= D / 4;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(delta_scan_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    ti_launch_after(delta_scan_kernel<G>, dim3((V + cols - 1) / cols, H, B), dim3(warps * 32), smem, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride,
+              cu_seqlens, seq_slots, H, GQ, D, V, vec);
 }
 
 extern "C" int ti_delta_scan(float* o, const float* qkv, long long ld, const float* ba, const float* a_log, const float* dt_bias, float* state,
                              long long state_stride, const int* cu_seqlens, const int* seq_slots, int n, int B, int H, int G, int D, int V,
                              cudaStream_t stream) {
     if (n == 0 || B == 0) return 0;
-    const int warps = (D + RS_ROWS - 1) / RS_ROWS;
-    TI_REQUIRE(D > 0 && V > 0 && warps <= RS_MAX_WARPS, "delta_scan: keys of %d (at most %d)", D, RS_MAX_WARPS * RS_ROWS);
+    TI_REQUIRE(D > 0 && V > 0 && D <= RS_MAX_KEY, "delta_scan: keys of %d (at most %d)", D, RS_MAX_KEY);
     TI_REQUIRE(H > 0 && G > 0 && H % G == 0, "delta_scan: %d heads do not divide into %d query/key heads", H, G);
-    if (n == B) {                                 // one token per sequence
-        ti_launch(delta_token_kernel, dim3((V + 31) / 32, H, B), dim3(warps * 32), 0, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride, seq_slots,
-                  H, G, D, V);
-        return ti_check_launch("delta_token");
-    }
-    // Very few (sequence, head) pairs: blocks of 16 or 8 columns, so that more SMs have one and a token's barrier joins fewer warps
-    // (with 64 blocks of 32 columns already, blocks of 16 were slower: 1,072 against 982 us; see the decay scan).
-    const long long blocks32 = (long long)((V + 31) / 32) * H * B;
-    const int sms = ti_sm_count();
-    if (blocks32 * 4 >= sms) launch_delta_scan<32>(o, qkv, ld, ba, a_log, dt_bias, state, state_stride, cu_seqlens, seq_slots, B, H, G, D, V, stream);
-    else if (blocks32 * 8 >= sms) launch_delta_scan<16>(o, qkv, ld, ba, a_log, dt_bias, state, state_stride, cu_seqlens, seq_slots, B, H, G, D, V, stream);
-    else launch_delta_scan<8>(o, qkv, ld, ba, a_log, dt_bias, state, state_stride, cu_seqlens, seq_slots, B, H, G, D, V, stream);
+    const ScanShape shape = scan_shape(RS_ROWS, D, V, (long long)H * B, 4, 1);
+#define RS_DELTA(GROUPS) launch_delta_scan<GROUPS>(o, qkv, ld, ba, a_log, dt_bias, state, state_stride, cu_seqlens, seq_slots, B, H, G, D, V, n == B, shape.warps, stream)
+    if (shape.groups == 1) RS_DELTA(1);
+    else if (shape.groups == 2) RS_DELTA(2);
+    else if (shape.groups == 4) RS_DELTA(4);
+    else if (shape.groups == 8) RS_DELTA(8);
+    else RS_DELTA(16);
+#undef RS_DELTA
     return ti_check_launch("delta_scan");
 }
 
