@@ -185,11 +185,15 @@ __global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(
     }
 }
 
+// The parts of a (sequence, head) merged: a block each, D elements over its threads. A part's weight is worked out by a lane of the first warp of its
+// own; every thread then goes over the parts in ascending order. What bounds it: one round trip to L2, so everything is asked for at once
+// (one thread's walk over the parts' maxima and sums, and later parts' outputs asked for late: 18 parts 6.3 us inside a step, now 2.2; 4 parts of 256 (sequence, head) 3.1 us, now 2.8).
+#define AC_AT_ONCE 32
 __global__ void attention_combine_kernel(bf16* __restrict__ out, const float* ws_o,
                                          const float* ws_ml, const int* seq_work, int D, int nq, int splits, const float* __restrict__ sink) {
     const size_t row = blockIdx.x;                          // (sequence, head)
-    __shared__ float sm[AD_MAX_SPLITS], sl[AD_MAX_SPLITS], sw[AD_MAX_SPLITS];
-    __shared__ float s_inv;
+    __shared__ float sl[AD_MAX_SPLITS], sw[AD_MAX_SPLITS];
+    __shared__ float s_max;
     // The parts of this (sequence, head) lie together: `splits` of them from row x splits on, or, with the
     // host's table (first slot << 8 | parts per sequence), `parts` from first slot x nq + head x parts on.
     size_t first = row * splits;
@@ -203,37 +207,51 @@ __global__ void attention_combine_kernel(bf16* __restrict__ out, const float* ws
     const float* part_o = ws_o + first * D;
     const float* ml = ws_ml + first * 2;
     pdl_enter();
-    // One round of loads: every thread's partial outputs (for up to 16 parts) are requested together
-    // with the parts' (m, l), before anything is computed.
     const int d0 = threadIdx.x;
-    float head_o[16];
+    float head_m[2], head_l[2];
+    if (d0 < 32) {
 #pragma unroll
-    for (int u = 0; u < 16; ++u) head_o[u] = (d0 < D && u < parts) ? __ldcg(part_o + (size_t)u * D + d0) : 0.f;
-    for (int s = threadIdx.x; s < parts; s += blockDim.x) {
-        sm[s] = __ldcg(ml + 2 * s);
-        sl[s] = __ldcg(ml + 2 * s + 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float M = -INFINITY;
-        for (int s = 0; s < parts; ++s) M = fmaxf(M, sm[s]);
-        float L = 0.f;
-        for (int s = 0; s < parts; ++s) {
-            sw[s] = M == -INFINITY ? 0.f : exp2f(sm[s] - M);     // no part saw a key (a sequence of length 0): zeros, not 0/0
-            L += sl[s] * sw[s];
+        for (int u = 0; u < 2; ++u) {
+            const int s = d0 + 32 * u;
+            head_m[u] = s < parts ? __ldcg(ml + 2 * s) : -INFINITY;
+            head_l[u] = s < parts ? __ldcg(ml + 2 * s + 1) : 0.f;
         }
-        if (sink != nullptr && L > 0.f) L += exp2f(sink[row % nq] * 1.4426950408889634f - M);
-        s_inv = L > 0.f ? 1.0f / L : 0.f;
+    }
+    float head_o[AC_AT_ONCE];
+#pragma unroll
+    for (int u0 = 0; u0 < AC_AT_ONCE; u0 += 4)
+        if (u0 < parts) {                                   // the same for every thread: few parts, few instructions
+#pragma unroll
+            for (int u = u0; u < u0 + 4; ++u) head_o[u] = (d0 < D && u < parts) ? __ldcg(part_o + (size_t)u * D + d0) : 0.f;
+        }
+    if (d0 < 32) {
+        const float M = warp_max(fmaxf(head_m[0], head_m[1]));
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int s = d0 + 32 * u;
+            if (s >= AD_MAX_SPLITS) break;
+            sw[s] = M == -INFINITY ? 0.f : exp2f(head_m[u] - M);     // no part saw a key (a sequence of length 0): zeros, not 0/0
+            sl[s] = head_l[u];
+        }
+        if (d0 == 0) s_max = M;
     }
     __syncthreads();
-    const float inv = s_inv;
+    float L = 0.f, O0 = 0.f;
+#pragma unroll
+    for (int u0 = 0; u0 < AC_AT_ONCE; u0 += 4)
+        if (u0 < parts) {
+#pragma unroll
+            for (int u = u0; u < u0 + 4; ++u) {             // beyond the last part: weights and values of zero
+                L += sl[u] * sw[u];
+                O0 += sw[u] * head_o[u];
+            }
+        }
+    for (int s = AC_AT_ONCE; s < parts; ++s) L += sl[s] * sw[s];
+    if (sink != nullptr && L > 0.f) L += exp2f(sink[row % nq] * 1.4426950408889634f - s_max);
+    const float inv = L > 0.f ? 1.0f / L : 0.f;
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        float O = 0.f;
-        if (d == d0) {
-#pragma unroll
-            for (int u = 0; u < 16; ++u) O += (u < parts ? sw[u] : 0.f) * head_o[u];
-        }
-        for (int s0 = d == d0 ? 16 : 0; s0 < parts; s0 += 8) {
+        float O = d == d0 ? O0 : 0.f;
+        for (int s0 = d == d0 ? AC_AT_ONCE : 0; s0 < parts; s0 += 8) {
             float v[8];
 #pragma unroll
             for (int u = 0; u < 8; ++u) v[u] = s0 + u < parts ? __ldcg(part_o + (size_t)(s0 + u) * D + d) : 0.f;
