@@ -23,13 +23,16 @@
 // not (every row of a product is computed alone, in ascending k), so results are the same bits from run to run.
 #include "tile_gemm.cuh"
 
+// The routers' shared memory is what a call needs (static arrays for 1,024 experts had the SMs of a step's few blocks split for 16 such blocks each,
+// most of it shared memory; blocks of the product behind them that come up there before they leave found 28 KB of L1 and took three times as long: both
+// streamed products of 13 plain units of 1,024 x 2,048 with router_select ahead of them 35 us, now 30).
 #define RT_THREADS 128
 #define RT_MAX_EXPERTS 1024
 
 template <typename T>
 __global__ void router_topk_kernel(const T* h, const T* __restrict__ wr, const float* logits, int width, int experts, int top,
                                    int always, int* __restrict__ ids, float* __restrict__ scores) {
-    __shared__ float z[RT_MAX_EXPERTS];
+    extern __shared__ float z[];                           // [experts]
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     pdl_enter();
     if (logits != nullptr) {                               // a product kernel has left the 32-bit sums
@@ -80,7 +83,7 @@ extern "C" int ti_router_topk(const void* h, const void* wr, const float* logits
                               int* ids, float* scores, int dtype, cudaStream_t stream) {
     if (n == 0) return 0;
     TI_REQUIRE(experts >= 1 && experts <= RT_MAX_EXPERTS && top >= 1 && top <= experts && always >= 0, "router_topk: top %d of %d experts", top, experts);
-    TI_DISPATCH_DTYPE(dtype, (ti_launch(router_topk_kernel<T>, dim3(n), dim3(RT_THREADS), 0, stream, (const T*)h, (const T*)wr, logits, width,
+    TI_DISPATCH_DTYPE(dtype, (ti_launch(router_topk_kernel<T>, dim3(n), dim3(RT_THREADS), experts * sizeof(float), stream, (const T*)h, (const T*)wr, logits, width,
                                         experts, top, always, ids, scores)));
     return ti_check_launch("router_topk");
 }
@@ -100,10 +103,11 @@ template <typename T>
 __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const float* z_in, long long ldz, int width, int experts, int total,
                                      int softmax, const float* __restrict__ z_bias, const float* __restrict__ correction, int groups, int keep, int group_best,
                                      int top, int renormalize, int always, int gate, int* __restrict__ ids, float* __restrict__ scores, float* __restrict__ pass_weight) {
-    __shared__ float z[RT_MAX_EXPERTS + 1], c[RT_MAX_EXPERTS], gs[RT_MAX_EXPERTS];
+    extern __shared__ float shared[];
     __shared__ float scratch[33];
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int columns = total + (gate ? 1 : 0);
+    float *z = shared, *c = z + columns, *gs = c + total;  // [columns], [total], [groups]
     pdl_enter();
     if (z_in != nullptr) {
         for (int e = threadIdx.x; e < columns; e += RT_THREADS) z[e] = __ldcg(z_in + (size_t)t * ldz + e);
@@ -161,6 +165,9 @@ __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const
     if (warp == 0) {
         float wsum = 0.f;
         const size_t out = (size_t)t * (top + always);
+        const bool few = top <= 32;                                 // lane j keeps choice j; of more they are kept in memory
+        int my_arg = 0;
+        float my_w = 0.f;
         for (int j = 0; j < top; ++j) {
             float best = -INFINITY;
             int arg = 0x7fffffff;
@@ -173,15 +180,40 @@ __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const
                 if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
             }
             if (arg >= total) arg = j;                              // only if nothing comparable is left (NaN)
+            const float w = z[arg];
+            if (lane == j) { my_arg = arg; my_w = w; }
             if (lane == 0) {
-                ids[out + j] = arg;
-                scores[out + j] = z[arg];
+                if (!few) { ids[out + j] = arg; scores[out + j] = w; }
                 c[arg] = -INFINITY;
             }
-            wsum += z[arg];
+            wsum += w;
             __syncwarp();
         }
-        if (softmax == 2 && lane == 0) {                            // the chosen logits come largest first
+        const float gw = gate ? 1.0f / (1.0f + expf(-z[total])) : 1.0f;
+        for (int a = lane; a < always; a += 32) {
+            ids[out + top + a] = experts + a;
+            scores[out + top + a] = gw;
+        }
+        if (few) {
+            if (softmax == 2) {                                     // the chosen logits come largest first
+                my_w = expf(my_w - __shfl_sync(0xffffffffu, my_w, 0));
+                wsum = 0.f;
+                for (int j = 0; j < top; ++j) wsum += __shfl_sync(0xffffffffu, my_w, j);
+            }
+            my_w /= renormalize ? wsum + 1e-20f : 1.0f;
+            float pass = 0.f;
+            for (int j = 0; j < top; ++j) {
+                const float w = __shfl_sync(0xffffffffu, my_w, j);
+                if (__shfl_sync(0xffffffffu, my_arg, j) >= experts) pass += w;
+            }
+            if (lane < top) {
+                ids[out + lane] = my_arg >= experts ? -1 : my_arg;
+                scores[out + lane] = my_w;
+            }
+            if (pass_weight != nullptr && lane == 0) pass_weight[t] = pass;
+            return;
+        }
+        if (softmax == 2 && lane == 0) {
             const float m = scores[out];
             wsum = 0.f;
             for (int j = 0; j < top; ++j) {
@@ -199,11 +231,6 @@ __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const
                 if (ids[out + j] >= experts) { pass += wgt; ids[out + j] = -1; }
             }
             if (pass_weight != nullptr) pass_weight[t] = pass;
-            const float gw = gate ? 1.0f / (1.0f + expf(-z[total])) : 1.0f;
-            for (int a = 0; a < always; ++a) {
-                ids[out + top + a] = experts + a;
-                scores[out + top + a] = gw;
-            }
         }
     }
 }
@@ -219,7 +246,7 @@ extern "C" int ti_router_select(const void* h, const void* wr, const float* z, l
                "router_select: %d of %d groups over %d choices for top %d", keep, groups, total, top);
     TI_REQUIRE(group_best == 1 || group_best == 2, "router_select: a group's score from its %d best", group_best);
     TI_REQUIRE(total == experts || pass_weight != nullptr, "router_select: pass choices need their weights' output");
-    TI_DISPATCH_DTYPE(dtype, (ti_launch(router_select_kernel<T>, dim3(n), dim3(RT_THREADS), 0, stream, (const T*)h, (const T*)wr, z, ldz, width, experts,
+    TI_DISPATCH_DTYPE(dtype, (ti_launch(router_select_kernel<T>, dim3(n), dim3(RT_THREADS), (2 * total + 1 + groups) * sizeof(float), stream, (const T*)h, (const T*)wr, z, ldz, width, experts,
                                         total, softmax, z_bias, correction, groups, keep, group_best, top, renormalize, always, gate, ids, scores, pass_weight)));
     return ti_check_launch("router_select");
 }
