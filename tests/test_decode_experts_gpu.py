@@ -60,6 +60,36 @@ def test_units_streamed_by_pair(units, out, k, tokens, per_token, gated):
             assert bool(((y2[p].cpu().to(F64) - want).abs() <= bound + 1e-7).all())
 
 
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("units,out,k,tokens,per_token", [(40, 1032, 72, 16, 2), (70, 24, 2056, 16, 4), (9, 40, 264, 16, 7), (300, 16, 40, 16, 20)])
+def test_units_listed_by_warp_block_and_launch(units, out, k, tokens, per_token, gated):
+    """32 pairs (listed by one warp), more, and more than one launch lists; several tiles a block; rows longer and shorter than the k blocks in
+    flight: every pair's result has the bits of the pair alone."""
+    from tileinfer_b200.kernels import fast
+    g = torch.Generator(device="cuda").manual_seed(units + k)
+    x = torch.randn(tokens, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(units, (2 if gated else 1) * out, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    ids = torch.randint(-1, units, (tokens, per_token), generator=g, device="cuda").int()
+    ids[::2, 0] = 3                                      # more than 8 pairs with one unit
+    scores = torch.rand(tokens, per_token, generator=g, device="cuda")
+    limits = torch.full((units,), 1.5, device="cuda")
+    pairs = tokens * per_token
+
+    def run(x, ids, scores, per_token):
+        y = torch.full((ids.numel(), out), 7.0, dtype=torch.bfloat16, device="cuda")
+        rows = torch.full(ids.shape, 99, dtype=torch.int32, device="cuda")
+        fast.grouped_stream(y, x, w, ids, scores, rows, per_token, gated=gated, relu2=not gated, limits=limits, slope=1.7, shift=1.0)
+        assert torch.equal(rows.flatten(), torch.where(ids.flatten() >= 0, torch.arange(ids.numel(), device="cuda"), -1).int())
+        return y
+
+    for s in (None, scores):
+        together = run(x, ids, s, per_token)
+        for p in range(pairs):
+            t, j = divmod(p, per_token)
+            one = run(x[t:t + 1].contiguous(), ids[t:t + 1, j:j + 1].contiguous(), s[t:t + 1, j:j + 1].contiguous() if s is not None else None, 1)
+            assert torch.equal(one[0], together[p]), p
+
+
 @pytest.mark.parametrize("heads,out,k", [(3, 40, 8), (16, 128, 64), (5, 24, 264), (2, 136, 2056), (64, 520, 128), (130, 264, 128)])
 @pytest.mark.parametrize("n", [1, 8, 9, 16, 17])
 def test_product_with_a_matrix_per_head(heads, out, k, n):
