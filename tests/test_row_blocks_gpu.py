@@ -153,3 +153,24 @@ def test_scans_have_the_bits_of_single_tokens(ops, H, D):
     for portions in ([17] * 4, [1] * 40):
         for got, want in zip(run(portions), whole):
             assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("out,k", [(248, 72), (256, 8), (264, 136), (520, 264), (1024, 2056), (2048, 128)])
+def test_grouped_products_on_pairs_of_sms(ops, out, k):
+    """Token tiles of 128 rows of one matrix each: from 256 weight rows on two SMs share a tile. Matrices without a tile and with several, fewer
+    tiles in use than there is room for, weight rows that are no whole tiles (the next matrix's lie behind them), k that ends inside a stage."""
+    from tileinfer_b200.kernels import fast
+    g = torch.Generator(device="cuda").manual_seed(out + k)
+    matrices, used, room = 5, [4, 0, 0, 2, 2, 2, 3], 12
+    x = torch.randn(room * 128, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(matrices, out, k, generator=g, device="cuda") * k ** -0.5).bfloat16()
+    y = torch.full((room * 128, out), 7.0, dtype=torch.bfloat16, device="cuda")
+    plan = torch.tensor([len(used)] + used + [99] * (room - len(used)), dtype=torch.int32, device="cuda")
+    assert fast.grouped_linear(y, x, w, plan, 128)
+    fast.check_status()
+    for t, m in enumerate(used):
+        rows = x[t * 128:(t + 1) * 128].double()
+        want, mass = rows @ w[m].double().t(), rows.abs() @ w[m].double().abs().t()
+        # 32-bit sums of k products in any order, then one rounding to bfloat16.
+        assert bool(((y[t * 128:(t + 1) * 128].double() - want).abs() <= k / 2 * 2.0 ** -24 * mass + want.abs() * 2.0 ** -8 + 1e-7).all()), t
+    assert bool((y[len(used) * 128:] == 7.0).all())

@@ -437,7 +437,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     const unsigned tmem_base = *tmem_slot;
 
     TileIter it;
-    it.id = blockIdx.x >> 1; it.step = gridDim.x >> 1; it.n_tiles = p.n_tiles; it.total = p.m_tiles * p.n_tiles * p.splits;
+    it.id = blockIdx.x >> 1; it.step = gridDim.x >> 1;
+    it.n_tiles = p.groups != nullptr ? min(__ldcg(p.groups), p.n_tiles) : p.n_tiles;
+    it.total = p.m_tiles * it.n_tiles * p.splits;
 
     if (warp == 0) {
         // ---------------------------------------------------------------- producer (TMA), in both blocks
@@ -445,6 +447,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         unsigned phase = 0;
         bool ok = true;
         while (lane == 0 && ok && it.next(p)) {             // one thread: see the producer of the kernel above
+            const int w_row = (p.groups != nullptr ? __ldcg(p.groups + 1 + it.n) * p.w_group_rows : 0) + (it.m * 2 + (int)rank) * BM;
             for (int kb = it.kb_lo; kb < it.kb_hi; ++kb) {
                 ok = mbar_wait(empty0 + 8 * stage, phase ^ 1, p.status, 1);
                 if (!ok) break;
@@ -453,7 +456,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
                 const unsigned a_dst = smem_addr(tiles + (size_t)stage * C::STAGE_BYTES);
 #pragma unroll
                 for (int a = 0; a < C::KB; ++a) {
-                    tma_load_2d_pair(a_dst + a * C::ATOM_BYTES, &map_w, (kb * C::KB + a) * BK, (it.m * 2 + (int)rank) * BM, bar);
+                    tma_load_2d_pair(a_dst + a * C::ATOM_BYTES, &map_w, (kb * C::KB + a) * BK, w_row, bar);
                     tma_load_2d_pair(a_dst + C::A_BYTES + a * C::ATOM_BYTES, &map_x, (kb * C::KB + a) * BK,
                                      it.n * tile_n + (int)rank * (tile_n / 2), bar);
                 }
@@ -669,18 +672,21 @@ int many_dispatch(void* y, long long ldy, const void* x, long long ldx, const vo
                   Params p, int* status, cudaStream_t stream) {
     p.N = n; p.K = in; p.M = out; p.tile_n = bn;
     p.m_fastest = p.groups != nullptr && bn >= 128;
-    // Token tiles of 128 with 256 weight rows per block: the token operand staged for a k block feeds two MMAs (tiles of
-    // 128 x 128 are bound by the fill of shared memory).
+    // Token tiles of 128 with 256 weight rows: the token operand staged for a k block feeds two MMAs (tiles of 128 x 128 are bound by the fill
+    // of shared memory). Matrices grouped by token tile take two SMs for such a tile, whose MMAs read a third less of each SM's shared
+    // memory and whose epilogue runs beside the next tile's (2,048 tokens x 6 of 34 matrices, 2,048 x 2,048 / 2,048 x 1,024 / 512 x 2,048
+    // 138 / 85 / 52 us on one SM a tile, 121 / 71 / 38 on two; 900 tokens 84 / 52, 77 / 46; 8,192 tokens 461, 403).
     const int mt = bn == 128 && out >= 2 * BM ? 2 : 1;
+    const bool pair = mt == 2 && p.groups != nullptr && pair_clusters(sm_count_cached()) > 0;
     p.m_tiles = (out + mt * BM - 1) / (mt * BM);
     p.n_tiles = (n + bn - 1) / bn;
-    p.k_blocks = (in + BK - 1) / BK;
+    p.k_blocks = pair ? (in + PairCfg::KB * BK - 1) / (PairCfg::KB * BK) : (in + BK - 1) / BK;
     p.splits = 1;
     p.ldy = ldy; p.epilogue = EPI_NONE; p.act = XieluParams{0.f, 0.f, 0.f, 0.f}; p.status = status;
     p.rotate = bn <= 64;
     CUtensorMap mw, mx, my;
     if (int rc = tensor_map(&mw, W, w_rows, in, in, BM)) return rc;
-    if (int rc = tensor_map(&mx, x, n, ldx, ldx, bn)) return rc;          // all columns of the rows: a batch picks its own
+    if (int rc = tensor_map(&mx, x, n, ldx, ldx, pair ? bn / 2 : bn)) return rc;          // all columns of the rows: a batch picks its own
     // Results leave by TMA stores in boxes of 32 features: a box must lie within one matrix's columns.
     p.tma_out = bn >= 128 && out % 32 == 0 && ldy % 8 == 0 && !((uintptr_t)y & 15);
     if (p.tma_out) {
@@ -688,6 +694,7 @@ int many_dispatch(void* y, long long ldy, const void* x, long long ldx, const vo
     } else {
         my = mx;
     }
+    if (pair) return launch_pair(y, mw, mx, my, p, stream);
     const int sms = sm_count_cached();
     switch (bn) {
         case 256: return launch<256, 1>(y, mw, mx, my, p, sms, stream);
