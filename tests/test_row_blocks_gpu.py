@@ -174,3 +174,37 @@ def test_grouped_products_on_pairs_of_sms(ops, out, k):
         # 32-bit sums of k products in any order, then one rounding to bfloat16.
         assert bool(((y[t * 128:(t + 1) * 128].double() - want).abs() <= k / 2 * 2.0 ** -24 * mass + want.abs() * 2.0 ** -8 + 1e-7).all()), t
     assert bool((y[len(used) * 128:] == 7.0).all())
+
+
+@pytest.mark.parametrize("D,nq,nkv,B", [(128, 8, 8, 50), (128, 40, 4, 100), (256, 16, 8, 45), (128, 6, 6, 90)])
+def test_decode_attention_on_half_pages(D, nq, nkv, B):
+    """So many unsplit sequences that blocks of half pages are taken: lengths on both sides of a page's and a half's end, a window, kept first
+    positions, a sink; against 64-bit arithmetic."""
+    from tileinfer_b200.kernels import fast
+    from tileinfer_b200.kernels.library import lib
+    g = torch.Generator(device="cuda").manual_seed(D + B)
+    R = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()                          # noqa: E731
+    lengths = [(1, 31, 32, 33, 63, 64, 65, 96, 97, 128, 129, 200)[i % 12] for i in range(B)]
+    pages = 4
+    k, v, q = R(B * pages, nkv, 64, D), R(B * pages, nkv, 64, D), R(B, nq, D)
+    table = torch.randperm(B * pages, generator=g, device="cuda").int().view(B, pages).contiguous()
+    slots, kv = torch.arange(B, device="cuda").int(), torch.tensor(lengths, device="cuda").int()
+    sink = torch.randn(nq, generator=g, device="cuda")
+    for window, keep, with_sink in ((0, 0, False), (40, 0, True), (70, 5, False)):
+        out = torch.empty(B, nq * D, dtype=torch.bfloat16, device="cuda")
+        rc = lib().ti_attention_decode_kept(out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), table.data_ptr(), pages, slots.data_ptr(), kv.data_ptr(), None, None, None,
+                                            None, D ** -0.5, B, nq, nkv, D, 64, 1, window, sink.data_ptr() if with_sink else None, 0, None, 0, 0.0, None, keep, fast._stream())
+        assert rc == 0
+        for b, n in enumerate(lengths):
+            keys, values = (c[table[b].long()].permute(1, 0, 2, 3).reshape(nkv, -1, D)[:, :n].double().repeat_interleave(nq // nkv, 0) for c in (k, v))
+            s = torch.einsum("hd,hnd->hn", q[b].double(), keys) * D ** -0.5
+            at = torch.arange(n, device="cuda")
+            if window:
+                s = s.masked_fill(~((at >= n - window) | (at < keep)), -float("inf"))
+            if with_sink:
+                s = torch.cat([s, sink.double()[:, None]], 1)
+            p = torch.softmax(s, -1)[:, :n]
+            want = torch.einsum("hn,hnd->hd", p, values)
+            # P is rounded to bfloat16, the result once more; scores and sums are 32-bit.
+            bound = 2.0 ** -8 * (torch.einsum("hn,hnd->hd", p, values.abs()) + want.abs()) + 1e-5
+            assert bool(((out[b].view(nq, D).double() - want).abs() <= bound).all()), (b, n, window)
