@@ -116,6 +116,52 @@ def test_delta_inputs_in_runs_of_tokens(ops, taps, G, D, HV):
         at += length
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("size", [40, 1000, 2048, 4100, 9000])
+def test_gated_rows_of_the_lightning_mixer_in_small_and_large_steps(ops, dtype, size):
+    g = torch.Generator(device="cuda").manual_seed(size)
+    n = 300                                                # more rows than SMs
+    o, w = torch.randn(n, size, generator=g, device="cuda"), torch.randn(size, generator=g, device="cuda").to(dtype)
+    gate = torch.randn(n, size, generator=g, device="cuda").to(dtype)
+    for z in (gate, None):
+        def run(lo, hi):
+            y = torch.empty(hi - lo, size, dtype=dtype, device="cuda")
+            ops.lightning_out(y, o[lo:hi].contiguous(), z[lo:hi] if z is not None else None, w, 1e-6)
+            return y
+
+        whole = run(0, n)
+        want = o.double() / torch.sqrt((o.double() ** 2).mean(-1, keepdim=True) + 1e-6) * w.double() * (torch.sigmoid(z.double()) if z is not None else 1.0)
+        # A sum of squares, a root, a quotient, an exponential; one rounding to the element type.
+        assert bool(((whole.double() - want).abs() <= want.abs() * ((2.0 ** -8 if dtype == torch.bfloat16 else 0) + 2.0 ** -18) + 1e-9).all())
+        for lo, hi in ((0, 1), (5, 9), (100, 248)):
+            assert torch.equal(run(lo, hi), whole[lo:hi])
+
+
+@pytest.mark.parametrize("tile", [32, 128])
+@pytest.mark.parametrize("n,per,units", [(1, 1, 1), (3, 2, 40), (2048, 6, 34), (1500, 8, 1000), (5000, 4, 65)])
+def test_plan_of_units(ops, n, per, units, tile):
+    """Up to as many pairs as the threads keep and more, experts beyond a warp's 32, units without pairs, choices without a unit."""
+    g = torch.Generator(device="cuda").manual_seed(n + units)
+    ids = torch.randint(-1, units, (n, per), generator=g, device="cuda").int()
+    ids[ids % 3 == 1] = units - 1
+    most, capacity = ops.expert_plan_sizes(n * per, units, tile)
+    pair_row, row_pair = torch.full((n, per), 77, dtype=torch.int32, device="cuda"), torch.full((capacity,), 77, dtype=torch.int32, device="cuda")
+    plan = torch.full((1 + most,), 77, dtype=torch.int32, device="cuda")
+    ops.expert_plan(ids, units, tile, pair_row, row_pair, plan)
+    flat, rows = ids.flatten().cpu(), pair_row.flatten().cpu()
+    counts = torch.bincount(flat[flat >= 0], minlength=units)
+    tiles = (counts + tile - 1) // tile
+    assert int(plan[0]) == int(tiles.sum())
+    assert torch.equal(plan[1:1 + int(tiles.sum())].cpu().long(), torch.repeat_interleave(torch.arange(units), tiles))
+    assert bool((rows[flat < 0] == -1).all())
+    has = flat >= 0
+    assert len(set(rows[has].tolist())) == int(has.sum())
+    assert torch.equal(plan[1:].cpu()[(rows[has] // tile).long()], flat[has])
+    back = torch.full((capacity,), -1, dtype=torch.int32)
+    back[rows[has].long()] = torch.arange(n * per, dtype=torch.int32)[has]
+    assert torch.equal(row_pair.cpu(), back)
+
+
 @pytest.mark.parametrize("H,D", [(3, 5), (2, 33), (32, 64), (1, 64), (5, 100), (2, 129), (1, 256)])
 def test_scans_have_the_bits_of_single_tokens(ops, H, D):
     """Batches of tokens, a batch's remainder and tokens one by one: the same bits, for every number of row groups and blocks of all sizes."""

@@ -255,35 +255,61 @@ extern "C" int ti_router_select(const void* h, const void* wr, const float* z, l
 // tile holds rows of one expert only (tensor-core kernels then treat a tile like any other; nobody reads the results of
 // padding rows). plan[0] = tiles in use, plan[1 + t] = the expert of tile t. pair_row[pair] = the pair's
 // row; row_pair[row] = the row's pair, or -1 for padding, for all `capacity` rows.
-__global__ void expert_plan_kernel(const int* ids, int pairs, int experts, int tile, int capacity, int* __restrict__ pair_row,
+// One block. What bounds it: round trips, so a thread's ids are asked for at once and kept, and the tiles are numbered by a warp, 32 experts at a
+// time (12,288 pairs of 34 units 14.2 -> 9.8 us, 160 of 64 6.3 -> 3.3).
+#define EP_KEPT 16
+__global__ void __launch_bounds__(1024) expert_plan_kernel(const int* ids, int pairs, int experts, int tile, int capacity, int* __restrict__ pair_row,
                                    int* __restrict__ row_pair, int* __restrict__ plan) {
     __shared__ int count[RT_MAX_EXPERTS], first[RT_MAX_EXPERTS];
     pdl_enter();
+    int kept[EP_KEPT];
+#pragma unroll
+    for (int k = 0; k < EP_KEPT; ++k) {
+        const int p = threadIdx.x + k * blockDim.x;
+        kept[k] = p < pairs ? __ldcg(ids + p) : -1;
+    }
     for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0;
     for (int r = threadIdx.x; r < capacity; r += blockDim.x) row_pair[r] = -1;
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+#pragma unroll
+    for (int k = 0; k < EP_KEPT; ++k)
+        if (kept[k] >= 0) atomicAdd(&count[kept[k]], 1);     // a negative id: a choice that needs no unit's matrices
+    for (int p = threadIdx.x + EP_KEPT * blockDim.x; p < pairs; p += blockDim.x) {
         const int e = __ldcg(ids + p);
-        if (e >= 0) atomicAdd(&count[e], 1);             // a negative id: a choice that needs no unit's matrices
+        if (e >= 0) atomicAdd(&count[e], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int tiles = 0;
-        for (int e = 0; e < experts; ++e) {
-            first[e] = tiles * tile;
-            for (int r = 0; r < count[e]; r += tile) plan[1 + tiles++] = e;
-            count[e] = 0;
+    if (threadIdx.x < 32) {
+        int tiles = 0;                                       // of the experts before these 32
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int e = e0 + (int)threadIdx.x, mine = e < experts ? (count[e] + tile - 1) / tile : 0;
+            int upto = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int before = __shfl_up_sync(0xffffffffu, upto, o);
+                if ((int)threadIdx.x >= o) upto += before;
+            }
+            if (e < experts) {
+                const int at = tiles + upto - mine;
+                first[e] = at * tile;
+                count[e] = 0;
+                for (int t = 0; t < mine; ++t) plan[1 + at + t] = e;
+            }
+            tiles += __shfl_sync(0xffffffffu, upto, 31);
         }
-        plan[0] = tiles;
+        if (threadIdx.x == 0) plan[0] = tiles;
     }
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        const int e = __ldcg(ids + p);
-        if (e < 0) { pair_row[p] = -1; continue; }
+    auto place = [&](int p, int e) {
+        if (e < 0) { pair_row[p] = -1; return; }
         const int row = first[e] + atomicAdd(&count[e], 1);
         pair_row[p] = row;
         row_pair[row] = p;
-    }
+    };
+#pragma unroll
+    for (int k = 0; k < EP_KEPT; ++k)
+        if (threadIdx.x + k * blockDim.x < pairs) place(threadIdx.x + k * blockDim.x, kept[k]);
+    for (int p = threadIdx.x + EP_KEPT * blockDim.x; p < pairs; p += blockDim.x) place(p, __ldcg(ids + p));
 }
 
 // The most tiles of `tile` rows that `pairs` pairs over `experts` experts can take: every tile holds at least one pair, and
