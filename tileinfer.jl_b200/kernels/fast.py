@@ -226,12 +226,11 @@ def grouped_linear(y, x, w, plan, tile) -> bool:
 
 # A step of so few tokens streams the matrices of the units in use (csrc/expert_stream.cu); with more, a unit's pairs no longer fit one
 # operand of 8 and its matrices are gone over again. Both products, streamed against planned and grouped: 32 gated units of 1,024 x 2,048
-# with two shared, 8 tokens 62 against 85 us, 16 tokens 89 against 91, 24 tokens 111 against 97; plain units, 16 tokens 50 against 62;
-# 64 units of 1,408 x 4,096, 4 tokens 141 against 157, 16 tokens 357 against 363, 24 tokens 421 against 397.
+# with two shared, 8 / 16 / 32 tokens 47 / 66 / 81 us against 85 / 91 / 94; plain units 30 / 41 / 45 against 51 / 63 / 66; 64 units of
+# 1,408 x 4,096 195 / 283 / 328 against 244 / 349 / 402. (So more tokens could be streamed too.)
 EXPERT_STREAM_TOKENS = 16
-# More units in use than this (as many as pairs drawn at random reach) take longer streamed, unless their matrices are small: 256 units of 2,048
-# x 256, 8 a token, 8 / 10 / 16 tokens 64 / 82 / 129 us against 67 / 75 / 100; 128 units of 2,048 x 768 10 / 12 / 16 tokens 130 / 151 / 192
-# against 137 / 146 / 179; 64 units of 2,048 x 512 16 tokens 95 against 96; 128 plain units of 512 x 128 16 tokens 24 against 31.
+# More units in use than this (as many as pairs drawn at random reach) go the other way, unless their matrices are small. (The line comes from an
+# earlier form of the kernel: 256 units of 2,048 x 256, 8 a token, 12 / 16 / 32 tokens now take 64 / 76 / 140 us streamed, 97 / 103 / 143 grouped.)
 EXPERT_STREAM_UNITS = 64
 EXPERT_STREAM_BYTES = 64 << 20
 
