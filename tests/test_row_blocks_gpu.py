@@ -117,7 +117,7 @@ def test_delta_inputs_in_runs_of_tokens(ops, taps, G, D, HV):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("size", [40, 1000, 2048, 4100, 9000])
+@pytest.mark.parametrize("size", [40, 1000, 2048, 4100, 9000, 12032, 12036, 12252, 12256, 12288, 12292])
 def test_gated_rows_of_the_lightning_mixer_in_small_and_large_steps(ops, dtype, size):
     g = torch.Generator(device="cuda").manual_seed(size)
     n = 300                                                # more rows than SMs

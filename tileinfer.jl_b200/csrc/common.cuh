@@ -77,6 +77,9 @@ inline cudaError_t ti_launch_after(void (*kernel)(KArgs...), dim3 grid, dim3 blo
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Dynamic shared memory that a launch may have unasked: 48 KB less a kernel's static arrays, which count too (less than 1 KB each).
+#define TI_SMEM_UNASKED (47 * 1024)
+
 #define TI_REQUIRE(cond, ...)                \
     do {                                     \
         if (!(cond)) return ti_fail(__VA_ARGS__); \
