@@ -116,6 +116,22 @@ def test_delta_inputs_in_runs_of_tokens(ops, taps, G, D, HV):
         at += length
 
 
+@pytest.mark.parametrize("n,G,D,HV", [(1500, 1, 1534, 0), (1500, 1, 1536, 8), (1500, 1, 1540, 8), (3, 1, 12288, 0)])
+def test_delta_inputs_of_rows_at_the_shared_memory_limit(ops, n, G, D, HV):
+    """A block's rows and its table of tokens fill 48 KB, or a little less or more."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    proj = torch.randn(n, 2 * G * D + HV, generator=g, device="cuda").bfloat16()
+    out = torch.empty(n, 2 * G * D + HV, device="cuda")
+    ops.delta_inputs(out, proj, None, 0, None, _step([n]), G, D, HV, 1e-6)
+    y = proj.double() * torch.sigmoid(proj.double())
+    heads = y[:, :2 * G * D].view(n, 2 * G, D)
+    heads = heads / torch.sqrt((heads * heads).sum(-1, keepdim=True) + 1e-6)
+    heads[:, :G] *= D ** -0.5
+    want = torch.cat([heads.reshape(n, -1), y[:, 2 * G * D:]], 1)
+    # An exponential, a quotient, and a head's sum of squares: 2^-24 for each of its D / 32 additions in a row.
+    assert float((out.double() - want).abs().max()) <= 2.0 ** -24 * (16 + D / 32) * float(y.abs().max())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("size", [40, 1000, 2048, 4100, 9000, 12032, 12036, 12252, 12256, 12288, 12292])
 def test_gated_rows_of_the_lightning_mixer_in_small_and_large_steps(ops, dtype, size):

@@ -678,11 +678,11 @@ extern "C" int ti_delta_inputs(float* out, const void* proj, long long ld, const
     // Heads' worth of channels a block: about DI_THREADS of them; eight tokens in a row once single ones would be some 20 blocks an SM (4,096
     // channels, single / eight: 100 tokens 5.7 / 6.8 us, 200 10.5 / 9.8, 2,048 89 / 54; 2,048 channels, 300 tokens 8.0 / 8.9, 600 14.7 / 11.9).
     const int heads = D >= DI_THREADS ? 1 : DI_THREADS / D, per = heads * D < C ? heads * D : C, parts = (C + per - 1) / per;
-    const bool runs = (long long)n * parts > 20LL * ti_sm_count() && (size_t)8 * per * sizeof(float) <= 48 * 1024;
+    const bool runs = (long long)n * parts > 20LL * ti_sm_count() && (size_t)8 * per * sizeof(float) <= TI_SMEM_UNASKED;
     const size_t smem = (size_t)(runs ? 8 : 1) * per * sizeof(float);
     TI_DISPATCH_DTYPE(dtype, {
         auto launch = [&](auto kernel) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             ti_launch(kernel, dim3(runs ? (n + 7) / 8 : n, parts), dim3(DI_THREADS), smem, stream, out, (const T*)proj, ld, (const T*)conv, taps, hist, hist_stride,
                       cu_seqlens, seq_slots, B, n, G, D, HV, unit_eps, per);
         };
