@@ -116,6 +116,31 @@ def test_delta_inputs_in_runs_of_tokens(ops, taps, G, D, HV):
         at += length
 
 
+def test_rows_of_steps_with_sequences_without_tokens(ops):
+    """As many sequences as tokens, some with none and some with several: the rows before are each sequence's own."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    W, G, D, HV, taps = 96, 1, 24, 48, 4
+    for lengths in ([0, 2], [2, 0], [1, 0, 0, 3], [1, 2, 0, 1]):
+        n, B = sum(lengths), len(lengths)
+        h, mu = torch.randn(n, W, generator=g, device="cuda"), torch.randn(2, W, generator=g, device="cuda")
+        prev, hist = torch.randn(B, W, generator=g, device="cuda"), torch.randn(B, (taps - 1) * W, generator=g, device="cuda")
+        conv = torch.randn(W, taps, generator=g, device="cuda")
+        state, out, rows = prev.clone(), torch.empty(2, n, W, device="cuda"), torch.empty(n, W, device="cuda")
+        ops.shift_blend(out, h, mu, state, _step(lengths))
+        ops.delta_inputs(rows, h, conv, taps, hist, _step(lengths), G, D, HV, 1e-6)
+        at = 0
+        for b, length in enumerate(lengths):
+            if not length:
+                assert torch.equal(state[b], prev[b])
+                continue
+            own = prev[b:b + 1].clone()
+            one, part = torch.empty(2, length, W, device="cuda"), torch.empty(length, W, device="cuda")
+            ops.shift_blend(one, h[at:at + length].contiguous(), mu, own, _step([length]))
+            ops.delta_inputs(part, h[at:at + length].contiguous(), conv, taps, hist[b:b + 1].contiguous(), _step([length]), G, D, HV, 1e-6)
+            assert torch.equal(out[:, at:at + length], one) and torch.equal(state[b], own[0]) and torch.equal(rows[at:at + length], part)
+            at += length
+
+
 @pytest.mark.parametrize("n,G,D,HV", [(1500, 1, 1534, 0), (1500, 1, 1536, 8), (1500, 1, 1540, 8), (3, 1, 12288, 0)])
 def test_delta_inputs_of_rows_at_the_shared_memory_limit(ops, n, G, D, HV):
     """A block's rows and its table of tokens fill 48 KB, or a little less or more."""

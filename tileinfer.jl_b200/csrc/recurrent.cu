@@ -24,22 +24,30 @@ __device__ __forceinline__ float rs_softplus(float z) { return z > 20.f ? z : lo
 
 // Where the RUN tokens from `first` on lie: every token's sequence's first token of the step, that sequence's slot and the one after its last token.
 // Asked by a whole block ahead of the wait (the step's tables were uploaded before its first kernel). One warp looks, a lane per token:
-// thousands of warps that each go through the same few words queue for them at L2. With one token a sequence there is nothing to look for.
+// thousands of warps that each go through the same few words queue for them at L2. Where the step has as many sequences as tokens, token t is
+// sequence t's only one, unless some sequence has none.
 template <int RUN> struct TokenRun {
     int t0[RUN], t1[RUN], slot[RUN];
     __device__ __forceinline__ void find(const int* cu, const int* slots, int B, int n, int first) {
         if (threadIdx.x < RUN && first + (int)threadIdx.x < n) {
             const int i = threadIdx.x, t = first + i;
-            int lo = 0, hi = B - 1;
-            if (n == B) lo = t;
-            else
+            bool found = false;
+            if (n == B) {
+                t0[i] = __ldcg(cu + t);
+                t1[i] = __ldcg(cu + t + 1);
+                slot[i] = __ldcg(slots + t);
+                found = t0[i] == t && t1[i] == t + 1;
+            }
+            if (!found) {
+                int lo = 0, hi = B - 1;
                 while (lo < hi) {
                     const int mid = (lo + hi + 1) >> 1;
                     if (__ldcg(cu + mid) <= t) lo = mid; else hi = mid - 1;
                 }
-            t0[i] = n == B ? t : __ldcg(cu + lo);
-            t1[i] = n == B ? t + 1 : __ldcg(cu + lo + 1);
-            slot[i] = __ldcg(slots + lo);
+                t0[i] = __ldcg(cu + lo);
+                t1[i] = __ldcg(cu + lo + 1);
+                slot[i] = __ldcg(slots + lo);
+            }
         }
         __syncthreads();
     }
