@@ -141,6 +141,16 @@ def test_rows_of_steps_with_sequences_without_tokens(ops):
             at += length
 
 
+@pytest.mark.parametrize("G,D,HV", [(0, 0, 300), (2, 0, 1000), (0, 24, 40), (0, 0, 0)])
+def test_delta_inputs_without_heads(ops, G, D, HV):
+    """Values alone: no head to norm, and none to divide a block's channels by."""
+    proj = torch.randn(5, HV, generator=torch.Generator(device="cuda").manual_seed(HV), device="cuda")
+    out = torch.empty(5, HV, device="cuda")
+    ops.delta_inputs(out, proj, None, 0, None, _step([5]), G, D, HV, 1e-6)
+    want = proj.double() * torch.sigmoid(proj.double())
+    assert HV == 0 or float((out.double() - want).abs().max()) <= 2.0 ** -20 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("n,G,D,HV", [(1500, 1, 1534, 0), (1500, 1, 1536, 8), (1500, 1, 1540, 8), (3, 1, 12288, 0)])
 def test_delta_inputs_of_rows_at_the_shared_memory_limit(ops, n, G, D, HV):
     """A block's rows and its table of tokens fill 48 KB, or a little less or more."""

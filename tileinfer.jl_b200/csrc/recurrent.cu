@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(DI_THREADS) delta_inputs_kernel(float* __restr
         }
     }
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head0 = c0 / D, heads = max(0, min(2 * G - head0, channels / D));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head0 = D > 0 ? c0 / D : 0, heads = D > 0 ? max(0, min(2 * G - head0, channels / D)) : 0;
     for (int e = warp; e < heads * count; e += DI_THREADS / 32) {              // a warp per q or k head of a token
         const int hd = head0 + e % heads;
         float* src = y + (e / heads) * per + (size_t)hd * D - c0;
@@ -681,11 +681,13 @@ extern "C" int ti_delta_inputs(float* out, const void* proj, long long ld, const
                                cudaStream_t stream) {
     if (n == 0) return 0;
     const int C = 2 * G * D + HV;
+    TI_REQUIRE(G >= 0 && D >= 0 && HV >= 0, "delta_inputs: %d heads of %d, %d values", G, D, HV);
     TI_REQUIRE(taps >= 0 && taps <= 64 && (taps <= 1 || hist != nullptr) && (taps == 0 || conv != nullptr), "delta_inputs: %d taps", taps);
     TI_REQUIRE((size_t)C * sizeof(float) <= 160 * 1024, "delta_inputs: %d channels", C);
+    if (C == 0) return 0;
     // Heads' worth of channels a block: about DI_THREADS of them; eight tokens in a row once single ones would be some 20 blocks an SM (4,096
     // channels, single / eight: 100 tokens 5.7 / 6.8 us, 200 10.5 / 9.8, 2,048 89 / 54; 2,048 channels, 300 tokens 8.0 / 8.9, 600 14.7 / 11.9).
-    const int heads = D >= DI_THREADS ? 1 : DI_THREADS / D, per = heads * D < C ? heads * D : C, parts = (C + per - 1) / per;
+    const int whole = D == 0 || D >= DI_THREADS ? 1 : DI_THREADS / D, want = D > 0 ? whole * D : DI_THREADS, per = want < C ? want : C, parts = (C + per - 1) / per;
     const bool runs = (long long)n * parts > 20LL * ti_sm_count() && (size_t)8 * per * sizeof(float) <= TI_SMEM_UNASKED;
     const size_t smem = (size_t)(runs ? 8 : 1) * per * sizeof(float);
     TI_DISPATCH_DTYPE(dtype, {
