@@ -274,9 +274,9 @@ def test_grouped_products_on_pairs_of_sms(ops, out, k):
 
 
 @pytest.mark.parametrize("D,nq,nkv,B", [(128, 8, 8, 50), (128, 40, 4, 100), (256, 16, 8, 45), (128, 6, 6, 90)])
-def test_decode_attention_on_half_pages(D, nq, nkv, B):
-    """So many unsplit sequences that blocks of half pages are taken: lengths on both sides of a page's and a half's end, a window, kept first
-    positions, a sink; against 64-bit arithmetic."""
+def test_decode_attention_of_many_unsplit_sequences(D, nq, nkv, B):
+    """A block per sequence and KV head, more of them than places: lengths on both sides of a page's end and of a warp's keys, a window, kept
+    first positions, a sink; against 64-bit arithmetic."""
     from tileinfer_b200.kernels import fast
     from tileinfer_b200.kernels.library import lib
     g = torch.Generator(device="cuda").manual_seed(D + B)

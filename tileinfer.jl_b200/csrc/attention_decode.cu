@@ -19,32 +19,29 @@
 
 #define AD_MAX_SPLITS 64
 
-// A block of WARPS warps walks tiles of 16 keys a warp: whole pages, or halves of them.
-template <int D, int WARPS> struct DecodeSmem {
+template <int D> struct DecodeSmem {
     static constexpr int STAGES = D <= 128 ? 3 : 2;
-    static constexpr int KEYS = 16 * WARPS;
-    static constexpr int TILE = KEYS * D;                    // elements of one K or V tile
+    static constexpr int TILE = AD_PAGE * D;                 // elements of one K or V tile
     static constexpr size_t BYTES = (size_t)STAGES * 2 * TILE * sizeof(bf16);
 };
 
-template <int D, int WARPS>
+template <int D>
 __device__ __forceinline__ void load_tile(bf16* dst, const bf16* src) {
     constexpr int CPR = D / 8;
-    for (int c = threadIdx.x; c < 16 * WARPS * CPR; c += 32 * WARPS) {
+    for (int c = threadIdx.x; c < AD_PAGE * CPR; c += AD_THREADS) {
         const int row = c / CPR, cc = c % CPR;
         cp_async16(smem_u32(dst + (row * CPR + swz<D>(row, cc)) * 8), src + (size_t)c * 8);
     }
 }
 
-template <int D, bool TABLE, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) attention_decode_kernel(
+template <int D, bool TABLE>
+__global__ void __launch_bounds__(AD_THREADS) attention_decode_kernel(
     bf16* __restrict__ out, const bf16* q, const bf16* k_cache, const bf16* v_cache,
     const int* block_table, int table_stride, const int* seq_slots,
     const int* kv_lens, const int* work, float* __restrict__ ws_o, float* __restrict__ ws_ml, float scale_log2e, int nq,
     int nkv, int splits, int window, const float* __restrict__ sink, AttnExtras ex) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    typedef DecodeSmem<D, WARPS> SM;
-    constexpr int KEYS = SM::KEYS, PER_PAGE = AD_PAGE / KEYS;
+    typedef DecodeSmem<D> SM;
     constexpr int KS = D / 16, NT = D / 8;
     bf16* tiles = reinterpret_cast<bf16*>(smem_raw);
 
@@ -73,9 +70,9 @@ __global__ void __launch_bounds__(32 * WARPS) attention_decode_kernel(
     // kernel that writes this step's key, value and query.
     int first_key = (window > 0 && kv_len > window) ? kv_len - window : 0;
     if (ex.chunk > 0 && kv_len > 0) first_key = max(first_key, ((kv_len - 1) / ex.chunk) * ex.chunk);       // the chunk of the step's token
-    const int t_begin = first_key / KEYS, t_end = (kv_len + KEYS - 1) / KEYS;
-    // The tiles to walk: those of the kept first keys that lie before the window's, then [t_begin, t_end).
-    const int kept = min((ex.keep + KEYS - 1) / KEYS, t_begin), n_tiles = kept + t_end - t_begin;
+    const int t_begin = first_key / AD_PAGE, t_end = (kv_len + AD_PAGE - 1) / AD_PAGE;
+    // The pages to walk: those of the kept first keys that lie before the window's, then [t_begin, t_end).
+    const int kept = min((ex.keep + AD_PAGE - 1) / AD_PAGE, t_begin), n_tiles = kept + t_end - t_begin;
     const int my_lo = (int)((long long)n_tiles * split / parts), my_hi = (int)((long long)n_tiles * (split + 1) / parts);
     auto tile_at = [&](int i) { return i < kept ? i : t_begin + i - kept; };
     const int* table = block_table + (size_t)__ldcg(seq_slots + b) * table_stride;
@@ -83,15 +80,14 @@ __global__ void __launch_bounds__(32 * WARPS) attention_decode_kernel(
 
     auto issue = [&](int i, int stage) {
         if (i < my_hi) {
-            if (i == n_tiles - 1 && !waited) {              // the tile that this step writes to
+            if (i == n_tiles - 1 && !waited) {              // the page that this step writes to
                 pdl_wait();
                 pdl_launch_dependents();
                 waited = true;
             }
-            const int at = tile_at(i);
-            const size_t base = (((size_t)__ldcg(table + at / PER_PAGE) * nkv + kvh) * AD_PAGE + at % PER_PAGE * KEYS) * D;
-            load_tile<D, WARPS>(tiles + (size_t)stage * 2 * SM::TILE, k_cache + base);
-            load_tile<D, WARPS>(tiles + (size_t)stage * 2 * SM::TILE + SM::TILE, v_cache + base);
+            const size_t base = ((size_t)__ldcg(table + tile_at(i)) * nkv + kvh) * AD_PAGE * D;
+            load_tile<D>(tiles + (size_t)stage * 2 * SM::TILE, k_cache + base);
+            load_tile<D>(tiles + (size_t)stage * 2 * SM::TILE + SM::TILE, v_cache + base);
         }
         cp_async_commit();
     };
@@ -138,7 +134,7 @@ __global__ void __launch_bounds__(32 * WARPS) attention_decode_kernel(
         const bf16* kt = tiles + (size_t)stage * 2 * SM::TILE;
         const bf16* vt = kt + SM::TILE;
 
-        decode_tile<D>(kt, vt, qf, o, m0, m1, l0, l1, tile * KEYS, warp, lane, kv_len, first_key, scale_log2e, bias0, bias1, ex.bias_len, ex,
+        decode_tile<D>(kt, vt, qf, o, m0, m1, l0, l1, tile, warp, lane, kv_len, first_key, scale_log2e, bias0, bias1, ex.bias_len, ex,
                        slope0, slope1);
     }
     cp_async_wait<0>();
@@ -162,15 +158,15 @@ __global__ void __launch_bounds__(32 * WARPS) attention_decode_kernel(
         }
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < group * D; e += 32 * WARPS) {
+    for (int e = threadIdx.x; e < group * D; e += AD_THREADS) {
         const int row = e / D, d = e % D;
         float M = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) M = fmaxf(M, mg[((size_t)w * 16 + row) * RS + D]);
+        for (int w = 0; w < AD_WARPS; ++w) M = fmaxf(M, mg[((size_t)w * 16 + row) * RS + D]);
         const float base = M == -INFINITY ? 0.f : M;
         float L = 0.f, O = 0.f;
 #pragma unroll
-        for (int w = 0; w < WARPS; ++w) {
+        for (int w = 0; w < AD_WARPS; ++w) {
             const float* src = mg + ((size_t)w * 16 + row) * RS;
             const float f = exp2f(src[D] - base);
             L += src[D + 1] * f;
@@ -270,35 +266,22 @@ template <int D>
 static int launch_decode(bf16* out, const bf16* q, const bf16* k, const bf16* v, const int* table, int table_stride,
                          const int* seq_slots, const int* kv_lens, const int* work, const int* seq_work, float* ws_o, float* ws_ml,
                          float scale, int B, int nq, int nkv, int splits, int window, const float* sink, AttnExtras ex, cudaStream_t stream) {
-    const int slabs = (nq / nkv + 15) / 16;
-    auto smem = [](int warps, size_t tiles) { const size_t merge = (size_t)warps * 16 * (D + 2) * 4; return tiles > merge ? tiles : merge; };
-    const size_t whole = smem(AD_WARPS, DecodeSmem<D, AD_WARPS>::BYTES), half = smem(AD_WARPS / 2, DecodeSmem<D, AD_WARPS / 2>::BYTES);
     static bool configured = false;
-    static int fit_whole = 1, fit_half = 1;                  // blocks that an SM holds
+    const size_t smem = DecodeSmem<D>::BYTES > (size_t)AD_WARPS * 16 * (D + 2) * 4 ? DecodeSmem<D>::BYTES
+                                                                                    : (size_t)AD_WARPS * 16 * (D + 2) * 4;
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<D, false, AD_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)whole);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_kernel<D, true, AD_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)whole);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_kernel<D, false, AD_WARPS / 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)half);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit_whole, attention_decode_kernel<D, false, AD_WARPS>, 32 * AD_WARPS, whole);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit_half, attention_decode_kernel<D, false, AD_WARPS / 2>, 16 * AD_WARPS, half);
+        cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(attention_decode_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return ti_fail("attention_decode: %s", cudaGetErrorString(e));
-        if (fit_whole < 1) fit_whole = 1;
-        if (fit_half < 1) fit_half = 1;
         configured = true;
     }
-    // Where a sequence's keys are not split, its blocks may need several rounds of the SMs. Blocks of half as many warps, on half pages, take 1.75
-    // times as long (head size 256: 2.2), but twice or three times as many fit: they are taken where their rounds come to less and the last round of whole ones is not
-    // nearly empty (with a margin: 200 sequences of 16 KV heads, 11 rounds against 6, take 4 % longer in halves), from head size 128 on (128, 8 KV heads, us, whole / half: 48 sequences of 200 / 1,024 positions 17.7 / 14.0, 49.4 / 48.3; 64 18.7 / 15.0, 52.0 /
-    // 49.6; 96 of 1,024 77.7 / 96.4; 256, 4 KV heads: 80 of 200 / 1,024 33.4 / 20.8, 90.4 / 69.4; 64, 8 KV heads: 96 of 1,024 46.6 / 54.6).
-    const long long blocks = (long long)B * nkv * slabs, place = (long long)fit_whole * ti_sm_count(), rounds = (blocks + place - 1) / place;
-    const long long half_rounds = (blocks + (long long)fit_half * ti_sm_count() - 1) / ((long long)fit_half * ti_sm_count());
-    const bool halves = splits == 1 && D >= 128 && (D > 128 ? 9 : 7.5) * half_rounds < 4 * rounds && 4 * (blocks - (rounds - 1) * place) >= place;
-#define AD_LAUNCH(TABLE, WARPS, GRID, SMEM) ti_launch(attention_decode_kernel<D, TABLE, WARPS>, GRID, dim3(32 * (WARPS)), SMEM, stream, out, q, k, v, table, table_stride, \
-                                                    seq_slots, kv_lens, work, ws_o, ws_ml, scale * 1.4426950408889634f, nq, nkv, splits, window, sink, ex)
-    if (work != nullptr && splits > 1) AD_LAUNCH(true, AD_WARPS, dim3(B * splits, nkv * slabs), whole);
-    else if (halves) AD_LAUNCH(false, AD_WARPS / 2, dim3(1, nkv * slabs, B), half);
-    else AD_LAUNCH(false, AD_WARPS, dim3(splits, nkv * slabs, B), whole);
-#undef AD_LAUNCH
+    const int slabs = (nq / nkv + 15) / 16;
+    if (work != nullptr && splits > 1)
+        ti_launch(attention_decode_kernel<D, true>, dim3(B * splits, nkv * slabs), dim3(AD_THREADS), smem, stream, out, q, k, v, table, table_stride,
+                  seq_slots, kv_lens, work, ws_o, ws_ml, scale * 1.4426950408889634f, nq, nkv, splits, window, sink, ex);
+    else
+        ti_launch(attention_decode_kernel<D, false>, dim3(splits, nkv * slabs, B), dim3(AD_THREADS), smem, stream, out, q, k, v, table, table_stride,
+                  seq_slots, kv_lens, work, ws_o, ws_ml, scale * 1.4426950408889634f, nq, nkv, splits, window, sink, ex);
     if (int rc = ti_check_launch("attention_decode")) return rc;
     if (splits > 1) {
         ti_launch(attention_combine_kernel, dim3(B * nq), dim3(D <= 64 ? 64 : 128), 0, stream, out, ws_o, ws_ml, seq_work, D, nq, splits, sink);

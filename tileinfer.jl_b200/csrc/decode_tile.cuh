@@ -1,16 +1,17 @@
-// One tile of decode attention (16 keys a warp of the block) for one warp: the warp takes its 16 keys of the tile, the rows of
+// One 64-key tile of decode attention for one warp: the warp takes 16 keys of the tile, the rows of
 // the MMA tiles are the query heads that share the KV head. Shared by the decode kernels.
 #pragma once
 #include "mma_util.cuh"
 
 #define AD_PAGE 64
 #define AD_WARPS 4
+#define AD_THREADS (AD_WARPS * 32)
 
-// first_of_tile: the tile's first key; kt, vt: the K and V tiles in (swizzled) shared memory; qf: the query fragments; o, m, l: this warp's
+// kt, vt: the K and V tiles in (swizzled) shared memory; qf: the query fragments; o, m, l: this warp's
 // running output, maximum and sum for rows g and g + 8 (32-bit).
 template <int D>
 __device__ __forceinline__ void decode_tile(const bf16* kt, const bf16* vt, const unsigned (&qf)[D / 16][4], float (&o)[D / 8][4],
-                                            float& m0, float& m1, float& l0, float& l1, int first_of_tile, int warp, int lane,
+                                            float& m0, float& m1, float& l0, float& l1, int tile, int warp, int lane,
                                             int kv_len, int first_key, float scale_log2e, const float* __restrict__ bias0 = nullptr,
                                             const float* __restrict__ bias1 = nullptr, int bias_len = 0, const AttnExtras& ex = AttnExtras{},
                                             float slope0 = 0.f, float slope1 = 0.f) {
@@ -32,7 +33,7 @@ __device__ __forceinline__ void decode_tile(const bf16* kt, const bf16* vt, cons
             mma16816(s[1], qf[ks], kb[2], kb[3]);
         }
     }
-    const int key0 = first_of_tile + warp * 16 + 2 * t;
+    const int key0 = tile * AD_PAGE + warp * 16 + 2 * t;
     float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
     for (int nt = 0; nt < 2; ++nt)
