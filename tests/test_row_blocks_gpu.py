@@ -168,6 +168,53 @@ def test_delta_inputs_of_rows_at_the_shared_memory_limit(ops, n, G, D, HV):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [2, 300])
+@pytest.mark.parametrize("fill", [11900, 12256, 12288, 12352])
+def test_rows_that_fill_the_shared_memory_a_launch_may_have_unasked(ops, dtype, n, fill):
+    """Kernels that keep ``fill`` floats of a row, or of two rows, in dynamic shared memory beside their static arrays, around 48 KB."""
+    g = torch.Generator(device="cuda").manual_seed(fill + n)
+    R = lambda *s, dtype=dtype: torch.randn(*s, generator=g, device="cuda").to(dtype)             # noqa: E731
+    rms = lambda t: t / torch.sqrt((t * t).mean(-1, keepdim=True) + 1e-6)                          # noqa: E731
+    step_of = 2.0 ** -8 if dtype == torch.bfloat16 else 0.0
+
+    def close(got, want, rounded):
+        # Sums of squares over a row, a root, a quotient and a few products; where the result is of the element type, one rounding more.
+        assert float(((got.double() - want).abs() - (step_of if rounded else 0.0) * want.abs()).max()) <= 2.0 ** -18 * float(want.abs().max())
+
+    for op in ("streams", "branch", "sum"):
+        x, d, w, w2, h = R(n, fill, dtype=torch.float32), R(n, fill), R(fill), R(fill), torch.empty(n, fill, dtype=dtype, device="cuda")
+        was, D = x.double(), d.double()
+        if op == "streams":
+            ops.streams_read_norm(h, x, torch.ones(1, device="cuda"), w, None, 1e-6, centred=False)
+            close(h, rms(was) * w.double(), True)
+            ops.streams_update(x, d, [0.5], [2.0], [1.0], h, w, None, 1e-6, centred=False)
+            want = 0.5 * was + 2.0 * D
+        elif op == "branch":
+            ops.branch_norm_add32(x, d, w2, 1e-6, 0.5, h=h, out_norm=(w, 1e-6, False))
+            want = was + 0.5 * rms(D) * w2.double()
+        else:
+            ops.sum_add_norm32(x, d, None, h, w, 1e-6)
+            want = was + D
+        close(x, want, False)
+        close(h, rms(want) * w.double(), True)
+    half = fill // 2
+    a, b, wa, wb, w, out = R(n, half), R(n, half), R(half), R(half), R(half), torch.empty(n, half, device="cuda")
+    pair = 0.5 * rms(a.double()) * wa.double() + 2.0 * rms(b.double()) * wb.double()
+    ops.pair_combine(out, a, b, wa, wb, 1e-6, 0.5, 2.0, dtype)
+    close(out, pair, False)
+    x, h = R(n, half, dtype=torch.float32), torch.empty(n, half, dtype=dtype, device="cuda")
+    want = x.double() + pair
+    ops.pair_add_norm32(x, a, b, wa, wb, 0.5, 2.0, 1e-6, 1.0, h, w, 1e-6)
+    close(x, want, False)
+    close(h, rms(want) * w.double(), True)
+    rows, q = R(n, fill), torch.empty(n, fill // 4, 4, dtype=dtype, device="cuda")
+    step = _step([n])
+    step.positions, step.kv_lens = torch.arange(n, device="cuda").int(), torch.tensor([n], device="cuda").int()
+    ops.conv_attention_inputs(rows, None, None, 0, None, None, None, 1e-6, None, q, None, None, step, None, fill // 4, 1, 4, 4, 4, 64, write_kv=False)
+    assert torch.equal(q.view(n, fill), rows)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("size", [40, 1000, 2048, 4100, 9000, 12032, 12036, 12252, 12256, 12288, 12292])
 def test_gated_rows_of_the_lightning_mixer_in_small_and_large_steps(ops, dtype, size):
     g = torch.Generator(device="cuda").manual_seed(size)

@@ -267,10 +267,10 @@ extern "C" int ti_conv_attention_inputs(const void* proj, long long ld, const vo
 #define CI_LAUNCH(TAPS)                                                                                                                       \
     do {                                                                                                                                      \
         if (quads) {                                                                                                                          \
-            if (smem > 48 * 1024) cudaFuncSetAttribute(conv_attention_inputs_kernel<T, TAPS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(conv_attention_inputs_kernel<T, TAPS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             CI_ONE(TAPS, true);                                                                                                               \
         } else {                                                                                                                              \
-            if (smem > 48 * 1024) cudaFuncSetAttribute(conv_attention_inputs_kernel<T, TAPS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(conv_attention_inputs_kernel<T, TAPS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             CI_ONE(TAPS, false);                                                                                                              \
         }                                                                                                                                     \
     } while (0)
@@ -288,7 +288,7 @@ extern "C" int ti_conv_attention_inputs(const void* proj, long long ld, const vo
             case 3: CI_LAUNCH(3); break;
             case 4: CI_LAUNCH(4); break;
             default:
-                if (smem > 48 * 1024) cudaFuncSetAttribute(conv_attention_inputs_kernel<T, -1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(conv_attention_inputs_kernel<T, -1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 CI_ONE(-1, false);
                 break;
         }

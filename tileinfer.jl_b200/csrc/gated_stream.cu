@@ -197,7 +197,7 @@ extern "C" int ti_gated_add_norm32(float* x, const void* d, const float* d_parti
         const uintptr_t mask = sizeof(T) == 2 ? 7 : 15;
         const bool vec = size % 4 == 0 && aligned16(x) && (((uintptr_t)h | (uintptr_t)w | (uintptr_t)conv | (uintptr_t)conv_out) & mask) == 0 &&
                          aligned16(hist) && hist_stride % 4 == 0 && row_vec_ok(db, sizeof(T)) && row_vec_ok(gb, sizeof(T));
-        if (smem > 48 * 1024) {
+        if (smem > TI_SMEM_UNASKED) {
             cudaFuncSetAttribute(gated_add_norm32_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             cudaFuncSetAttribute(gated_add_norm32_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         }
@@ -270,7 +270,7 @@ extern "C" int ti_pair_add_norm32(float* x, const void* a, const float* a_partia
         const uintptr_t mask = sizeof(T) == 2 ? 7 : 15;
         const bool vec = size % 4 == 0 && aligned16(x) && (((uintptr_t)h | (uintptr_t)w | (uintptr_t)wa | (uintptr_t)wb) & mask) == 0 && row_vec_ok(p.a, sizeof(T)) &&
                          row_vec_ok(p.b, sizeof(T));
-        if (smem > 48 * 1024) {
+        if (smem > TI_SMEM_UNASKED) {
             cudaFuncSetAttribute(pair_add_norm32_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             cudaFuncSetAttribute(pair_add_norm32_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         }

@@ -204,7 +204,7 @@ extern "C" int ti_streams_read_norm(void* h, const float* x, const float* a, int
     const size_t smem = (size_t)size * sizeof(float);
     TI_REQUIRE(smem <= 160 * 1024, "streams_read_norm: rows of %d", size);
     TI_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(streams_read_norm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(streams_read_norm_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ti_launch(streams_read_norm_kernel<T>, dim3(n), dim3(hs_block(size, n)), smem, stream, (T*)h, x, a, S, (const T*)w, (const T*)b, eps, centred, size,
                   hs_threads(size));
     });
@@ -229,7 +229,7 @@ extern "C" int ti_streams_update(float* x, const void* delta, const float* parti
     const int threads = hs_block(size, n);
     TI_DISPATCH_DTYPE(dtype, {
         auto launch = [&](auto kernel) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             ti_launch(kernel, dim3(n), dim3(threads), smem, stream, x, (const T*)delta, partials, n_partials, (size_t)partial_stride, tab, S, (T*)h,
                       (const T*)w, (const T*)b, eps, centred, size, hs_threads(size));
         };

@@ -315,7 +315,7 @@ static void launch_decay_scan(float* o, const T* rkv, long long ld, int r_off, i
     const int cols = warps * (32 / G);
     const size_t smem = (size_t)(2 * 3 * RS_BATCH * G * (R + 4) + 2 * RS_BATCH * cols + RS_BATCH * warps * 32) * sizeof(float);
     auto launch = [&](auto kernel) {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ti_launch_after(kernel, dim3((D + cols - 1) / cols, H, B), dim3(warps * 32), smem, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u, state, state_stride,
                   cu_seqlens, seq_slots, H, D);
     };
@@ -522,7 +522,7 @@ static void launch_delta_scan(float* o, const float* qkv, long long ld, const fl
     const int cols = warps * (32 / G);
     const size_t smem = (size_t)(4 * RS_BATCH * G * (RS_ROWS + 4) + 2 * RS_BATCH * cols + 4 * RS_BATCH + RS_BATCH * warps * 32) * sizeof(float);
     const int vec = D % 4 == 0 && ld % 4 == 0 && aligned16(qkv) && warps * 32 >= D / 4;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(delta_scan_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(delta_scan_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     ti_launch_after(delta_scan_kernel<G>, dim3((V + cols - 1) / cols, H, B), dim3(warps * 32), smem, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride,
               cu_seqlens, seq_slots, H, GQ, D, V, vec);
 }
@@ -843,7 +843,7 @@ extern "C" int ti_pair_combine(float* out, const void* a, const float* pa, int n
     const size_t smem = (size_t)2 * size * sizeof(float);
     TI_REQUIRE(smem <= 160 * 1024, "pair_combine: rows of %d", size);
     TI_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(pair_combine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(pair_combine_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         const int sum_threads = size >= 1024 ? 256 : 128, all = size > 1024 ? 1024 : (size + 31) / 32 * 32;
         const int threads = n <= ti_sm_count() && all > sum_threads ? all : sum_threads;
         ti_launch(pair_combine_kernel<T>, dim3(n), dim3(threads), smem, stream, out, (const T*)a, pa, na, (size_t)sa_stride, (const T*)b,

@@ -328,7 +328,7 @@ extern "C" int ti_ssm_gate_norm(void* out, const float* y, const void* z, long l
     const size_t smem = (size_t)((size + 3) / 4 * 4 + parts + (parts > threads / 32 ? parts : threads / 32)) * sizeof(float);
     TI_DISPATCH_DTYPE(dtype, {
         const bool vec = size % 4 == 0 && ldz % 4 == 0 && aligned16(y) && (((uintptr_t)out | (uintptr_t)z | (uintptr_t)w) & (sizeof(T) == 2 ? 7 : 15)) == 0;
-        if (smem > 48 * 1024) {
+        if (smem > TI_SMEM_UNASKED) {
             cudaFuncSetAttribute(ssm_gate_norm_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             cudaFuncSetAttribute(ssm_gate_norm_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         }

@@ -501,10 +501,11 @@ extern "C" int ti_branch_norm_add32(float* x, const void* delta, const float* pa
     const int threads = row_threads(size);
     const size_t smem = (size_t)size * sizeof(float);
     TI_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) {
+        if (smem > TI_SMEM_UNASKED) {
             static bool raised = false;       // per element type (this block is instantiated once for each)
             if (!raised) {
                 cudaFuncSetAttribute(branch_norm_add32_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                cudaFuncSetAttribute(branch_norm_add32_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
                 raised = true;
             }
         }
@@ -625,7 +626,10 @@ extern "C" int ti_sum_add_norm32(float* x, const void* d1, const float* p1, int 
     TI_REQUIRE(h == nullptr || w_out != nullptr, "sum_add_norm32: the next input needs its norm's weight");
     const size_t smem = (size_t)size * sizeof(float);
     TI_DISPATCH_DTYPE(dtype, {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(sum_add_norm32_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        if (smem > TI_SMEM_UNASKED) {
+            cudaFuncSetAttribute(sum_add_norm32_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            cudaFuncSetAttribute(sum_add_norm32_vec_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 48 * 1024);
+        }
         const bool vec = sizeof(T) == 2 && size % 4 == 0 && smem <= 48 * 1024 && aligned16(x) && (p1 == nullptr || (aligned16(p1) && s1 % 4 == 0)) &&
                          (p2 == nullptr || (aligned16(p2) && s2 % 4 == 0)) &&
                          (((uintptr_t)d1 | (uintptr_t)d2 | (uintptr_t)h | (uintptr_t)w_out) & 7) == 0;
