@@ -184,8 +184,8 @@ extern "C" int ti_lightning_out(void* y, const float* o, const void* g, long lon
     TI_REQUIRE(size > 0, "lightning_out: size %d", size);
     const int sum_threads = size >= 4096 ? 512 : size >= 1024 ? 256 : 128, all = size > 1024 ? 1024 : (size + 31) / 32 * 32;
     const size_t kept = (size_t)size * sizeof(float);
-    // (Kept rows and the kernel's static arrays fit what a launch may have unasked.)
-    const int threads = n <= ti_sm_count() && all > sum_threads && kept <= TI_SMEM_UNASKED ? all : sum_threads;
+    // (Kept rows and the kernel's static arrays, less than 256 bytes, fit the 48 KB that a launch may have unasked.)
+    const int threads = n <= ti_sm_count() && all > sum_threads && kept + 256 <= 48 * 1024 ? all : sum_threads;
     TI_DISPATCH_DTYPE(dtype, (ti_launch(lightning_out_kernel<T>, dim3(n), dim3(threads), threads > sum_threads ? kept : 0, stream, (T*)y, o, (const T*)g, ldg,
                                         (const T*)w, eps, size, sum_threads)));
     return ti_check_launch("lightning_out");
