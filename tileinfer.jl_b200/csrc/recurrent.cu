@@ -8,10 +8,11 @@
 //
 // S is [dim][vdim] (key rows, value columns). A warp owns CB value columns of one (sequence, head) with all their key rows: G = 32 / CB groups
 // of R rows a column, a lane has the rows of one group in registers (G is the least power of two that holds the key size). What a token
-// reads out of the state is added up over a column's groups by shuffles, so the warps of a block share nothing but the staged inputs.
-// A step's tokens are walked in order from the state that earlier steps left, in batches of RS_BATCH tokens staged in shared memory. The
-// sums over the groups have one order (partners G / 2, ..., 2, 1 apart), in the one-token kernels too, so a result depends on the token's
-// place in its sequence alone, not on the batch or on how the prompt was cut.
+// reads out of the state is added up over a column's groups by shuffles, so the warps of a block share nothing but the staged inputs. (The decay
+// scan of keys above 64 shares a column's rows out among warps instead: see there.) A step's tokens are walked in order from the state that earlier
+// steps left, in batches of RS_BATCH tokens staged in shared memory. The groups' sums are added in ascending order everywhere, in the one-token
+// kernels too, and only those of groups that have rows of the key, so a result depends on the token's place in its sequence alone, not on the
+// batch or on how the prompt was cut.
 #include "mma_util.cuh"
 #include "packed_f32.cuh"
 
@@ -55,31 +56,42 @@ template <int RUN> struct TokenRun {
 
 // ------------------------------------------------------------------------------------------------ what both scans share
 // The launch of a scan: G groups of R rows hold a key of D elements; a block has `warps` warps of 32 / G columns.
-struct ScanShape { int groups, warps; };
+struct ScanShape { int groups, warps, through; };
 // Blocks of `most` warps share the staged rows of a head; where so few leave most SMs idle, smaller ones (a token's time is its warp's own
 // chain, and staging takes a small part of it).
 static ScanShape scan_shape(int rows, int D, int cols, long long heads, int most, int least) {
-    ScanShape s = {1, most};
+    ScanShape s = {1, most, 0};
     while (s.groups * rows < D) s.groups *= 2;
     auto blocks = [&] { const int per = s.warps * (32 / s.groups); return (cols + per - 1) / per * heads; };
+    if (blocks() > 4LL * ti_sm_count())                     // so many that warps without a column, which help with staging, take room from others
+        while (s.warps > 1 && s.warps / 2 * (32 / s.groups) >= cols) s.warps /= 2;
     while (s.warps > least && 2 * blocks() < ti_sm_count()) s.warps /= 2;
+    s.through = s.groups >= 8 && blocks() > 4LL * ti_sm_count();
     return s;
 }
-template <int G> __device__ __forceinline__ float groups_sum(float v) {      // lanes of a column are 32 / G apart
+// The sum over the groups of a column, whose lanes are 32 / G apart, in every lane of it; groups without rows of the key give zero. (One shuffle a
+// group: they do not wait for one another as a tree's would, and their additions in a row take no longer than its round trips.)
+template <int G> __device__ __forceinline__ float groups_sum(float v) {
+    const int first = (threadIdx.x & 31) % (32 / G);
+    float t[G], total = 0.f;
 #pragma unroll
-    for (int m = 16; m >= 32 / G; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-    return v;
+    for (int i = 0; i < G; ++i) t[i] = __shfl_sync(0xffffffffu, v, first + i * (32 / G));
+#pragma unroll
+    for (int i = 0; i < G; ++i) total += t[i];
+    return total;
 }
-// The same sum of G values that lie `stride` apart.
+// The same of the first `used` groups' values, which lie `stride` apart.
+__device__ __forceinline__ float groups_sum(const float* from, int stride, int used) {
+    float total = 0.f;
+    for (int i = 0; i < used; ++i) total += from[i * stride];
+    return total;
+}
+// All G of them.
 template <int G> __device__ __forceinline__ float groups_sum(const float* from, int stride) {
-    float v[G];
+    float total = 0.f;
 #pragma unroll
-    for (int i = 0; i < G; ++i) v[i] = from[i * stride];
-#pragma unroll
-    for (int m = G / 2; m >= 1; m >>= 1)
-#pragma unroll
-        for (int i = 0; i < m; ++i) v[i] += v[i + m];
-    return v[0];
+    for (int i = 0; i < G; ++i) total += from[i * stride];
+    return total;
 }
 // A staged row: a group's rows lie four floats further apart than they are many, so that a warp's 16-byte reads fall into different banks.
 template <int R> __device__ __forceinline__ int staged_at(int d) { return d + d / R * 4; }
@@ -88,21 +100,6 @@ template <int R> __device__ __forceinline__ void read_rows(f32x2 (&to)[R / 2], c
     for (int r = 0; r < R; r += 4) {
         const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(from + r);
         to[r / 2] = t.x; to[r / 2 + 1] = t.y;
-    }
-}
-template <int R> __device__ __forceinline__ void load_state(f32x2 (&s)[R / 2], const float* S, int row0, int col, int D, int V) {
-#pragma unroll
-    for (int r = 0; r < R; r += 2)
-        s[r / 2] = pack2(row0 + r < D && col < V ? __ldcg(S + (size_t)(row0 + r) * V + col) : 0.f,
-                         row0 + r + 1 < D && col < V ? __ldcg(S + (size_t)(row0 + r + 1) * V + col) : 0.f);
-}
-template <int R> __device__ __forceinline__ void store_state(float* S, const f32x2 (&s)[R / 2], int row0, int col, int D, int V) {
-#pragma unroll
-    for (int r = 0; r < R; r += 2) {
-        float lo, hi;
-        unpack2(s[r / 2], lo, hi);
-        if (row0 + r < D && col < V) S[(size_t)(row0 + r) * V + col] = lo;
-        if (row0 + r + 1 < D && col < V) S[(size_t)(row0 + r + 1) * V + col] = hi;
     }
 }
 __device__ __forceinline__ float rows_sum(f32x2 a, f32x2 b) {
@@ -125,6 +122,62 @@ __device__ __forceinline__ bf16 load_now(const bf16* p) {
 __device__ __forceinline__ void copy4(float* dst, const float* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src));
 }
+// A block's columns of the state. Where many blocks have few tokens each and a warp few columns (`through`), they pass through shared memory: a warp's
+// own columns are 8 or 16 bytes of a row, the block's a whole sector or more (64 sequences of two tokens, straight into the lanes / through: 16 heads of
+// 256 x 256 726 / 325 us, 32 of 128 x 128 225 / 142). A group's rows lie CB floats further apart than they are long, so that a warp's reads fall into
+// different banks. A thread carries R elements.
+template <int R, int G> struct StateTile {
+    static constexpr int CB = 32 / G;
+    float* area;                                   // [R * G][cols] and the gaps: 32 R floats a warp and 32 more
+    float* S;                                      // [D][V], from the block's first column on
+    int cols_log2, D, V, cols_left;
+    __device__ __forceinline__ int place(int row, int c) const { return (row << cols_log2) + row / R * CB + c; }
+    __device__ __forceinline__ void ask(float (&t)[R]) const {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int e = threadIdx.x + j * blockDim.x, row = e >> cols_log2, c = e & ((1 << cols_log2) - 1);
+            t[j] = row < D && c < cols_left ? load_now(S + (size_t)row * V + c) : 0.f;
+        }
+    }
+    __device__ __forceinline__ void lay(const float (&t)[R]) const {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int e = threadIdx.x + j * blockDim.x;
+            area[place(e >> cols_log2, e & ((1 << cols_log2) - 1))] = t[j];
+        }
+    }
+    __device__ __forceinline__ void take(f32x2 (&s)[R / 2], int row0, int cl) const {
+#pragma unroll
+        for (int r = 0; r < R; r += 2) s[r / 2] = pack2(area[place(row0 + r, cl)], area[place(row0 + r + 1, cl)]);
+    }
+    __device__ __forceinline__ void give(const f32x2 (&s)[R / 2], int row0, int cl) const {
+#pragma unroll
+        for (int r = 0; r < R; r += 2) unpack2(s[r / 2], area[place(row0 + r, cl)], area[place(row0 + r + 1, cl)]);
+    }
+    __device__ __forceinline__ void leave() const {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int e = threadIdx.x + j * blockDim.x, row = e >> cols_log2, c = e & ((1 << cols_log2) - 1);
+            if (row < D && c < cols_left) S[(size_t)row * V + c] = area[place(row, c)];
+        }
+    }
+    // Straight between global memory and the lanes.
+    __device__ __forceinline__ void load(f32x2 (&s)[R / 2], int row0, int cl) const {
+#pragma unroll
+        for (int r = 0; r < R; r += 2)
+            s[r / 2] = pack2(row0 + r < D && cl < cols_left ? __ldcg(S + (size_t)(row0 + r) * V + cl) : 0.f,
+                             row0 + r + 1 < D && cl < cols_left ? __ldcg(S + (size_t)(row0 + r + 1) * V + cl) : 0.f);
+    }
+    __device__ __forceinline__ void store(const f32x2 (&s)[R / 2], int row0, int cl) const {
+#pragma unroll
+        for (int r = 0; r < R; r += 2) {
+            float lo, hi;
+            unpack2(s[r / 2], lo, hi);
+            if (row0 + r < D && cl < cols_left) S[(size_t)(row0 + r) * V + cl] = lo;
+            if (row0 + r + 1 < D && cl < cols_left) S[(size_t)(row0 + r + 1) * V + cl] = hi;
+        }
+    }
+};
 
 // ------------------------------------------------------------------------------------------------ decay scan
 // rkv [n][ld] of T: r at r_off, k at k_off, v at v_off, heads of `D` side by side; dlog [n][H * D] float: the decay's logit
@@ -135,11 +188,12 @@ __device__ __forceinline__ void copy4(float* dst, const float* src) {
 // per batch. A prompt of 1,500 tokens (with 333, 64 and 7 beside it), 32 heads of 64, inside the step: 423 -> 309 us, against blocks of 32 columns
 // whose warps shared a column's rows; 2,048 tokens alone 405 -> 313, 8 heads 800 -> 392.
 template <typename T, int R, int G, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
+__global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? 4 : 1) decay_scan_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
                                   const float* __restrict__ w0, const float* __restrict__ u, float* state, long long state_stride,
-                                  const int* cu_seqlens, const int* seq_slots, int H, int D) {
+                                  const int* cu_seqlens, const int* seq_slots, int H, int D, int through) {
     extern __shared__ __align__(16) float sm[];
     constexpr int CB = 32 / G, Dp = R * G, ROW = G * (R + 4), THREADS = 32 * WARPS, COLS = WARPS * CB;
+    constexpr int AT_ONCE = 4;                                                             // tokens whose reads are in flight
     constexpr int CHANNELS = Dp < THREADS ? Dp : THREADS, STEP = THREADS / CHANNELS;       // threads of a row, rows at a time
     constexpr int PER = RS_BATCH / STEP, PASSES = Dp / CHANNELS;                           // rows of a thread's channel, channels of a thread
     constexpr int PV = (RS_BATCH * COLS + THREADS - 1) / THREADS;
@@ -147,11 +201,11 @@ __global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restric
     float* sk = sr + 2 * RS_BATCH * ROW;
     float* sw = sk + 2 * RS_BATCH * ROW;
     float* sv = sw + 2 * RS_BATCH * ROW;          // [2][RS_BATCH][COLS]
-    float* so = sv + 2 * RS_BATCH * COLS;         // [WARPS][RS_BATCH][32]
+    float* so = sv + 2 * RS_BATCH * COLS;         // [WARPS][RS_BATCH][32], and before and after the tokens the state
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = warp * CB + lane % CB, sub = lane / CB;
-    const int col0 = blockIdx.x * COLS, col = col0 + cl, h = blockIdx.y, b = blockIdx.z, row0 = sub * R;
+    const int col0 = blockIdx.x * COLS, h = blockIdx.y, b = blockIdx.z, row0 = sub * R, used = (D + R - 1) / R;
     const int t0 = __ldcg(cu_seqlens + b), t1 = __ldcg(cu_seqlens + b + 1);
-    float* S = state + (size_t)__ldcg(seq_slots + b) * state_stride + (size_t)h * D * D;
+    const StateTile<R, G> tile = {so, state + (size_t)__ldcg(seq_slots + b) * state_stride + (size_t)h * D * D + col0, __ffs(COLS) - 1, D, D, D - col0};
     const int ch = threadIdx.x % CHANNELS, i0 = threadIdx.x / CHANNELS;
     float shift[PASSES];
 #pragma unroll
@@ -162,7 +216,8 @@ __global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restric
         bonus[r / 2] = pack2(row0 + r < D ? u[h * D + row0 + r] : 0.f, row0 + r + 1 < D ? u[h * D + row0 + r + 1] : 0.f);
     pdl_enter();
     f32x2 s[R / 2];
-    load_state<R>(s, S, row0, col, D, D);
+    float asked[R];
+    if (through) tile.ask(asked); else tile.load(s, row0, cl);
     // Fetched values stay as they were loaded (no conversion, no branch): a use right behind a load would make the warp wait for it,
     // one round trip to memory per load instead of one per batch. Rows outside the batch or the head read a valid address and
     // are zeroed when they are laid into shared memory.
@@ -214,11 +269,18 @@ __global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restric
         const int count = min(RS_BATCH, t1 - t0);
         fetch(t0, count, 0);
         fetch_values(t0, count);
+        if (through) tile.lay(asked);
         stash(0, count, 0);
         stash_values(0, count);
         rest(0, t0, count);
+    } else {
+        return;                                   // no token: the state stays as it is
     }
     __syncthreads();
+    if (through) {
+        tile.take(s, row0, cl);
+        __syncthreads();
+    }
     int buf = 0;
     float* mine = so + warp * RS_BATCH * 32;
     for (int base = t0; base < t1; base += RS_BATCH, buf ^= 1) {
@@ -227,17 +289,16 @@ __global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restric
             fetch(next, next_count, 0);
             fetch_values(next, next_count);
         }
-        // Whole batches (tokens beyond the last leave the state as it is: k = 0, v = 0, w = 1), several tokens' reads in flight: a token
-        // waits for the one before only in the state, one multiply-add an element.
-#pragma unroll 4
-        for (int i = 0; i < RS_BATCH; ++i) {
+        // Tokens AT_ONCE at a time (those beyond the last leave the state as it is: k = 0, v = 0, w = 1), their reads in flight together: a token
+        // waits for the one before only in the state, one multiply-add an element. (A loop of known length lets the next reads start earlier.)
+        auto token = [&](int i) {
             const int at = (buf * RS_BATCH + i) * ROW + sub * (R + 4);
             const float v = sv[(buf * RS_BATCH + i) * COLS + cl];
+            const f32x2 v2 = pack2(v, v);
             f32x2 rr[R / 2], kk[R / 2], ww[R / 2], part[2] = {0ull, 0ull};
             read_rows<R>(rr, sr + at);
             read_rows<R>(kk, sk + at);
             read_rows<R>(ww, sw + at);
-            const f32x2 v2 = pack2(v, v);
 #pragma unroll
             for (int r = 0; r < R / 2; ++r) {
                 const f32x2 kv = mul2(kk[r], v2);
@@ -245,11 +306,19 @@ __global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restric
                 s[r] = fma2(ww[r], s[r], kv);
             }
             mine[i * 32 + lane] = rows_sum(part[0], part[1]);
+        };
+        if (count == RS_BATCH) {
+#pragma unroll AT_ONCE
+            for (int i = 0; i < RS_BATCH; ++i) token(i);
+        } else {
+            for (int i0 = 0; i0 < count; i0 += AT_ONCE)
+#pragma unroll
+                for (int i1 = 0; i1 < AT_ONCE; ++i1) token(i0 + i1);
         }
         __syncwarp();
         for (int e = lane; e < count * CB; e += 32) {         // a warp's own columns leave once per batch
             const int i = e / CB, c = e % CB, to = col0 + warp * CB + c;
-            if (to < D) o[(size_t)(base + i) * H * D + h * D + to] = groups_sum<G>(mine + i * 32 + c, CB);
+            if (to < D) o[(size_t)(base + i) * H * D + h * D + to] = used == G ? groups_sum<G>(mine + i * 32 + c, CB) : groups_sum(mine + i * 32 + c, CB, used);
         }
         if (next < t1) {
             stash(buf ^ 1, next_count, 0);
@@ -258,16 +327,143 @@ __global__ void __launch_bounds__(32 * WARPS) decay_scan_kernel(float* __restric
         }
         __syncthreads();
     }
-    store_state<R>(S, s, row0, col, D, D);
+    if (through) {
+        tile.give(s, row0, cl);
+        __syncthreads();
+        tile.leave();
+    } else {
+        tile.store(s, row0, cl);
+    }
+}
+
+// Keys above 64. Every block stages all key rows of its head, and what that takes grows with the key, so a block has 32 columns here (8 or 16 where few
+// blocks would leave most SMs idle): R rows a lane, a column's rows shared out among the warps, and among a warp's lanes too where the columns are
+// fewer; their sums meet in shared memory once per batch. 2,048 tokens here / in the kernel above: 32 heads of 128 576 / 1,112 us, 16 of 256 985 / 4,019;
+// for 64 and less the other way round (32 heads of 64 405 / 281).
+template <typename T, int R, int CB>
+__global__ void decay_scan_wide_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
+                                  const float* __restrict__ w0, const float* __restrict__ u, float* state, long long state_stride,
+                                  const int* cu_seqlens, const int* seq_slots, int H, int D) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int SUBS = 32 / CB;                 // a warp's lanes: CB columns x SUBS groups of R rows
+    constexpr int PER = RS_BATCH * R * SUBS / 32; // staged elements of r, k, w per thread and batch: RS_BATCH * Dp / threads
+    constexpr int PV = (RS_BATCH * CB + 127) / 128;
+    const int warps = blockDim.x >> 5, Dp = warps * R * SUBS, threads = blockDim.x;
+    float* sr = sm;                               // [2][RS_BATCH][Dp]
+    float* sk = sr + 2 * RS_BATCH * Dp;
+    float* sw = sk + 2 * RS_BATCH * Dp;
+    float* sv = sw + 2 * RS_BATCH * Dp;           // [2][RS_BATCH][CB]
+    float* red = sv + 2 * RS_BATCH * CB;          // [2][RS_BATCH][warps][32]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = lane % CB, sub = lane / CB;
+    const int col0 = blockIdx.x * CB, col = col0 + cl, h = blockIdx.y, b = blockIdx.z;
+    const int row0 = (warp * SUBS + sub) * R;
+    const int used = (D + R - 1) / R;
+    const bool early_v = threads >= 128;          // enough threads to fetch a batch's values ahead in PV registers each
+    pdl_enter();
+    const int t0 = __ldcg(cu_seqlens + b), t1 = __ldcg(cu_seqlens + b + 1);
+    float* S = state + (size_t)__ldcg(seq_slots + b) * state_stride + (size_t)h * D * D;
+    float s[R], bonus[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const bool in = row0 + r < D && col < D;
+        s[r] = in ? __ldcg(S + (size_t)(row0 + r) * D + col) : 0.f;
+        bonus[r] = row0 + r < D ? u[h * D + row0 + r] : 0.f;
+    }
+    // Fetched values stay as they were loaded (no conversion, no branch): a use right behind a load would make the warp wait for it,
+    // one round trip to memory per load instead of one per batch. Rows outside the batch or the head read a valid address and
+    // are zeroed when they are laid into shared memory.
+    T fr[PER], fk[PER], fv[PV];
+    float fd[PER];
+    auto fetch = [&](int base, int count) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int e = threadIdx.x + j * threads, i = e / Dp, d = e - i * Dp;
+            const bool in = i < count && d < D;
+            const size_t at = in ? (size_t)(base + i) * ld + h * D + d : 0;
+            fr[j] = __ldcg(rkv + at + r_off);
+            fk[j] = __ldcg(rkv + at + k_off);
+            fd[j] = __ldcg(dlog + (in ? (size_t)(base + i) * H * D + h * D + d : 0));
+        }
+        if (early_v) {
+#pragma unroll
+            for (int j = 0; j < PV; ++j) {
+                const int e = threadIdx.x + j * threads, i = e / CB, c = col0 + e % CB;
+                const bool in = e < RS_BATCH * CB && i < count && c < D;
+                fv[j] = __ldcg(rkv + (in ? (size_t)(base + i) * ld + v_off + h * D + c : 0));
+            }
+        }
+    };
+    auto stash = [&](int buf, int base, int count) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int e = threadIdx.x + j * threads, i = e / Dp, d = e - i * Dp;
+            const bool in = i < count && d < D;
+            sr[buf * RS_BATCH * Dp + e] = in ? to_f32(fr[j]) : 0.f;
+            sk[buf * RS_BATCH * Dp + e] = in ? to_f32(fk[j]) : 0.f;
+            sw[buf * RS_BATCH * Dp + e] = in ? expf(-expf(fd[j] + w0[h * D + d])) : 1.f;
+        }
+        if (early_v) {
+#pragma unroll
+            for (int j = 0; j < PV; ++j) {
+                const int e = threadIdx.x + j * threads, i = e / CB, c = col0 + e % CB;
+                if (e < RS_BATCH * CB) sv[buf * RS_BATCH * CB + e] = (i < count && c < D) ? to_f32(fv[j]) : 0.f;
+            }
+        } else {                                  // a block of few threads (a small key size) reads its values late
+            for (int e = threadIdx.x; e < RS_BATCH * CB; e += threads) {
+                const int i = e / CB, c = col0 + e % CB;
+                sv[buf * RS_BATCH * CB + e] = (i < count && c < D) ? to_f32(__ldcg(rkv + (size_t)(base + i) * ld + v_off + h * D + c)) : 0.f;
+            }
+        }
+    };
+    if (t0 < t1) {
+        fetch(t0, min(RS_BATCH, t1 - t0));
+        stash(0, t0, min(RS_BATCH, t1 - t0));
+    }
+    __syncthreads();
+    int it = 0;
+    for (int base = t0; base < t1; base += RS_BATCH, ++it) {
+        const int count = min(RS_BATCH, t1 - base), buf = it & 1;
+        const int next = base + RS_BATCH, next_count = min(RS_BATCH, t1 - next);
+        if (next < t1) fetch(next, next_count);
+        float* my_red = red + (size_t)buf * RS_BATCH * warps * 32;
+        for (int i = 0; i < count; ++i) {
+            const float v = sv[(buf * RS_BATCH + i) * CB + cl];
+            const float4* pr = reinterpret_cast<const float4*>(sr + (buf * RS_BATCH + i) * Dp + row0);
+            const float4* pk = reinterpret_cast<const float4*>(sk + (buf * RS_BATCH + i) * Dp + row0);
+            const float4* pw = reinterpret_cast<const float4*>(sw + (buf * RS_BATCH + i) * Dp + row0);
+            float part[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int q = 0; q < R / 4; ++q) {
+                const float4 r4 = pr[q], k4 = pk[q], w4 = pw[q];
+                const float rr[4] = {r4.x, r4.y, r4.z, r4.w}, kk[4] = {k4.x, k4.y, k4.z, k4.w}, ww[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const float kv = kk[c] * v;
+                    part[c] = fmaf(fmaf(bonus[4 * q + c], kv, s[4 * q + c]), rr[c], part[c]);
+                    s[4 * q + c] = fmaf(ww[c], s[4 * q + c], kv);
+                }
+            }
+            my_red[(i * warps + warp) * 32 + lane] = (part[0] + part[1]) + (part[2] + part[3]);
+        }
+        if (next < t1) stash(buf ^ 1, next, next_count);
+        __syncthreads();
+        for (int e = threadIdx.x; e < count * CB; e += threads) {
+            const int i = e / CB, c = col0 + e % CB;
+            if (c < D) o[(size_t)(base + i) * H * D + h * D + c] = groups_sum(my_red + i * warps * 32 + e % CB, CB, used);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (row0 + r < D && col < D) S[(size_t)(row0 + r) * D + col] = s[r];
 }
 
 // One token per sequence (a decode step): no staging; a warp has one group of rows of 32 columns, its lanes read the same r, k and decay
 // logits; the groups' sums meet in a small array and are added in the scan's order.
-template <typename T, int R, int G>
+template <typename T, int R>
 __global__ void decay_token_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
                                    const float* __restrict__ w0, const float* __restrict__ u, float* state, long long state_stride,
                                    const int* seq_slots, int H, int D) {
-    __shared__ float red[G * 32];
+    __shared__ float red[RS_MAX_KEY / R * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int col = blockIdx.x * 32 + lane, h = blockIdx.y, t = blockIdx.z;
     const int row0 = warp * R;
@@ -300,27 +496,36 @@ __global__ void decay_token_kernel(float* __restrict__ o, const T* rkv, long lon
     for (int r = 0; r < R; ++r)
         if (row0 + r < D && col < D) S[(size_t)(row0 + r) * D + col] = s[r];
     __syncthreads();
-    if (warp == 0 && col < D) o[(size_t)t * H * D + h * D + col] = groups_sum<G>(red + lane, 32);
+    if (warp == 0 && col < D) o[(size_t)t * H * D + h * D + col] = groups_sum(red + lane, 32, blockDim.x >> 5);
 }
 
-template <typename T, int R, int G>
+template <typename T, int G>
 static void launch_decay_scan(float* o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog, const float* w0, const float* u,
-                              float* state, long long state_stride, const int* cu_seqlens, const int* seq_slots, int B, int H, int D, bool one_token,
-                              int warps, cudaStream_t stream) {
-    if (one_token) {
-        ti_launch(decay_token_kernel<T, R, G>, dim3((D + 31) / 32, H, B), dim3(G * 32), 0, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u, state,
-                  state_stride, seq_slots, H, D);
-        return;
-    }
-    const int cols = warps * (32 / G);
-    const size_t smem = (size_t)(2 * 3 * RS_BATCH * G * (R + 4) + 2 * RS_BATCH * cols + RS_BATCH * warps * 32) * sizeof(float);
+                              float* state, long long state_stride, const int* cu_seqlens, const int* seq_slots, int B, int H, int D, ScanShape shape, cudaStream_t stream) {
+    constexpr int R = 8;
+    const int warps = shape.warps, cols = warps * (32 / G);
+    const size_t smem = (size_t)(2 * 3 * RS_BATCH * G * (R + 4) + 2 * RS_BATCH * cols + RS_BATCH * warps * 32 + 32) * sizeof(float);
     auto launch = [&](auto kernel) {
         if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ti_launch_after(kernel, dim3((D + cols - 1) / cols, H, B), dim3(warps * 32), smem, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u, state, state_stride,
-                  cu_seqlens, seq_slots, H, D);
+                        cu_seqlens, seq_slots, H, D, shape.through);
     };
-    if (warps >= 4) launch(decay_scan_kernel<T, R, G, 4>);
+    if constexpr (G <= 2) {                       // a warp or two hold all columns of such heads
+        if (warps == 1) return launch(decay_scan_kernel<T, R, G, 1>);
+    }
+    if (warps == 4) launch(decay_scan_kernel<T, R, G, 4>);
     else launch(decay_scan_kernel<T, R, G, 2>);
+}
+
+template <typename T, int R, int CB>
+static void launch_decay_scan_wide(float* o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog, const float* w0, const float* u,
+                                   float* state, long long state_stride, const int* cu_seqlens, const int* seq_slots, int B, int H, int D, cudaStream_t stream) {
+    constexpr int RW = R * (32 / CB);             // key rows of a warp
+    const int warps = (D + RW - 1) / RW;
+    const size_t smem = (size_t)(2 * 3 * RS_BATCH * warps * RW + 2 * RS_BATCH * CB + 2 * RS_BATCH * warps * 32) * sizeof(float);
+    if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(decay_scan_wide_kernel<T, R, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    ti_launch_after(decay_scan_wide_kernel<T, R, CB>, dim3((D + CB - 1) / CB, H, B), dim3(warps * 32), smem, stream, o, rkv, ld, r_off, k_off, v_off, dlog, w0, u,
+                    state, state_stride, cu_seqlens, seq_slots, H, D);
 }
 
 extern "C" int ti_decay_scan(float* o, const void* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog, const float* w0,
@@ -328,19 +533,31 @@ extern "C" int ti_decay_scan(float* o, const void* rkv, long long ld, int r_off,
                              int H, int D, int dtype, cudaStream_t stream) {
     if (n == 0 || B == 0) return 0;
     TI_REQUIRE(D > 0 && D <= RS_MAX_KEY && H > 0, "decay_scan: %d heads of %d (at most %d)", H, D, RS_MAX_KEY);
-    // 8 rows a lane up to key size 128 (more warps for the same work), 16 beyond.
-    const ScanShape shape = scan_shape(D <= 128 ? 8 : 16, D, D, (long long)H * B, 4, 2);
-#define RS_DECAY(R, G) launch_decay_scan<T, R, G>(o, (const T*)rkv, ld, r_off, k_off, v_off, dlog, w0, u, state, state_stride, cu_seqlens, seq_slots, B, H, D, n == B, shape.warps, stream)
+    if (n == B) {                                 // one token per sequence
+        TI_DISPATCH_DTYPE(dtype, {
+            auto launch = [&](auto kernel, int rows) {
+                ti_launch(kernel, dim3((D + 31) / 32, H, B), dim3((D + rows - 1) / rows * 32), 0, stream, o, (const T*)rkv, ld, r_off, k_off, v_off, dlog, w0, u,
+                          state, state_stride, seq_slots, H, D);
+            };
+            if (D <= 128) launch(decay_token_kernel<T, 8>, 8); else launch(decay_token_kernel<T, 16>, 16);
+        });
+        return ti_check_launch("decay_token");
+    }
+    const ScanShape shape = scan_shape(8, D, D, (long long)H * B, 4, 2);
+    const long long blocks32 = (long long)((D + 31) / 32) * H * B;
+    const int sms = ti_sm_count();
+#define RS_ARGS o, (const T*)rkv, ld, r_off, k_off, v_off, dlog, w0, u, state, state_stride, cu_seqlens, seq_slots, B, H, D
     TI_DISPATCH_DTYPE(dtype, {
-        if (D <= 128) {
-            if (shape.groups == 1) RS_DECAY(8, 1);
-            else if (shape.groups == 2) RS_DECAY(8, 2);
-            else if (shape.groups == 4) RS_DECAY(8, 4);
-            else if (shape.groups == 8) RS_DECAY(8, 8);
-            else RS_DECAY(8, 16);
-        } else RS_DECAY(16, 16);
+        if (D > 128) launch_decay_scan_wide<T, 16, 32>(RS_ARGS, stream);
+        else if (D > 64 && blocks32 * 4 >= sms) launch_decay_scan_wide<T, 8, 32>(RS_ARGS, stream);
+        else if (D > 64 && blocks32 * 8 >= sms) launch_decay_scan_wide<T, 8, 16>(RS_ARGS, stream);
+        else if (D > 64) launch_decay_scan_wide<T, 8, 8>(RS_ARGS, stream);
+        else if (shape.groups == 8) launch_decay_scan<T, 8>(RS_ARGS, shape, stream);
+        else if (shape.groups == 4) launch_decay_scan<T, 4>(RS_ARGS, shape, stream);
+        else if (shape.groups == 2) launch_decay_scan<T, 2>(RS_ARGS, shape, stream);
+        else launch_decay_scan<T, 1>(RS_ARGS, shape, stream);
     });
-#undef RS_DECAY
+#undef RS_ARGS
     return ti_check_launch("decay_scan");
 }
 
@@ -352,32 +569,48 @@ extern "C" int ti_decay_scan(float* o, const void* rkv, long long ld, int r_off,
 // ahead, the products with q are off the chain, and pairs of rows share an instruction. A prompt of 1,500 tokens
 // (with 333, 64 and 7 beside it), 16 heads of 128 x 128, inside the step: 965 -> 412 us, against blocks of 32 columns whose warps shared a column's rows
 // and met at a barrier per token; 2,048 tokens alone 972 -> 436, 4 heads 1,407 -> 451.
-template <int G>
-__global__ void __launch_bounds__(128) delta_scan_kernel(float* __restrict__ o, const float* qkv, long long ld, const float* ba, const float* __restrict__ a_log,
+// FULL: every group has rows of the key. FEW: so few blocks that a token's chain is all that counts; the state then always goes through shared memory, which
+// leaves the compiler twice the registers to read ahead into (2 heads of 256 x 256, 2,048 tokens 741 -> 484 us; 16 heads, with more warps an SM, 1,282 -> 1,411).
+template <int G, bool FULL, bool FEW>
+__global__ void __launch_bounds__(G == 16 ? 256 : 128) delta_scan_kernel(float* __restrict__ o, const float* qkv, long long ld, const float* ba, const float* __restrict__ a_log,
                                   const float* __restrict__ dt_bias, float* state, long long state_stride, const int* cu_seqlens,
-                                  const int* seq_slots, int H, int GQ, int D, int V, int vec) {
+                                  const int* seq_slots, int H, int GQ, int D, int V, int vec, int many) {
     extern __shared__ __align__(16) float sm[];
     constexpr int R = RS_ROWS, CB = 32 / G, ROW = G * (R + 4);
+    const bool through = FEW || many;
     const int threads = blockDim.x, cols = (threads >> 5) * CB;
     float* sq = sm;                               // [2][RS_BATCH][ROW]
     float* sk = sq + 2 * RS_BATCH * ROW;
     float* sv = sk + 2 * RS_BATCH * ROW;          // [2][RS_BATCH][cols]
     float* sg = sv + 2 * RS_BATCH * cols;         // [2][RS_BATCH][2]: decay, beta
-    float* so = sg + 2 * RS_BATCH * 2;            // [warps][RS_BATCH][32]
+    float* so = sg + 2 * RS_BATCH * 2;            // [warps][RS_BATCH][32], and before and after the tokens the state
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cl = warp * CB + lane % CB, sub = lane / CB;
-    const int col0 = blockIdx.x * cols, col = col0 + cl, h = blockIdx.y, b = blockIdx.z;
-    const int g = h / (H / GQ), row0 = sub * R;
+    const int col0 = blockIdx.x * cols, h = blockIdx.y, b = blockIdx.z;
+    const int g = h / (H / GQ), row0 = sub * R, used = (D + R - 1) / R;
     const int t0 = __ldcg(cu_seqlens + b), t1 = __ldcg(cu_seqlens + b + 1);
-    float* S = state + (size_t)__ldcg(seq_slots + b) * state_stride + (size_t)h * D * V;
+    if (t0 >= t1) return;                         // no token: the state stays as it is
+    const StateTile<R, G> tile = {so, state + (size_t)__ldcg(seq_slots + b) * state_stride + (size_t)h * D * V + col0, __ffs(cols) - 1, D, V, V - col0};
     const float rate = expf(a_log[h]), shift = dt_bias[h];
     // 16-byte pieces: a thread has one column of rows `vec_rows` apart (threads beyond whole rows have none).
     const int pieces = max(1, D >> 2), vec_rows = threads / pieces, vec_col = (int)threadIdx.x % pieces * 4;
     const int vec_row = (int)threadIdx.x < vec_rows * pieces ? (int)threadIdx.x / pieces : RS_BATCH;
-    for (int e = threadIdx.x; e < 4 * RS_BATCH * ROW + 2 * RS_BATCH * cols; e += threads) sm[e] = 0.f;      // what lies beyond the last key or column stays zero
-    __syncthreads();
+    // What lies beyond the last key or column stays zero, in the rows that the step's tokens use.
+    if (D < R * G) {
+        const int rows = min(RS_BATCH, t1 - t0), rest = R * G - D, bits = 32 - __clz(rest - 1);
+#pragma unroll 4
+        for (int e = threadIdx.x; e < rows << bits; e += threads) {
+            const int d = D + (e & ((1 << bits) - 1)), at = (e >> bits) * ROW + staged_at<R>(d);
+            if (d < R * G)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) sm[k * RS_BATCH * ROW + at] = 0.f;      // both halves of q and of k
+        }
+    }
+    if (col0 + cols > V)
+        for (int e = threadIdx.x; e < 2 * RS_BATCH * cols; e += threads) sv[e] = 0.f;
     pdl_enter();
     f32x2 s[R / 2];
-    load_state<R>(s, S, row0, col, D, V);
+    float asked[R];
+    if (through) tile.ask(asked); else tile.load(s, row0, cl);
     float fg[2] = {0.f, 0.f};
     auto fetch = [&](int buf, int base, int count) {
         const float* from = qkv + (size_t)base * ld + g * D;
@@ -412,9 +645,13 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(float* __restrict__ o, 
         cp_async_wait<0>();
         __syncthreads();
     };
-    if (t0 < t1) {
-        fetch(0, t0, min(RS_BATCH, t1 - t0));
-        land(0, min(RS_BATCH, t1 - t0));
+    if (col0 + cols > V) __syncthreads();         // the zeros lie before the values
+    fetch(0, t0, min(RS_BATCH, t1 - t0));
+    if (through) tile.lay(asked);
+    land(0, min(RS_BATCH, t1 - t0));
+    if (through) {
+        tile.take(s, row0, cl);
+        __syncthreads();
     }
     int buf = 0;
     float* mine = so + warp * RS_BATCH * 32;
@@ -438,7 +675,7 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(float* __restrict__ o, 
             read_rows<R>(kn, rows_k + after * ROW);
             read_rows<R>(qq, rows_q + i * ROW);
             decay_n = gates[after * 2];
-            const float write = beta * (v - groups_sum<G>(rows_sum(part[0], part[1])));
+            const float write = beta * (v - groups_sum<G>(FULL || sub < used ? rows_sum(part[0], part[1]) : 0.f));
             const f32x2 write2 = pack2(write, write);
 #pragma unroll
             for (int r = 0; r < R / 2; ++r) {
@@ -459,22 +696,28 @@ __global__ void __launch_bounds__(128) delta_scan_kernel(float* __restrict__ o, 
         __syncwarp();
         for (int e = lane; e < count * CB; e += 32) {         // a warp's own columns leave once per batch
             const int i = e / CB, c = e % CB, to = col0 + warp * CB + c;
-            if (to < V) o[(size_t)(base + i) * H * V + h * V + to] = groups_sum<G>(mine + i * 32 + c, CB);
+            if (to < V) o[(size_t)(base + i) * H * V + h * V + to] = FULL ? groups_sum<G>(mine + i * 32 + c, CB) : groups_sum(mine + i * 32 + c, CB, used);
         }
         __syncwarp();
         if (next < t1) land(buf ^ 1, next_count);
     }
-    store_state<R>(S, s, row0, col, D, V);
+    if (through) {
+        __syncthreads();
+        tile.give(s, row0, cl);
+        __syncthreads();
+        tile.leave();
+    } else {
+        tile.store(s, row0, cl);
+    }
 }
 
 // One token per sequence: as the scan's step for one token, without staging; a warp has one group of rows of 32 columns.
-template <int G>
 __global__ void delta_token_kernel(float* __restrict__ o, const float* qkv, long long ld, const float* ba, const float* __restrict__ a_log,
                                    const float* __restrict__ dt_bias, float* state, long long state_stride, const int* seq_slots, int H, int GQ,
                                    int D, int V) {
     constexpr int R = RS_ROWS;
-    __shared__ float red[2 * G * 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ float red[2 * (RS_MAX_KEY / RS_ROWS) * 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, used = blockDim.x >> 5;
     const int col = blockIdx.x * 32 + lane, h = blockIdx.y, t = blockIdx.z;
     const int g = h / (H / GQ), row0 = warp * R;
     float* S = state + (size_t)__ldg(seq_slots + t) * state_stride + (size_t)h * D * V;
@@ -495,7 +738,7 @@ __global__ void delta_token_kernel(float* __restrict__ o, const float* qkv, long
     }
     red[warp * 32 + lane] = (part[0] + part[1]) + (part[2] + part[3]);
     __syncthreads();
-    const float write = beta * (v - groups_sum<G>(red + lane, 32));
+    const float write = beta * (v - groups_sum(red + lane, 32, used));
     float out[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -504,27 +747,34 @@ __global__ void delta_token_kernel(float* __restrict__ o, const float* qkv, long
         out[r & 3] = fmaf(s[r], qq, out[r & 3]);
         if (row0 + r < D && col < V) S[(size_t)(row0 + r) * V + col] = s[r];
     }
-    float* red_o = red + G * 32;
+    float* red_o = red + used * 32;
     red_o[warp * 32 + lane] = (out[0] + out[1]) + (out[2] + out[3]);
     __syncthreads();
-    if (warp == 0 && col < V) o[(size_t)t * H * V + h * V + col] = groups_sum<G>(red_o + lane, 32);
+    if (warp == 0 && col < V) o[(size_t)t * H * V + h * V + col] = groups_sum(red_o + lane, 32, used);
 }
 
 template <int G>
 static void launch_delta_scan(float* o, const float* qkv, long long ld, const float* ba, const float* a_log, const float* dt_bias, float* state,
                               long long state_stride, const int* cu_seqlens, const int* seq_slots, int B, int H, int GQ, int D, int V, bool one_token,
-                              int warps, cudaStream_t stream) {
+                              ScanShape shape, cudaStream_t stream) {
     if (one_token) {
-        ti_launch(delta_token_kernel<G>, dim3((V + 31) / 32, H, B), dim3(G * 32), 0, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride, seq_slots,
+        ti_launch(delta_token_kernel, dim3((V + 31) / 32, H, B), dim3((D + RS_ROWS - 1) / RS_ROWS * 32), 0, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride, seq_slots,
                   H, GQ, D, V);
         return;
     }
-    const int cols = warps * (32 / G);
-    const size_t smem = (size_t)(4 * RS_BATCH * G * (RS_ROWS + 4) + 2 * RS_BATCH * cols + 4 * RS_BATCH + RS_BATCH * warps * 32) * sizeof(float);
+    const int warps = shape.warps, cols = warps * (32 / G);
+    const size_t smem = (size_t)(4 * RS_BATCH * G * (RS_ROWS + 4) + 2 * RS_BATCH * cols + 4 * RS_BATCH + RS_BATCH * warps * 32 + 32) * sizeof(float);
     const int vec = D % 4 == 0 && ld % 4 == 0 && aligned16(qkv) && warps * 32 >= D / 4;
-    if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(delta_scan_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ti_launch_after(delta_scan_kernel<G>, dim3((V + cols - 1) / cols, H, B), dim3(warps * 32), smem, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride,
-              cu_seqlens, seq_slots, H, GQ, D, V, vec);
+    auto launch = [&](auto kernel) {
+        if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        ti_launch_after(kernel, dim3((V + cols - 1) / cols, H, B), dim3(warps * 32), smem, stream, o, qkv, ld, ba, a_log, dt_bias, state, state_stride,
+                        cu_seqlens, seq_slots, H, GQ, D, V, vec, shape.through);
+    };
+    const bool full = D > RS_ROWS * (G - 1);
+    if constexpr (G == 16) {
+        if (!shape.through) return full ? launch(delta_scan_kernel<G, true, true>) : launch(delta_scan_kernel<G, false, true>);
+    }
+    if (full) launch(delta_scan_kernel<G, true, false>); else launch(delta_scan_kernel<G, false, false>);
 }
 
 extern "C" int ti_delta_scan(float* o, const float* qkv, long long ld, const float* ba, const float* a_log, const float* dt_bias, float* state,
@@ -533,8 +783,8 @@ extern "C" int ti_delta_scan(float* o, const float* qkv, long long ld, const flo
     if (n == 0 || B == 0) return 0;
     TI_REQUIRE(D > 0 && V > 0 && D <= RS_MAX_KEY, "delta_scan: keys of %d (at most %d)", D, RS_MAX_KEY);
     TI_REQUIRE(H > 0 && G > 0 && H % G == 0, "delta_scan: %d heads do not divide into %d query/key heads", H, G);
-    const ScanShape shape = scan_shape(RS_ROWS, D, V, (long long)H * B, 4, 1);
-#define RS_DELTA(GROUPS) launch_delta_scan<GROUPS>(o, qkv, ld, ba, a_log, dt_bias, state, state_stride, cu_seqlens, seq_slots, B, H, G, D, V, n == B, shape.warps, stream)
+    const ScanShape shape = scan_shape(RS_ROWS, D, V, (long long)H * B, D > 128 ? 8 : 4, 1);
+#define RS_DELTA(GROUPS) launch_delta_scan<GROUPS>(o, qkv, ld, ba, a_log, dt_bias, state, state_stride, cu_seqlens, seq_slots, B, H, G, D, V, n == B, shape, stream)
     if (shape.groups == 1) RS_DELTA(1);
     else if (shape.groups == 2) RS_DELTA(2);
     else if (shape.groups == 4) RS_DELTA(4);
