@@ -858,11 +858,12 @@ extern "C" int ti_shift_blend(void* out, const void* h, const void* mu, int K, f
 // the step's own rows or from `hist`: the sequence's last taps - 1 rows, state rows `hist_stride` floats apart) and SiLU; then
 // every q and k head becomes a unit vector x / sqrt(sum x^2 + unit_eps), q also times D^(-1/2). out [n][C] float.
 // A block has RUN tokens in a row and `per` channels, whole heads among the q and k channels. A thread reads a channel's rows and weights once
-// for all of them (TAPS weights, 0: so many that they are read again for every token), its loads in flight together
+// for all of them (TAPS weights; -1: more than 4, four at a time), its loads in flight together
 // (4,096 channels, 4 taps, against a block that goes through a token's channels: 4 tokens 13.6 -> 2.3 us, 2,048 tokens 60 -> 54).
 #define DI_THREADS 256
+#define DI_MOST_THREADS 512
 template <typename T, int RUN, int TAPS>
-__global__ void __launch_bounds__(DI_THREADS) delta_inputs_kernel(float* __restrict__ out, const T* proj, long long ld, const T* __restrict__ conv,
+__global__ void __launch_bounds__(DI_MOST_THREADS) delta_inputs_kernel(float* __restrict__ out, const T* proj, long long ld, const T* __restrict__ conv,
                                                                    int taps, const float* hist, long long hist_stride, const int* cu_seqlens,
                                                                    const int* seq_slots, int B, int n, int G, int D, int HV, float unit_eps, int per) {
     extern __shared__ float y[];                             // [RUN][per]
@@ -870,17 +871,17 @@ __global__ void __launch_bounds__(DI_THREADS) delta_inputs_kernel(float* __restr
     const int t = blockIdx.x * RUN, C = 2 * G * D + HV, c0 = blockIdx.y * per, channels = min(per, C - c0), count = min(RUN, n - t);
     run.find(cu_seqlens, seq_slots, B, n, t);
     pdl_enter();
-    for (int i = threadIdx.x; i < channels; i += DI_THREADS) {
+    for (int i = threadIdx.x; i < channels; i += blockDim.x) {
         const int c = c0 + i;
         // The row `back` before token t + j: of the step, or of the sequence's history, whose row taps - 1 - (t0 - token) counts back from the newest.
         auto older = [&](int j, int back) {
             return __ldcg(hist + (size_t)run.slot[j] * hist_stride + (size_t)(taps - 1 - (run.t0[j] - (t + j - back))) * C + c);
         };
-        if (TAPS > 0) {
+        if (TAPS >= 0) {
             constexpr int KEEP = TAPS > 0 ? TAPS - 1 : 0;
             float row[RUN + KEEP], weight[KEEP + 1];
 #pragma unroll
-            for (int k = 0; k < TAPS; ++k) weight[k] = to_f32(conv[(size_t)c * TAPS + k]);
+            for (int k = 0; k < (TAPS > 0 ? TAPS : 0); ++k) weight[k] = to_f32(conv[(size_t)c * taps + k]);
 #pragma unroll
             for (int j = 0; j < RUN + KEEP; ++j) {
                 const int tj = t + j - KEEP;
@@ -889,30 +890,53 @@ __global__ void __launch_bounds__(DI_THREADS) delta_inputs_kernel(float* __restr
 #pragma unroll
             for (int j = 0; j < RUN; ++j) {
                 if (j >= count) break;
-                float acc = 0.f;
+                float acc = TAPS == 0 ? row[j] : 0.f;
 #pragma unroll
-                for (int k = 0; k < TAPS; ++k) {
+                for (int k = 0; k < (TAPS > 0 ? TAPS : 0); ++k) {
                     const int back = KEEP - k;
                     acc = fmaf(weight[k], t + j - back >= run.t0[j] ? row[j + k] : older(j, back), acc);
                 }
                 y[j * per + i] = rs_silu(acc);
             }
-        } else {
-            for (int j = 0; j < count; ++j) {
-                float acc = 0.f;
-                if (taps <= 0) acc = to_f32(__ldcg(proj + (size_t)(t + j) * ld + c));
-                for (int k = 0; k < taps; ++k) {
-                    const int back = taps - 1 - k;
-                    const float x = t + j - back >= run.t0[j] ? to_f32(__ldcg(proj + (size_t)(t + j - back) * ld + c)) : older(j, back);
-                    acc = fmaf(to_f32(conv[(size_t)c * taps + k]), x, acc);
-                }
-                y[j * per + i] = rs_silu(acc);
+        } else if (RUN == 1) {
+            float acc = 0.f;
+            for (int k = 0; k < taps; ++k) {
+                const int back = taps - 1 - k;
+                const float x = t - back >= run.t0[0] ? to_f32(__ldcg(proj + (size_t)(t - back) * ld + c)) : older(0, back);
+                acc = fmaf(to_f32(conv[(size_t)c * taps + k]), x, acc);
             }
+            y[i] = rs_silu(acc);
+        } else {
+            // Four taps at a time: their rows lie in a row, a token's one after the one before's.
+            float acc[RUN];
+#pragma unroll
+            for (int j = 0; j < RUN; ++j) acc[j] = 0.f;
+            for (int k0 = 0; k0 < taps; k0 += 4) {
+                const int far = taps - 1 - k0;               // rows back of the first of them
+                float row[RUN + 3], weight[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) weight[k] = k0 + k < taps ? to_f32(conv[(size_t)c * taps + k0 + k]) : 0.f;
+#pragma unroll
+                for (int j = 0; j < RUN + 3; ++j) {
+                    const int tj = t + j - far;
+                    row[j] = tj >= run.t0[0] && tj < t + count ? to_f32(__ldcg(proj + (size_t)tj * ld + c)) : 0.f;
+                }
+#pragma unroll
+                for (int j = 0; j < RUN; ++j) {
+                    if (j >= count) break;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (k0 + k < taps) acc[j] = fmaf(weight[k], t + j - far + k >= run.t0[j] ? row[j + k] : older(j, far - k), acc[j]);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < RUN; ++j)
+                if (j < count) y[j * per + i] = rs_silu(acc[j]);
         }
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, head0 = D > 0 ? c0 / D : 0, heads = D > 0 ? max(0, min(2 * G - head0, channels / D)) : 0;
-    for (int e = warp; e < heads * count; e += DI_THREADS / 32) {              // a warp per q or k head of a token
+    for (int e = warp; e < heads * count; e += blockDim.x >> 5) {              // a warp per q or k head of a token
         const int hd = head0 + e % heads;
         float* src = y + (e / heads) * per + (size_t)hd * D - c0;
         float ss = 0.f;
@@ -923,7 +947,7 @@ __global__ void __launch_bounds__(DI_THREADS) delta_inputs_kernel(float* __restr
     }
     __syncthreads();
     for (int j = 0; j < count; ++j)
-        for (int i = threadIdx.x; i < channels; i += DI_THREADS) out[(size_t)(t + j) * C + c0 + i] = y[j * per + i];
+        for (int i = threadIdx.x; i < channels; i += blockDim.x) out[(size_t)(t + j) * C + c0 + i] = y[j * per + i];
 }
 
 extern "C" int ti_delta_inputs(float* out, const void* proj, long long ld, const void* conv, int taps, const float* hist, long long hist_stride,
@@ -940,15 +964,24 @@ extern "C" int ti_delta_inputs(float* out, const void* proj, long long ld, const
     const int whole = D == 0 || D >= DI_THREADS ? 1 : DI_THREADS / D, want = D > 0 ? whole * D : DI_THREADS, per = want < C ? want : C, parts = (C + per - 1) / per;
     const bool runs = (long long)n * parts > 20LL * ti_sm_count() && (size_t)8 * per * sizeof(float) <= TI_SMEM_UNASKED;
     const size_t smem = (size_t)(runs ? 8 : 1) * per * sizeof(float);
+    const int threads = per > DI_MOST_THREADS ? DI_MOST_THREADS : (per + 31) / 32 * 32;
+#define DI_TAPS(TAPS) do { if (runs) launch(delta_inputs_kernel<T, 8, TAPS>); else launch(delta_inputs_kernel<T, 1, TAPS>); } while (0)
     TI_DISPATCH_DTYPE(dtype, {
         auto launch = [&](auto kernel) {
             if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            ti_launch(kernel, dim3(runs ? (n + 7) / 8 : n, parts), dim3(DI_THREADS), smem, stream, out, (const T*)proj, ld, (const T*)conv, taps, hist, hist_stride,
+            ti_launch(kernel, dim3(runs ? (n + 7) / 8 : n, parts), dim3(threads), smem, stream, out, (const T*)proj, ld, (const T*)conv, taps, hist, hist_stride,
                       cu_seqlens, seq_slots, B, n, G, D, HV, unit_eps, per);
         };
-        if (taps == 4) { if (runs) launch(delta_inputs_kernel<T, 8, 4>); else launch(delta_inputs_kernel<T, 1, 4>); }
-        else { if (runs) launch(delta_inputs_kernel<T, 8, 0>); else launch(delta_inputs_kernel<T, 1, 0>); }
+        switch (taps) {
+            case 0: DI_TAPS(0); break;
+            case 1: DI_TAPS(1); break;
+            case 2: DI_TAPS(2); break;
+            case 3: DI_TAPS(3); break;
+            case 4: DI_TAPS(4); break;
+            default: DI_TAPS(-1); break;
+        }
     });
+#undef DI_TAPS
     return ti_check_launch("delta_inputs");
 }
 
