@@ -133,8 +133,8 @@ extern "C" int ti_lightning_scan(float* o, const void* qkv, long long ld, int q_
 
 // The squares are added as by `sum_threads` threads, element i by thread i modulo it, whatever a block's size is. The first LO_AHEAD elements of a thread
 // and their gates are asked for at once and kept. With no more rows than SMs a block has up to 1,024 threads (2,048 elements, 1 / 2,048 rows 5.7 / 14.1 -> 3.1 / 12.2 us).
-#define LO_AHEAD 4
-template <typename T>
+#define LO_AHEAD 4                 // (1 where a thread has no more)
+template <typename T, int AHEAD>
 __global__ void __launch_bounds__(1024) lightning_out_kernel(T* __restrict__ y, const float* o, const T* g, long long ldg, const T* __restrict__ w, float eps, int size,
                                                              int sum_threads) {
     extern __shared__ float squares[];                  // [size], where the block is larger than sum_threads
@@ -142,25 +142,25 @@ __global__ void __launch_bounds__(1024) lightning_out_kernel(T* __restrict__ y, 
     const float* row = o + (size_t)blockIdx.x * size;
     const T* gate = g != nullptr ? g + (size_t)blockIdx.x * ldg : nullptr;
     pdl_enter();
-    float v[LO_AHEAD], gv[LO_AHEAD], ss = 0.f;
+    float v[AHEAD], gv[AHEAD], ss = 0.f;
 #pragma unroll
-    for (int k = 0; k < LO_AHEAD; ++k) {
+    for (int k = 0; k < AHEAD; ++k) {
         const int i = threadIdx.x + k * blockDim.x;
         v[k] = i < size ? __ldcg(row + i) : 0.f;
         gv[k] = gate != nullptr && i < size ? to_f32(__ldcg(gate + i)) : 0.f;
     }
-    const bool wide = blockDim.x != sum_threads;
+    if (blockDim.x == sum_threads) {
 #pragma unroll
-    for (int k = 0; k < LO_AHEAD; ++k) {
-        const int i = threadIdx.x + k * blockDim.x;
-        if (wide) { if (i < size) squares[i] = v[k]; }
-        else ss = fmaf(v[k], v[k], ss);
-    }
-    for (int i = threadIdx.x + LO_AHEAD * blockDim.x; i < size; i += blockDim.x) {
-        const float t = __ldcg(row + i);
-        if (wide) squares[i] = t; else ss = fmaf(t, t, ss);
-    }
-    if (wide) {
+        for (int k = 0; k < AHEAD; ++k) ss = fmaf(v[k], v[k], ss);
+        for (int i = threadIdx.x + AHEAD * blockDim.x; i < size; i += blockDim.x) {
+            const float t = __ldcg(row + i);
+            ss = fmaf(t, t, ss);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k)
+            if (threadIdx.x + k * blockDim.x < size) squares[threadIdx.x + k * blockDim.x] = v[k];
+        for (int i = threadIdx.x + AHEAD * blockDim.x; i < size; i += blockDim.x) squares[i] = __ldcg(row + i);
         __syncthreads();
         for (int i = threadIdx.x < sum_threads ? threadIdx.x : size; i < size; i += sum_threads) ss = fmaf(squares[i], squares[i], ss);
     }
@@ -172,9 +172,9 @@ __global__ void __launch_bounds__(1024) lightning_out_kernel(T* __restrict__ y, 
         y[(size_t)blockIdx.x * size + i] = from_f32<T>(r);
     };
 #pragma unroll
-    for (int k = 0; k < LO_AHEAD; ++k)
+    for (int k = 0; k < AHEAD; ++k)
         if (threadIdx.x + k * blockDim.x < size) leave(threadIdx.x + k * blockDim.x, v[k], gv[k]);
-    for (int i = threadIdx.x + LO_AHEAD * blockDim.x; i < size; i += blockDim.x) leave(i, __ldcg(row + i), gate != nullptr ? to_f32(__ldcg(gate + i)) : 0.f);
+    for (int i = threadIdx.x + AHEAD * blockDim.x; i < size; i += blockDim.x) leave(i, __ldcg(row + i), gate != nullptr ? to_f32(__ldcg(gate + i)) : 0.f);
 }
 
 // y [n, size] = T(o / rms(o) * w * sigmoid(g)); o [n, size] float, g [n, ldg] of T (null: no gate), w [size].
@@ -186,7 +186,12 @@ extern "C" int ti_lightning_out(void* y, const float* o, const void* g, long lon
     const size_t kept = (size_t)size * sizeof(float);
     // (Kept rows and the kernel's static arrays, less than 256 bytes, fit the 48 KB that a launch may have unasked.)
     const int threads = n <= ti_sm_count() && all > sum_threads && kept + 256 <= 48 * 1024 ? all : sum_threads;
-    TI_DISPATCH_DTYPE(dtype, (ti_launch(lightning_out_kernel<T>, dim3(n), dim3(threads), threads > sum_threads ? kept : 0, stream, (T*)y, o, (const T*)g, ldg,
-                                        (const T*)w, eps, size, sum_threads)));
+    TI_DISPATCH_DTYPE(dtype, {
+        auto launch = [&](auto kernel) {
+            ti_launch(kernel, dim3(n), dim3(threads), threads > sum_threads ? kept : 0, stream, (T*)y, o, (const T*)g, ldg, (const T*)w, eps, size, sum_threads);
+        };
+        if (size <= threads) launch(lightning_out_kernel<T, 1>);
+        else launch(lightning_out_kernel<T, LO_AHEAD>);
+    });
     return ti_check_launch("lightning_out");
 }
