@@ -109,13 +109,16 @@ extern "C" int ti_lightning_scan(float* o, const void* qkv, long long ld, int q_
     TI_REQUIRE(H <= 65535 && B <= 65535, "lightning_scan: %d heads, %d sequences", H, B);
     if (n_tokens == B && V % 4 == 0 && D <= 2048) {      // one token per sequence: the kernel that streams the states
         const size_t smem1 = (size_t)(2 * D + LT_WARPS * 128) * sizeof(float);
-        // Eight rows at once are all of a warp's up to 64, and leave room for more blocks (64 sequences of 16 heads of 64 x 64 13.6 us with 16).
+        // Eight rows at once are all of a warp's up to 64, and leave room for more blocks (64 sequences of 16 heads of 64 x 64 13.6 us with 16); four once there
+        // are blocks for many rounds of heads whose values are few, where an SM's blocks hide one another's latency (256 sequences of them 26.7, with eight 30.5).
+        const bool many = V <= 72 && (long long)((V + 127) / 128) * H * B > 5LL * ti_sm_count();
         TI_DISPATCH_DTYPE(dtype, {
             auto launch = [&](auto kernel) {
                 ti_launch(kernel, dim3((V + 127) / 128, H, B), dim3(LT_WARPS * 32), smem1, stream, o, (const T*)qkv, ld, q_off, k_off, v_off, state, decay,
                           seq_slots, H, D, V, act);
             };
-            if (D <= 8 * LT_WARPS) launch(lightning_token_kernel<T, 8>);
+            if (many) launch(lightning_token_kernel<T, 4>);
+            else if (D <= 8 * LT_WARPS) launch(lightning_token_kernel<T, 8>);
             else launch(lightning_token_kernel<T, 16>);
         });
         return ti_check_launch("lightning_scan");
