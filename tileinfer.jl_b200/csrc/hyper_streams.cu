@@ -228,20 +228,25 @@ extern "C" int ti_streams_update(float* x, const void* delta, const float* parti
     TI_REQUIRE(smem <= 160 * 1024, "streams_update: rows of %d", size);
     const int threads = hs_block(size, n);
     TI_DISPATCH_DTYPE(dtype, {
-        auto launch = [&](auto kernel) {
+        auto launch = [&](auto kernel, int block) {
             if (smem > TI_SMEM_UNASKED) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            ti_launch(kernel, dim3(n), dim3(threads), smem, stream, x, (const T*)delta, partials, n_partials, (size_t)partial_stride, tab, S, (T*)h,
+            ti_launch(kernel, dim3(n), dim3(block), smem, stream, x, (const T*)delta, partials, n_partials, (size_t)partial_stride, tab, S, (T*)h,
                       (const T*)w, (const T*)b, eps, centred, size, hs_threads(size));
         };
+        // A thread asks for no more elements at once than it has: one in blocks as large as the row, four of rows up to 4,096 in blocks of 512 (two copies of
+        // 2,048, 4 rows: 5.3 us in blocks of 1,024 with four, whose 64 registers do not hold them, 3.7 so; longer rows take less all the same in blocks of
+        // 1,024: 4,096 9.1 and 5.7). Three copies and more: one at a time (four of 8,192, 4 rows 13.1 us with two, 10.2).
         // Many rows of 4,096 and more, or of many copies: their blocks' memory traffic is the bound, and a thread that asks for more at once only
         // takes room from other blocks (2,048 rows of 4,096, two copies, four elements at once: 73 us
-        // against 65; four copies, two elements: 112 against 80).
-        if (n <= ti_sm_count()) {
-            if (S <= 2) launch(streams_update_rows_kernel<T, 2, 4, 1024>);
-            else if (S <= 4) launch(streams_update_rows_kernel<T, 4, 2, 1024>);
-            else launch(streams_update_rows_kernel<T, HS_MAX_STREAMS, 1, 1024>);
-        } else if (S <= 2 && size < 4096) launch(streams_update_rows_kernel<T, 2, 4, 256>);
-        else launch(streams_update_kernel<T>);
+        // against 65; four copies, two elements: 112 against 80); rows of one or two elements a thread have none to ask for.
+        if (threads > hs_threads(size)) {
+            if (S <= 2 && size <= 1024) launch(streams_update_rows_kernel<T, 2, 1, 1024>, threads);
+            else if (S <= 2 && size < 4096) launch(streams_update_rows_kernel<T, 2, 4, 512>, 512);
+            else if (S <= 2) launch(streams_update_rows_kernel<T, 2, 4, 1024>, threads);
+            else if (S <= 4) launch(streams_update_rows_kernel<T, 4, 1, 1024>, threads);
+            else launch(streams_update_rows_kernel<T, HS_MAX_STREAMS, 1, 1024>, threads);
+        } else if (n > ti_sm_count() && S <= 2 && size < 4096 && size > 2 * threads) launch(streams_update_rows_kernel<T, 2, 4, 256>, threads);
+        else launch(streams_update_kernel<T>, threads);
     });
     return ti_check_launch("streams_update");
 }
