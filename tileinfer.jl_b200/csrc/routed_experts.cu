@@ -99,7 +99,8 @@ extern "C" int ti_router_topk(const void* h, const void* wr, const float* logits
 // ids [n, top + always]: the chosen expert, or -1 for a pass choice (the last `total - experts`: their output is the input
 // itself), whose weights are summed into pass_weight[n]; then `always` units numbered from `experts` on with the weight
 // sigmoid(gate logit), or 1 without a gate.
-template <typename T>
+// FEW: at most 32 are chosen, and lane j of the first warp keeps choice j; of more they are kept in memory.
+template <typename T, bool FEW>
 __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const float* z_in, long long ldz, int width, int experts, int total,
                                      int softmax, const float* __restrict__ z_bias, const float* __restrict__ correction, int groups, int keep, int group_best,
                                      int top, int renormalize, int always, int gate, int* __restrict__ ids, float* __restrict__ scores, float* __restrict__ pass_weight) {
@@ -165,7 +166,6 @@ __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const
     if (warp == 0) {
         float wsum = 0.f;
         const size_t out = (size_t)t * (top + always);
-        const bool few = top <= 32;                                 // lane j keeps choice j; of more they are kept in memory
         int my_arg = 0;
         float my_w = 0.f;
         for (int j = 0; j < top; ++j) {
@@ -180,12 +180,10 @@ __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const
                 if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
             }
             if (arg >= total) arg = j;                              // only if nothing comparable is left (NaN)
+            if (lane == 0) c[arg] = -INFINITY;                      // first: the next round waits for it alone
             const float w = z[arg];
-            if (lane == j) { my_arg = arg; my_w = w; }
-            if (lane == 0) {
-                if (!few) { ids[out + j] = arg; scores[out + j] = w; }
-                c[arg] = -INFINITY;
-            }
+            if (FEW && lane == j) { my_arg = arg; my_w = w; }
+            if (!FEW && lane == 0) { ids[out + j] = arg; scores[out + j] = w; }
             wsum += w;
             __syncwarp();
         }
@@ -194,7 +192,7 @@ __global__ void router_select_kernel(const T* h, const T* __restrict__ wr, const
             ids[out + top + a] = experts + a;
             scores[out + top + a] = gw;
         }
-        if (few) {
+        if (FEW) {
             if (softmax == 2) {                                     // the chosen logits come largest first
                 my_w = expf(my_w - __shfl_sync(0xffffffffu, my_w, 0));
                 wsum = 0.f;
@@ -246,8 +244,13 @@ extern "C" int ti_router_select(const void* h, const void* wr, const float* z, l
                "router_select: %d of %d groups over %d choices for top %d", keep, groups, total, top);
     TI_REQUIRE(group_best == 1 || group_best == 2, "router_select: a group's score from its %d best", group_best);
     TI_REQUIRE(total == experts || pass_weight != nullptr, "router_select: pass choices need their weights' output");
-    TI_DISPATCH_DTYPE(dtype, (ti_launch(router_select_kernel<T>, dim3(n), dim3(RT_THREADS), (2 * total + 1 + groups) * sizeof(float), stream, (const T*)h, (const T*)wr, z, ldz, width, experts,
-                                        total, softmax, z_bias, correction, groups, keep, group_best, top, renormalize, always, gate, ids, scores, pass_weight)));
+    TI_DISPATCH_DTYPE(dtype, {
+        auto launch = [&](auto kernel) {
+            ti_launch(kernel, dim3(n), dim3(RT_THREADS), (2 * total + 1 + groups) * sizeof(float), stream, (const T*)h, (const T*)wr, z, ldz, width, experts, total, softmax,
+                      z_bias, correction, groups, keep, group_best, top, renormalize, always, gate, ids, scores, pass_weight);
+        };
+        if (top <= 32) launch(router_select_kernel<T, true>); else launch(router_select_kernel<T, false>);
+    });
     return ti_check_launch("router_select");
 }
 
