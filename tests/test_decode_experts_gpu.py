@@ -61,10 +61,12 @@ def test_units_streamed_by_pair(units, out, k, tokens, per_token, gated):
 
 
 @pytest.mark.parametrize("gated", [True, False])
-@pytest.mark.parametrize("units,out,k,tokens,per_token", [(40, 1032, 72, 16, 2), (70, 24, 2056, 16, 4), (9, 40, 264, 16, 7), (300, 16, 40, 16, 20)])
+@pytest.mark.parametrize("units,out,k,tokens,per_token", [(40, 1032, 72, 16, 2), (70, 24, 2056, 16, 4), (9, 40, 264, 16, 7), (300, 16, 40, 16, 20), (100, 16, 40, 16, 40),
+                                                          (5, 4096, 40, 9, 13)])
 def test_units_listed_by_warp_block_and_launch(units, out, k, tokens, per_token, gated):
-    """32 pairs (listed by one warp), more, and more than one launch lists; several tiles a block; rows longer and shorter than the k blocks in
-    flight: every pair's result has the bits of the pair alone."""
+    """32 pairs (listed by one warp), more, as many as a block's threads and more, and more than one launch lists; few units that many pairs chose;
+    several tiles a block, and a block per unit and tile; rows longer and shorter than the k blocks in flight: every pair's result has the bits of
+    the pair alone."""
     from tileinfer_b200.kernels import fast
     g = torch.Generator(device="cuda").manual_seed(units + k)
     x = torch.randn(tokens, k, generator=g, device="cuda").bfloat16()

@@ -260,18 +260,17 @@ def test_plan_of_units(ops, n, per, units, tile):
     assert torch.equal(row_pair.cpu(), back)
 
 
-@pytest.mark.parametrize("H,D", [(3, 5), (2, 33), (32, 64), (1, 64), (5, 100), (2, 129), (1, 256)])
-def test_scans_have_the_bits_of_single_tokens(ops, H, D):
-    """Batches of tokens, a batch's remainder and tokens one by one: the same bits, for every number of row groups and blocks of all sizes."""
+@pytest.mark.parametrize("H,D,G,V", [(3, 5, 3, 8), (2, 33, 2, 36), (32, 64, 32, 67), (1, 64, 1, 67), (5, 100, 5, 103), (2, 129, 2, 132), (1, 256, 1, 259),
+                                     (4, 16, 2, 64), (4, 128, 2, 128), (1, 128, 1, 132), (2, 256, 1, 64), (8, 192, 4, 36), (64, 64, 32, 64), (24, 128, 12, 128), (24, 256, 12, 128)])
+def test_scans_have_the_bits_of_single_tokens(ops, H, D, G, V):
+    """Batches of tokens, a batch's remainder and tokens one by one: the same bits, for every number of row groups and blocks of all sizes, the state
+    straight into the lanes and through shared memory, rows of the delta rule in pieces of 16 bytes and of 4, heads that share queries and keys."""
     g = torch.Generator(device="cuda").manual_seed(D)
     R = lambda *s: torch.randn(*s, generator=g, device="cuda")                                     # noqa: E731
-    lengths, G, V = [37, 16, 1, 30], H, D + 3
+    lengths = [37, 16, 1, 30]
     n = sum(lengths)
     rkv, dlog, w0, u = R(n, 3 * H * D).bfloat16(), R(n, H * D), R(H * D) - 2, R(H * D)
-    C = 2 * G * D + H * V
-    wide = torch.zeros(n, (C + 3) // 4 * 4 + 4, device="cuda")
-    wide[:, :C] = R(n, C) * D ** -0.5
-    qkv = wide[:, :C].contiguous()
+    qkv = R(n, 2 * G * D + H * V) * D ** -0.5
     ba, a_log, dt = R(n, 2 * H), R(H) * 0.5, R(H) - 1
 
     def run(portions):
