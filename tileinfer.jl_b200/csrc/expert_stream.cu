@@ -15,7 +15,7 @@
 // after the other is asked for, in the next tile where this one ends, so the sums over the warps and the epilogue of a tile cost little bandwidth.
 // (Six sets of one k block took 31 % longer: a warp has few counters for loads in flight, and sets that share one wait for one another.) Both products
 // of units of 1,024 x 2,048 out of 32, each token in 4, on weights that are not in L2, against a block per tile of 32 rows: plain units, 4 tokens
-// 28.1 -> 24.1 us, 8 tokens 38.0 -> 31.4; gated ones with two more that every token takes, 8 tokens 61.5 -> 47.4 (289 MB: 6.1 TB/s), 16 tokens 86 -> 66.
+// 28.1 -> 24.1 us, 8 tokens 38.0 -> 30.2; gated ones with two more that every token takes, 8 tokens 61.5 -> 47.4 (289 MB: 6.1 TB/s), 16 tokens 86 -> 66.
 #include "expert_stream.h"
 
 #define ES_WARPS 8

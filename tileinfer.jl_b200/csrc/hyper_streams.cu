@@ -13,7 +13,7 @@
 // depend on the step it is in.
 static int hs_threads(int size) { return size >= 4096 ? 512 : size >= 1024 ? 256 : 128; }
 // Threads of a row's block. With no more rows than SMs a row's time is the round trips of one thread's loads, one after the other: blocks as
-// large as the row, up to 1,024 threads (4 rows of 2,048, two copies: update 8.4 -> 5.3 us, read 6.1 -> 3.6).
+// large as the row, up to 1,024 threads (4 rows of 2,048, two copies: update 8.4 -> 3.7 us, read 6.1 -> 3.6).
 static int hs_block(int size, int n) {
     if (n > ti_sm_count()) return hs_threads(size);
     const int all = (size + 31) / 32 * 32;

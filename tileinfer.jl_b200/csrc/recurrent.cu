@@ -124,7 +124,7 @@ __device__ __forceinline__ void copy4(float* dst, const float* src) {
 }
 // A block's columns of the state. Where many blocks have few tokens each and a warp few columns (`through`), they pass through shared memory: a warp's
 // own columns are 8 or 16 bytes of a row, the block's a whole sector or more (64 sequences of two tokens, straight into the lanes / through: 16 heads of
-// 256 x 256 726 / 325 us, 32 of 128 x 128 225 / 142). A group's rows lie CB floats further apart than they are long, so that a warp's reads fall into
+// 256 x 256 726 / 301 us, 32 of 128 x 128 225 / 144). A group's rows lie CB floats further apart than they are long, so that a warp's reads fall into
 // different banks. A thread carries R elements.
 template <int R, int G> struct StateTile {
     static constexpr int CB = 32 / G;
@@ -185,8 +185,8 @@ template <int R, int G> struct StateTile {
 // The next batch's rows are fetched into registers before this batch is worked on and laid into the other half of the staging buffers
 // after it, so their latency hides behind the recurrence; one barrier per batch. A thread stages one channel of tokens STEP apart.
 // What bounds it: instructions issued, a warp or two per scheduler, a third of them staging. The lanes' sums of a token meet in shared memory once
-// per batch. A prompt of 1,500 tokens (with 333, 64 and 7 beside it), 32 heads of 64, inside the step: 423 -> 309 us, against blocks of 32 columns
-// whose warps shared a column's rows; 2,048 tokens alone 405 -> 313, 8 heads 800 -> 392.
+// per batch. A prompt of 1,500 tokens (with 333, 64 and 7 beside it), 32 heads of 64, alone 373 -> 270 us, against blocks of 32 columns
+// whose warps shared a column's rows; 2,048 tokens 406 -> 274, 8 heads 799 -> 355.
 template <typename T, int R, int G, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? 4 : 1) decay_scan_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
                                   const float* __restrict__ w0, const float* __restrict__ u, float* state, long long state_stride,
@@ -338,8 +338,8 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? 4 : 1) decay_scan_ker
 
 // Keys above 64. Every block stages all key rows of its head, and what that takes grows with the key, so a block has 32 columns here (8 or 16 where few
 // blocks would leave most SMs idle): R rows a lane, a column's rows shared out among the warps, and among a warp's lanes too where the columns are
-// fewer; their sums meet in shared memory once per batch. 2,048 tokens here / in the kernel above: 32 heads of 128 576 / 1,112 us, 16 of 256 985 / 4,019;
-// for 64 and less the other way round (32 heads of 64 405 / 281).
+// fewer; their sums meet in shared memory once per batch. 2,048 tokens here / in the kernel above: 32 heads of 128 576 / 1,111 us, 16 of 256 986 / 4,027;
+// for 64 and less the other way round (32 heads of 64 406 / 274).
 template <typename T, int R, int CB>
 __global__ void decay_scan_wide_kernel(float* __restrict__ o, const T* rkv, long long ld, int r_off, int k_off, int v_off, const float* dlog,
                                   const float* __restrict__ w0, const float* __restrict__ u, float* state, long long state_stride,
@@ -567,10 +567,10 @@ extern "C" int ti_decay_scan(float* o, const void* rkv, long long ld, int r_off,
 // on their way (cp.async, 16 bytes where `vec` says that all rows allow it) while this batch is worked on; one barrier per batch.
 // What bounds it: one token's chain, decay, products with k, their sum over the lanes of a column, the write. So the next token's k is read
 // ahead, the products with q are off the chain, and pairs of rows share an instruction. A prompt of 1,500 tokens
-// (with 333, 64 and 7 beside it), 16 heads of 128 x 128, inside the step: 965 -> 412 us, against blocks of 32 columns whose warps shared a column's rows
-// and met at a barrier per token; 2,048 tokens alone 972 -> 436, 4 heads 1,407 -> 451.
+// (with 333, 64 and 7 beside it), 16 heads of 128 x 128, alone 804 -> 405 us, against blocks of 32 columns whose warps shared a column's rows
+// and met at a barrier per token; 2,048 tokens 973 -> 402, 4 heads 1,408 -> 405.
 // FULL: every group has rows of the key. FEW: so few blocks that a token's chain is all that counts; the state then always goes through shared memory, which
-// leaves the compiler twice the registers to read ahead into (2 heads of 256 x 256, 2,048 tokens 741 -> 484 us; 16 heads, with more warps an SM, 1,282 -> 1,411).
+// leaves the compiler twice the registers to read ahead into (2 heads of 256 x 256, 2,048 tokens 741 -> 476 us; 16 heads, with more warps an SM, 1,282 -> 1,411).
 template <int G, bool FULL, bool FEW>
 __global__ void __launch_bounds__(G == 16 ? 256 : 128) delta_scan_kernel(float* __restrict__ o, const float* qkv, long long ld, const float* ba, const float* __restrict__ a_log,
                                   const float* __restrict__ dt_bias, float* state, long long state_stride, const int* cu_seqlens,

@@ -224,13 +224,14 @@ def grouped_linear(y, x, w, plan, tile) -> bool:
     return True
 
 
-# A step of so few tokens streams the matrices of the units in use (csrc/expert_stream.cu); with more, a unit's pairs no longer fit one
-# operand of 8 and its matrices are gone over again. Both products, streamed against planned and grouped: 32 gated units of 1,024 x 2,048
-# with two shared, 8 / 16 / 32 tokens 47 / 66 / 81 us against 85 / 91 / 94; plain units 30 / 41 / 45 against 51 / 63 / 66; 64 units of
-# 1,408 x 4,096 195 / 283 / 328 against 244 / 349 / 402. (So more tokens could be streamed too.)
+# Steps of so few tokens stream the matrices of the units in use (csrc/expert_stream.cu). Both limits were drawn for an earlier form of that kernel; the
+# present one takes less beyond them too, and they stand where they were because the two paths add their sums in different orders, and steps
+# beyond them have not been compared over all designs on the other path. Both products, streamed against planned and grouped: 32 gated units of
+# 1,024 x 2,048 with two shared, 8 / 16 / 32 tokens 47 / 66 / 81 us against 85 / 91 / 94; plain units 30 / 41 / 45 against 51 / 63 / 66; 64 units of
+# 1,408 x 4,096 195 / 283 / 328 against 244 / 349 / 402.
 EXPERT_STREAM_TOKENS = 16
-# More units in use than this (as many as pairs drawn at random reach) go the other way, unless their matrices are small. (The line comes from an
-# earlier form of the kernel: 256 units of 2,048 x 256, 8 a token, 12 / 16 / 32 tokens now take 64 / 76 / 140 us streamed, 97 / 103 / 143 grouped.)
+# More units in use than this (as many as pairs drawn at random reach) go the other way, unless their matrices are small (256 units of 2,048 x 256, 8 a
+# token, 12 / 16 / 32 tokens 64 / 76 / 140 us streamed, 97 / 103 / 143 grouped).
 EXPERT_STREAM_UNITS = 64
 EXPERT_STREAM_BYTES = 64 << 20
 
